@@ -3,9 +3,9 @@
 // Three kernels behind one launcher:
 //   k_dense_rows   up to 4 tokens (decode): one warp streams one weight row with 16-byte loads and keeps one fp32 accumulator per token;
 //                  the launch is bound by the HBM read of W
-//   k_dense_tc     bf16, 5 tokens and more (decode batches, prompts): tcgen05.mma with the accumulator in TMEM (dense_tc.cu)
+//   dense_tc.cu    bf16, 5 tokens and more (decode batches, prompts): TMA and tcgen05.mma, K cut over a cluster where tiles are few
 //   k_dense_tile   everything else (true-fp32 products, ragged shapes): shared-memory tiles, fp32 fused multiply-add
-// No kernel splits K across CTAs or uses atomics: an output element is one fixed-order sum, whatever else is in the batch.
+// No kernel uses atomics: an output element is one sum in an order that the sizes of the call fix (dense_tc.cu may cut K).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

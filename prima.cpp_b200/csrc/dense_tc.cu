@@ -1,14 +1,24 @@
-// prima.cpp_b200/csrc/dense_tc.cu — bf16 dense product for prompts on the 5th-generation tensor cores:
+// prima.cpp_b200/csrc/dense_tc.cu — bf16 dense product for decode batches and prompts on the 5th-generation tensor cores:
 //   C[t][n] = alpha * sum_k A[t][k] W[n][k] (+ bias[n]) (+ resid[t][n]),   A [T][K], W [N][K] row-major bf16, C f32.
-// One CTA computes a tile of 128 weight rows x BN tokens: tcgen05.mma kind::f16 (bf16 operands, M = 128, N = BN, K = 16) with the fp32
-// accumulator in TMEM, both operands staged from their row-major global layout into the swizzle-128B K-major shared-memory image by
-// 16-byte cp.async pieces (4 producer warps, 4 to 8 stages of 64 k: narrow token tiles keep more of them in flight), one elected thread issuing the MMAs, tcgen05.commit handing stages back,
-// and all 8 warps reading the accumulator out with tcgen05.ld for the epilogue (lane = weight row, so a warp stores 32 consecutive
-// floats of one token's row).  K is never split: an output element is one fixed-order sum.  Every wait is bounded (common.cuh).
+// Weight rows are the M side of tcgen05.mma (lane of the accumulator = weight row, so a warp of the epilogue stores 32 consecutive floats of
+// one token's row), tokens the N side.  Both operands travel from their row-major layout into the swizzle-128B K-major shared-memory image by
+// tiled TMA loads (one elected thread; rows and k beyond the matrix read zeros), one elected thread issues the MMAs, tcgen05.commit hands
+// stages back.  Two kernels:
+//   k_dense_pair   products that fill the machine: a CTA pair shares 256 weight rows x 256 tokens (cta_group::2), each CTA staging half of both
+//                  operands, persistent over the tiles with two accumulators, so that a tile is read out while the next one is multiplied
+//   k_dense_split  the others: 128 weight rows x BN tokens per CTA; a cluster of up to 8 CTAs cuts K into equal consecutive parts and adds the
+//                  partial sums in the parts' order through distributed shared memory
+// What bounds them: all SMs together take about 12.5 TB/s from L2, and a 64-k step of a tile loads (rows + tokens) * 128 bytes: 128 x 256 tiles
+// are held to 0.65 of the tensor rate by that, the pair's 256 x 256 to 0.87; small batches are bound by the weights' way from HBM.  Measured
+// (2048 x 28672 x 4096): 870 us with cp.async producers and 128 x 256 tiles before, 360 us with the pair.  No atomics: the sum of an
+// element has one order, fixed by (T, N, K).  Every wait is bounded (common.cuh).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cstdlib>
 
 #include "launch.h"
 #include "layers.h"
@@ -17,30 +27,30 @@
 namespace pb {
 namespace {
 
-constexpr int TC_BM = 128, TC_BK = 64, TC_MAX_STAGES = 8, TC_PRODUCERS = 128, TC_THREADS = 256;
-
-// Stages: up to 192 KB of them while every CTA has an SM to itself; with more tiles than SMs the narrow tile takes four, so that two CTAs share one.
+constexpr int TC_BM = 128, TC_BK = 64, TC_MAX_STAGES = 10;
+constexpr int TC_A_BYTES = TC_BM * 128;                       // one stage of weights: 128 rows x 64 bf16
+constexpr int PAIR_BN = 256, PAIR_STAGES = 6, PAIR_THREADS = 320, PAIR_STAGE = TC_A_BYTES + PAIR_BN / 2 * 128;
+constexpr int SPLIT_THREADS = 256, MAX_SPLIT = 8;
 
 struct TcCtl {
-    uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], acc_ready;
+    uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], acc_full[2], acc_empty[2];
     uint32_t tmem_base;
     int abort;
 };
 
 struct TcParams {
-    const __nv_bfloat16 * A; int64_t lda;
-    const __nv_bfloat16 * W; int64_t ldw;
     float * C; int64_t ldc;
     const float * bias; const float * resid; int64_t ldr;
     float alpha;
     int T, N, K;
     int * abort_flag;
-    // grouped: rows [grp_start[g], + grp_count[g]) of A times the g-th matrix of W (grp_w_stride elements apart) into the same rows of C.
-    // The counts live on the device: blockIdx.y numbers the token tiles of all groups in a row (group 0's tiles, then group 1's, ...), the
-    // grid has room for the most tiles there can be (rows / BN + groups) and a CTA past the last tile leaves at once.
-    const int32_t * grp_start; const int32_t * grp_count; int64_t grp_w_stride; int groups;
-    // planes: weight rows [p * plane_rows, + plane_rows) meet the operand a_plane * p elements further on (plane_rows a multiple of the row tile)
-    int plane_rows; int64_t a_plane;
+    // grouped: rows [grp_start[g], + grp_count[g]) of A times the g-th matrix of W into the same rows of C.  The counts live on the device:
+    // blockIdx.y numbers the token tiles of all groups in a row (group 0's tiles, then group 1's, ...), the grid has room for the most tiles
+    // there can be (rows / BN + groups) and a CTA past the last tile leaves at once.
+    const int32_t * grp_start; const int32_t * grp_count; int groups;
+    int plane_rows;        // planes: weight rows [p * plane_rows, + plane_rows) meet the p-th operand (a multiple of the row tile)
+    int splits;            // CTAs of a cluster that share a tile's K
+    int row_tiles, tok_tiles;
     DenseAct act;
 };
 
@@ -52,87 +62,172 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {   // K-major, S
     d |= (uint64_t) 2 << 61;
     return d;
 }
+template <int CG>
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (CG == 1)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "setp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+            "}\n" ::"r"(tmem_d),
+            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "setp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+            "}\n" ::"r"(tmem_d),
+            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t * bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// completion of all prior MMAs of the pair -> the barrier at this offset in both CTAs
+__device__ __forceinline__ void mma_commit_pair(uint64_t * bar) {
+    const uint16_t mask = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask)
+                 : "memory");
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// 16 bytes global -> shared; bytes = 0 writes zeros (rows / k beyond the matrix)
-__device__ __forceinline__ void cp16(uint32_t dst, const void * src, uint32_t bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(saddr), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void prefetch_map(const CUtensorMap * m) { asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory"); }
+// box of 64 k x rows at (k, row, plane); bar: shared-memory address in the cluster's window (CG 2: either CTA of the pair)
+template <int CG>
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap * m, int k, int row, int plane, uint32_t bar) {
+    if constexpr (CG == 1)
+        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(m), "r"(k),
+                     "r"(row), "r"(plane), "r"(bar)
+                     : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(m),
+                     "r"(k), "r"(row), "r"(plane), "r"(bar)
+                     : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// rows [r0, r0 + ROWS) x k [k0, k0 + 64) of a row-major bf16 matrix -> swizzle-128B image at `dst` (1024-byte aligned)
-template <int ROWS>
-__device__ __forceinline__ void stage_rows(uint32_t dst, const __nv_bfloat16 * M, int64_t ld, int r0, int nrows, int k0, int K, int p) {
+// epilogue of NT tokens t, t + 1, ... of the warp's 32 consecutive weight rows (lane: row n); v: the sums.  FULL: all NT tokens exist (the
+// test per token is a fifth of the instructions, and instructions are what bounds this part: 46 a warp and stored row before the
+// paths were split, 11 us of a 256-token tile).  Residuals are fetched together before the first store: C may be the same memory, and
+// every load behind a store would wait for it.
+struct Finish {
+    float bias, xp, xn;
+    __device__ __forceinline__ Finish(const TcParams & P, int n) {
+        bias = (P.bias && n < P.N) ? P.bias[n] : 0.f;
+        xp = P.act.xielu ? softplus_f(P.act.xielu[0]) : 0.f;
+        xn = P.act.xielu ? 0.5f + softplus_f(P.act.xielu[1]) : 0.f;
+    }
+    template <int NT, bool FULL>
+    __device__ __forceinline__ void store(const TcParams & P, float * Cm, int n, int t, int Tn, const float (&v)[NT]) const {
+        if (P.act.silu_glu) {   // neighbouring lanes hold a gate and its value: of two tokens the even lane finishes the first, the odd one the second
+            const int odd = threadIdx.x & 1;
+            __nv_bfloat16 * y = (__nv_bfloat16 *) P.act.y + (int64_t) (t + odd) * P.act.ldy + n / 2;
+            const int64_t step = 2 * P.act.ldy;
 #pragma unroll
-    for (int j = 0; j < ROWS * 8 / TC_PRODUCERS; j++) {
-        const int i = p + TC_PRODUCERS * j;
-        const int row = i >> 3, c = i & 7;
-        const bool ok = r0 + row < nrows && k0 + c * 8 < K;
-        const __nv_bfloat16 * src = ok ? M + (int64_t) (r0 + row) * ld + k0 + c * 8 : M;
-        cp16(dst + (uint32_t) ((row >> 3) * 1024 + (row & 7) * 128 + ((c ^ (row & 7)) << 4)), src, ok ? 16u : 0u);
+            for (int i = 0; i < NT; i += 2, y += step) {
+                const float v0 = P.alpha * v[i], v1 = i + 1 < NT ? P.alpha * v[i + 1 < NT ? i + 1 : 0] : 0.f;
+                const float mine = odd ? v1 : v0, other = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+                const float g = odd ? other : mine, u = odd ? mine : other;
+                // the fast exponential and quotient are far more accurate than the operand type the result is rounded to
+                if (n < P.N && i + odd < NT && (FULL || t + i + odd < Tn)) *y = __float2bfloat16_rn(__fdividef(g, 1.f + __expf(-g)) * u);
+            }
+            return;
+        }
+        if (n >= P.N) return;
+        if (P.act.xielu) {
+            __nv_bfloat16 * y = (__nv_bfloat16 *) P.act.y + (int64_t) t * P.act.ldy + n;
+#pragma unroll
+            for (int i = 0; i < NT; i++, y += P.act.ldy)
+                if (FULL || t + i < Tn) *y = __float2bfloat16_rn(xielu_f(fmaf(P.alpha, v[i], bias), xp, xn));
+            return;
+        }
+        float * c = Cm + (int64_t) t * P.ldc + n;
+        if (P.resid) {
+            const float * rp = P.resid + (int64_t) t * P.ldr + n;
+            float r[NT];
+#pragma unroll
+            for (int i = 0; i < NT; i++, rp += P.ldr) r[i] = FULL || t + i < Tn ? *rp : 0.f;
+#pragma unroll
+            for (int i = 0; i < NT; i++, c += P.ldc)
+                if (FULL || t + i < Tn) *c = fmaf(P.alpha, v[i], bias) + r[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < NT; i++, c += P.ldc)
+                if (FULL || t + i < Tn) *c = fmaf(P.alpha, v[i], bias);
+        }
     }
-}
-
-// waits until at most n of this thread's newest copy groups are still in flight
-__device__ __forceinline__ void cp_wait(int n) {
-    switch (n) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+    // NT columns of the accumulator from column address `taddr` on
+    template <int NT>
+    __device__ __forceinline__ void columns(const TcParams & P, float * Cm, int n, int t, int Tn, uint32_t taddr) const {
+        uint32_t v[NT];
+        tmem_ld(taddr, v);
+        float f[NT];
+#pragma unroll
+        for (int i = 0; i < NT; i++) f[i] = __uint_as_float(v[i]);
+        if (t + NT <= Tn) store<NT, true>(P, Cm, n, t, Tn, f);
+        else store<NT, false>(P, Cm, n, t, Tn, f);
     }
-}
+};
 
-template <int BN, int TC_STAGES>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_dense_tc(const __grid_constant__ TcParams P) {
-    const __nv_bfloat16 * Am = P.A, * Wm = P.W;
+// ---------------------------------------------------------------------------------------------------------------
+// 128 weight rows x BN tokens, K cut over the cluster.  Warp 0: TMA producer, warp 1: MMA issuer and owner of the TMEM columns; all 8 warps read
+// the accumulator out (TMEM quadrant = warp % 4, token halves).
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1)
+    k_dense_split(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ TcParams P) {
+    constexpr int B_BYTES = BN * 128, STAGE = TC_A_BYTES + B_BYTES, COLS = BN < 32 ? 32 : BN;
     float * Cm = P.C;
-    int Tn = P.T, tile_y = blockIdx.y;
-    if (P.plane_rows > 0) Am += (int64_t) ((blockIdx.x * TC_BM) / P.plane_rows) * P.a_plane;
+    int Tn = P.T, tile_y = blockIdx.y, grp = 0, a_row0 = 0;
     if (P.grp_count) {
-        int g = 0;
-        for (; g < P.groups; g++) {
-            const int nt = (P.grp_count[g] + BN - 1) / BN;
+        for (; grp < P.groups; grp++) {
+            const int nt = (P.grp_count[grp] + BN - 1) / BN;
             if (tile_y < nt) break;
             tile_y -= nt;
         }
-        if (g >= P.groups) return;   // the whole CTA, before any barrier or TMEM allocation
-        Tn = P.grp_count[g];
-        const int64_t r0 = P.grp_start[g];
-        Am += r0 * P.lda; Cm += r0 * P.ldc; Wm += (int64_t) g * P.grp_w_stride;
+        if (grp >= P.groups) return;   // the whole cluster, before any barrier or TMEM allocation
+        Tn = P.grp_count[grp];
+        a_row0 = P.grp_start[grp];
+        Cm += (int64_t) a_row0 * P.ldc;
     }
     extern __shared__ uint8_t smem_raw[];
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    constexpr int TC_LAG = TC_STAGES - 2;
-    constexpr int A_BYTES = TC_BM * 128, B_BYTES = BN * 128, STAGE = A_BYTES + B_BYTES;
-    TcCtl * ctl = reinterpret_cast<TcCtl *>(smem + TC_STAGES * STAGE);
+    TcCtl * ctl = reinterpret_cast<TcCtl *>(smem + STAGES * STAGE);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.x * TC_BM, t0 = tile_y * BN;
-    const int nk = (P.K + TC_BK - 1) / TC_BK;
+    const int S = P.splits, part = blockIdx.x % S;
+    const int n0 = (blockIdx.x / S) * TC_BM, t0 = tile_y * BN;
+    const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
+    const int nk = (P.K + TC_BK - 1) / TC_BK, u0 = nk * part / S, nu = nk * (part + 1) / S - u0;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < TC_STAGES; i++) { mbar_init(&ctl->full[i], TC_PRODUCERS); mbar_init(&ctl->empty[i], 1); }
-        mbar_init(&ctl->acc_ready, 1);
+        prefetch_map(&map_w);
+        prefetch_map(&map_a);
+        for (int i = 0; i < STAGES; i++) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], 1); }
+        mbar_init(&ctl->acc_full[0], 1);
         ctl->abort = 0;
         mbar_fence_init();
     }
-    if (warp == 4) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(BN) : "memory");
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     fence_before();
@@ -141,120 +236,302 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_dense_tc(const __grid_constan
     const uint32_t tmem = *(volatile uint32_t *) &ctl->tmem_base;
     volatile int * cta_abort = &ctl->abort;
 
-    if (warp < 4) {
-        // ---- producers: stage u of A (weights) and B (activations) into its ring slot ----
-        const int p = threadIdx.x;
-        int signalled = 0;
-        auto signal = [&](int u) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copies above are read by the tensor core's async proxy
-            mbar_arrive(&ctl->full[u % TC_STAGES]);
-        };
-        for (int u = 0; u < nk; u++) {
-            const int s = u % TC_STAGES;
-            if (u >= TC_STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / TC_STAGES - 1) & 1), cta_abort, P.abort_flag);
-            const uint32_t base = smem_u32(smem + s * STAGE);
-            stage_rows<TC_BM>(base, Wm, P.ldw, n0, P.N, u * TC_BK, P.K, p);
-            stage_rows<BN>(base + A_BYTES, Am, P.lda, t0, Tn, u * TC_BK, P.K, p);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (u - signalled >= TC_LAG) {
-                cp_wait(TC_LAG);
-                signal(signalled++);
+    if (warp == 0) {
+        if (lane == 0) {
+            auto load_w = [&](int u) { tma_load<1>(smem_u32(smem + (u % STAGES) * STAGE), &map_w, (u0 + u) * TC_BK, n0, grp, smem_u32(&ctl->full[u % STAGES])); };
+            auto load_a = [&](int u) {
+                tma_load<1>(smem_u32(smem + (u % STAGES) * STAGE + TC_A_BYTES), &map_a, (u0 + u) * TC_BK, a_row0 + t0, plane, smem_u32(&ctl->full[u % STAGES]));
+            };
+            for (int u = 0; u < nu; u++) {
+                if (u >= STAGES) mbar_wait(&ctl->empty[u % STAGES], (uint32_t) ((u / STAGES - 1) & 1), cta_abort, P.abort_flag);
+                if (*cta_abort) break;
+                mbar_arrive_expect_tx(&ctl->full[u % STAGES], STAGE);
+                load_w(u);
+                load_a(u);
             }
         }
-        while (signalled < nk) {
-            cp_wait(nk - 1 - signalled);
-            signal(signalled++);
-        }
-    } else if (warp == 4) {
-        // ---- one thread issues the MMAs ----
+        __syncwarp();
+    } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (BN >> 3) << 17) | ((uint32_t) (TC_BM >> 4) << 24);
-            for (int u = 0; u < nk; u++) {
-                const int s = u % TC_STAGES;
-                mbar_wait(&ctl->full[s], (uint32_t) ((u / TC_STAGES) & 1), cta_abort, P.abort_flag);
+            for (int u = 0; u < nu; u++) {
+                const int s = u % STAGES;
+                mbar_wait(&ctl->full[s], (uint32_t) ((u / STAGES) & 1), cta_abort, P.abort_flag);
                 fence_after();
-                const uint64_t da = desc_sw128(smem_u32(smem + s * STAGE)), db = desc_sw128(smem_u32(smem + s * STAGE + A_BYTES));
+                const uint64_t da = desc_sw128(smem_u32(smem + s * STAGE)), db = desc_sw128(smem_u32(smem + s * STAGE + TC_A_BYTES));
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; k++) mma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (uint32_t) ((u | k) != 0));
+                for (int k = 0; k < TC_BK / 16; k++) mma_bf16<1>(tmem, da + 2 * k, db + 2 * k, idesc, (uint32_t) ((u | k) != 0));
                 mma_commit(&ctl->empty[s]);        // arrives once the MMAs above have read the stage
             }
-            mma_commit(&ctl->acc_ready);
+            mma_commit(&ctl->acc_full[0]);
         }
         __syncwarp();
     }
-    // ---- epilogue: every warp reads its TMEM quadrant (lanes = weight rows), warps 0-3 the first half of the tokens, 4-7 the second ----
-    mbar_wait(&ctl->acc_ready, 0u, cta_abort, P.abort_flag);
+    mbar_wait(&ctl->acc_full[0], 0u, cta_abort, P.abort_flag);
+    __syncwarp();
     fence_after();
     {
-        const int quad = warp & 3, half = warp >> 2;
-        const int n = n0 + quad * 32 + lane;
-        const float bias = (P.bias && n < P.N) ? P.bias[n] : 0.f;
-        const float * pq = P.act.xielu;
-        const float xp = pq ? softplus_f(pq[0]) : 0.f, xn = pq ? 0.5f + softplus_f(pq[1]) : 0.f;
-        __nv_bfloat16 * ya = (__nv_bfloat16 *) P.act.y;
-        for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
-            if (t0 + c0 >= Tn) break;                                   // uniform over the warp
-            uint32_t v[16];
-            const uint32_t taddr = tmem + ((uint32_t) (quad * 32) << 16) + (uint32_t) c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-                  "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(taddr)
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (P.act.silu_glu) {   // neighbouring lanes hold a gate and its value: of two tokens the even lane finishes the first, the odd one the second
-                const bool odd = lane & 1, ok = n < P.N && !*cta_abort;
-                __nv_bfloat16 * yp = ya + (int64_t) (t0 + c0 + (odd ? 1 : 0)) * P.act.ldy + n / 2;
+        const int quad = warp & 3, half = warp >> 2, r = quad * 32 + lane, n = n0 + r;
+        const Finish finish(P, n);
+        const uint32_t tq = tmem + ((uint32_t) (quad * 32) << 16);
+        constexpr int HC = BN >= 32 ? BN / 2 : BN;   // columns per warp: halves of the tile, or all of a 16-token tile for the first four warps
+        const int c_lo = half * HC, c_hi = c_lo + HC;
+        if (S == 1) {
+            for (int c0 = c_lo; c0 < c_hi && c0 < BN && t0 + c0 < Tn; c0 += 16) finish.template columns<16>(P, Cm, n, t0 + c0, Tn, tq + (uint32_t) c0);
+        } else {
+            // partial sums [token][row] in the stages' memory (every load and MMA of this CTA is done); token t is added up by CTA t % S
+            float * red = reinterpret_cast<float *>(smem);
+            for (int c0 = c_lo; c0 < c_hi && c0 < BN && t0 + c0 < Tn; c0 += 16) {
+                uint32_t v[16];
+                tmem_ld(tq + (uint32_t) c0, v);
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    const float mine = P.alpha * __uint_as_float(odd ? v[i + 1] : v[i]);
-                    const float other = __shfl_xor_sync(0xffffffffu, P.alpha * __uint_as_float(odd ? v[i] : v[i + 1]), 1);
-                    const float g = odd ? other : mine, u = odd ? mine : other;
-                    // the fast exponential and quotient are far more accurate than the operand type the result is rounded to
-                    if (ok && t0 + c0 + i + (odd ? 1 : 0) < Tn) yp[(int64_t) i * P.act.ldy] = __float2bfloat16_rn(__fdividef(g, 1.f + __expf(-g)) * u);
-                }
-                continue;
+                for (int i = 0; i < 16; i++) red[(c0 + i) * TC_BM + r] = __uint_as_float(v[i]);
             }
-            if (n < P.N && !*cta_abort) {
+            __syncwarp();
+            cluster_barrier();
+            const int tn = min(BN, Tn - t0);
+            for (int t = part + S * half; t < tn; t += 2 * S) {
+                const uint32_t at = smem_u32(red + t * TC_BM + r);
+                float f[MAX_SPLIT], v[1] = {0.f};
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int t = t0 + c0 + i;
-                    if (t < Tn) {
-                        float y = P.alpha * __uint_as_float(v[i]) + bias;
-                        if (P.resid) y += P.resid[(int64_t) t * P.ldr + n];
-                        if (pq) put(ya, (int64_t) t * P.act.ldy + n, xielu_f(y, xp, xn));
-                        else Cm[(int64_t) t * P.ldc + n] = y;
-                    }
+                for (int c = 0; c < MAX_SPLIT; c++) {
+                    f[c] = 0.f;
+                    if (c < S) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f[c]) : "r"(cluster_addr(at, (uint32_t) c)));
                 }
+#pragma unroll
+                for (int c = 0; c < MAX_SPLIT; c++)
+                    if (c < S) v[0] += f[c];
+                finish.template store<1, true>(P, Cm, n, t0 + t, Tn, v);
             }
+            __syncwarp();
+            cluster_barrier();   // no CTA leaves while another one reads its partial sums
         }
     }
     fence_before();
     __syncthreads();
-    if (warp == 4) {
+    if (warp == 1) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
     }
 }
 
-template <int BN, int STAGES> constexpr size_t tc_smem() { return 1024 + (size_t) STAGES * (TC_BM * 128 + BN * 128) + sizeof(TcCtl) + 64; }
+// ---------------------------------------------------------------------------------------------------------------
+// CTA pair: 256 weight rows x 256 tokens a tile, tiles token-first so that the pairs at work share weight rows in L2.  The leader (rank 0) issues
+// the MMAs of both; its full barriers count the bytes of both CTAs' loads.  Warp 0: TMA producer, warp 1: MMA issuer (leader), TMEM owner;
+// warps 2 .. 9 read accumulators out.
+__global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
+    k_dense_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ TcParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    TcCtl * ctl = reinterpret_cast<TcCtl *>(smem + PAIR_STAGES * PAIR_STAGE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int tiles = P.row_tiles * P.tok_tiles;
+    const int nk = (P.K + TC_BK - 1) / TC_BK;
+
+    if (threadIdx.x == 0) {
+        prefetch_map(&map_w);
+        prefetch_map(&map_a);
+        for (int i = 0; i < PAIR_STAGES; i++) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(&ctl->acc_full[i], 1); mbar_init(&ctl->acc_empty[i], 16); }
+        ctl->abort = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    cluster_barrier();   // both CTAs' barriers exist before anything arrives on them from the other CTA
+    fence_after();
+    const uint32_t tmem = *(volatile uint32_t *) &ctl->tmem_base;
+    volatile int * cta_abort = &ctl->abort;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int u = 0;
+            for (int i = pair; i < tiles; i += pairs) {
+                const int n0 = (i / P.tok_tiles) * 2 * TC_BM, t0 = (i % P.tok_tiles) * PAIR_BN;
+                const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
+                for (int k = 0; k < nk; k++, u++) {
+                    const int s = u % PAIR_STAGES;
+                    if (u >= PAIR_STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / PAIR_STAGES - 1) & 1), cta_abort, P.abort_flag);
+                    if (*cta_abort) break;
+                    if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * PAIR_STAGE);
+                    const uint32_t dst = smem_u32(smem + s * PAIR_STAGE), bar = cluster_addr(smem_u32(&ctl->full[s]), 0);
+                    tma_load<2>(dst, &map_w, k * TC_BK, n0 + rank * TC_BM, 0, bar);
+                    tma_load<2>(dst + TC_A_BYTES, &map_a, k * TC_BK, t0 + rank * (PAIR_BN / 2), plane, bar);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (PAIR_BN >> 3) << 17) | ((uint32_t) ((2 * TC_BM) >> 4) << 24);
+            int u = 0, j = 0;
+            for (int i = pair; i < tiles; i += pairs, j++) {
+                const int buf = j & 1;
+                if (j >= 2) mbar_wait(&ctl->acc_empty[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+                if (*cta_abort) break;
+                fence_after();
+                for (int k = 0; k < nk; k++, u++) {
+                    const int s = u % PAIR_STAGES;
+                    mbar_wait(&ctl->full[s], (uint32_t) ((u / PAIR_STAGES) & 1), cta_abort, P.abort_flag);
+                    fence_after();
+                    const uint64_t da = desc_sw128(smem_u32(smem + s * PAIR_STAGE)), db = desc_sw128(smem_u32(smem + s * PAIR_STAGE + TC_A_BYTES));
+#pragma unroll
+                    for (int q = 0; q < TC_BK / 16; q++) mma_bf16<2>(tmem + buf * PAIR_BN, da + 2 * q, db + 2 * q, idesc, (uint32_t) ((k | q) != 0));
+                    mma_commit_pair(&ctl->empty[s]);
+                }
+                mma_commit_pair(&ctl->acc_full[buf]);
+            }
+        }
+        __syncwarp();
+    } else {
+        const int quad = warp & 3, half = (warp - 2) >> 2, r = quad * 32 + lane;
+        int j = 0;
+        for (int i = pair; i < tiles; i += pairs, j++) {
+            const int buf = j & 1;
+            const int n = (i / P.tok_tiles) * 2 * TC_BM + rank * TC_BM + r, t0 = (i % P.tok_tiles) * PAIR_BN;
+            const Finish finish(P, n);
+            mbar_wait(&ctl->acc_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            const uint32_t tq = tmem + ((uint32_t) (quad * 32) << 16) + (uint32_t) (buf * PAIR_BN);
+            for (int c0 = half * (PAIR_BN / 2); c0 < (half + 1) * (PAIR_BN / 2) && t0 + c0 < P.T; c0 += 16)
+                finish.template columns<16>(P, P.C, n, t0 + c0, P.T, tq + (uint32_t) c0);
+            fence_before();
+            __syncwarp();
+            if (lane == 0)   // the leader may overwrite this accumulator
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(smem_u32(&ctl->acc_empty[buf]), 0)) : "memory");
+        }
+    }
+    fence_before();
+    __syncthreads();
+    cluster_barrier();   // the pair leaves together: MMAs, commits and loads of one CTA reach into the other's shared memory
+    if (warp == 1) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void * p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+        return (EncodeTiled) p;
+    }();
+    return fn;
+}
+// planes x rows x K bf16, boxes of 64 k x box_rows in the swizzle-128B image
+int make_map(CUtensorMap & m, const void * base, int64_t K, int64_t rows, int64_t planes, int64_t ld, int64_t plane, int box_rows) {
+    const EncodeTiled fn = encode_tiled();
+    if (!fn) return (int) cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, (cuuint64_t) planes};
+    const cuuint64_t strides[2] = {(cuuint64_t) ld * 2, (cuuint64_t) (planes > 1 ? plane : rows * ld) * 2};
+    const cuuint32_t box[3] = {(cuuint32_t) TC_BK, (cuuint32_t) box_rows, 1}, one[3] = {1, 1, 1};
+    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *) base, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : (int) cudaErrorInvalidValue;
+}
+
+struct TcOperands {
+    const __nv_bfloat16 * A; int64_t lda, a_rows, a_planes, a_plane;
+    const __nv_bfloat16 * W; int64_t ldw, w_rows, w_planes, w_plane;
+};
+
+template <int BN, int STAGES> constexpr size_t split_smem() { return 1024 + (size_t) STAGES * (TC_A_BYTES + BN * 128) + sizeof(TcCtl) + 64; }
 
 template <int BN, int STAGES>
-int launch_tc_stages(const TcParams & P, const dim3 & grid, cudaStream_t st) {
+int launch_split_stages(const TcParams & P, const TcOperands & o, const dim3 & grid, cudaStream_t st) {
     static FuncAttrCache cache;
-    cudaError_t e = ensure_dyn_smem(cache, (const void *) k_dense_tc<BN, STAGES>, tc_smem<BN, STAGES>(), BN == 256);
+    const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_dense_split<BN, STAGES>, split_smem<BN, STAGES>(), true);
     if (e != cudaSuccess) return (int) e;
+    CUtensorMap mw, ma;
+    int rc = make_map(mw, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
+    if (!rc) rc = make_map(ma, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, BN);
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(SPLIT_THREADS);
+    cfg.dynamicSmemBytes = split_smem<BN, STAGES>();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned) P.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     g_launches++;
-    k_dense_tc<BN, STAGES><<<grid, TC_THREADS, tc_smem<BN, STAGES>(), st>>>(P);
+    return (int) cudaLaunchKernelEx(&cfg, k_dense_split<BN, STAGES>, mw, ma, P);
+}
+// Stages: while every CTA has an SM to itself as many as fit; with more CTAs than SMs (at most 96 KB each) two of them share one, so that one's
+// prologue and epilogue lie beside the other's loads.
+int launch_split(int bn, TcParams P, const TcOperands & o, cudaStream_t st) {
+    const dim3 grid((unsigned) ((P.N + TC_BM - 1) / TC_BM * P.splits), (unsigned) ((P.T + bn - 1) / bn + (P.grp_count ? P.groups : 0)));
+    const bool shared = (int64_t) grid.x * grid.y > sm_count() || P.splits == MAX_SPLIT;
+    switch (bn) {
+    case 16: return shared ? launch_split_stages<16, 5>(P, o, grid, st) : launch_split_stages<16, 10>(P, o, grid, st);
+    case 32: return shared ? launch_split_stages<32, 5>(P, o, grid, st) : launch_split_stages<32, 10>(P, o, grid, st);
+    case 64: return shared ? launch_split_stages<64, 4>(P, o, grid, st) : launch_split_stages<64, 8>(P, o, grid, st);
+    case 128: return shared ? launch_split_stages<128, 3>(P, o, grid, st) : launch_split_stages<128, 6>(P, o, grid, st);
+    default: return launch_split_stages<256, 4>(P, o, grid, st);
+    }
+}
+int launch_pair(TcParams P, const TcOperands & o, cudaStream_t st) {
+    constexpr size_t smem = 1024 + (size_t) PAIR_STAGES * PAIR_STAGE + sizeof(TcCtl) + 64;
+    static FuncAttrCache cache;
+    const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_dense_pair, smem, true);
+    if (e != cudaSuccess) return (int) e;
+    P.row_tiles = (P.N + 2 * TC_BM - 1) / (2 * TC_BM);
+    P.tok_tiles = (P.T + PAIR_BN - 1) / PAIR_BN;
+    CUtensorMap mw, ma;
+    int rc = make_map(mw, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
+    if (!rc) rc = make_map(ma, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, PAIR_BN / 2);
+    if (rc) return rc;
+    const int64_t tiles = (int64_t) P.row_tiles * P.tok_tiles;
+    const int pairs = (int) (tiles < sm_count() / 2 ? tiles : sm_count() / 2);
+    g_launches++;
+    k_dense_pair<<<dim3((unsigned) (2 * pairs)), PAIR_THREADS, smem, st>>>(mw, ma, P);
     return (int) cudaGetLastError();
 }
-template <int BN>
-int launch_tc(const TcParams & P, cudaStream_t st) {
-    const dim3 grid((unsigned) ((P.N + TC_BM - 1) / TC_BM), (unsigned) ((P.T + BN - 1) / BN + (P.grp_count ? P.groups : 0)));
-    if (BN == 256) return launch_tc_stages<256, 4>(P, grid, st);
-    if (BN == 128) return launch_tc_stages<128, 6>(P, grid, st);
-    return (int64_t) grid.x * grid.y <= 148 ? launch_tc_stages<64, 8>(P, grid, st) : launch_tc_stages<64, 4>(P, grid, st);
+
+// Which kernel, token tile and cut of K: the one with the least time by a model of what was measured on a B200 (148 SMs, 1.9 GHz, all tiles of
+// T 8 .. 2048, N 256 .. 32000, K 512 .. 14336, launches back to back in a graph; within 15 % of every time):
+//   an SM takes 0.265 us for a 64-k step of one tile up to 128 tokens wide (the MMA's time does not fall below that of 256 tokens by
+//   more), 0.29 us for 256; all SMs together take 12.5 TB/s from L2 and 6.5 TB/s of weights from HBM;
+//   a launch costs 3 us + 0.01 us per token of the tile (9 us with the pair's two accumulators), a cut of K 2 us + 0.02 us per token more.
+// Examples, us: 8 x 2048 x 8192 uncut 37.9, cut in 4 13.7, in 8 11.7; 512 x 2048 x 8192 pair 47.4, 128 tokens 39.5, cut in 4 26.0;
+// 1488 x 16384 x 2048 pair 84.7, 256 tokens 105, 128 tokens 119.  rows: tokens (grouped: expected ones of a group).
+struct TcPlan { int pair, bn, splits; };
+TcPlan plan_tc(int rows, int groups, int N, int K, int plane_rows) {
+    const int64_t nk = (K + TC_BK - 1) / TC_BK, sms = sm_count();
+    const double hbm = (double) N * K * 2 * groups / 6.5e6;
+    TcPlan best{0, 64, 1};
+    double best_us = 1e30;
+    auto consider = [&](const TcPlan & p, int64_t steps_of_an_sm, double step_us, int64_t steps, int step_bytes, double fixed_us) {
+        const double us = std::max({(double) steps_of_an_sm * step_us, (double) steps * step_bytes / 12.5e6, hbm}) + fixed_us;
+        if (us < best_us) { best_us = us; best = p; }
+    };
+    if (groups == 1 && rows > 128 && plane_rows % (2 * TC_BM) == 0) {
+        const int64_t tiles = (int64_t) ((N + 2 * TC_BM - 1) / (2 * TC_BM)) * ((rows + PAIR_BN - 1) / PAIR_BN), waves = (tiles + sms / 2 - 1) / (sms / 2);
+        consider({1, PAIR_BN, 1}, waves * nk, 0.29, tiles * nk, 2 * PAIR_STAGE, 9.0);
+    }
+    for (int bn = 16; bn <= 256; bn *= 2) {
+        if (bn > 16 && rows <= bn / 2) break;
+        const int64_t tiles = (int64_t) ((N + TC_BM - 1) / TC_BM) * ((rows + bn - 1) / bn) * groups;
+        for (int s = 1; s <= MAX_SPLIT && s <= nk; s *= 2) {
+            if (s > 1 && (bn > 128 || groups > 1 || tiles * s > 2 * sms)) break;
+            const int64_t per_sm = (tiles * s + sms - 1) / sms;
+            consider({0, bn, s}, per_sm * ((nk + s - 1) / s), bn > 128 ? 0.29 : 0.265, tiles * nk, (TC_BM + bn) * 128,
+                     3.0 + 0.01 * bn + (s > 1 ? 2.0 + 0.02 * bn : 0.0) + (bn > 128 ? 2.5 * (double) (per_sm - 1) : 0.0));
+        }
+    }
+    return best;
 }
 
 }  // namespace
@@ -266,27 +543,23 @@ bool dense_tc_ok(int T, int N, int K, int64_t lda, int64_t ldw, const void * A, 
 
 int launch_dense_tc(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
                     const float * resid, int64_t ldr, float alpha, cudaStream_t st, int plane_rows, int64_t a_plane, DenseAct act) {
-    TcParams P{A, lda, W, ldw, C, ldc, bias, resid, ldr, alpha, T, N, K, abort_flag(), nullptr, nullptr, 0, 0, plane_rows, a_plane, act};
-    if (T <= 64) return launch_tc<64>(P, st);
-    // token tile: the one whose waves of CTAs cost least, a k step of a tile being about its tokens plus the weight rows' share of the loads.  Few
-    // weight rows leave most SMs idle under wide tiles; an element's sum runs over k in the same order under any of them.
-    int best = 0;
-    int64_t best_cost = 0;
-    for (const int bn : {256, 128, 64}) {
-        if (bn > 64 && T <= bn / 2) continue;
-        const int64_t tiles = (int64_t) ((N + TC_BM - 1) / TC_BM) * ((T + bn - 1) / bn), cost = (tiles + 147) / 148 * (bn + 48);
-        if (!best || cost < best_cost) { best = bn; best_cost = cost; }
-    }
-    return best == 64 ? launch_tc<64>(P, st) : best == 128 ? launch_tc<128>(P, st) : launch_tc<256>(P, st);
+    TcParams P{C, ldc, bias, resid, ldr, alpha, T, N, K, abort_flag(), nullptr, nullptr, 1, plane_rows, 1, 0, 0, act};
+    const TcOperands o{A, lda, T, plane_rows > 0 ? N / plane_rows : 1, a_plane, W, ldw, N, 1, 0};
+    const TcPlan p = plan_tc(T, 1, N, K, plane_rows);
+    if (p.pair) return launch_pair(P, o, st);
+    P.splits = p.splits;
+    return launch_split(p.bn, P, o, st);
 }
 
 int launch_dense_tc_grouped(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, int64_t w_stride, float * C, int64_t ldc,
                             const int32_t * start, const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st) {
     if (groups <= 0 || max_rows <= 0) return 0;
     // T bounds the grid only (all groups together hold max_rows rows); the kernel reads each group's own count
-    TcParams P{A, lda, W, ldw, C, ldc, nullptr, nullptr, 0, 1.f, max_rows, N, K, abort_flag(), start, count, w_stride, groups, 0, 0, DenseAct()};
-    const int avg = (max_rows + groups - 1) / groups;   // the token tile follows the expected rows of a group
-    return avg <= 64 ? launch_tc<64>(P, st) : avg <= 128 ? launch_tc<128>(P, st) : launch_tc<256>(P, st);
+    TcParams P{C, ldc, nullptr, nullptr, 0, 1.f, max_rows, N, K, abort_flag(), start, count, groups, 0, 1, 0, 0, DenseAct()};
+    const TcOperands o{A, lda, max_rows, 1, 0, W, ldw, N, groups, w_stride};
+    const TcPlan p = plan_tc((max_rows + groups - 1) / groups, groups, N, K, 0);   // the tile follows the expected rows of a group
+    P.splits = 1;
+    return launch_split(p.bn, P, o, st);
 }
 
 }  // namespace pb
