@@ -10,9 +10,8 @@
 //                  partial sums in the parts' order through distributed shared memory
 // What bounds them: all SMs together take about 12.5 TB/s from L2, and a 64-k step of a tile loads (rows + tokens) * 128 bytes: 128 x 256 tiles
 // are held to 0.65 of the tensor rate by that, the pair's 256 x 256 to 0.87; small batches are bound by the weights' way from HBM.  Measured
-// (2048 x 28672 x 4096): 870 us with cp.async producers and 128 x 256 tiles before, 360 us with the pair.  No atomics: the sum of an
+// (2048 x 28672 x 4096): 870 us with cp.async producers and 128 x 256 tiles before, 330 us with the pair.  No atomics: the sum of an
 // element has one order, fixed by (T, N, K).  Every wait is bounded (common.cuh).
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -23,6 +22,7 @@
 #include "launch.h"
 #include "layers.h"
 #include "mixers.cuh"
+#include "tc.cuh"
 
 namespace pb {
 namespace {
@@ -53,78 +53,6 @@ struct TcParams {
     int row_tiles, tok_tiles;
     DenseAct act;
 };
-
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {   // K-major, SWIZZLE_128B: rows of 128 B, 8-row groups 1024 B apart
-    uint64_t d = (uint64_t) ((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t) 1 << 16;
-    d |= (uint64_t) (1024 >> 4) << 32;
-    d |= (uint64_t) 1 << 46;
-    d |= (uint64_t) 2 << 61;
-    return d;
-}
-template <int CG>
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (CG == 1)
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "setp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n" ::"r"(tmem_d),
-            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-            : "memory");
-    else
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "setp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n" ::"r"(tmem_d),
-            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t * bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// completion of all prior MMAs of the pair -> the barrier at this offset in both CTAs
-__device__ __forceinline__ void mma_commit_pair(uint64_t * bar) {
-    const uint16_t mask = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask)
-                 : "memory");
-}
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(saddr), "r"(rank));
-    return ra;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void prefetch_map(const CUtensorMap * m) { asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory"); }
-// box of 64 k x rows at (k, row, plane); bar: shared-memory address in the cluster's window (CG 2: either CTA of the pair)
-template <int CG>
-__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap * m, int k, int row, int plane, uint32_t bar) {
-    if constexpr (CG == 1)
-        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(m), "r"(k),
-                     "r"(row), "r"(plane), "r"(bar)
-                     : "memory");
-    else
-        asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(m),
-                     "r"(k), "r"(row), "r"(plane), "r"(bar)
-                     : "memory");
-}
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // epilogue of NT tokens t, t + 1, ... of the warp's 32 consecutive weight rows (lane: row n); v: the sums.  FULL: all NT tokens exist (the
 // test per token is a fifth of the instructions, and instructions are what bounds this part: 46 a warp and stored row before the
@@ -212,7 +140,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     extern __shared__ uint8_t smem_raw[];
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     TcCtl * ctl = reinterpret_cast<TcCtl *>(smem + STAGES * STAGE);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int S = P.splits, part = blockIdx.x % S;
     const int n0 = (blockIdx.x / S) * TC_BM, t0 = tile_y * BN;
     const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
@@ -237,35 +165,36 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     volatile int * cta_abort = &ctl->abort;
 
     if (warp == 0) {
-        if (lane == 0) {
-            auto load_w = [&](int u) { tma_load<1>(smem_u32(smem + (u % STAGES) * STAGE), &map_w, (u0 + u) * TC_BK, n0, grp, smem_u32(&ctl->full[u % STAGES])); };
-            auto load_a = [&](int u) {
-                tma_load<1>(smem_u32(smem + (u % STAGES) * STAGE + TC_A_BYTES), &map_a, (u0 + u) * TC_BK, a_row0 + t0, plane, smem_u32(&ctl->full[u % STAGES]));
-            };
-            for (int u = 0; u < nu; u++) {
-                if (u >= STAGES) mbar_wait(&ctl->empty[u % STAGES], (uint32_t) ((u / STAGES - 1) & 1), cta_abort, P.abort_flag);
-                if (*cta_abort) break;
-                mbar_arrive_expect_tx(&ctl->full[u % STAGES], STAGE);
-                load_w(u);
-                load_a(u);
+        for (int u = 0; u < nu; u++) {
+            const int s = u % STAGES;
+            if (u >= STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / STAGES - 1) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            if (elect_one()) {
+                const uint32_t dst = smem_u32(smem + s * STAGE), bar = smem_u32(&ctl->full[s]);
+                mbar_arrive_expect_tx(&ctl->full[s], STAGE);
+                tma_load<1>(dst, &map_w, (u0 + u) * TC_BK, n0, grp, bar);
+                tma_load<1>(dst + TC_A_BYTES, &map_a, (u0 + u) * TC_BK, a_row0 + t0, plane, bar);
             }
+            __syncwarp();
+            if (*cta_abort) break;
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (BN >> 3) << 17) | ((uint32_t) (TC_BM >> 4) << 24);
-            for (int u = 0; u < nu; u++) {
-                const int s = u % STAGES;
-                mbar_wait(&ctl->full[s], (uint32_t) ((u / STAGES) & 1), cta_abort, P.abort_flag);
-                fence_after();
-                const uint64_t da = desc_sw128(smem_u32(smem + s * STAGE)), db = desc_sw128(smem_u32(smem + s * STAGE + TC_A_BYTES));
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (BN >> 3) << 17) | ((uint32_t) (TC_BM >> 4) << 24);
+        for (int u = 0; u < nu; u++) {
+            const int s = u % STAGES;
+            mbar_wait(&ctl->full[s], (uint32_t) ((u / STAGES) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            const uint64_t da = desc_sw128(smem_u32(smem + s * STAGE)), db = desc_sw128(smem_u32(smem + s * STAGE + TC_A_BYTES));
+            if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; k++) mma_bf16<1>(tmem, da + 2 * k, db + 2 * k, idesc, (uint32_t) ((u | k) != 0));
+                for (int k = 0; k < TC_BK / 16; k++) mma_f16<1>(tmem, da + 2 * k, db + 2 * k, idesc, (uint32_t) ((u | k) != 0));
                 mma_commit(&ctl->empty[s]);        // arrives once the MMAs above have read the stage
+                if (u == nu - 1) mma_commit(&ctl->acc_full[0]);
             }
-            mma_commit(&ctl->acc_full[0]);
+            __syncwarp();
         }
-        __syncwarp();
     }
     mbar_wait(&ctl->acc_full[0], 0u, cta_abort, P.abort_flag);
     __syncwarp();
@@ -324,7 +253,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     extern __shared__ uint8_t smem_raw[];
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     TcCtl * ctl = reinterpret_cast<TcCtl *>(smem + PAIR_STAGES * PAIR_STAGE);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles = P.row_tiles * P.tok_tiles;
     const int nk = (P.K + TC_BK - 1) / TC_BK;
@@ -349,42 +278,49 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     volatile int * cta_abort = &ctl->abort;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int u = 0;
-            for (int i = pair; i < tiles; i += pairs) {
-                const int n0 = (i / P.tok_tiles) * 2 * TC_BM, t0 = (i % P.tok_tiles) * PAIR_BN;
-                const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
-                for (int k = 0; k < nk; k++, u++) {
-                    const int s = u % PAIR_STAGES;
-                    if (u >= PAIR_STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / PAIR_STAGES - 1) & 1), cta_abort, P.abort_flag);
-                    if (*cta_abort) break;
-                    if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * PAIR_STAGE);
+        int u = 0;
+        for (int i = pair; i < tiles && !*cta_abort; i += pairs) {
+            const int n0 = (i / P.tok_tiles) * 2 * TC_BM, t0 = (i % P.tok_tiles) * PAIR_BN;
+            const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
+            for (int k = 0; k < nk; k++, u++) {
+                const int s = u % PAIR_STAGES;
+                if (u >= PAIR_STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / PAIR_STAGES - 1) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
+                if (elect_one()) {
                     const uint32_t dst = smem_u32(smem + s * PAIR_STAGE), bar = cluster_addr(smem_u32(&ctl->full[s]), 0);
+                    if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * PAIR_STAGE);
                     tma_load<2>(dst, &map_w, k * TC_BK, n0 + rank * TC_BM, 0, bar);
                     tma_load<2>(dst + TC_A_BYTES, &map_a, k * TC_BK, t0 + rank * (PAIR_BN / 2), plane, bar);
                 }
+                __syncwarp();
+                if (*cta_abort) break;
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (PAIR_BN >> 3) << 17) | ((uint32_t) ((2 * TC_BM) >> 4) << 24);
             int u = 0, j = 0;
             for (int i = pair; i < tiles; i += pairs, j++) {
                 const int buf = j & 1;
                 if (j >= 2) mbar_wait(&ctl->acc_empty[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
                 if (*cta_abort) break;
                 fence_after();
                 for (int k = 0; k < nk; k++, u++) {
                     const int s = u % PAIR_STAGES;
                     mbar_wait(&ctl->full[s], (uint32_t) ((u / PAIR_STAGES) & 1), cta_abort, P.abort_flag);
+                    __syncwarp();
                     fence_after();
                     const uint64_t da = desc_sw128(smem_u32(smem + s * PAIR_STAGE)), db = desc_sw128(smem_u32(smem + s * PAIR_STAGE + TC_A_BYTES));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int q = 0; q < TC_BK / 16; q++) mma_bf16<2>(tmem + buf * PAIR_BN, da + 2 * q, db + 2 * q, idesc, (uint32_t) ((k | q) != 0));
-                    mma_commit_pair(&ctl->empty[s]);
+                        for (int q = 0; q < TC_BK / 16; q++) mma_f16<2>(tmem + buf * PAIR_BN, da + 2 * q, db + 2 * q, idesc, (uint32_t) ((k | q) != 0));
+                        mma_commit_pair(&ctl->empty[s]);
+                        if (k == nk - 1) mma_commit_pair(&ctl->acc_full[buf]);
+                    }
+                    __syncwarp();
                 }
-                mma_commit_pair(&ctl->acc_full[buf]);
             }
         }
         __syncwarp();
@@ -417,29 +353,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encode_tiled() {
-    static const EncodeTiled fn = [] {
-        void * p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-        return (EncodeTiled) p;
-    }();
-    return fn;
-}
-// planes x rows x K bf16, boxes of 64 k x box_rows in the swizzle-128B image
-int make_map(CUtensorMap & m, const void * base, int64_t K, int64_t rows, int64_t planes, int64_t ld, int64_t plane, int box_rows) {
-    const EncodeTiled fn = encode_tiled();
-    if (!fn) return (int) cudaErrorNotSupported;
-    const cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, (cuuint64_t) planes};
-    const cuuint64_t strides[2] = {(cuuint64_t) ld * 2, (cuuint64_t) (planes > 1 ? plane : rows * ld) * 2};
-    const cuuint32_t box[3] = {(cuuint32_t) TC_BK, (cuuint32_t) box_rows, 1}, one[3] = {1, 1, 1};
-    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *) base, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int) cudaErrorInvalidValue;
-}
-
 struct TcOperands {
     const __nv_bfloat16 * A; int64_t lda, a_rows, a_planes, a_plane;
     const __nv_bfloat16 * W; int64_t ldw, w_rows, w_planes, w_plane;
@@ -453,8 +366,8 @@ int launch_split_stages(const TcParams & P, const TcOperands & o, const dim3 & g
     const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_dense_split<BN, STAGES>, split_smem<BN, STAGES>(), true);
     if (e != cudaSuccess) return (int) e;
     CUtensorMap mw, ma;
-    int rc = make_map(mw, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
-    if (!rc) rc = make_map(ma, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, BN);
+    int rc = make_map(mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
+    if (!rc) rc = make_map(ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, BN);
     if (rc) return rc;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -490,8 +403,8 @@ int launch_pair(TcParams P, const TcOperands & o, cudaStream_t st) {
     P.row_tiles = (P.N + 2 * TC_BM - 1) / (2 * TC_BM);
     P.tok_tiles = (P.T + PAIR_BN - 1) / PAIR_BN;
     CUtensorMap mw, ma;
-    int rc = make_map(mw, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
-    if (!rc) rc = make_map(ma, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, PAIR_BN / 2);
+    int rc = make_map(mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.W, P.K, o.w_rows, o.w_planes, o.ldw, o.w_plane, TC_BM);
+    if (!rc) rc = make_map(ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.A, P.K, o.a_rows, o.a_planes, o.lda, o.a_plane, PAIR_BN / 2);
     if (rc) return rc;
     const int64_t tiles = (int64_t) P.row_tiles * P.tok_tiles;
     const int pairs = (int) (tiles < sm_count() / 2 ? tiles : sm_count() / 2);
@@ -502,11 +415,11 @@ int launch_pair(TcParams P, const TcOperands & o, cudaStream_t st) {
 
 // Which kernel, token tile and cut of K: the one with the least time by a model of what was measured on a B200 (148 SMs, 1.9 GHz, all tiles of
 // T 8 .. 2048, N 256 .. 32000, K 512 .. 14336, launches back to back in a graph; within 15 % of every time):
-//   an SM takes 0.265 us for a 64-k step of one tile up to 128 tokens wide (the MMA's time does not fall below that of 256 tokens by
-//   more), 0.29 us for 256; all SMs together take 12.5 TB/s from L2 and 6.5 TB/s of weights from HBM;
-//   a launch costs 3 us + 0.01 us per token of the tile (9 us with the pair's two accumulators), a cut of K 2 us + 0.02 us per token more.
-// Examples, us: 8 x 2048 x 8192 uncut 37.9, cut in 4 13.7, in 8 11.7; 512 x 2048 x 8192 pair 47.4, 128 tokens 39.5, cut in 4 26.0;
-// 1488 x 16384 x 2048 pair 84.7, 256 tokens 105, 128 tokens 119.  rows: tokens (grouped: expected ones of a group).
+//   an SM takes 0.2 us for a 64-k step of one tile up to 128 tokens wide (what issuing and waiting cost), 0.28 us for 256 (its MMAs);
+//   all SMs together take 12.5 TB/s from L2 and 6.5 TB/s of weights from HBM;
+//   a launch costs 3 us + 0.01 us per token of the tile (9 us with the pair's two accumulators), a cut of K 1.5 us + 0.015 us per token more.
+// Examples, us: 8 x 2048 x 8192 uncut 37.9, cut in 4 13.7, in 8 10.6; 512 x 2048 x 8192 pair 47.4, 128 tokens 31.2, cut in 4 24.1;
+// 1488 x 16384 x 2048 pair 81.8, 256 tokens 105, 128 tokens 119.  rows: tokens (grouped: expected ones of a group).
 struct TcPlan { int pair, bn, splits; };
 TcPlan plan_tc(int rows, int groups, int N, int K, int plane_rows) {
     const int64_t nk = (K + TC_BK - 1) / TC_BK, sms = sm_count();
@@ -515,11 +428,11 @@ TcPlan plan_tc(int rows, int groups, int N, int K, int plane_rows) {
     double best_us = 1e30;
     auto consider = [&](const TcPlan & p, int64_t steps_of_an_sm, double step_us, int64_t steps, int step_bytes, double fixed_us) {
         const double us = std::max({(double) steps_of_an_sm * step_us, (double) steps * step_bytes / 12.5e6, hbm}) + fixed_us;
-        if (us < best_us) { best_us = us; best = p; }
+        if (us <= best_us) { best_us = us; best = p; }   // of equals the finer cut: two CTAs to an SM hide each other's start and end
     };
     if (groups == 1 && rows > 128 && plane_rows % (2 * TC_BM) == 0) {
         const int64_t tiles = (int64_t) ((N + 2 * TC_BM - 1) / (2 * TC_BM)) * ((rows + PAIR_BN - 1) / PAIR_BN), waves = (tiles + sms / 2 - 1) / (sms / 2);
-        consider({1, PAIR_BN, 1}, waves * nk, 0.29, tiles * nk, 2 * PAIR_STAGE, 9.0);
+        consider({1, PAIR_BN, 1}, waves * nk, 0.28, tiles * nk, 2 * PAIR_STAGE, 9.0);
     }
     for (int bn = 16; bn <= 256; bn *= 2) {
         if (bn > 16 && rows <= bn / 2) break;
@@ -527,8 +440,8 @@ TcPlan plan_tc(int rows, int groups, int N, int K, int plane_rows) {
         for (int s = 1; s <= MAX_SPLIT && s <= nk; s *= 2) {
             if (s > 1 && (bn > 128 || groups > 1 || tiles * s > 2 * sms)) break;
             const int64_t per_sm = (tiles * s + sms - 1) / sms;
-            consider({0, bn, s}, per_sm * ((nk + s - 1) / s), bn > 128 ? 0.29 : 0.265, tiles * nk, (TC_BM + bn) * 128,
-                     3.0 + 0.01 * bn + (s > 1 ? 2.0 + 0.02 * bn : 0.0) + (bn > 128 ? 2.5 * (double) (per_sm - 1) : 0.0));
+            consider({0, bn, s}, per_sm * ((nk + s - 1) / s), bn > 128 ? 0.28 : 0.2, tiles * nk, (TC_BM + bn) * 128,
+                     3.0 + 0.01 * bn + (s > 1 ? 1.5 + 0.015 * bn : 0.0) + (bn > 128 ? 2.5 * (double) (per_sm - 1) : 0.0));
         }
     }
     return best;
