@@ -85,6 +85,10 @@ int attn_scratch_floats(int n_head, int n_ctx);
 // batched form for prompt processing: token t (q row t, out row t) attends to cache rows [0, pos_dev[t]]
 int launch_attn_batch(const float * q, const __half * kcache, const __half * vcache, float * out, int n_head, int n_head_kv, int D,
                       const int32_t * pos_dev, int n_tok, int n_kv_max, float scale, cudaStream_t stream);
+// the same on the tensor cores (attn_tc.cu): head size 128, any GQA group up to 128, 16-byte aligned arrays
+bool attn_prefill_tc_ok(const float * q, const __half * kcache, const __half * vcache, const float * out, int n_head, int n_head_kv, int D, int n_kv_max);
+int launch_attn_prefill_tc(const float * q, const __half * kcache, const __half * vcache, float * out, int n_head, int n_head_kv, const int32_t * pos_dev, int n_tok,
+                           int n_kv_max, float scale, cudaStream_t stream);
 // rope(q), rope(k) -> f16 K row, v -> f16 V row, cache store and attention in one launch (the engine's per-token path)
 int launch_attn_fused(const float * q, const float * k, const float * v, __half * kcache, __half * vcache, float * out, int n_head, int n_head_kv,
                       int D, const int32_t * pos_dev, int n_ctx, const RopeParams & rp, const float * freq_factors, float scale, cudaStream_t stream,

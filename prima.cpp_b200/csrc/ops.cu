@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) k_attn_decode(const float * __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Tiled prompt-processing attention: one CTA per (kv head, ATT_TQ consecutive tokens; 4, or 2 / 1 for long contexts).  Warp w =
+// Tiled prompt-processing attention for arrays that the tensor-core kernel (attn_tc.cu) does not take (queries at 4-byte boundaries): one CTA per (kv head, ATT_TQ consecutive tokens; 4, or 2 / 1 for long contexts).  Warp w =
 // q head w of the GQA group (loops when gqa > 8) for those tokens; K and V stream through shared memory in 32-position tiles and every tile is used by all
 // gqa x 4 query rows (a per-(head, token) grid re-reads K/V for every row: measured L2-bound at 7 TB/s, 0.6 ms per 70B layer at T = 512).  Numerics are the CPU
 // graph's (FA off): q and the probabilities rounded to f16, softmax sum in double; scores of all rows live in shared memory,
@@ -1310,8 +1310,11 @@ int launch_attn_decode(const float * q, const __half * kcache, const __half * vc
 int launch_attn_batch(const float * q, const __half * kcache, const __half * vcache, float * out, int n_head, int n_head_kv, int D,
                       const int32_t * pos_dev, int n_tok, int n_kv_max, float scale, cudaStream_t stream) {
     if (D != 128 || n_tok <= 0 || n_tok > 65535) return (int) cudaErrorInvalidValue;
-    static const int attn_mode = getenv("PB200_ATTN_MODE") ? atoi(getenv("PB200_ATTN_MODE")) : 0;   // A/B switch: 1 = the per-(head, token) grid of k_attn_decode
-    if (attn_mode == 0 && n_head % n_head_kv == 0) {   // tiled kernel: all score rows of gqa x TQ queries in shared memory
+    static const int attn_mode = getenv("PB200_ATTN_MODE") ? atoi(getenv("PB200_ATTN_MODE")) : 0;   // A/B switch: 1 = the per-(head, token) grid of k_attn_decode, 2 = the tiled kernel of this file
+    // one kernel for every length, so that a row's bits do not depend on how a prompt is cut (prompts of 32 tokens and less lose 1 to 3 us of 6 by it)
+    if (attn_mode == 0 && attn_prefill_tc_ok(q, kcache, vcache, out, n_head, n_head_kv, D, n_kv_max))
+        return launch_attn_prefill_tc(q, kcache, vcache, out, n_head, n_head_kv, pos_dev, n_tok, n_kv_max, scale, stream);
+    if ((attn_mode == 0 || attn_mode == 2) && n_head % n_head_kv == 0) {   // tiled kernel: all score rows of gqa x TQ queries in shared memory
         const int gqa = n_head / n_head_kv;
         const int n_kv_pad = (n_kv_max + 31) & ~31;
         auto smem_for = [&](int tq) { return (size_t) gqa * tq * n_kv_pad * 4 + (size_t) gqa * tq * D * 4 + (size_t) ATT_TK * ATT_KSTRIDE * 2; };
