@@ -1,0 +1,522 @@
+// prima.cpp_b200/csrc/attn_split.cu — prompt attention of the layer-list models (windows, kept first tokens, chunks, soft-cap, sinks, gates, grouped
+// heads, keys with a shared tail, another layer's cache) on the 5th-generation tensor cores, with fp32 inputs kept to 22 bits and more:
+// every fp32 operand x is two f16 numbers, hi = f16(x s) and lo = f16(x s - hi) with s a power of two per row that puts the row's largest
+// entry between 2^13 and 2^14, and a product is hi hi + hi lo + lo hi with fp32 accumulation.  What is dropped (lo lo and the rounding of lo) is
+// 2^-22 of the row's entries and less.  Scores, softmax, its running maximum and sum and the weighted sum across key tiles stay in fp32
+// registers; the weights are split like the other operands.
+// Two launches: k_split_kv writes keys and values once, split and laid out as the operands' shared-memory images; k_attn_split walks them.
+// Only models that compute in bf16 come here (the result is rounded to 2^-9 next); float32 models keep the fp32 FMA kernels of mixers.cu.
+// Against float64 in models where nothing else rounds below fp32, over windows, chunks, sinks and 40 .. 700 keys: 2.9e-7 .. 5.8e-7 off, the FMA
+// kernel, whose sums round once a term, 2.9e-7 .. 5.8e-7 (at most 6 % less or more case by case; tests/test_gpu_attn_split.py).
+// Measured with the split pass: 2048 tokens, 16 heads of 128 over 4, causal 1516 -> 105 us; 512 tokens 176 -> 44; latent heads, prompts of 1111,
+// 300 and 77 tokens 522 -> 94.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <atomic>
+
+#include "launch.h"
+#include "layers.h"
+#include "mixers.cuh"
+#include "tc.cuh"
+
+namespace pb {
+namespace {
+
+constexpr int SP_KEYS = 128;                   // positions of a key tile
+constexpr int SP_K_UNIT = 2 * SP_KEYS * 128;   // 64 head entries of a tile's keys: hi, lo, each 128 rows of 128 bytes
+constexpr int SP_MAX_ND = 3, SP_MAX_NV = 2;    // head sizes up to 192, value sizes up to 128
+constexpr int SP_SCALES = 1040;                // key scales [128], value ratios [128], value factor [4] of a tile
+constexpr int SP_THREADS = 320, SP_SM_THREADS = 256;
+
+__host__ __device__ inline int sp_v_unit(int nv) { return 2 * nv * 64 * 128; }   // 64 positions of a tile's values: hi, lo, each nv blocks of 64 rows of 128 bytes
+__host__ __device__ inline int64_t sp_tile_bytes(int nd, int nv) { return (int64_t) nd * SP_K_UNIT + 2 * sp_v_unit(nv) + SP_SCALES; }
+
+struct SplitParams {
+    AttnIO io;
+    AttnParams a;
+    const int32_t * off;
+    uint8_t * ws;              // [kv head][tile slot][sp_tile_bytes]; entry e's first slot: off[e] / 128 + e
+    int slots;
+    void * out;
+    int nd, nv, gqa, tok_per_cta, stages;
+    int * abort_flag;
+};
+
+// power of two that puts the largest entry (bits of its magnitude) in [2^13, 2^14); e: the clamped exponent it follows from
+__device__ __forceinline__ float split_scale(uint32_t max_bits, int lowest, int & e) {
+    e = min(max((int) (max_bits >> 23), lowest), 254);
+    return __uint_as_float((uint32_t) max(267 - e, 1) << 23);
+}
+__device__ __forceinline__ void split2(float x, float y, uint32_t & hi, uint32_t & lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+// One CTA: a tile of 128 positions of one kv head and entry; a warp takes a position at a time, a lane two neighbouring entries of every 64.
+__global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitParams P) {
+    __shared__ int ev[SP_KEYS];
+    const int e = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x;
+    const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
+    if (tile * SP_KEYS >= n) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const AttnIO & io = P.io;
+    const int D = P.a.dim, DN = P.a.dim - P.a.shared_dim, DV = P.a.vdim;
+    const int64_t at = io.kv_slot ? (int64_t) io.kv_slot[e] * io.kv_slot_stride : 0;
+    const float * kb = io.k + (io.kv_slot ? at : (int64_t) t_begin * io.ldk) + (int64_t) kvh * DN;
+    const float * vb = io.v + (io.kv_slot ? at : (int64_t) t_begin * io.ldv) + (int64_t) kvh * DV;
+    const float * ks = io.ks ? io.ks + (int64_t) t_begin * io.ldks : nullptr;
+    uint8_t * dst = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e + tile) * sp_tile_bytes(P.nd, P.nv);
+    uint8_t * dv = dst + P.nd * SP_K_UNIT;
+    float * sc = reinterpret_cast<float *>(dv + 2 * sp_v_unit(P.nv));
+    const int blk_b = sp_v_unit(P.nv) / 2;                         // the lo half of a unit of values
+    constexpr int ROWS = 4;
+    for (int r0 = warp * 16; r0 < warp * 16 + 16; r0 += ROWS) {
+        float k[ROWS][SP_MAX_ND][2], v[ROWS][SP_MAX_NV][2];
+#pragma unroll
+        for (int j = 0; j < ROWS; j++) {
+            const int64_t p = (int64_t) tile * SP_KEYS + r0 + j;
+            const bool live = p < n;
+#pragma unroll
+            for (int c = 0; c < SP_MAX_ND; c++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int d = 64 * c + 2 * lane + i;
+                    k[j][c][i] = live && d < D ? (d < DN ? kb[p * io.ldk + d] : ks[p * io.ldks + d - DN]) : 0.f;
+                }
+#pragma unroll
+            for (int c = 0; c < SP_MAX_NV; c++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int d = 64 * c + 2 * lane + i;
+                    v[j][c][i] = live && d < DV ? vb[p * io.ldv + d] : 0.f;
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; j++) {
+            const int r = r0 + j;
+            uint32_t mk = 0u, mv = 0u;
+#pragma unroll
+            for (int c = 0; c < SP_MAX_ND; c++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) mk = max(mk, __float_as_uint(k[j][c][i]) & 0x7fffffffu);
+#pragma unroll
+            for (int c = 0; c < SP_MAX_NV; c++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) mv = max(mv, __float_as_uint(v[j][c][i]) & 0x7fffffffu);
+            mk = __reduce_max_sync(0xffffffffu, mk);
+            mv = __reduce_max_sync(0xffffffffu, mv);
+            int ek, e_v;
+            const float sk = split_scale(mk, 14, ek), sv = split_scale(mv, 28, e_v);
+            const uint32_t in_row = (uint32_t) ((((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+#pragma unroll
+            for (int c = 0; c < SP_MAX_ND; c++)
+                if (c < P.nd) {
+                    uint32_t hi, lo;
+                    split2(k[j][c][0] * sk, k[j][c][1] * sk, hi, lo);
+                    uint8_t * o = dst + c * SP_K_UNIT + (r >> 3) * 1024 + (r & 7) * 128 + in_row;
+                    *reinterpret_cast<uint32_t *>(o) = hi;
+                    *reinterpret_cast<uint32_t *>(o + SP_K_UNIT / 2) = lo;
+                }
+            const int rv = r & 63;
+#pragma unroll
+            for (int c = 0; c < SP_MAX_NV; c++)
+                if (c < P.nv) {
+                    uint32_t hi, lo;
+                    split2(v[j][c][0] * sv, v[j][c][1] * sv, hi, lo);
+                    uint8_t * o = dv + (r >> 6) * sp_v_unit(P.nv) + c * 8192 + (rv >> 3) * 1024 + (rv & 7) * 128 + in_row;
+                    *reinterpret_cast<uint32_t *>(o) = hi;
+                    *reinterpret_cast<uint32_t *>(o + blk_b) = lo;
+                }
+            if (lane == 0) {
+                sc[r] = __uint_as_float((uint32_t) (ek - 13) << 23);
+                ev[r] = e_v;
+            }
+        }
+    }
+    __syncthreads();
+    // the values' powers of two meet the weights: relative to the tile's largest one, times 2^14 (weights are at most 1, f16 reaches 2^16)
+    if (warp < 4) {
+        int top = max(max(ev[lane], ev[lane + 32]), max(ev[lane + 64], ev[lane + 96]));
+        top = __reduce_max_sync(0xffffffffu, top);
+        const int r = warp * 32 + lane, f = 141 + ev[r] - top;
+        sc[SP_KEYS + r] = f >= 1 ? __uint_as_float((uint32_t) f << 23) : 0.f;
+        if (r < 4) sc[2 * SP_KEYS + r] = __uint_as_float((uint32_t) (top - 27) << 23);
+    }
+}
+
+struct SpCtl {
+    uint64_t full[4], empty[4], sc_full[2], sc_empty[2], s_full[2], p_full[2], o_full[2], o_free[2];
+    uint32_t tmem_base;
+    int abort;
+    float row_max[2][2][128];      // [tile parity][half of the keys][row]
+    float q_scale[128];
+    float row_l[2][128];
+};
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int h, int d, int DV) {
+    if (io.gate_mode == 1) return sigmoid_f(io.gate[row * io.ldg + h]);
+    if (io.gate_mode == 2) return sigmoid_f(io.gate[row * io.ldg + (int64_t) h * DV + d]);
+    return 1.f;
+}
+
+// One CTA: 128 query rows (the heads of a GQA group x 128 / group consecutive tokens) of one entry and kv head.  Tensor memory: S twice (2 x 128
+// columns; the split weights go over the scores they come from), the tile's weighted sum twice (2 x 128).
+//   warp 0       key units (64 head entries of 128 keys, hi and lo: 32 KB), value units (64 positions, hi and lo) by bulk copies of the split images
+//   warp 1       MMA issuer, owner of the tensor memory; S(j + 1) goes before P(j) V(j)
+//   warps 2 - 9  softmax: thread = (row, half of the tile's keys); the weighted sum [row][half of the value columns] in registers
+// Bound: 24 MMAs of 107 clocks for S (operand A from shared memory) and 24 of 74 for P V a 128 x 128 tile of 128-wide heads, 4300 clocks; the
+// softmax warps take about half of that. 
+template <typename OT, bool CAP>
+__global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_constant__ SplitParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    const AttnIO & io = P.io;
+    const AttnParams & a = P.a;
+    const int e = blockIdx.z, kvh = blockIdx.x;
+    const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
+    const int q0 = ((int) gridDim.y - 1 - (int) blockIdx.y) * P.tok_per_cta;      // long rows first
+    if (q0 >= n) return;
+    const int toks = min(P.tok_per_cta, n - q0), rows = toks * P.gqa;
+    uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int nd = P.nd, nv = P.nv, stages = P.stages, v_unit = sp_v_unit(nv), q_piece = nd * 16384;
+    uint8_t * q_s = smem, * ring = smem + 2 * q_piece;                            // queries: hi, lo, each nd blocks of 128 rows of 128 bytes
+    float * scales = reinterpret_cast<float *>(ring + stages * SP_K_UNIT);       // [2][SP_SCALES]
+    SpCtl * ctl = reinterpret_cast<SpCtl *>(ring + stages * SP_K_UNIT + 2 * SP_SCALES);
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    volatile int * cta_abort = &ctl->abort;
+    // key tiles some row sees: the kept first tokens' ones, then from the window's (chunk's) first position to the last query
+    const int w_lo = attn_first_visible(a, q0), s_hi = min(a.keep_first, w_lo);
+    const int kept = (s_hi + SP_KEYS - 1) / SP_KEYS, first = max(w_lo / SP_KEYS, kept), last = (q0 + toks - 1) / SP_KEYS;
+    const int nt = kept + last - first + 1;
+    auto tile_of = [&](int j) { return j < kept ? j : first + j - kept; };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; i++) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], 1); }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&ctl->sc_full[i], 1); mbar_init(&ctl->sc_empty[i], 8); mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_full[i], 8);
+            mbar_init(&ctl->o_full[i], 1); mbar_init(&ctl->o_free[i], 8);
+        }
+        ctl->abort = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else if (warp >= 2) {
+        const int w = warp - 2, D = a.dim;
+        for (int r0 = w * 16; r0 < w * 16 + 16; r0 += 4) {
+            float x[4][SP_MAX_ND][2];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int r = r0 + j;
+                const float * src = io.q + (int64_t) (t_begin + q0 + r / P.gqa) * io.ldq + (int64_t) (kvh * P.gqa + r % P.gqa) * D;
+#pragma unroll
+                for (int c = 0; c < SP_MAX_ND; c++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const int d = 64 * c + 2 * lane + i;
+                        x[j][c][i] = r < rows && d < D ? src[d] : 0.f;
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int r = r0 + j;
+                uint32_t m = 0u;
+#pragma unroll
+                for (int c = 0; c < SP_MAX_ND; c++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) m = max(m, __float_as_uint(x[j][c][i]) & 0x7fffffffu);
+                m = __reduce_max_sync(0xffffffffu, m);
+                int eq;
+                const float s = split_scale(m, 14, eq);
+#pragma unroll
+                for (int c = 0; c < SP_MAX_ND; c++)
+                    if (c < nd) {
+                        uint32_t hi, lo;
+                        split2(x[j][c][0] * s, x[j][c][1] * s, hi, lo);
+                        uint8_t * o = q_s + c * 16384 + (r >> 3) * 1024 + (r & 7) * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4;
+                        *reinterpret_cast<uint32_t *>(o) = hi;
+                        *reinterpret_cast<uint32_t *>(o + q_piece) = lo;
+                    }
+                if (lane == 0) ctl->q_scale[r] = __uint_as_float((uint32_t) (eq - 13) << 23);
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *(volatile uint32_t *) &ctl->tmem_base;
+    constexpr uint32_t O0 = 256;
+
+    if (warp == 0) {
+        const uint8_t * src0 = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
+        int u = 0;
+        auto load = [&](const uint8_t * src, uint32_t bytes) {
+            const int s = u % stages;
+            if (u >= stages) mbar_wait(&ctl->empty[s], (uint32_t) ((u / stages - 1) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&ctl->full[s], bytes);
+                bulk_load(smem_u32(ring + s * SP_K_UNIT), src, bytes, smem_u32(&ctl->full[s]));
+            }
+            __syncwarp();
+            u++;
+        };
+        for (int j = 0; j <= nt && !*cta_abort; j++) {   // K(0) K(1) V(0) K(2) V(1) ...
+            if (j < nt) {
+                const uint8_t * src = src0 + (int64_t) tile_of(j) * sp_tile_bytes(nd, nv);
+                if (j >= 2) mbar_wait(&ctl->sc_empty[j & 1], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&ctl->sc_full[j & 1], SP_SCALES);
+                    bulk_load(smem_u32(scales) + (j & 1) * SP_SCALES, src + nd * SP_K_UNIT + 2 * v_unit, SP_SCALES, smem_u32(&ctl->sc_full[j & 1]));
+                }
+                __syncwarp();
+                for (int c = 0; c < nd; c++) load(src + c * SP_K_UNIT, SP_K_UNIT);
+            }
+            if (j > 0) {
+                const uint8_t * src = src0 + (int64_t) tile_of(j - 1) * sp_tile_bytes(nd, nv) + nd * SP_K_UNIT;
+                for (int c = 0; c < 2; c++) load(src + c * v_unit, (uint32_t) v_unit);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t) (SP_KEYS >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+        const uint32_t idesc_v = (1u << 4) | (1u << 16) | ((uint32_t) (nv * 64 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+        const uint64_t dq = desc_sw128(smem_u32(q_s));
+        const uint32_t q_lo = (uint32_t) (q_piece >> 4);
+        int u = 0;
+        auto scores = [&](int j) {
+            const uint32_t d = tmem + (uint32_t) ((j & 1) * 128);
+            for (int c = 0; c < nd; c++, u++) {
+                const int s = u % stages;
+                mbar_wait(&ctl->full[s], (uint32_t) ((u / stages) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
+                fence_after();
+                const uint64_t hk = desc_sw128(smem_u32(ring + s * SP_K_UNIT)), lk = hk + (SP_K_UNIT / 2 >> 4), hq = dq + c * (16384 >> 4), lq = hq + q_lo;
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16<1>(d, lq + 2 * k, hk + 2 * k, idesc, (uint32_t) ((c | k) != 0));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, lk + 2 * k, idesc, 1u);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, hk + 2 * k, idesc, 1u);
+                    mma_commit(&ctl->empty[s]);
+                    if (c == nd - 1) mma_commit(&ctl->s_full[j & 1]);
+                }
+                __syncwarp();
+            }
+        };
+        scores(0);
+        for (int j = 0; j < nt && !*cta_abort; j++) {
+            if (j + 1 < nt) scores(j + 1);       // its columns held P(j - 1), whose products precede it in the pipe
+            const int buf = j & 1;
+            mbar_wait(&ctl->p_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+            if (j >= 2) mbar_wait(&ctl->o_free[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            const uint32_t d = tmem + O0 + (uint32_t) (buf * 128);
+            for (int h = 0; h < 2; h++, u++) {
+                const int s = u % stages;
+                mbar_wait(&ctl->full[s], (uint32_t) ((u / stages) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
+                fence_after();
+                const uint64_t hv = desc_sw128_mn(smem_u32(ring + s * SP_K_UNIT), 8192), lv = hv + (v_unit / 2 >> 4);
+                const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);          // 16 columns hi, 16 columns lo of 32 keys, then the next 32
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + 16 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, (uint32_t) ((h | k) != 0));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, lv + k * (2048 >> 4), idesc_v, 1u);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, 1u);
+                    mma_commit(&ctl->empty[s]);
+                    if (h == 1) mma_commit(&ctl->o_full[buf]);
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    } else {
+        const int quad = warp & 3, part = (warp - 2) >> 2, row = quad * 32 + lane;
+        const int qi = row < rows ? q0 + row / P.gqa : -1;                       // the row's position; -1: sees nothing
+        const int lo_q = qi >= 0 ? attn_first_visible(a, qi) : 0;
+        const int h = kvh * P.gqa + (row < rows ? row % P.gqa : 0);
+        const uint32_t mine = tmem + ((uint32_t) (quad * 32) << 16);
+        constexpr float LOG2E = 1.4426950408889634f;
+        const float qs = CAP ? ctl->q_scale[row] * a.scale / a.softcap : ctl->q_scale[row] * a.scale * LOG2E, cap = a.softcap * LOG2E;
+        const int all_from = attn_first_visible(a, q0 + toks - 1), all_to = q0;   // positions in [all_from, all_to] are visible to every row
+        float o[64], m = -INFINITY, l = 0.f, corr1 = 0.f, f1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 64; i++) o[i] = 0.f;
+        auto add_tile = [&](int j, float corr, float f) {                        // o = o * corr + f * (tile j's weighted sum)
+            mbar_wait(&ctl->o_full[j & 1], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            uint32_t v[32];
+            if (part < nv) {
+                const uint32_t at = mine + O0 + (uint32_t) ((j & 1) * 128 + part * 64);
+#pragma unroll
+                for (int c = 0; c < 64; c += 32) {
+                    TMEM_LD32(at + c, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; i++) o[c + i] = fmaf(o[c + i], corr, __uint_as_float(v[i]) * f);
+                }
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl->o_free[j & 1]);
+        };
+        for (int j = 0; j < nt; j++) {   // to the end also after an abort (waits return at once then): the warps meet at a barrier in every round
+            const int buf = j & 1, k0 = tile_of(j) * SP_KEYS + part * 64;
+            const float * sc = scales + buf * (SP_SCALES / 4) + part * 64;
+            mbar_wait(&ctl->sc_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+            mbar_wait(&ctl->s_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            float t[64];
+            uint32_t * v = reinterpret_cast<uint32_t *>(t);
+            const uint32_t at = mine + (uint32_t) (buf * 128 + part * 64);
+            TMEM_LD32(at, v);
+            TMEM_LD32(at + 32, v + 32);
+            tmem_wait_ld();
+            const bool every = k0 >= all_from && k0 + 63 <= all_to;
+            float tm = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 64; i += 4) {
+                const float4 s4 = *reinterpret_cast<const float4 *>(sc + i);
+                const float f[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float x = t[i + q] * f[q] * qs;
+                    if constexpr (CAP) x = cap * tanhf(x);
+                    if (!every) {
+                        const int kj = k0 + i + q;
+                        if (!(kj <= qi && (kj >= lo_q || kj < a.keep_first))) x = -INFINITY;
+                    }
+                    t[i + q] = x;
+                    tm = fmaxf(tm, x);
+                }
+            }
+            ctl->row_max[buf][part][row] = tm;
+            asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
+            const float mn = fmaxf(m, fmaxf(tm, ctl->row_max[buf][part ^ 1][row]));
+            const float ref = mn == -INFINITY ? 0.f : mn;
+            const float corr = m == -INFINITY ? 0.f : ex2(m - ref);
+            float e4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 64; c += 32) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 r4 = *reinterpret_cast<const float4 *>(sc + SP_KEYS + c + i);
+                    const float r[4] = {r4.x, r4.y, r4.z, r4.w};
+                    float p[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        p[q] = ex2(t[c + i + q] - ref);
+                        e4[q] += p[q];
+                        p[q] *= r[q];
+                    }
+                    split2(p[0], p[1], hi[i / 2], lo[i / 2]);
+                    split2(p[2], p[3], hi[i / 2 + 1], lo[i / 2 + 1]);
+                }
+                TMEM_ST16(at + c, hi);
+                TMEM_ST16(at + c + 16, lo);
+            }
+            tmem_wait_st();
+            const float f = scales[buf * (SP_SCALES / 4) + 2 * SP_KEYS];
+            fence_before();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&ctl->p_full[buf]); mbar_arrive(&ctl->sc_empty[buf]); }
+            l = l * corr + ((e4[0] + e4[1]) + (e4[2] + e4[3]));
+            m = mn;
+            if (j > 0) add_tile(j - 1, corr1, f1);
+            corr1 = corr;
+            f1 = f;
+        }
+        add_tile(nt - 1, corr1, f1);
+        ctl->row_l[part][row] = l;
+        asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
+        l = ctl->row_l[0][row] + ctl->row_l[1][row];
+        if (a.sink && m != -INFINITY) l += ex2((io.sink ? io.sink[h] : 0.f) * LOG2E - m);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        // through the ring's memory (every unit has been used; a row's 16-byte pieces rotated by the row), so that a warp stores whole rows
+        float * os = reinterpret_cast<float *>(ring);
+        if (part < nv) {
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                *reinterpret_cast<float4 *>(os + row * 128 + ((part * 16 + i + row) & 31) * 4) = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
+        const int DV = a.vdim, w = warp - 2;
+        for (int r = w * 16; r < w * 16 + 16 && r < rows; r++) {
+            const int64_t tok = t_begin + q0 + r / P.gqa;
+            const int hh = kvh * P.gqa + r % P.gqa;
+#pragma unroll
+            for (int c = 0; c < 128; c += 32) {
+                const int d = c + lane;
+                if (d < DV) put((OT *) P.out, tok * ((int64_t) a.heads * DV) + (int64_t) hh * DV + d, os[r * 128 + (((d >> 2) + r) & 31) * 4 + (d & 3)] * gate_factor(io, tok, hh, d, DV));
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+template <typename OT, bool CAP>
+int launch_typed(const SplitParams & P, const dim3 & grid, size_t smem, cudaStream_t st) {
+    static FuncAttrCache cache;
+    const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_attn_split<OT, CAP>, smem, true);
+    if (e != cudaSuccess) return (int) e;
+    k_attn_split<OT, CAP><<<grid, SP_THREADS, smem, st>>>(P);
+    return (int) cudaGetLastError();
+}
+int split_slots(int n_tokens, int n_entries) { return n_tokens / SP_KEYS + n_entries; }   // floor(off / 128) + e are distinct runs of slots
+
+}  // namespace
+
+// scratch that a batch of n_tokens prompt tokens in up to n_tokens / 128 + 16 entries needs
+size_t attn_split_bytes(const AttnParams & a, int n_tokens) {
+    if (a.dim > 64 * SP_MAX_ND || a.vdim > 64 * SP_MAX_NV || a.dim <= 0 || a.vdim <= 0 || a.kv_heads <= 0) return 0;
+    return (size_t) a.kv_heads * (size_t) split_slots(n_tokens, n_tokens / SP_KEYS + 16) * (size_t) sp_tile_bytes((a.dim + 63) / 64, (a.vdim + 63) / 64);
+}
+bool attn_split_ok(const AttnIO & io, const BatchView & b, const AttnParams & a) {
+    if (!io.split_ws || a.dim > 64 * SP_MAX_ND || a.vdim > 64 * SP_MAX_NV || a.heads / a.kv_heads > 128 || b.n_entries > 65535) return false;
+    const size_t need = (size_t) a.kv_heads * (size_t) split_slots(b.n_tokens, b.n_entries) * (size_t) sp_tile_bytes((a.dim + 63) / 64, (a.vdim + 63) / 64);
+    return need <= io.split_bytes;
+}
+int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t st) {
+    SplitParams P{};
+    P.io = io; P.a = a; P.off = b.off;
+    P.ws = (uint8_t *) io.split_ws;
+    P.slots = split_slots(b.n_tokens, b.n_entries);
+    P.out = out;
+    P.nd = (a.dim + 63) / 64; P.nv = (a.vdim + 63) / 64;
+    P.gqa = a.heads / a.kv_heads;
+    P.tok_per_cta = 128 / P.gqa;
+    P.stages = P.nd == 3 ? 3 : 4;
+    P.abort_flag = abort_flag();
+    g_launches += 2;
+    k_split_kv<<<dim3((unsigned) ((b.max_n + SP_KEYS - 1) / SP_KEYS), (unsigned) a.kv_heads, (unsigned) b.n_entries), 256, 0, st>>>(P);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int) e;
+    const size_t smem = 1024 + (size_t) P.nd * 32768 + (size_t) P.stages * SP_K_UNIT + 2 * SP_SCALES + sizeof(SpCtl);
+    const dim3 grid((unsigned) a.kv_heads, (unsigned) ((b.max_n + P.tok_per_cta - 1) / P.tok_per_cta), (unsigned) b.n_entries);
+    if (otype == T_BF16) return a.softcap > 0.f ? launch_typed<__nv_bfloat16, true>(P, grid, smem, st) : launch_typed<__nv_bfloat16, false>(P, grid, smem, st);
+    return a.softcap > 0.f ? launch_typed<float, true>(P, grid, smem, st) : launch_typed<float, false>(P, grid, smem, st);
+}
+
+}  // namespace pb

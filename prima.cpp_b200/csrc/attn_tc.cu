@@ -43,48 +43,6 @@ struct AtParams {
     int * abort_flag;
 };
 
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {   // A in tensor memory
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// operand in shared memory, N contiguous (values [key][dim]), SWIZZLE_128B: rows of 64 entries, 8-key groups 1024 bytes apart, blocks of 64 entries AT_BLOCK apart
-__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr) {
-    uint64_t d = (uint64_t) ((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t) (AT_BLOCK >> 4) << 16;
-    d |= (uint64_t) (1024 >> 4) << 32;
-    d |= (uint64_t) 1 << 46;
-    d |= (uint64_t) 2 << 61;
-    return d;
-}
-#define TMEM_LD32(addr, v)                                                                                                                              \
-    asm volatile(                                                                                                                                       \
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, "   \
-        "%22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"                                                                                     \
-        : "=r"((v)[0]), "=r"((v)[1]), "=r"((v)[2]), "=r"((v)[3]), "=r"((v)[4]), "=r"((v)[5]), "=r"((v)[6]), "=r"((v)[7]), "=r"((v)[8]), "=r"((v)[9]),     \
-          "=r"((v)[10]), "=r"((v)[11]), "=r"((v)[12]), "=r"((v)[13]), "=r"((v)[14]), "=r"((v)[15]), "=r"((v)[16]), "=r"((v)[17]), "=r"((v)[18]),          \
-          "=r"((v)[19]), "=r"((v)[20]), "=r"((v)[21]), "=r"((v)[22]), "=r"((v)[23]), "=r"((v)[24]), "=r"((v)[25]), "=r"((v)[26]), "=r"((v)[27]),          \
-          "=r"((v)[28]), "=r"((v)[29]), "=r"((v)[30]), "=r"((v)[31])                                                                                    \
-        : "r"(addr)                                                                                                                                     \
-        : "memory")
-#define TMEM_ST16(addr, v)                                                                                                                              \
-    asm volatile(                                                                                                                                       \
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr), "r"((v)[0]), \
-        "r"((v)[1]), "r"((v)[2]), "r"((v)[3]), "r"((v)[4]), "r"((v)[5]), "r"((v)[6]), "r"((v)[7]), "r"((v)[8]), "r"((v)[9]), "r"((v)[10]), "r"((v)[11]),  \
-        "r"((v)[12]), "r"((v)[13]), "r"((v)[14]), "r"((v)[15])                                                                                          \
-        : "memory")
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -209,7 +167,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2)
             mbar_wait(&ctl->p_full, (uint32_t) (i & 1), cta_abort, P.abort_flag);
             __syncwarp();
             fence_after();
-            const uint64_t dv = desc_sw128_mn(smem_u32(ring + s * AT_STAGE));
+            const uint64_t dv = desc_sw128_mn(smem_u32(ring + s * AT_STAGE), AT_BLOCK);
             if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < 8; k++) mma_f16_ts(tmem + O0, tmem + S0 + (k >> 2) * 64 + (k & 3) * 8, dv + k * (2048 >> 4), idesc_v, (uint32_t) ((i | k) != 0));

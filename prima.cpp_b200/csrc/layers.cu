@@ -217,6 +217,8 @@ struct LayerList {
     float *x = nullptr, *x0 = nullptr, *xalt = nullptr, *big = nullptr, *msub = nullptr, *xbc = nullptr, *yssm = nullptr, *logits = nullptr;
     void *act = nullptr, *act2 = nullptr, *actw = nullptr;
     // FRAME_PRENORM and its mixers: results of all layers [layers + 1][capT][width]; further fp32 and operand-type scratch
+    void * split_ws = nullptr;      // split keys and values of a prompt (attn_split.cu); bf16 models with an attention layer that fits
+    size_t split_bytes = 0;
     float *hist = nullptr, *big2 = nullptr, *big3 = nullptr, *big4 = nullptr, *krb = nullptr;
     float * lat_part = nullptr;     // partial results of the split decode attention kernels: latent [entries][splits][heads][kv_rank + 2], windowed [entries][heads][splits][vdim + 2]
     size_t lat_part_cap = 0;
@@ -1951,6 +1953,21 @@ static int ll_reserve(pb200_model * m, int T, int nW, int nE) {
             if (!ll.moe_count_host) CK(cudaMallocHost((void **) &ll.moe_count_host, (size_t) 2 * 4096 * 4));
         }
         CK(grab(&ll.actw, (size_t) cW * W * es));
+        ll.split_ws = nullptr; ll.split_bytes = 0;
+        // PB200_ATTN_SPLIT: 0 = prompts keep the fp32 FMA attention, 1 = float32 models take the split kernel as well (A/B runs, tests)
+        const char * sp = getenv("PB200_ATTN_SPLIT");
+        if (cT > 16 && (sp ? atoi(sp) != 0 : ll.ctype == T_BF16)) {
+            size_t need = 0;
+            for (const LLayer & L : ll.layers) {
+                AttnParams ap = L.att;
+                if (L.weights_of >= 0) continue;
+                if (L.kind == MIX_LATENT) { ap.kv_heads = L.lat.heads; ap.dim = L.lat.dim + L.lat.rot_dim; ap.vdim = L.lat.vdim; }
+                else if (L.kind != MIX_ATTENTION && L.kind != MIX_DUAL) continue;
+                need = std::max(need, attn_split_bytes(ap, cT));
+            }
+            if (need) CK(grab(&ll.split_ws, need));
+            ll.split_bytes = need;
+        }
         CK(grab((void **) &ll.logits, (size_t) cW * (size_t) ll.vocab * 4));
         CK(grab((void **) &ll.greedy_dev, (size_t) cW * 4));
         if (ll.greedy_host) cudaFreeHost(ll.greedy_host);
@@ -2053,6 +2070,7 @@ static int mix_attention(pb200_model * m, const BatchView & b, bool prefill, con
         io.v = vc; io.ldv = io.v_row;
         io.kv_slot = b.slot; io.kv_slot_stride = ll.slot_floats;
     }
+    io.split_ws = ll.split_ws; io.split_bytes = ll.split_bytes;
     if (prefill) CK(launch_attn_prefill_io(io, b, a, ll.act, ct, st));
     else CK(launch_attn_decode_io(io, b, a, kc, vc, ll.slot_floats, ll.act, ct, st, ll.lat_part));
     CAT(CAT_DENSE);
@@ -2137,6 +2155,7 @@ static int mix_latent(pb200_model * m, const BatchView & b, bool prefill, const 
         io.ks = ll.krb; io.ldks = a.rot_dim;
         io.v = ll.big3 + (int64_t) H * a.dim; io.ldv = KV;
         io.gate = gate; io.ldg = C; io.gate_mode = a.gate_mode;
+        io.split_ws = ll.split_ws; io.split_bytes = ll.split_bytes;
         CK(launch_attn_prefill_io(io, b, ap, ll.act, ct, st));
     } else if (T == b.n_entries && R <= 512) {   // one token per entry: the key up-projection folded into the query, rows split over CTAs
         CK(launch_latent_absorb_q(q, ldq, b, wuk, ct, a, L.rot_freq.data, ll.big3, st));
@@ -2301,6 +2320,7 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     if (!post) { io.gate = ll.big + d.c_g; io.ldg = C; io.gate_mode = d.gate_mode; }
     void * att_out = post ? (void *) ll.big2 : ll.act;
     const int att_type = post ? T_F32 : ct;
+    io.split_ws = ll.split_ws; io.split_bytes = ll.split_bytes;
     if (prefill) CK(launch_attn_prefill_io(io, b, a, att_out, att_type, st));
     else CK(launch_attn_decode_io(io, b, a, kc, vc, ll.slot_floats, att_out, att_type, st, ll.lat_part));
     const int64_t ldo = sum ? OD + RV : OD;

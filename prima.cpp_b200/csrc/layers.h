@@ -143,6 +143,8 @@ struct AttnIO {
     // set: prompt kernels read keys and values of position p from row p of the entry's slot (k / v: the cache's base, ldk / ldv its row strides;
     // a cache that holds every position) instead of the batch
     const int32_t * kv_slot = nullptr;  int64_t kv_slot_stride = 0;
+    // scratch of the prompt kernel on the tensor cores (attn_split.cu), for models that compute in bf16; without it the fp32 FMA kernels run
+    void * split_ws = nullptr;  size_t split_bytes = 0;
 };
 // floats of a cached value row (none of its own when a key is its own value)
 __host__ __device__ inline int attn_v_row(const AttnParams & a) { return a.tied_v ? 0 : a.kv_heads * a.vdim; }
@@ -185,6 +187,11 @@ int launch_attn_window_decode(const float * qkvg, const BatchView & b, const Att
 int launch_attn_prefill_io(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t stream);
 int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnParams & a, const float * kcache, const float * vcache, int64_t slot_stride,
                           void * out, int otype, cudaStream_t stream, float * part = nullptr);
+
+// prompt attention with every operand as two f16 numbers on the tensor cores (attn_split.cu): head sizes up to 192, value sizes up to 128
+size_t attn_split_bytes(const AttnParams & a, int n_tokens);   // scratch for prompt batches of up to n_tokens tokens (0: the shape is not taken)
+bool attn_split_ok(const AttnIO & io, const BatchView & b, const AttnParams & a);
+int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t stream);
 
 // ---- Mamba-2 ----
 struct Mamba2Params {

@@ -1056,6 +1056,7 @@ int launch_attn_prefill_io(const AttnIO & io, const BatchView & b, const AttnPar
         (a.shared_dim > 0 && !io.ks))
         return (int) cudaErrorInvalidValue;
     static const bool no_tiled = getenv("PB200_ATTN_ROWWISE") != nullptr;   // A/B: the one-warp-per-query kernel for every length
+    if (b.max_n > 16 && !no_tiled && attn_split_ok(io, b, a)) return launch_attn_split(io, b, a, out, otype, st);
     const size_t tiled_smem = attn_tiled_smem(a.dim, a.vdim);
     if (b.max_n > 16 && !no_tiled && tiled_smem <= 220 * 1024) {   // long entries: 64-query tiles; the same numbers up to fp32 summation order
         const int nvc = (a.vdim + 15) / 16;

@@ -100,6 +100,49 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {   // A in tensor memory
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// operand in shared memory, N contiguous (values [key][dim]), SWIZZLE_128B: rows of 64 entries, 8-key groups 1024 bytes apart, blocks of 64 entries `block` bytes apart
+__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t block) {
+    uint64_t d = (uint64_t) ((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t) (block >> 4) << 16;
+    d |= (uint64_t) (1024 >> 4) << 32;
+    d |= (uint64_t) 1 << 46;
+    d |= (uint64_t) 2 << 61;
+    return d;
+}
+#define TMEM_LD32(addr, v)                                                                                                                              \
+    asm volatile(                                                                                                                                       \
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, "   \
+        "%22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"                                                                                     \
+        : "=r"((v)[0]), "=r"((v)[1]), "=r"((v)[2]), "=r"((v)[3]), "=r"((v)[4]), "=r"((v)[5]), "=r"((v)[6]), "=r"((v)[7]), "=r"((v)[8]), "=r"((v)[9]),     \
+          "=r"((v)[10]), "=r"((v)[11]), "=r"((v)[12]), "=r"((v)[13]), "=r"((v)[14]), "=r"((v)[15]), "=r"((v)[16]), "=r"((v)[17]), "=r"((v)[18]),          \
+          "=r"((v)[19]), "=r"((v)[20]), "=r"((v)[21]), "=r"((v)[22]), "=r"((v)[23]), "=r"((v)[24]), "=r"((v)[25]), "=r"((v)[26]), "=r"((v)[27]),          \
+          "=r"((v)[28]), "=r"((v)[29]), "=r"((v)[30]), "=r"((v)[31])                                                                                    \
+        : "r"(addr)                                                                                                                                     \
+        : "memory")
+#define TMEM_ST16(addr, v)                                                                                                                              \
+    asm volatile(                                                                                                                                       \
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr), "r"((v)[0]), \
+        "r"((v)[1]), "r"((v)[2]), "r"((v)[3]), "r"((v)[4]), "r"((v)[5]), "r"((v)[6]), "r"((v)[7]), "r"((v)[8]), "r"((v)[9]), "r"((v)[10]), "r"((v)[11]),  \
+        "r"((v)[12]), "r"((v)[13]), "r"((v)[14]), "r"((v)[15])                                                                                          \
+        : "memory")
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // ---- host: tensor maps (the encoder comes from the driver at run time, nothing links against it) ----
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
