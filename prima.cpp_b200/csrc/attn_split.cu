@@ -60,6 +60,7 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t & hi, uint32_t
 // One CTA: a tile of 128 positions of one kv head and entry; a warp takes a position at a time, a lane two neighbouring entries of every 64.
 __global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitParams P) {
     __shared__ int ev[SP_KEYS];
+    pdl_enter();
     const int e = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x;
     const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
     if (tile * SP_KEYS >= n) return;
@@ -176,6 +177,7 @@ __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int
 // softmax warps take about half of that. 
 template <typename OT, bool CAP>
 __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_constant__ SplitParams P) {
+    pdl_enter();
     extern __shared__ uint8_t smem_raw[];
     const AttnIO & io = P.io;
     const AttnParams & a = P.a;
@@ -481,8 +483,7 @@ int launch_typed(const SplitParams & P, const dim3 & grid, size_t smem, cudaStre
     static FuncAttrCache cache;
     const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_attn_split<OT, CAP>, smem, true);
     if (e != cudaSuccess) return (int) e;
-    k_attn_split<OT, CAP><<<grid, SP_THREADS, smem, st>>>(P);
-    return (int) cudaGetLastError();
+    return launch_dep(k_attn_split<OT, CAP>, grid, dim3(SP_THREADS), smem, st, P);
 }
 int split_slots(int n_tokens, int n_entries) { return n_tokens / SP_KEYS + n_entries; }   // floor(off / 128) + e are distinct runs of slots
 
@@ -510,9 +511,8 @@ int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams &
     P.stages = P.nd == 3 ? 3 : 4;
     P.abort_flag = abort_flag();
     g_launches += 2;
-    k_split_kv<<<dim3((unsigned) ((b.max_n + SP_KEYS - 1) / SP_KEYS), (unsigned) a.kv_heads, (unsigned) b.n_entries), 256, 0, st>>>(P);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int) e;
+    const int rc = launch_dep(k_split_kv, dim3((unsigned) ((b.max_n + SP_KEYS - 1) / SP_KEYS), (unsigned) a.kv_heads, (unsigned) b.n_entries), dim3(256), 0, st, P);
+    if (rc) return rc;
     const size_t smem = 1024 + (size_t) P.nd * 32768 + (size_t) P.stages * SP_K_UNIT + 2 * SP_SCALES + sizeof(SpCtl);
     const dim3 grid((unsigned) a.kv_heads, (unsigned) ((b.max_n + P.tok_per_cta - 1) / P.tok_per_cta), (unsigned) b.n_entries);
     if (otype == T_BF16) return a.softcap > 0.f ? launch_typed<__nv_bfloat16, true>(P, grid, smem, st) : launch_typed<__nv_bfloat16, false>(P, grid, smem, st);

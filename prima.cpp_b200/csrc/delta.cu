@@ -23,6 +23,7 @@ template <int N> constexpr int ds_stage_floats() { return DS_CHUNK * (3 * N + DS
 template <int N>
 __global__ void __launch_bounds__(DS_COLS / 2 * (N / DS_NREG)) k_delta_scan(GatedLinIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                                            GatedLinParams p, float * __restrict__ state, int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];   // [stages][ q [16][N] | k [16][N] | g [16][N] | v [16][16] | beta [16] ]
     constexpr int LN = N / DS_NREG, NT = DS_COLS / 2 * LN, STAGE = ds_stage_floats<N>();
     const int P = p.vdim, inner = p.heads * P, ptiles = (P + DS_COLS - 1) / DS_COLS;
@@ -146,7 +147,7 @@ int delta_scan_launch(const GatedLinIO & io, const BatchView & b, const GatedLin
     const int rc = raise_smem(k_delta_scan<N>, smem);
     if (rc) return rc;
     const dim3 grid((unsigned) (p.heads * ((p.vdim + DS_COLS - 1) / DS_COLS)), (unsigned) b.n_entries);
-    return ck_launch([&] { k_delta_scan<N><<<grid, DS_COLS / 2 * (N / DS_NREG), smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });
+    return ck_launch([&] { launch_dep(k_delta_scan<N>, dim3(grid), dim3(DS_COLS / 2 * (N / DS_NREG)), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });
 }
 
 }  // namespace

@@ -37,6 +37,7 @@ template <typename WT>
 __global__ void __launch_bounds__(256) k_dense_tile(const WT * __restrict__ A, int64_t lda, const WT * __restrict__ W, int64_t ldw, float * C, int64_t ldc,
                                                     int T, int N, int K, const float * __restrict__ bias, const float * resid, int64_t ldr, float alpha,
                                                     DenseAct act) {
+    pdl_enter();
     __shared__ float As[TK][TM + 4];
     __shared__ float Ws[TK][TN + 4];
     const int t0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, i
     const int rows_per_cta = (blockDim.x >> 5) / KS;
     const int n = blockIdx.x * rows_per_cta + warp / KS, part = warp % KS;
     const bool live = n < N;
+    pdl_trigger();
     if (plane_rows > 0) A += (int64_t) (n / plane_rows) * a_plane;   // several products over operands of their own (n < N: a valid plane)
     constexpr int V = Vec16<WT>::n;
     const int Kc = KS == 1 ? K : ((K + KS - 1) / KS + 32 * V - 1) / (32 * V) * (32 * V);
@@ -136,12 +138,26 @@ __global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, i
     float acc[R * TB];                       // row r of the pair, token t at r * TB + t
 #pragma unroll
     for (int t = 0; t < R * TB; t++) acc[t] = 0.f;
+    // one token: the row's first step is on its way before the kernel in front has ended (its result is A), later ones one step ahead; more of them cost
+    // warps in flight (2048 x 8192, us: none ahead 9.1, one 8.9, two 11.0, four 10.3; a step of a six-layer model 453, 440, 455, 452)
+    constexpr int AHEAD = VEC && TB == 1 ? 1 : 0;
+    uint4 pre[AHEAD > 0 ? AHEAD : 1][R];
+    auto fetch = [&](uint4 (&raw)[R], int k) {                       // weights: streamed once, not kept in L1
+#pragma unroll
+        for (int r = 0; r < R; r++) raw[r] = __ldcs(reinterpret_cast<const uint4 *>(w + r * ldw + k));
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++) {
+        const int k = k_begin + (lane + 32 * i) * V;
+        if (live && k < k_end) fetch(pre[i], k);
+    }
+    pdl_wait();
     if (live) {
-        if (VEC) {
-            for (int k = k_begin + lane * V; k < k_end; k += 32 * V) {
+        if constexpr (VEC) {
+            auto step = [&](const uint4 (&raw)[R], int k) {
                 float wf[R][V];
 #pragma unroll
-                for (int r = 0; r < R; r++) unpack<V>(__ldcs(reinterpret_cast<const uint4 *>(w + r * ldw + k)), wf[r], WT());   // streamed once: do not keep in L1
+                for (int r = 0; r < R; r++) unpack<V>(raw[r], wf[r], WT());
 #pragma unroll
                 for (int t = 0; t < TB; t++) {
                     if (t < T) {
@@ -152,6 +168,31 @@ __global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, i
 #pragma unroll
                             for (int i = 0; i < V; i++) acc[r * TB + t] = fmaf(af[i], wf[r][i], acc[r * TB + t]);
                     }
+                }
+            };
+            int k = k_begin + lane * V;
+            if constexpr (AHEAD > 0) {
+                // the next AHEAD steps are fetched in front of the ones at hand
+                for (; k < k_end; k += 32 * AHEAD * V) {
+                    uint4 cur[AHEAD][R];
+#pragma unroll
+                    for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+                        for (int r = 0; r < R; r++) cur[i][r] = pre[i][r];
+#pragma unroll
+                    for (int i = 0; i < AHEAD; i++) {
+                        const int kn = k + 32 * (AHEAD + i) * V;
+                        if (kn < k_end) fetch(pre[i], kn);
+                    }
+#pragma unroll
+                    for (int i = 0; i < AHEAD; i++)
+                        if (k + 32 * i * V < k_end) step(cur[i], k + 32 * i * V);
+                }
+            } else {
+                for (; k < k_end; k += 32 * V) {
+                    uint4 raw[R];
+                    fetch(raw, k);
+                    step(raw, k);
                 }
             }
         } else {
@@ -237,7 +278,7 @@ int dense_typed(const WT * A, int64_t lda, const WT * W, int64_t ldw, float * C,
         while (KS < 8 && (int64_t) N * KS < 6144 && K / (2 * KS) >= 1024) KS *= 2;
         const dim3 grid((unsigned) ((N + 8 / KS - 1) / (8 / KS))), block(256);
         g_launches++;
-#define PB_ROWS(TB, VEC, GLU) k_dense_rows<WT, TB, VEC, GLU><<<grid, block, 0, st>>>(A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, KS, plane_rows, a_plane, act)
+#define PB_ROWS(TB, VEC, GLU) launch_dep(k_dense_rows<WT, TB, VEC, GLU>, grid, block, 0, st, A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, KS, plane_rows, a_plane, act)
 #define PB_ROWS_TB(TB)                          \
     do {                                        \
         if (glu) {                              \
@@ -255,7 +296,7 @@ int dense_typed(const WT * A, int64_t lda, const WT * W, int64_t ldw, float * C,
     }
     const dim3 grid((unsigned) ((N + TN - 1) / TN), (unsigned) ((T + TM - 1) / TM)), block(256);
     g_launches++;
-    k_dense_tile<WT><<<grid, block, 0, st>>>(A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, act);
+    launch_dep(k_dense_tile<WT>, grid, block, 0, st, A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, act);
     return (int) cudaGetLastError();
 }
 

@@ -126,7 +126,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     constexpr int B_BYTES = BN * 128, STAGE = TC_A_BYTES + B_BYTES, COLS = BN < 32 ? 32 : BN;
     float * Cm = P.C;
     int Tn = P.T, tile_y = blockIdx.y, grp = 0, a_row0 = 0;
+    pdl_trigger();
     if (P.grp_count) {
+        pdl_wait();                    // the counts come from the kernels in front
         for (; grp < P.groups; grp++) {
             const int nt = (P.grp_count[grp] + BN - 1) / BN;
             if (tile_y < nt) break;
@@ -165,16 +167,28 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     volatile int * cta_abort = &ctl->abort;
 
     if (warp == 0) {
-        for (int u = 0; u < nu; u++) {
+        // the weights of the first stages are on their way before the kernel in front has ended; its result is A
+        const int ahead = min(nu, STAGES);
+        auto load_w = [&](int u) {
             const int s = u % STAGES;
-            if (u >= STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / STAGES - 1) & 1), cta_abort, P.abort_flag);
+            mbar_arrive_expect_tx(&ctl->full[s], STAGE);
+            tma_load<1>(smem_u32(smem + s * STAGE), &map_w, (u0 + u) * TC_BK, n0, grp, smem_u32(&ctl->full[s]));
+        };
+        auto load_a = [&](int u) {
+            const int s = u % STAGES;
+            tma_load<1>(smem_u32(smem + s * STAGE + TC_A_BYTES), &map_a, (u0 + u) * TC_BK, a_row0 + t0, plane, smem_u32(&ctl->full[s]));
+        };
+        if (elect_one())
+            for (int u = 0; u < ahead; u++) load_w(u);
+        __syncwarp();
+        pdl_wait();
+        if (elect_one())
+            for (int u = 0; u < ahead; u++) load_a(u);
+        __syncwarp();
+        for (int u = ahead; u < nu; u++) {
+            mbar_wait(&ctl->empty[u % STAGES], (uint32_t) ((u / STAGES - 1) & 1), cta_abort, P.abort_flag);
             __syncwarp();
-            if (elect_one()) {
-                const uint32_t dst = smem_u32(smem + s * STAGE), bar = smem_u32(&ctl->full[s]);
-                mbar_arrive_expect_tx(&ctl->full[s], STAGE);
-                tma_load<1>(dst, &map_w, (u0 + u) * TC_BK, n0, grp, bar);
-                tma_load<1>(dst + TC_A_BYTES, &map_a, (u0 + u) * TC_BK, a_row0 + t0, plane, bar);
-            }
+            if (elect_one()) { load_w(u); load_a(u); }
             __syncwarp();
             if (*cta_abort) break;
         }
@@ -196,6 +210,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
             __syncwarp();
         }
     }
+    pdl_wait();                        // residual rows are read and results written behind it
     mbar_wait(&ctl->acc_full[0], 0u, cta_abort, P.abort_flag);
     __syncwarp();
     fence_after();
@@ -257,6 +272,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles = P.row_tiles * P.tok_tiles;
     const int nk = (P.K + TC_BK - 1) / TC_BK;
+    pdl_trigger();
 
     if (threadIdx.x == 0) {
         prefetch_map(&map_w);
@@ -279,6 +295,15 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
 
     if (warp == 0) {
         int u = 0;
+        const int ahead = pair < tiles ? min(nk, PAIR_STAGES) : 0;   // stages whose weights are on their way before the kernel in front has ended
+        auto load_w = [&](int s, int k, int n0) {
+            if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * PAIR_STAGE);
+            tma_load<2>(smem_u32(smem + s * PAIR_STAGE), &map_w, k * TC_BK, n0 + rank * TC_BM, 0, cluster_addr(smem_u32(&ctl->full[s]), 0));
+        };
+        if (elect_one())
+            for (int k = 0; k < ahead; k++) load_w(k, k, (pair / P.tok_tiles) * 2 * TC_BM);
+        __syncwarp();
+        pdl_wait();
         for (int i = pair; i < tiles && !*cta_abort; i += pairs) {
             const int n0 = (i / P.tok_tiles) * 2 * TC_BM, t0 = (i % P.tok_tiles) * PAIR_BN;
             const int plane = P.plane_rows > 0 ? n0 / P.plane_rows : 0;
@@ -287,10 +312,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
                 if (u >= PAIR_STAGES) mbar_wait(&ctl->empty[s], (uint32_t) ((u / PAIR_STAGES - 1) & 1), cta_abort, P.abort_flag);
                 __syncwarp();
                 if (elect_one()) {
-                    const uint32_t dst = smem_u32(smem + s * PAIR_STAGE), bar = cluster_addr(smem_u32(&ctl->full[s]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * PAIR_STAGE);
-                    tma_load<2>(dst, &map_w, k * TC_BK, n0 + rank * TC_BM, 0, bar);
-                    tma_load<2>(dst + TC_A_BYTES, &map_a, k * TC_BK, t0 + rank * (PAIR_BN / 2), plane, bar);
+                    if (u >= ahead) load_w(s, k, n0);
+                    tma_load<2>(smem_u32(smem + s * PAIR_STAGE + TC_A_BYTES), &map_a, k * TC_BK, t0 + rank * (PAIR_BN / 2), plane, cluster_addr(smem_u32(&ctl->full[s]), 0));
                 }
                 __syncwarp();
                 if (*cta_abort) break;
@@ -327,6 +350,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     } else {
         const int quad = warp & 3, half = (warp - 2) >> 2, r = quad * 32 + lane;
         int j = 0;
+        pdl_wait();
         for (int i = pair; i < tiles; i += pairs, j++) {
             const int buf = j & 1;
             const int n = (i / P.tok_tiles) * 2 * TC_BM + rank * TC_BM + r, t0 = (i % P.tok_tiles) * PAIR_BN;
@@ -374,11 +398,13 @@ int launch_split_stages(const TcParams & P, const TcOperands & o, const dim3 & g
     cfg.blockDim = dim3(SPLIT_THREADS);
     cfg.dynamicSmemBytes = split_smem<BN, STAGES>();
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned) P.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = g_pdl ? 2 : 1;
     g_launches++;
     return (int) cudaLaunchKernelEx(&cfg, k_dense_split<BN, STAGES>, mw, ma, P);
 }
@@ -409,8 +435,7 @@ int launch_pair(TcParams P, const TcOperands & o, cudaStream_t st) {
     const int64_t tiles = (int64_t) P.row_tiles * P.tok_tiles;
     const int pairs = (int) (tiles < sm_count() / 2 ? tiles : sm_count() / 2);
     g_launches++;
-    k_dense_pair<<<dim3((unsigned) (2 * pairs)), PAIR_THREADS, smem, st>>>(mw, ma, P);
-    return (int) cudaGetLastError();
+    return launch_dep(k_dense_pair, dim3((unsigned) (2 * pairs)), dim3(PAIR_THREADS), smem, st, mw, ma, P);
 }
 
 // Which kernel, token tile and cut of K: the one with the least time by a model of what was measured on a B200 (148 SMs, 1.9 GHz, all tiles of

@@ -49,6 +49,7 @@ __global__ void k_embed_bigram(const WT * __restrict__ table, const WT * __restr
 __global__ void k_causal_conv(const float * __restrict__ u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                               const int32_t * __restrict__ entry_of, int channels, int taps, const float * __restrict__ w, int silu_from,
                               float * __restrict__ conv_state, int64_t slot_stride, float * __restrict__ out, int64_t ldo, int advance) {
+    pdl_enter();
     const int t = blockIdx.x;
     const int e = entry_of[t];
     const int lt = t - off[e];
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(1024) k_dual_prep_store(RecPrep rc, float * __
                                                          float * __restrict__ v, int64_t ldv, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                          const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, AttnParams a, AttnPrep pr,
                                                          float * __restrict__ kcache, float * __restrict__ vcache, int64_t slot_stride, int staged) {
+    pdl_enter();
     extern __shared__ float sm[];
     __shared__ float red[33];
     const int t = blockIdx.x;
@@ -254,6 +256,7 @@ template <typename OT>
 __global__ void k_attn_unrotate_gate(const float * __restrict__ o, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
                                      const int32_t * __restrict__ entry_of, int heads, int vdim, int v_layout, const float * __restrict__ v_freq,
                                      const float * __restrict__ gate, int64_t ldg, int gate_mode, float out_scale, OT * __restrict__ out, int64_t ldo) {
+    pdl_enter();
     const int t = blockIdx.x, h = blockIdx.y;
     const int e = entry_of[t];
     const float fp = (float) (pos0[e] + (t - off[e]));
@@ -285,11 +288,13 @@ __global__ void k_attn_unrotate_gate(const float * __restrict__ o, const int32_t
 __global__ void __launch_bounds__(256) k_delta_prep(float * __restrict__ q, int64_t ldq, float * __restrict__ k, int64_t ldk, float * __restrict__ beta,
                                                     int64_t ldb, float * __restrict__ a, int64_t lda, const float * __restrict__ A_log,
                                                     const float * __restrict__ dt_bias, int qk_heads, int heads, int dim) {
+    pdl_enter();
     const int64_t t = blockIdx.x;
     delta_prep_rows(q + t * ldq, k + t * ldk, beta + t * ldb, a ? a + t * lda : nullptr, A_log, dt_bias, qk_heads, heads, dim);
 }
 __global__ void k_hgrn2_prep(float * __restrict__ q, int64_t ldq, float * __restrict__ f, int64_t ldf, const float * __restrict__ f_bias,
                              const float * __restrict__ lower, int n) {
+    pdl_enter();
     const int64_t t = blockIdx.x;
     hgrn2_prep_rows(q + t * ldq, f + t * ldf, f_bias, lower, n);
 }
@@ -303,6 +308,7 @@ __global__ void __launch_bounds__(128) k_dual_post(const float * __restrict__ o,
                                                    const float * __restrict__ gate, int64_t ldg, int gate_mode, float left_scale, const float * __restrict__ y,
                                                    int r_heads, int r_vdim, const float * __restrict__ r_gate, int64_t ldrg, const float * __restrict__ r_w,
                                                    int r_gate_act, float eps, float right_scale, OT * __restrict__ out, int64_t ldo) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x;
     if ((int) blockIdx.y < heads) {
@@ -358,6 +364,7 @@ enum : int { GL_DELTA = 0, GL_TIED = 1, GL_BONUS = 2, GL_DELTA_CH = 3 };
 template <int NREG, int LN, int MODE>
 __global__ void __launch_bounds__(GCOLS * LN) k_gated_linattn_reg(GatedLinIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                                   GatedLinParams p, float * __restrict__ state, int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     constexpr bool DELTA = MODE == GL_DELTA, TIED = MODE == GL_TIED, BONUS = MODE == GL_BONUS, DELTA_CH = MODE == GL_DELTA_CH;
     constexpr bool ROWS3 = BONUS || DELTA_CH;   // the decay per channel is a third staged row
@@ -541,6 +548,7 @@ __global__ void __launch_bounds__(GCOLS * LN) k_gated_linattn_reg(GatedLinIO io,
 constexpr int GSCOLS = 64;
 __global__ void __launch_bounds__(256) k_gated_linattn_smem(GatedLinIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, GatedLinParams p,
                                                             float * __restrict__ state, int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int N = p.dim, P = p.vdim, inner = p.heads * p.vdim;
     const int ptiles = (P + GSCOLS - 1) / GSCOLS;
@@ -616,6 +624,7 @@ template <typename OT>
 __global__ void __launch_bounds__(256) k_rmsnorm_pair_residual(const float * __restrict__ a, int64_t lda, const float * __restrict__ bb, int64_t ldb,
                                                                const float * __restrict__ wa, const float * __restrict__ wb, float mult, float eps,
                                                                float * __restrict__ x, const float * __restrict__ wn, OT * __restrict__ y, int width) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const float * ar = a + (int64_t) t * lda, * br = bb + (int64_t) t * ldb;
@@ -638,6 +647,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_pair_residual(const float * __r
 template <typename OT>
 __global__ void __launch_bounds__(256) k_stream_add_rmsnorm(float * __restrict__ x, const float * __restrict__ x0, const float * __restrict__ vec,
                                                             const float * __restrict__ w, float eps, OT * __restrict__ y, int width) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x;
     float * xr = x + (int64_t) t * width;
@@ -660,8 +670,8 @@ int launch_stream_add_rmsnorm(float * x, const float * x0, const float * vec, co
     if (n_rows <= 0) return 0;
     if (!x || !w || !y) return (int) cudaErrorInvalidValue;
     return ck_launch([&] {
-        if (otype == T_BF16) k_stream_add_rmsnorm<__nv_bfloat16><<<n_rows, 256, 0, st>>>(x, x0, vec, w, eps, (__nv_bfloat16 *) y, width);
-        else k_stream_add_rmsnorm<float><<<n_rows, 256, 0, st>>>(x, x0, vec, w, eps, (float *) y, width);
+        if (otype == T_BF16) launch_dep(k_stream_add_rmsnorm<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, st, x, x0, vec, w, eps, (__nv_bfloat16 *) y, width);
+        else launch_dep(k_stream_add_rmsnorm<float>, dim3(n_rows), dim3(256), 0, st, x, x0, vec, w, eps, (float *) y, width);
     });
 }
 
@@ -684,7 +694,7 @@ int launch_causal_conv(const float * u, int64_t ldu, const BatchView & b, int ch
     const int tiles = b.n_tokens >= 512 ? 1 : std::min((channels + 127) / 128, 32);   // few tokens: a token's channels spread over CTAs
     const int advance = b.max_n == 1 && taps > 1;   // one-token entries: the same kernel moves the state on
     int rc = ck_launch([&] {
-        k_causal_conv<<<dim3((unsigned) b.n_tokens, (unsigned) tiles), 128, 0, st>>>(u, ldu, b.slot, b.off, b.entry_of, channels, taps, w, silu_from, conv_state,
+        launch_dep(k_causal_conv, dim3((unsigned) b.n_tokens, (unsigned) tiles), dim3(128), 0, st, u, ldu, b.slot, b.off, b.entry_of, channels, taps, w, silu_from, conv_state,
                                                                                      slot_stride, out, ldo, advance);
     });
     if (rc || taps == 1 || advance) return rc;
@@ -709,7 +719,7 @@ static int dual_prep_launch(const RecPrep & rc, float * q, int64_t ldq, float * 
     int e = raise_smem(k_dual_prep_store, smem);
     if (e) return e;
     return ck_launch([&] {
-        k_dual_prep_store<<<b.n_tokens, row_threads(b.n_tokens, (int) floats / 2), smem, st>>>(rc, q, ldq, k, ldk, v, ldv, b.slot, b.off, b.pos0, b.entry_of, a, pr, kcache, vcache, slot_stride, staged);
+        launch_dep(k_dual_prep_store, dim3(b.n_tokens), dim3(row_threads(b.n_tokens, (int) floats / 2)), smem, st, rc, q, ldq, k, ldk, v, ldv, b.slot, b.off, b.pos0, b.entry_of, a, pr, kcache, vcache, slot_stride, staged);
     });
 }
 int launch_attn_prep_store(float * q, int64_t ldq, float * k, int64_t ldk, float * v, int64_t ldv, const BatchView & b, const AttnParams & a,
@@ -726,9 +736,9 @@ int launch_attn_unrotate_gate(const float * o, const BatchView & b, int heads, i
     const int threads = vdim / 2 >= 128 ? 128 : vdim / 2 >= 64 ? 64 : 32;
     return ck_launch([&] {
         if (otype == T_BF16)
-            k_attn_unrotate_gate<__nv_bfloat16><<<grid, threads, 0, st>>>(o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, out_scale,
+            launch_dep(k_attn_unrotate_gate<__nv_bfloat16>, dim3(grid), dim3(threads), 0, st, o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, out_scale,
                                                                          (__nv_bfloat16 *) out, ldo);
-        else k_attn_unrotate_gate<float><<<grid, threads, 0, st>>>(o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, out_scale,
+        else launch_dep(k_attn_unrotate_gate<float>, dim3(grid), dim3(threads), 0, st, o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, out_scale,
                                                                    (float *) out, ldo);
     });
 }
@@ -737,12 +747,12 @@ int launch_delta_prep(float * q, int64_t ldq, float * k, int64_t ldk, float * be
                       const float * dt_bias, int qk_heads, int heads, int dim, int n_tokens, cudaStream_t st) {
     if (n_tokens <= 0) return 0;
     if (qk_heads <= 0 || heads <= 0 || dim <= 0 || (a && (!A_log || !dt_bias))) return (int) cudaErrorInvalidValue;
-    return ck_launch([&] { k_delta_prep<<<n_tokens, 256, 0, st>>>(q, ldq, k, ldk, beta, ldb, a, lda, A_log, dt_bias, qk_heads, heads, dim); });
+    return ck_launch([&] { launch_dep(k_delta_prep, dim3(n_tokens), dim3(256), 0, st, q, ldq, k, ldk, beta, ldb, a, lda, A_log, dt_bias, qk_heads, heads, dim); });
 }
 int launch_hgrn2_prep(float * q, int64_t ldq, float * f, int64_t ldf, const float * f_bias, const float * lower, int n, int n_tokens, cudaStream_t st) {
     if (n_tokens <= 0 || n <= 0) return 0;
     if (!f_bias || !lower) return (int) cudaErrorInvalidValue;
-    return ck_launch([&] { k_hgrn2_prep<<<n_tokens, 256, 0, st>>>(q, ldq, f, ldf, f_bias, lower, n); });
+    return ck_launch([&] { launch_dep(k_hgrn2_prep, dim3(n_tokens), dim3(256), 0, st, q, ldq, f, ldf, f_bias, lower, n); });
 }
 
 int launch_gated_linattn(const GatedLinIO & io, const BatchView & b, const GatedLinParams & p, float * state, int64_t slot_stride, float * y, cudaStream_t st) {
@@ -768,15 +778,15 @@ int launch_gated_linattn(const GatedLinIO & io, const BatchView & b, const Gated
         if (p.bonus) {                                                                                                                               \
             const int rc = raise_smem(k_gated_linattn_reg<NR, LNV, GL_BONUS>, smem);                                                                 \
             if (rc) return rc;                                                                                                                       \
-            return ck_launch([&] { k_gated_linattn_reg<NR, LNV, GL_BONUS><<<grid, GCOLS * LNV, smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });            \
+            return ck_launch([&] { launch_dep(k_gated_linattn_reg<NR, LNV, GL_BONUS>, dim3(grid), dim3(GCOLS * LNV), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });            \
         }                                                                                                                                            \
         if (delta_ch) {                                                                                                                              \
             const int rc = raise_smem(k_gated_linattn_reg<NR, LNV, GL_DELTA_CH>, smem);                                                              \
             if (rc) return rc;                                                                                                                       \
-            return ck_launch([&] { k_gated_linattn_reg<NR, LNV, GL_DELTA_CH><<<grid, GCOLS * LNV, smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });         \
+            return ck_launch([&] { launch_dep(k_gated_linattn_reg<NR, LNV, GL_DELTA_CH>, dim3(grid), dim3(GCOLS * LNV), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });         \
         }                                                                                                                                            \
-        if (p.delta) return ck_launch([&] { k_gated_linattn_reg<NR, LNV, GL_DELTA><<<grid, GCOLS * LNV, smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); }); \
-        return ck_launch([&] { k_gated_linattn_reg<NR, LNV, GL_TIED><<<grid, GCOLS * LNV, smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });            \
+        if (p.delta) return ck_launch([&] { launch_dep(k_gated_linattn_reg<NR, LNV, GL_DELTA>, dim3(grid), dim3(GCOLS * LNV), smem, st, io, b.slot, b.off, p, state, slot_stride, y); }); \
+        return ck_launch([&] { launch_dep(k_gated_linattn_reg<NR, LNV, GL_TIED>, dim3(grid), dim3(GCOLS * LNV), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });            \
     } while (0)
 #define PB_GL_LN(LNV)                 \
     do {                              \
@@ -796,7 +806,7 @@ int launch_gated_linattn(const GatedLinIO & io, const BatchView & b, const Gated
     int rc = raise_smem(k_gated_linattn_smem, smem);
     if (rc) return rc;
     const dim3 grid((unsigned) (p.heads * ((p.vdim + GSCOLS - 1) / GSCOLS)), (unsigned) b.n_entries);
-    return ck_launch([&] { k_gated_linattn_smem<<<grid, 256, smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });
+    return ck_launch([&] { launch_dep(k_gated_linattn_smem, dim3(grid), dim3(256), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });
 }
 
 int launch_dual_prep_store(int rec_kind, float * rq, int64_t ldrq, float * rk, int64_t ldrk, float * beta, int64_t ldb, float * ra, int64_t lda, const float * p0,
@@ -822,10 +832,10 @@ int launch_dual_post(const float * o, const BatchView & b, int heads, int vdim, 
     const dim3 grid((unsigned) b.n_tokens, (unsigned) (heads + r_heads));
     return ck_launch([&] {
         if (otype == T_BF16)
-            k_dual_post<__nv_bfloat16><<<grid, 128, 0, st>>>(o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, left_scale, y, r_heads,
+            launch_dep(k_dual_post<__nv_bfloat16>, dim3(grid), dim3(128), 0, st, o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, left_scale, y, r_heads,
                                                             r_vdim, r_gate, ldrg, r_w, r_gate_act, eps, right_scale, (__nv_bfloat16 *) out, ldo);
         else
-            k_dual_post<float><<<grid, 128, 0, st>>>(o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, left_scale, y, r_heads, r_vdim,
+            launch_dep(k_dual_post<float>, dim3(grid), dim3(128), 0, st, o, b.off, b.pos0, b.entry_of, heads, vdim, v_layout, v_freq, gate, ldg, gate_mode, left_scale, y, r_heads, r_vdim,
                                                     r_gate, ldrg, r_w, r_gate_act, eps, right_scale, (float *) out, ldo);
     });
 }
@@ -836,8 +846,8 @@ int launch_rmsnorm_pair_residual(const float * a, int64_t lda, const float * bb,
     if (!a || !bb || !wa || !wb || !x || (y && !wn)) return (int) cudaErrorInvalidValue;
     return ck_launch([&] {
         if (otype == T_BF16)
-            k_rmsnorm_pair_residual<__nv_bfloat16><<<n_rows, 256, 0, st>>>(a, lda, bb, ldb, wa, wb, mult, eps, x, wn, (__nv_bfloat16 *) y, width);
-        else k_rmsnorm_pair_residual<float><<<n_rows, 256, 0, st>>>(a, lda, bb, ldb, wa, wb, mult, eps, x, wn, (float *) y, width);
+            launch_dep(k_rmsnorm_pair_residual<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, st, a, lda, bb, ldb, wa, wb, mult, eps, x, wn, (__nv_bfloat16 *) y, width);
+        else launch_dep(k_rmsnorm_pair_residual<float>, dim3(n_rows), dim3(256), 0, st, a, lda, bb, ldb, wa, wb, mult, eps, x, wn, (float *) y, width);
     });
 }
 

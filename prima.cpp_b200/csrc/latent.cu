@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(1024) k_latent_prep(float * __restrict__ proj,
                                                      const float * __restrict__ wq, const float * __restrict__ wkv, const float * __restrict__ freq, float eps,
                                                      OT * __restrict__ cq, float * __restrict__ cache, int64_t slot_stride, OT * __restrict__ lat,
                                                      float * __restrict__ kr, int turn_q) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const int e = entry_of[t];
@@ -123,6 +124,7 @@ template <typename WT>
 __global__ void __launch_bounds__(512) k_latent_absorb_q(const float * __restrict__ q, int64_t ldq, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
                                                          const int32_t * __restrict__ entry_of, const WT * __restrict__ wuk, LatentParams p,
                                                          const float * __restrict__ freq, float * __restrict__ qa) {
+    pdl_enter();
     extern __shared__ float qs[];   // [dim]
     __shared__ float quarter[4][128];
     const int h = blockIdx.x, t = blockIdx.y;
@@ -170,6 +172,7 @@ __global__ void __launch_bounds__(512) k_latent_absorb_q(const float * __restric
 template <typename WT, typename OT>
 __global__ void __launch_bounds__(256) k_latent_up_v(const float * __restrict__ olat, const WT * __restrict__ wuv, LatentParams p,
                                                      const float * __restrict__ gate, int64_t ldg, OT * __restrict__ out) {
+    pdl_enter();
     extern __shared__ float os[];   // [kv_rank]
     const int h = blockIdx.x, t = blockIdx.y;
     const int R = p.kv_rank, DV = p.vdim;
@@ -202,6 +205,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(256) k_latent_decode_split(const float * __restrict__ qa, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                              const int32_t * __restrict__ pos0, LatentParams p, const float * __restrict__ cache,
                                                              int64_t slot_stride, int splits, float * __restrict__ part) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int s = blockIdx.x, e = blockIdx.y, h0 = blockIdx.z * LT_HEADS;
     const int H = p.heads, R = p.kv_rank, RW = R + p.rot_dim, RWP = latent_row_stride(p);
@@ -339,6 +343,7 @@ __global__ void __launch_bounds__(256) k_latent_merge_up_v(const float * __restr
                                                            const int32_t * __restrict__ pos0, const WT * __restrict__ wuv,
                                                            LatentParams p, const float * __restrict__ sink, const float * __restrict__ gate, int64_t ldg,
                                                            OT * __restrict__ out) {
+    pdl_enter();
     extern __shared__ float os[];   // [kv_rank], then [64] weights of the splits
     const int h = blockIdx.x, e = blockIdx.y, t = off[e];
     const int R = p.kv_rank, DV = p.vdim, H = p.heads;
@@ -394,10 +399,10 @@ int launch_latent_prep(float * proj, const BatchView & b, const LatentParams & p
     const int threads = row_threads(b.n_tokens, std::max(p.q_rank, p.kv_rank));
     return ck_launch([&] {
         if (otype == T_BF16)
-            k_latent_prep<__nv_bfloat16><<<b.n_tokens, threads, 0, st>>>(proj, b.slot, b.off, b.pos0, b.entry_of, p, wq, wkv, freq, eps, (__nv_bfloat16 *) cq, cache,
+            launch_dep(k_latent_prep<__nv_bfloat16>, dim3(b.n_tokens), dim3(threads), 0, st, proj, b.slot, b.off, b.pos0, b.entry_of, p, wq, wkv, freq, eps, (__nv_bfloat16 *) cq, cache,
                                                                      slot_stride, (__nv_bfloat16 *) lat, kr, turn_q);
         else
-            k_latent_prep<float><<<b.n_tokens, threads, 0, st>>>(proj, b.slot, b.off, b.pos0, b.entry_of, p, wq, wkv, freq, eps, (float *) cq, cache, slot_stride,
+            launch_dep(k_latent_prep<float>, dim3(b.n_tokens), dim3(threads), 0, st, proj, b.slot, b.off, b.pos0, b.entry_of, p, wq, wkv, freq, eps, (float *) cq, cache, slot_stride,
                                                              (float *) lat, kr, turn_q);
     });
 }
@@ -423,8 +428,8 @@ int launch_latent_absorb_q(const float * q, int64_t ldq, const BatchView & b, co
     const dim3 grid((unsigned) p.heads, (unsigned) n_tokens, (unsigned) ((p.kv_rank + 127) / 128));
     const size_t smem = (size_t) p.dim * sizeof(float);
     return ck_launch([&] {
-        if (wtype == T_BF16) k_latent_absorb_q<__nv_bfloat16><<<grid, 512, smem, st>>>(q, ldq, b.off, b.pos0, b.entry_of, (const __nv_bfloat16 *) wuk, p, freq, qa);
-        else k_latent_absorb_q<float><<<grid, 512, smem, st>>>(q, ldq, b.off, b.pos0, b.entry_of, (const float *) wuk, p, freq, qa);
+        if (wtype == T_BF16) launch_dep(k_latent_absorb_q<__nv_bfloat16>, dim3(grid), dim3(512), smem, st, q, ldq, b.off, b.pos0, b.entry_of, (const __nv_bfloat16 *) wuk, p, freq, qa);
+        else launch_dep(k_latent_absorb_q<float>, dim3(grid), dim3(512), smem, st, q, ldq, b.off, b.pos0, b.entry_of, (const float *) wuk, p, freq, qa);
     });
 }
 int launch_latent_up_v(const float * olat, const void * wuv, int wtype, const LatentParams & p, const float * gate, int64_t ldg, void * out, int otype,
@@ -435,11 +440,11 @@ int launch_latent_up_v(const float * olat, const void * wuv, int wtype, const La
     const size_t smem = (size_t) p.kv_rank * sizeof(float);
     return ck_launch([&] {
         if (wtype == T_BF16) {
-            if (otype == T_BF16) k_latent_up_v<__nv_bfloat16, __nv_bfloat16><<<grid, 256, smem, st>>>(olat, (const __nv_bfloat16 *) wuv, p, gate, ldg, (__nv_bfloat16 *) out);
-            else k_latent_up_v<__nv_bfloat16, float><<<grid, 256, smem, st>>>(olat, (const __nv_bfloat16 *) wuv, p, gate, ldg, (float *) out);
+            if (otype == T_BF16) launch_dep(k_latent_up_v<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(256), smem, st, olat, (const __nv_bfloat16 *) wuv, p, gate, ldg, (__nv_bfloat16 *) out);
+            else launch_dep(k_latent_up_v<__nv_bfloat16, float>, dim3(grid), dim3(256), smem, st, olat, (const __nv_bfloat16 *) wuv, p, gate, ldg, (float *) out);
         } else {
-            if (otype == T_BF16) k_latent_up_v<float, __nv_bfloat16><<<grid, 256, smem, st>>>(olat, (const float *) wuv, p, gate, ldg, (__nv_bfloat16 *) out);
-            else k_latent_up_v<float, float><<<grid, 256, smem, st>>>(olat, (const float *) wuv, p, gate, ldg, (float *) out);
+            if (otype == T_BF16) launch_dep(k_latent_up_v<float, __nv_bfloat16>, dim3(grid), dim3(256), smem, st, olat, (const float *) wuv, p, gate, ldg, (__nv_bfloat16 *) out);
+            else launch_dep(k_latent_up_v<float, float>, dim3(grid), dim3(256), smem, st, olat, (const float *) wuv, p, gate, ldg, (float *) out);
         }
     });
 }
@@ -455,8 +460,8 @@ int launch_latent_decode(const float * qa, const BatchView & b, const LatentPara
     if (rc) return rc;
     const dim3 grid((unsigned) splits, (unsigned) b.n_entries, (unsigned) ((p.heads + LT_HEADS - 1) / LT_HEADS));
     rc = ck_launch([&] {
-        if (vec) k_latent_decode_split<true><<<grid, 256, smem, st>>>(qa, b.slot, b.off, b.pos0, p, cache, slot_stride, splits, part);
-        else k_latent_decode_split<false><<<grid, 256, smem, st>>>(qa, b.slot, b.off, b.pos0, p, cache, slot_stride, splits, part);
+        if (vec) launch_dep(k_latent_decode_split<true>, dim3(grid), dim3(256), smem, st, qa, b.slot, b.off, b.pos0, p, cache, slot_stride, splits, part);
+        else launch_dep(k_latent_decode_split<false>, dim3(grid), dim3(256), smem, st, qa, b.slot, b.off, b.pos0, p, cache, slot_stride, splits, part);
     });
     if (rc) return rc;
     // shares: enough CTAs for the machine when heads and entries are few (an output row is the same sum under any number of them)
@@ -465,11 +470,11 @@ int launch_latent_decode(const float * qa, const BatchView & b, const LatentPara
     const size_t smem2 = ((size_t) p.kv_rank + 64) * sizeof(float);
     return ck_launch([&] {
         if (wtype == T_BF16) {
-            if (otype == T_BF16) k_latent_merge_up_v<__nv_bfloat16, __nv_bfloat16><<<grid2, 256, smem2, st>>>(part, splits, b.off, b.pos0, (const __nv_bfloat16 *) wuv, p, sink, gate, ldg, (__nv_bfloat16 *) out);
-            else k_latent_merge_up_v<__nv_bfloat16, float><<<grid2, 256, smem2, st>>>(part, splits, b.off, b.pos0, (const __nv_bfloat16 *) wuv, p, sink, gate, ldg, (float *) out);
+            if (otype == T_BF16) launch_dep(k_latent_merge_up_v<__nv_bfloat16, __nv_bfloat16>, dim3(grid2), dim3(256), smem2, st, part, splits, b.off, b.pos0, (const __nv_bfloat16 *) wuv, p, sink, gate, ldg, (__nv_bfloat16 *) out);
+            else launch_dep(k_latent_merge_up_v<__nv_bfloat16, float>, dim3(grid2), dim3(256), smem2, st, part, splits, b.off, b.pos0, (const __nv_bfloat16 *) wuv, p, sink, gate, ldg, (float *) out);
         } else {
-            if (otype == T_BF16) k_latent_merge_up_v<float, __nv_bfloat16><<<grid2, 256, smem2, st>>>(part, splits, b.off, b.pos0, (const float *) wuv, p, sink, gate, ldg, (__nv_bfloat16 *) out);
-            else k_latent_merge_up_v<float, float><<<grid2, 256, smem2, st>>>(part, splits, b.off, b.pos0, (const float *) wuv, p, sink, gate, ldg, (float *) out);
+            if (otype == T_BF16) launch_dep(k_latent_merge_up_v<float, __nv_bfloat16>, dim3(grid2), dim3(256), smem2, st, part, splits, b.off, b.pos0, (const float *) wuv, p, sink, gate, ldg, (__nv_bfloat16 *) out);
+            else launch_dep(k_latent_merge_up_v<float, float>, dim3(grid2), dim3(256), smem2, st, part, splits, b.off, b.pos0, (const float *) wuv, p, sink, gate, ldg, (float *) out);
         }
     });
 }

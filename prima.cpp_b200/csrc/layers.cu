@@ -42,6 +42,7 @@
 #include "arch.h"
 #include "json.h"
 #include "layers.h"
+#include "pdl.h"
 #include "model.h"
 
 extern std::atomic<uint64_t> g_launches;
@@ -2289,6 +2290,7 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
         mp.ldd = mp.ldg = ldrg = (int64_t) rp.heads * rp.dim + RV;
         mp.decay = ll.big3; mp.gate = ll.big3 + (int64_t) rp.heads * rp.dim;
         r_gate = mp.gate;
+        const PdlScope plain(g_pdl && !forked);   // a kernel behind an event of another stream has two dependencies
         CK(launch_lowrank_maps(mp, T, rst));
     }
     CAT(CAT_SCAN);
@@ -2303,9 +2305,13 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     } else {
         gi.decay = rk; gi.ldd = ldr;
     }
-    CK(launch_gated_linattn(gi, b, rp, rec_state, ll.slot_floats, ll.yssm, rst));
+    {
+        const PdlScope plain(g_pdl && !forked);
+        CK(launch_gated_linattn(gi, b, rp, rec_state, ll.slot_floats, ll.yssm, rst));
+    }
     if (!sum) {   // every head by its own root mean square with the weight all heads share -> operand of the branch's own output product
         CAT(CAT_NORM);
+        const PdlScope plain(g_pdl && !forked);
         CK(launch_norm_gate(ll.yssm, r_gate, ldrg, rp.heads, L.onorm.data, r_gate ? d.r_gate_act : -1, ll.eps, ll.act2, ct, T, RV, rst, RV, 1.f));
     }
     if (forked) CK(cudaEventRecord(ll.ev_join, rst));
@@ -2331,6 +2337,7 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     if (forked) CK(cudaStreamWaitEvent(st, ll.ev_join, 0));
     CAT(CAT_NORM);
     if (sum && unfused) {
+        const PdlScope plain(g_pdl && !forked);
         CK(launch_attn_unrotate_gate(ll.big2, b, a.heads, a.vdim, d.rot_layout, d.v_rot ? L.vrot_freq.data : nullptr, ll.big + d.c_g, C, d.gate_mode, d.left_scale,
                                      ll.act, ldo, ct, st));
         CK(launch_norm_gate(ll.yssm, r_gate, ldrg, rp.heads, L.onorm.data, r_gate ? d.r_gate_act : -1, ll.eps,
@@ -2341,14 +2348,20 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     if (sum) {
         // attention heads turned back and gated; recurrence heads by their own root mean square, the weight all heads share, the SiLU gate; both
         // with their branch's factor, side by side as the operand of the one output product
+        {
+        const PdlScope plain(g_pdl && !forked);
         CK(launch_dual_post(ll.big2, b, a.heads, a.vdim, d.rot_layout, d.v_rot ? L.vrot_freq.data : nullptr, ll.big + d.c_g, C, d.gate_mode, d.left_scale, ll.yssm,
                             rp.heads, rp.vdim, r_gate, ldrg, L.onorm.data, r_gate ? d.r_gate_act : -1, ll.eps, d.right_scale,
                             ll.act, ldo, ct, st));
+        }
         CAT(CAT_DENSE);
         return launch_dense(ct, ll.act, ldo, L.out.data, ldo, x, W, T, W, (int) ldo, nullptr, x, W, mult, st);
     }
     CAT(CAT_DENSE);
+    {
+    const PdlScope plain(g_pdl && !forked);
     CK(launch_dense(ct, ll.act, OD, L.out.data, OD, ll.big4, 2 * W, T, W, OD, nullptr, nullptr, 0, 1.f, st));
+    }
     CK(launch_dense(ct, ll.act2, RV, L.out_r.data, RV, ll.big4 + W, 2 * W, T, W, RV, nullptr, nullptr, 0, 1.f, st));
     CAT(CAT_NORM);
     return launch_rmsnorm_pair_residual(ll.big4, 2 * W, ll.big4 + W, 2 * W, L.join_wl.data, L.join_wr.data, mult * d.left_scale, ll.eps, x, next_norm,
@@ -2645,6 +2658,8 @@ static int ll_forward(pb200_model * m, const BatchView & b, bool prefill, const 
     cudaStream_t st = m->stream;
     ll.prof_cat.clear();
     CK(tap_prepare(m, b.n_tokens));
+    static const bool no_pdl = getenv("PB200_NO_PDL") != nullptr;   // A/B
+    const PdlScope pdl(!no_pdl && !ll.prof_on && !ll.tap_on);
     if (ll.frame == FRAME_PRENORM) return ll_forward_prenorm(m, b, prefill, tokens_dev, want_dev, nW, lrow0);
     if (ll.frame == FRAME_POSTNORM) return ll_forward_postnorm(m, b, prefill, tokens_dev, want_dev, nW, lrow0);
     if (ll.frame == FRAME_PRERMS) return ll_forward_prerms(m, b, prefill, tokens_dev, want_dev, nW, lrow0);

@@ -28,6 +28,7 @@ template <int NREG, int LN>
 __global__ void __launch_bounds__(DCOLS * LN) k_decay_attn_reg(DecayIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, DecayAttnParams p,
                                                                const float * __restrict__ decay, float * __restrict__ state, int64_t slot_stride,
                                                                float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     constexpr int NT = DCOLS * LN;                                 // threads
     constexpr int NV = (DCHUNK * DCOLS + NT - 1) / NT;             // staged v elements per thread
@@ -115,6 +116,7 @@ constexpr int SCOLS = 64;
 __global__ void __launch_bounds__(256) k_decay_attn_smem(DecayIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, DecayAttnParams p,
                                                          const float * __restrict__ decay, float * __restrict__ state, int64_t slot_stride,
                                                          float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int N = p.dim, P = p.vdim, inner = p.heads * p.vdim;
     const int ptiles = (P + SCOLS - 1) / SCOLS;
@@ -174,7 +176,7 @@ int launch_decay_attn(const float * qkv, int64_t ld, int q_off, int k_off, int v
         const int nreg = (p.dim + ln - 1) / ln;
         const size_t smem = ((size_t) 2 * DCHUNK * p.dim + DCHUNK * DCOLS) * sizeof(float);
         const dim3 grid((unsigned) (p.heads * ((p.vdim + DCOLS - 1) / DCOLS)), (unsigned) b.n_entries);
-#define PB_DECAY(NR, LNV) return ck_launch([&] { k_decay_attn_reg<NR, LNV><<<grid, DCOLS * LNV, smem, st>>>(io, b.slot, b.off, p, decay, state, slot_stride, y); })
+#define PB_DECAY(NR, LNV) return ck_launch([&] { launch_dep(k_decay_attn_reg<NR, LNV>, dim3(grid), dim3(DCOLS * LNV), smem, st, io, b.slot, b.off, p, decay, state, slot_stride, y); })
 #define PB_DECAY_LN(LNV)           \
     do {                           \
         if (nreg <= 1) PB_DECAY(1, LNV); \
@@ -193,7 +195,7 @@ int launch_decay_attn(const float * qkv, int64_t ld, int q_off, int k_off, int v
     int rc = raise_smem(k_decay_attn_smem, smem);
     if (rc) return rc;
     const dim3 grid((unsigned) (p.heads * ((p.vdim + SCOLS - 1) / SCOLS)), (unsigned) b.n_entries);
-    return ck_launch([&] { k_decay_attn_smem<<<grid, 256, smem, st>>>(io, b.slot, b.off, p, decay, state, slot_stride, y); });
+    return ck_launch([&] { launch_dep(k_decay_attn_smem, dim3(grid), dim3(256), smem, st, io, b.slot, b.off, p, decay, state, slot_stride, y); });
 }
 
 }  // namespace pb

@@ -13,6 +13,7 @@
 #include "mixers.cuh"
 
 namespace pb {
+thread_local bool g_pdl = false;
 namespace {
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(1024) k_embed_rmsnorm(const WT * __restrict__ 
 
 template <typename OT>
 __global__ void k_cast(const float * __restrict__ x, OT * __restrict__ y, int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) put(y, i, x[i]);
 }
@@ -64,6 +66,7 @@ __global__ void k_cast(const float * __restrict__ x, OT * __restrict__ y, int64_
 template <typename OT, bool RESID>
 __global__ void __launch_bounds__(256) k_layernorm(const float * __restrict__ x, const int32_t * __restrict__ rows, const float * __restrict__ w,
                                                    const float * __restrict__ bias, float eps, OT * __restrict__ y, float * __restrict__ xres, int width) {
+    pdl_enter();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const float * in = x + (int64_t) (rows ? rows[r] : r) * width;
@@ -86,6 +89,7 @@ __global__ void __launch_bounds__(256) k_layernorm(const float * __restrict__ x,
 template <typename OT>
 __global__ void __launch_bounds__(256) k_layernorm_residual_next(const float * __restrict__ m, const float * __restrict__ wa, const float * __restrict__ wb,
                                                                  float eps, float * __restrict__ x, OT * __restrict__ y, int width) {
+    pdl_enter();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const float * in = m + (int64_t) r * width;
@@ -114,6 +118,7 @@ __global__ void __launch_bounds__(256) k_layernorm_residual_next(const float * _
 template <typename OT>
 __global__ void __launch_bounds__(256) k_layernorm_affine_residual(const float * __restrict__ m, const float * __restrict__ w, const float * __restrict__ bias,
                                                                    float mult, float eps, float * __restrict__ x, OT * __restrict__ xa, int width) {
+    pdl_enter();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const float * in = m + (int64_t) r * width;
@@ -133,6 +138,7 @@ __global__ void __launch_bounds__(256) k_layernorm_affine_residual(const float *
 
 template <typename OT>
 __global__ void k_relu2(const float * __restrict__ u, OT * __restrict__ y, int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = fmaxf(u[i], 0.f);
@@ -140,11 +146,13 @@ __global__ void k_relu2(const float * __restrict__ u, OT * __restrict__ y, int64
 }
 template <typename OT>
 __global__ void k_xielu(const float * __restrict__ u, const float * __restrict__ pq, OT * __restrict__ y, int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     put(y, i, xielu_f(u[i], softplus_f(pq[0]), 0.5f + softplus_f(pq[1])));
 }
 __global__ void k_softcap(float * __restrict__ x, int64_t n, float cap) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = cap * tanhf(x[i] / cap);
 }
@@ -168,6 +176,7 @@ __global__ void k_embed_pos(const WT * __restrict__ table, const WT * __restrict
 
 template <typename OT>
 __global__ void k_gelu_mul(const float * __restrict__ gu, OT * __restrict__ y, int n_tokens, int ff) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t) n_tokens * ff) return;
     const int64_t t = i / ff, j = i - t * ff;
@@ -244,6 +253,7 @@ __device__ __forceinline__ float attn_gate(const AttnIO & io, int64_t row, int h
 __global__ void k_attn_kv_store(const float * __restrict__ qkvg, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                 const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, AttnParams a, float * __restrict__ kcache,
                                 float * __restrict__ vcache, int64_t slot_stride) {
+    pdl_enter();
     const int t = blockIdx.x;
     const int e = entry_of[t];
     const int n = off[e + 1] - off[e];
@@ -266,6 +276,7 @@ __global__ void __launch_bounds__(256) k_attn_qknorm_kv_store(float * __restrict
                                                               const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, AttnParams a,
                                                               const float * __restrict__ wq, const float * __restrict__ wk, float eps,
                                                               float * __restrict__ kcache, float * __restrict__ vcache, int64_t slot_stride) {
+    pdl_enter();
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int KD = a.kv_heads * a.dim, VD = a.kv_heads * a.vdim, C = attn_qkvg_cols(a);
@@ -553,6 +564,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) k_attn_window_decode(const Att
                                                                        const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, AttnParams a,
                                                                        const float * __restrict__ kcache, const float * __restrict__ vcache,
                                                                        int64_t slot_stride, OT * __restrict__ out, float * __restrict__ part, int chunk) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int e = blockIdx.y, h = blockIdx.x;
     const int t = off[e];
@@ -686,6 +698,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) k_attn_window_decode(const Att
 template <typename OT>
 __global__ void __launch_bounds__(128) k_attn_decode_merge(const AttnIO io, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, AttnParams a,
                                                            const float * __restrict__ part, int all_splits, int chunk, OT * __restrict__ out) {
+    pdl_enter();
     __shared__ float w[64];
     const int e = blockIdx.y, h = blockIdx.x, DV = a.vdim;
     const int t = off[e];
@@ -726,6 +739,7 @@ __global__ void __launch_bounds__(128) k_attn_decode_merge(const AttnIO io, cons
 __global__ void k_mamba2_conv(const float * __restrict__ u, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                               const int32_t * __restrict__ entry_of, Mamba2Params p, const float * __restrict__ w, const float * __restrict__ bias,
                               const float * __restrict__ conv_state, int64_t slot_stride, float * __restrict__ xbc) {
+    pdl_enter();
     const int t = blockIdx.x;
     const int e = entry_of[t];
     const int lt = t - off[e];
@@ -760,6 +774,7 @@ __global__ void __launch_bounds__(256) k_mamba2_scan(const float * __restrict__ 
                                                      const int32_t * __restrict__ off, Mamba2Params p, const float * __restrict__ dt_bias,
                                                      const float * __restrict__ A_log, const float * __restrict__ Dp, float * __restrict__ ssm_state,
                                                      int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int h = blockIdx.x, e = blockIdx.y;
     const int N = p.state, P = p.vdim, inner = mamba2_inner(p), CH = mamba2_conv_channels(p), U = mamba2_in_cols(p);
@@ -810,6 +825,7 @@ __global__ void __launch_bounds__(128) k_mamba2_scan_reg(const float * __restric
                                                          const int32_t * __restrict__ off, Mamba2Params p, const float * __restrict__ dt_bias,
                                                          const float * __restrict__ A_log, const float * __restrict__ Dp, float * __restrict__ ssm_state,
                                                          int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int N = p.state, P = p.vdim, inner = mamba2_inner(p), CH = mamba2_conv_channels(p), U = mamba2_in_cols(p);
     const int ptiles = (P + SCAN_COLS - 1) / SCAN_COLS;
@@ -889,6 +905,7 @@ __global__ void __launch_bounds__(128) k_mamba2_scan_reg(const float * __restric
 template <typename OT>
 __global__ void __launch_bounds__(256) k_mamba2_gate_norm(const float * __restrict__ y, const float * __restrict__ u, Mamba2Params p, const float * __restrict__ w,
                                                           float eps, OT * __restrict__ out) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x, grp = blockIdx.y;
     const int inner = mamba2_inner(p), U = mamba2_in_cols(p), part = inner / p.norm_groups;
@@ -923,39 +940,39 @@ int launch_cast(const float * x, void * y, int otype, int64_t n, cudaStream_t st
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_cast<__nv_bfloat16><<<grid, 256, 0, st>>>(x, (__nv_bfloat16 *) y, n);
-        else k_cast<float><<<grid, 256, 0, st>>>(x, (float *) y, n);
+        if (otype == T_BF16) launch_dep(k_cast<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, x, (__nv_bfloat16 *) y, n);
+        else launch_dep(k_cast<float>, dim3(grid), dim3(256), 0, st, x, (float *) y, n);
     });
 }
 int launch_layernorm(const float * x, const int32_t * rows, const float * w, float eps, void * y, int otype, int n_rows, int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
     return ck_launch([&] {
-        if (otype == T_BF16) k_layernorm<__nv_bfloat16, false><<<n_rows, 256, 0, st>>>(x, rows, w, nullptr, eps, (__nv_bfloat16 *) y, nullptr, width);
-        else k_layernorm<float, false><<<n_rows, 256, 0, st>>>(x, rows, w, nullptr, eps, (float *) y, nullptr, width);
+        if (otype == T_BF16) launch_dep(k_layernorm<__nv_bfloat16, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, nullptr, eps, (__nv_bfloat16 *) y, nullptr, width);
+        else launch_dep(k_layernorm<float, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, nullptr, eps, (float *) y, nullptr, width);
     });
 }
 int launch_layernorm_affine(const float * x, const int32_t * rows, const float * w, const float * bias, float eps, void * y, int otype, int n_rows, int width,
                             cudaStream_t st) {
     if (n_rows <= 0) return 0;
     return ck_launch([&] {
-        if (otype == T_BF16) k_layernorm<__nv_bfloat16, false><<<n_rows, 256, 0, st>>>(x, rows, w, bias, eps, (__nv_bfloat16 *) y, nullptr, width);
-        else k_layernorm<float, false><<<n_rows, 256, 0, st>>>(x, rows, w, bias, eps, (float *) y, nullptr, width);
+        if (otype == T_BF16) launch_dep(k_layernorm<__nv_bfloat16, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, bias, eps, (__nv_bfloat16 *) y, nullptr, width);
+        else launch_dep(k_layernorm<float, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, bias, eps, (float *) y, nullptr, width);
     });
 }
 int launch_layernorm_affine_residual(const float * m, const float * w, const float * bias, float mult, float eps, float * x, void * xa, int otype, int n_rows,
                                      int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
     return ck_launch([&] {
-        if (otype == T_BF16) k_layernorm_affine_residual<__nv_bfloat16><<<n_rows, 256, 0, st>>>(m, w, bias, mult, eps, x, (__nv_bfloat16 *) xa, width);
-        else k_layernorm_affine_residual<float><<<n_rows, 256, 0, st>>>(m, w, bias, mult, eps, x, (float *) xa, width);
+        if (otype == T_BF16) launch_dep(k_layernorm_affine_residual<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, st, m, w, bias, mult, eps, x, (__nv_bfloat16 *) xa, width);
+        else launch_dep(k_layernorm_affine_residual<float>, dim3(n_rows), dim3(256), 0, st, m, w, bias, mult, eps, x, (float *) xa, width);
     });
 }
 int launch_relu2(const float * u, void * y, int otype, int64_t n, cudaStream_t st) {
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_relu2<__nv_bfloat16><<<grid, 256, 0, st>>>(u, (__nv_bfloat16 *) y, n);
-        else k_relu2<float><<<grid, 256, 0, st>>>(u, (float *) y, n);
+        if (otype == T_BF16) launch_dep(k_relu2<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, u, (__nv_bfloat16 *) y, n);
+        else launch_dep(k_relu2<float>, dim3(grid), dim3(256), 0, st, u, (float *) y, n);
     });
 }
 int launch_xielu(const float * u, const float * pq, void * y, int otype, int64_t n, cudaStream_t st) {
@@ -963,13 +980,13 @@ int launch_xielu(const float * u, const float * pq, void * y, int otype, int64_t
     if (!pq) return (int) cudaErrorInvalidValue;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_xielu<__nv_bfloat16><<<grid, 256, 0, st>>>(u, pq, (__nv_bfloat16 *) y, n);
-        else k_xielu<float><<<grid, 256, 0, st>>>(u, pq, (float *) y, n);
+        if (otype == T_BF16) launch_dep(k_xielu<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, u, pq, (__nv_bfloat16 *) y, n);
+        else launch_dep(k_xielu<float>, dim3(grid), dim3(256), 0, st, u, pq, (float *) y, n);
     });
 }
 int launch_softcap(float * x, int64_t n, float cap, cudaStream_t st) {
     if (n <= 0 || !(cap > 0.f)) return 0;
-    return ck_launch([&] { k_softcap<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(x, n, cap); });
+    return ck_launch([&] { launch_dep(k_softcap, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, x, n, cap); });
 }
 int launch_embed_pos(const void * table, const void * pos_table, int type, int width, const int32_t * tokens, const BatchView & b, float * x, void * xa,
                      int otype, cudaStream_t st) {
@@ -986,14 +1003,14 @@ int launch_embed_pos(const void * table, const void * pos_table, int type, int w
 }
 int launch_layernorm_residual(const float * m, const float * w, float eps, float * x, int n_rows, int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
-    return ck_launch([&] { k_layernorm<float, true><<<n_rows, 256, 0, st>>>(m, nullptr, w, nullptr, eps, nullptr, x, width); });
+    return ck_launch([&] { launch_dep(k_layernorm<float, true>, dim3(n_rows), dim3(256), 0, st, m, nullptr, w, nullptr, eps, nullptr, x, width); });
 }
 int launch_layernorm_residual_next(const float * m, const float * wa, const float * wb, float eps, float * x, void * y, int otype, int n_rows, int width,
                                    cudaStream_t st) {
     if (n_rows <= 0) return 0;
     return ck_launch([&] {
-        if (otype == T_BF16) k_layernorm_residual_next<__nv_bfloat16><<<n_rows, 256, 0, st>>>(m, wa, wb, eps, x, (__nv_bfloat16 *) y, width);
-        else k_layernorm_residual_next<float><<<n_rows, 256, 0, st>>>(m, wa, wb, eps, x, (float *) y, width);
+        if (otype == T_BF16) launch_dep(k_layernorm_residual_next<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, st, m, wa, wb, eps, x, (__nv_bfloat16 *) y, width);
+        else launch_dep(k_layernorm_residual_next<float>, dim3(n_rows), dim3(256), 0, st, m, wa, wb, eps, x, (float *) y, width);
     });
 }
 int launch_gelu_mul(const float * gu, void * y, int otype, int n_tokens, int ff, cudaStream_t st) {
@@ -1001,8 +1018,8 @@ int launch_gelu_mul(const float * gu, void * y, int otype, int n_tokens, int ff,
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_gelu_mul<__nv_bfloat16><<<grid, 256, 0, st>>>(gu, (__nv_bfloat16 *) y, n_tokens, ff);
-        else k_gelu_mul<float><<<grid, 256, 0, st>>>(gu, (float *) y, n_tokens, ff);
+        if (otype == T_BF16) launch_dep(k_gelu_mul<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, gu, (__nv_bfloat16 *) y, n_tokens, ff);
+        else launch_dep(k_gelu_mul<float>, dim3(grid), dim3(256), 0, st, gu, (float *) y, n_tokens, ff);
     });
 }
 int launch_argmax_rows(const float * logits, int n, int n_rows, int32_t * out, cudaStream_t st) {
@@ -1012,7 +1029,7 @@ int launch_argmax_rows(const float * logits, int n, int n_rows, int32_t * out, c
 
 int launch_attn_kv_store(const float * qkvg, const BatchView & b, const AttnParams & a, float * kcache, float * vcache, int64_t slot_stride, cudaStream_t st) {
     if (b.n_tokens <= 0) return 0;
-    return ck_launch([&] { k_attn_kv_store<<<b.n_tokens, 128, 0, st>>>(qkvg, b.slot, b.off, b.pos0, b.entry_of, a, kcache, vcache, slot_stride); });
+    return ck_launch([&] { launch_dep(k_attn_kv_store, dim3(b.n_tokens), dim3(128), 0, st, qkvg, b.slot, b.off, b.pos0, b.entry_of, a, kcache, vcache, slot_stride); });
 }
 
 int launch_attn_qknorm_kv_store(float * qkvg, const BatchView & b, const AttnParams & a, const float * wq, const float * wk, float eps, float * kcache,
@@ -1020,7 +1037,7 @@ int launch_attn_qknorm_kv_store(float * qkvg, const BatchView & b, const AttnPar
     if (b.n_tokens <= 0) return 0;
     if (!wq || !wk) return (int) cudaErrorInvalidValue;
     return ck_launch([&] {
-        k_attn_qknorm_kv_store<<<b.n_tokens, 256, 0, st>>>(qkvg, b.slot, b.off, b.pos0, b.entry_of, a, wq, wk, eps, kcache, vcache, slot_stride);
+        launch_dep(k_attn_qknorm_kv_store, dim3(b.n_tokens), dim3(256), 0, st, qkvg, b.slot, b.off, b.pos0, b.entry_of, a, wq, wk, eps, kcache, vcache, slot_stride);
     });
 }
 
@@ -1088,11 +1105,11 @@ static int attn_decode_typed(const AttnIO & io, const BatchView & b, const AttnP
     if (rc) return rc;
     const dim3 grid((unsigned) a.heads, (unsigned) b.n_entries, (unsigned) splits);
     rc = ck_launch([&] {
-        k_attn_window_decode<OT, NV, TIED><<<grid, nw * 32, smem, st>>>(io, b.slot, b.off, b.pos0, a, kc, vc, stride, out, part, attn_decode_chunk(a.cache_rows));
+        launch_dep(k_attn_window_decode<OT, NV, TIED>, dim3(grid), dim3(nw * 32), smem, st, io, b.slot, b.off, b.pos0, a, kc, vc, stride, out, part, attn_decode_chunk(a.cache_rows));
     });
     if (rc || splits == 1) return rc;
     const dim3 mgrid((unsigned) a.heads, (unsigned) b.n_entries);
-    return ck_launch([&] { k_attn_decode_merge<OT><<<mgrid, 128, 0, st>>>(io, b.off, b.pos0, a, part, splits, attn_decode_chunk(a.cache_rows), out); });
+    return ck_launch([&] { launch_dep(k_attn_decode_merge<OT>, dim3(mgrid), dim3(128), 0, st, io, b.off, b.pos0, a, part, splits, attn_decode_chunk(a.cache_rows), out); });
 }
 int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnParams & a, const float * kcache, const float * vcache, int64_t slot_stride,
                           void * out, int otype, cudaStream_t st, float * part) {
@@ -1134,7 +1151,7 @@ int launch_mamba2_conv(const float * u, const BatchView & b, const Mamba2Params 
     // few tokens (decode): spread the channels of a token over several CTAs
     const int CHn = mamba2_conv_channels(p);
     const dim3 cgrid((unsigned) b.n_tokens, (unsigned) (b.n_tokens >= 64 ? 1 : std::min(16, (CHn + 255) / 256)));
-    int rc = ck_launch([&] { k_mamba2_conv<<<cgrid, 256, 0, st>>>(u, b.slot, b.off, b.entry_of, p, w, bias, conv_state, slot_stride, xbc); });
+    int rc = ck_launch([&] { launch_dep(k_mamba2_conv, dim3(cgrid), dim3(256), 0, st, u, b.slot, b.off, b.entry_of, p, w, bias, conv_state, slot_stride, xbc); });
     if (rc || p.conv < 2) return rc;
     const dim3 grid((unsigned) ((mamba2_conv_channels(p) + 127) / 128), (unsigned) b.n_entries);
     return ck_launch([&] { k_mamba2_conv_state<<<grid, 128, 0, st>>>(u, b.slot, b.off, p, conv_state, slot_stride); });
@@ -1147,7 +1164,7 @@ int launch_mamba2_scan(const float * u, const float * xbc, const BatchView & b, 
         const size_t sm2 = ((size_t) 2 * SCAN_CHUNK * p.state + SCAN_CHUNK * SCAN_COLS + 2 * SCAN_CHUNK) * sizeof(float);
         const dim3 grid2((unsigned) (p.heads * ((p.vdim + SCAN_COLS - 1) / SCAN_COLS)), (unsigned) b.n_entries);
         const int nreg = (p.state + 7) / 8;
-#define PB_SCAN(NR) return ck_launch([&] { k_mamba2_scan_reg<NR><<<grid2, 128, sm2, st>>>(u, xbc, b.slot, b.off, p, dt_bias, A_log, D, ssm_state, slot_stride, y); })
+#define PB_SCAN(NR) return ck_launch([&] { launch_dep(k_mamba2_scan_reg<NR>, dim3(grid2), dim3(128), sm2, st, u, xbc, b.slot, b.off, p, dt_bias, A_log, D, ssm_state, slot_stride, y); })
         if (nreg <= 1) PB_SCAN(1);
         if (nreg <= 2) PB_SCAN(2);
         if (nreg <= 4) PB_SCAN(4);
@@ -1159,7 +1176,7 @@ int launch_mamba2_scan(const float * u, const float * xbc, const BatchView & b, 
     int rc = raise_smem(k_mamba2_scan, smem);
     if (rc) return rc;
     const dim3 grid((unsigned) p.heads, (unsigned) b.n_entries);
-    return ck_launch([&] { k_mamba2_scan<<<grid, 256, smem, st>>>(u, xbc, b.slot, b.off, p, dt_bias, A_log, D, ssm_state, slot_stride, y); });
+    return ck_launch([&] { launch_dep(k_mamba2_scan, dim3(grid), dim3(256), smem, st, u, xbc, b.slot, b.off, p, dt_bias, A_log, D, ssm_state, slot_stride, y); });
 }
 int launch_mamba2_gate_norm(const float * y, const float * u, const Mamba2Params & p, const float * w, float eps, void * out, int otype, int n_tokens,
                             cudaStream_t st) {
@@ -1167,8 +1184,8 @@ int launch_mamba2_gate_norm(const float * y, const float * u, const Mamba2Params
     if (p.norm_groups <= 0 || mamba2_inner(p) % p.norm_groups != 0) return (int) cudaErrorInvalidValue;
     const dim3 grid((unsigned) n_tokens, (unsigned) p.norm_groups);
     return ck_launch([&] {
-        if (otype == T_BF16) k_mamba2_gate_norm<__nv_bfloat16><<<grid, 256, 0, st>>>(y, u, p, w, eps, (__nv_bfloat16 *) out);
-        else k_mamba2_gate_norm<float><<<grid, 256, 0, st>>>(y, u, p, w, eps, (float *) out);
+        if (otype == T_BF16) launch_dep(k_mamba2_gate_norm<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, y, u, p, w, eps, (__nv_bfloat16 *) out);
+        else launch_dep(k_mamba2_gate_norm<float>, dim3(grid), dim3(256), 0, st, y, u, p, w, eps, (float *) out);
     });
 }
 

@@ -7,10 +7,16 @@
 
 #include <atomic>
 
+#include "common.cuh"
+#include "pdl.h"
+
 extern std::atomic<uint64_t> g_launches;
 
 namespace pb {
+
 namespace {
+
+__device__ __forceinline__ void pdl_enter() { pdl_trigger(); pdl_wait(); }
 
 __device__ __forceinline__ void put(float * p, int64_t i, float v) { p[i] = v; }
 __device__ __forceinline__ void put(__nv_bfloat16 * p, int64_t i, float v) { p[i] = __float2bfloat16_rn(v); }

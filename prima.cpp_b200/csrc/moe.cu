@@ -53,6 +53,7 @@ __device__ __forceinline__ float dot_part(const WT * __restrict__ w, const WT * 
 template <typename HT>
 __global__ void __launch_bounds__(256) k_moe_route(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ bias, MoeParams p,
                                                    int width, int32_t * __restrict__ idx, float * __restrict__ wt) {
+    pdl_enter();
     extern __shared__ float sm[];
     float * hs = sm;            // [width]
     float * z = hs + width;     // [experts]
@@ -112,6 +113,7 @@ template <typename HT>
 __global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p,
                                                            int width, const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt,
                                                            float * __restrict__ sg_out) {
+    pdl_enter();
     extern __shared__ float sm[];
     float * hs = sm;                 // [width]
     float * sc = hs + width;         // [experts] sigmoid scores
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restric
 template <typename WT, bool VEC>
 __global__ void __launch_bounds__(256) k_moe_gateup_rows(const WT * __restrict__ h, const WT * __restrict__ gateup, const int32_t * __restrict__ idx, MoeParams p,
                                                          int width, WT * __restrict__ y, const float * __restrict__ in_wt) {
+    pdl_enter();
     const int pair = blockIdx.y, t = pair / p.top;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = blockIdx.x * 8 + warp;
@@ -206,6 +209,7 @@ template <typename WT, bool VEC>
 __global__ void __launch_bounds__(256) k_moe_down_rows(const WT * __restrict__ y, const WT * __restrict__ down, const int32_t * __restrict__ idx,
                                                        const float * __restrict__ wt, MoeParams p, int width, float * __restrict__ x, int base,
                                                        const float * __restrict__ xscale, float out_scale) {
+    pdl_enter();
     const int t = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + warp;
@@ -286,6 +290,7 @@ __global__ void k_moe_combine(const float * __restrict__ ds, const int32_t * __r
 template <typename OT>
 __global__ void k_silu_mul(const float * __restrict__ gu, OT * __restrict__ y, int n_rows, int ff, const float * __restrict__ in_wt, const int32_t * __restrict__ perm,
                            int interleaved) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t) n_rows * ff) return;
     const int64_t r = i / ff, j = i - r * ff;
@@ -310,11 +315,11 @@ int launch_moe_route(const void * h, int htype, const float * wr, const float * 
     if (htype == T_BF16) {
         int rc = raise_smem(k_moe_route<__nv_bfloat16>, smem);
         if (rc) return rc;
-        return ck_launch([&] { k_moe_route<__nv_bfloat16><<<n_tokens, 256, smem, st>>>((const __nv_bfloat16 *) h, wr, bias, p, width, idx, wt); });
+        return ck_launch([&] { launch_dep(k_moe_route<__nv_bfloat16>, dim3(n_tokens), dim3(256), smem, st, (const __nv_bfloat16 *) h, wr, bias, p, width, idx, wt); });
     }
     int rc = raise_smem(k_moe_route<float>, smem);
     if (rc) return rc;
-    return ck_launch([&] { k_moe_route<float><<<n_tokens, 256, smem, st>>>((const float *) h, wr, bias, p, width, idx, wt); });
+    return ck_launch([&] { launch_dep(k_moe_route<float>, dim3(n_tokens), dim3(256), smem, st, (const float *) h, wr, bias, p, width, idx, wt); });
 }
 int launch_moe_route_sigmoid(const void * h, int htype, const float * wr, const float * correction, const MoeParams & p, int width, const float * shared_gate,
                              int32_t * idx, float * wt, float * sg_out, int n_tokens, cudaStream_t st) {
@@ -330,12 +335,12 @@ int launch_moe_route_sigmoid(const void * h, int htype, const float * wr, const 
         int rc = raise_smem(k_moe_route_sigmoid<__nv_bfloat16>, smem);
         if (rc) return rc;
         return ck_launch([&] {
-            k_moe_route_sigmoid<__nv_bfloat16><<<n_tokens, threads, smem, st>>>((const __nv_bfloat16 *) h, wr, correction, p, width, shared_gate, idx, wt, sg_out);
+            launch_dep(k_moe_route_sigmoid<__nv_bfloat16>, dim3(n_tokens), dim3(threads), smem, st, (const __nv_bfloat16 *) h, wr, correction, p, width, shared_gate, idx, wt, sg_out);
         });
     }
     int rc = raise_smem(k_moe_route_sigmoid<float>, smem);
     if (rc) return rc;
-    return ck_launch([&] { k_moe_route_sigmoid<float><<<n_tokens, threads, smem, st>>>((const float *) h, wr, correction, p, width, shared_gate, idx, wt, sg_out); });
+    return ck_launch([&] { launch_dep(k_moe_route_sigmoid<float>, dim3(n_tokens), dim3(threads), smem, st, (const float *) h, wr, correction, p, width, shared_gate, idx, wt, sg_out); });
 }
 int launch_silu_mul(const float * gu, void * y, int otype, int n_rows, int ff, const float * in_wt, const int32_t * perm, cudaStream_t st,
                     int interleaved) {
@@ -343,8 +348,8 @@ int launch_silu_mul(const float * gu, void * y, int otype, int n_rows, int ff, c
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_silu_mul<__nv_bfloat16><<<grid, 256, 0, st>>>(gu, (__nv_bfloat16 *) y, n_rows, ff, in_wt, perm, interleaved);
-        else k_silu_mul<float><<<grid, 256, 0, st>>>(gu, (float *) y, n_rows, ff, in_wt, perm, interleaved);
+        if (otype == T_BF16) launch_dep(k_silu_mul<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, gu, (__nv_bfloat16 *) y, n_rows, ff, in_wt, perm, interleaved);
+        else launch_dep(k_silu_mul<float>, dim3(grid), dim3(256), 0, st, gu, (float *) y, n_rows, ff, in_wt, perm, interleaved);
     });
 }
 int launch_moe_gateup_rows(const void * h, int type, const void * gateup, const int32_t * idx, const MoeParams & p, int width, void * y, int n_tokens,
@@ -355,11 +360,11 @@ int launch_moe_gateup_rows(const void * h, int type, const void * gateup, const 
     return ck_launch([&] {
         if (type == T_BF16) {
             using B = __nv_bfloat16;
-            if (vec_ok<B>(h, gateup, width)) k_moe_gateup_rows<B, true><<<grid, 256, 0, st>>>((const B *) h, (const B *) gateup, idx, p, width, (B *) y, in_wt);
-            else k_moe_gateup_rows<B, false><<<grid, 256, 0, st>>>((const B *) h, (const B *) gateup, idx, p, width, (B *) y, in_wt);
+            if (vec_ok<B>(h, gateup, width)) launch_dep(k_moe_gateup_rows<B, true>, dim3(grid), dim3(256), 0, st, (const B *) h, (const B *) gateup, idx, p, width, (B *) y, in_wt);
+            else launch_dep(k_moe_gateup_rows<B, false>, dim3(grid), dim3(256), 0, st, (const B *) h, (const B *) gateup, idx, p, width, (B *) y, in_wt);
         } else {
-            if (vec_ok<float>(h, gateup, width)) k_moe_gateup_rows<float, true><<<grid, 256, 0, st>>>((const float *) h, (const float *) gateup, idx, p, width, (float *) y, in_wt);
-            else k_moe_gateup_rows<float, false><<<grid, 256, 0, st>>>((const float *) h, (const float *) gateup, idx, p, width, (float *) y, in_wt);
+            if (vec_ok<float>(h, gateup, width)) launch_dep(k_moe_gateup_rows<float, true>, dim3(grid), dim3(256), 0, st, (const float *) h, (const float *) gateup, idx, p, width, (float *) y, in_wt);
+            else launch_dep(k_moe_gateup_rows<float, false>, dim3(grid), dim3(256), 0, st, (const float *) h, (const float *) gateup, idx, p, width, (float *) y, in_wt);
         }
     });
 }
@@ -371,11 +376,11 @@ int launch_moe_down_rows(const void * y, int type, const void * down, const int3
     return ck_launch([&] {
         if (type == T_BF16) {
             using B = __nv_bfloat16;
-            if (vec_ok<B>(y, down, p.ff)) k_moe_down_rows<B, true><<<grid, 256, 0, st>>>((const B *) y, (const B *) down, idx, wt, p, width, x, base, xscale, out_scale);
-            else k_moe_down_rows<B, false><<<grid, 256, 0, st>>>((const B *) y, (const B *) down, idx, wt, p, width, x, base, xscale, out_scale);
+            if (vec_ok<B>(y, down, p.ff)) launch_dep(k_moe_down_rows<B, true>, dim3(grid), dim3(256), 0, st, (const B *) y, (const B *) down, idx, wt, p, width, x, base, xscale, out_scale);
+            else launch_dep(k_moe_down_rows<B, false>, dim3(grid), dim3(256), 0, st, (const B *) y, (const B *) down, idx, wt, p, width, x, base, xscale, out_scale);
         } else {
-            if (vec_ok<float>(y, down, p.ff)) k_moe_down_rows<float, true><<<grid, 256, 0, st>>>((const float *) y, (const float *) down, idx, wt, p, width, x, base, xscale, out_scale);
-            else k_moe_down_rows<float, false><<<grid, 256, 0, st>>>((const float *) y, (const float *) down, idx, wt, p, width, x, base, xscale, out_scale);
+            if (vec_ok<float>(y, down, p.ff)) launch_dep(k_moe_down_rows<float, true>, dim3(grid), dim3(256), 0, st, (const float *) y, (const float *) down, idx, wt, p, width, x, base, xscale, out_scale);
+            else launch_dep(k_moe_down_rows<float, false>, dim3(grid), dim3(256), 0, st, (const float *) y, (const float *) down, idx, wt, p, width, x, base, xscale, out_scale);
         }
     });
 }

@@ -42,6 +42,7 @@ __device__ __forceinline__ void group_inv_rms(const float * __restrict__ row, in
 template <typename OT>
 __global__ void __launch_bounds__(1024) k_group_rmsnorm(const float * __restrict__ x, const int32_t * __restrict__ rows, const float * __restrict__ w, int groups,
                                                        float eps, OT * __restrict__ y, int width) {
+    pdl_enter();
     __shared__ float red[33];
     __shared__ float inv[MAX_NORM_GROUPS];
     const int r = blockIdx.x;
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(256) k_group_rmsnorm_shift(const float * __res
                                                              const int32_t * __restrict__ entry_of, const float * __restrict__ w, int groups, float eps,
                                                              const float * __restrict__ mu, float * __restrict__ shift_state, int64_t slot_stride,
                                                              OT * __restrict__ y, int width) {
+    pdl_enter();
     __shared__ float red[33];
     __shared__ float inv[MAX_NORM_GROUPS], invp[MAX_NORM_GROUPS];
     const int t = blockIdx.x;
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(1024) k_rmsnorm_token_mix(const float * __rest
                                                             const int32_t * __restrict__ entry_of, const float * __restrict__ w, float eps,
                                                             const float * __restrict__ mu, int n_planes, float * __restrict__ shift_state, int64_t slot_stride,
                                                             OT * __restrict__ y, int64_t plane, float * __restrict__ yf, int width) {
+    pdl_enter();
     __shared__ float red[33];
     __shared__ float inv[1], invp[1];
     const int t = blockIdx.x;
@@ -130,6 +133,7 @@ __device__ __forceinline__ float depth_sum(const float * __restrict__ planes, in
 }
 __global__ void k_depth_average(const float * __restrict__ planes, int64_t plane_stride, const float * __restrict__ coef, int n, float * __restrict__ out,
                                 int64_t count) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     out[i] = depth_sum(planes, plane_stride, coef, n, i);
@@ -141,6 +145,7 @@ __global__ void __launch_bounds__(256) k_depth_average_norm_shift(const float * 
                                                                   float * __restrict__ x, const int32_t * __restrict__ slot, const float * __restrict__ w,
                                                                   int groups, float eps, const float * __restrict__ mu, float * __restrict__ shift_state,
                                                                   int64_t slot_stride, OT * __restrict__ y, int width) {
+    pdl_enter();
     extern __shared__ __align__(16) float row[];   // [width]
     __shared__ float red[33];
     __shared__ float inv[MAX_NORM_GROUPS];
@@ -196,6 +201,7 @@ template <typename OT>
 __global__ void __launch_bounds__(256) k_norm_gate(const float * __restrict__ y, const float * __restrict__ gate, int64_t ldg, int part,
                                                    const float * __restrict__ w, int gate_act, float eps, OT * __restrict__ out, int inner, int64_t ldo,
                                                    float out_scale) {
+    pdl_enter();
     __shared__ float red[33];
     const int t = blockIdx.x, grp = blockIdx.y;
     const float * yr = y + (int64_t) t * inner + grp * part;
@@ -213,6 +219,7 @@ __global__ void __launch_bounds__(256) k_norm_gate(const float * __restrict__ y,
 
 template <typename OT>
 __global__ void k_clamped_glu(const float * __restrict__ gu, OT * __restrict__ y, int n_tokens, int ff, float limit) {
+    pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t) n_tokens * ff) return;
     const int64_t t = i / ff, j = i - t * ff;
@@ -228,8 +235,8 @@ int launch_group_rmsnorm(const float * x, const int32_t * rows, const float * w,
     if (n_rows <= 0) return 0;
     if (groups <= 0 || groups > MAX_NORM_GROUPS || width % groups != 0) return (int) cudaErrorInvalidValue;
     return ck_launch([&] {
-        if (otype == T_BF16) k_group_rmsnorm<__nv_bfloat16><<<n_rows, row_threads(n_rows, width), 0, st>>>(x, rows, w, groups, eps, (__nv_bfloat16 *) y, width);
-        else k_group_rmsnorm<float><<<n_rows, row_threads(n_rows, width), 0, st>>>(x, rows, w, groups, eps, (float *) y, width);
+        if (otype == T_BF16) launch_dep(k_group_rmsnorm<__nv_bfloat16>, dim3(n_rows), dim3(row_threads(n_rows, width)), 0, st, x, rows, w, groups, eps, (__nv_bfloat16 *) y, width);
+        else launch_dep(k_group_rmsnorm<float>, dim3(n_rows), dim3(row_threads(n_rows, width)), 0, st, x, rows, w, groups, eps, (float *) y, width);
     });
 }
 int launch_group_rmsnorm_shift(const float * x, const BatchView & b, const float * w, int groups, float eps, const float * mu, float * shift_state,
@@ -239,9 +246,9 @@ int launch_group_rmsnorm_shift(const float * x, const BatchView & b, const float
     if (groups <= 0 || groups > MAX_NORM_GROUPS || width % groups != 0 || !shift_state) return (int) cudaErrorInvalidValue;
     int rc = ck_launch([&] {
         if (otype == T_BF16)
-            k_group_rmsnorm_shift<__nv_bfloat16><<<b.n_tokens, 256, 0, st>>>(x, b.slot, b.off, b.entry_of, w, groups, eps, mu, shift_state, slot_stride,
+            launch_dep(k_group_rmsnorm_shift<__nv_bfloat16>, dim3(b.n_tokens), dim3(256), 0, st, x, b.slot, b.off, b.entry_of, w, groups, eps, mu, shift_state, slot_stride,
                                                                              (__nv_bfloat16 *) y, width);
-        else k_group_rmsnorm_shift<float><<<b.n_tokens, 256, 0, st>>>(x, b.slot, b.off, b.entry_of, w, groups, eps, mu, shift_state, slot_stride, (float *) y, width);
+        else launch_dep(k_group_rmsnorm_shift<float>, dim3(b.n_tokens), dim3(256), 0, st, x, b.slot, b.off, b.entry_of, w, groups, eps, mu, shift_state, slot_stride, (float *) y, width);
     });
     if (rc || b.max_n <= 1) return rc;   // one-token entries have written their state themselves
     return ck_launch([&] { k_shift_state<<<b.n_entries, 256, 0, st>>>(x, b.slot, b.off, w, groups, eps, shift_state, slot_stride, width); });
@@ -253,10 +260,10 @@ int launch_rmsnorm_token_mix(const float * x, const BatchView & b, const float *
     const int threads = row_threads(b.n_tokens, width);
     int rc = ck_launch([&] {
         if (otype == T_BF16)
-            k_rmsnorm_token_mix<__nv_bfloat16><<<b.n_tokens, threads, 0, st>>>(x, b.slot, b.off, b.entry_of, w, eps, mu, n_planes, shift_state, slot_stride,
+            launch_dep(k_rmsnorm_token_mix<__nv_bfloat16>, dim3(b.n_tokens), dim3(threads), 0, st, x, b.slot, b.off, b.entry_of, w, eps, mu, n_planes, shift_state, slot_stride,
                                                                                (__nv_bfloat16 *) y, plane, yf, width);
         else
-            k_rmsnorm_token_mix<float><<<b.n_tokens, threads, 0, st>>>(x, b.slot, b.off, b.entry_of, w, eps, mu, n_planes, shift_state, slot_stride, (float *) y,
+            launch_dep(k_rmsnorm_token_mix<float>, dim3(b.n_tokens), dim3(threads), 0, st, x, b.slot, b.off, b.entry_of, w, eps, mu, n_planes, shift_state, slot_stride, (float *) y,
                                                                        plane, yf, width);
     });
     if (rc || b.max_n <= 1) return rc;   // one-token entries have written their state themselves
@@ -264,7 +271,7 @@ int launch_rmsnorm_token_mix(const float * x, const BatchView & b, const float *
 }
 int launch_depth_average(const float * planes, int64_t plane_stride, const float * coef, int n, float * out, int64_t count, cudaStream_t st) {
     if (count <= 0 || n <= 0) return 0;
-    return ck_launch([&] { k_depth_average<<<(unsigned) ((count + 255) / 256), 256, 0, st>>>(planes, plane_stride, coef, n, out, count); });
+    return ck_launch([&] { launch_dep(k_depth_average, dim3((unsigned) ((count + 255) / 256)), dim3(256), 0, st, planes, plane_stride, coef, n, out, count); });
 }
 int launch_depth_average_norm_shift(const float * planes, int64_t plane_stride, const float * coef, int n, float * x, const BatchView & b, const float * w,
                                     int groups, float eps, const float * mu, float * shift_state, int64_t slot_stride, void * y, int otype, int width,
@@ -277,14 +284,14 @@ int launch_depth_average_norm_shift(const float * planes, int64_t plane_stride, 
         int rc = raise_smem(k_depth_average_norm_shift<__nv_bfloat16>, smem);
         if (rc) return rc;
         return ck_launch([&] {
-            k_depth_average_norm_shift<__nv_bfloat16><<<b.n_tokens, 256, smem, st>>>(planes, plane_stride, coef, n, x, b.slot, w, groups, eps, mu, shift_state,
+            launch_dep(k_depth_average_norm_shift<__nv_bfloat16>, dim3(b.n_tokens), dim3(256), smem, st, planes, plane_stride, coef, n, x, b.slot, w, groups, eps, mu, shift_state,
                                                                                      slot_stride, (__nv_bfloat16 *) y, width);
         });
     }
     int rc = raise_smem(k_depth_average_norm_shift<float>, smem);
     if (rc) return rc;
     return ck_launch([&] {
-        k_depth_average_norm_shift<float><<<b.n_tokens, 256, smem, st>>>(planes, plane_stride, coef, n, x, b.slot, w, groups, eps, mu, shift_state, slot_stride,
+        launch_dep(k_depth_average_norm_shift<float>, dim3(b.n_tokens), dim3(256), smem, st, planes, plane_stride, coef, n, x, b.slot, w, groups, eps, mu, shift_state, slot_stride,
                                                                          (float *) y, width);
     });
 }
@@ -296,8 +303,8 @@ int launch_norm_gate(const float * y, const float * gate, int64_t ldg, int group
     if (ldo <= 0) ldo = inner;
     const dim3 grid((unsigned) n_tokens, (unsigned) groups);
     return ck_launch([&] {
-        if (otype == T_BF16) k_norm_gate<__nv_bfloat16><<<grid, 256, 0, st>>>(y, gate, ldg, inner / groups, w, gate_act, eps, (__nv_bfloat16 *) out, inner, ldo, out_scale);
-        else k_norm_gate<float><<<grid, 256, 0, st>>>(y, gate, ldg, inner / groups, w, gate_act, eps, (float *) out, inner, ldo, out_scale);
+        if (otype == T_BF16) launch_dep(k_norm_gate<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, y, gate, ldg, inner / groups, w, gate_act, eps, (__nv_bfloat16 *) out, inner, ldo, out_scale);
+        else launch_dep(k_norm_gate<float>, dim3(grid), dim3(256), 0, st, y, gate, ldg, inner / groups, w, gate_act, eps, (float *) out, inner, ldo, out_scale);
     });
 }
 int launch_clamped_glu(const float * gu, void * y, int otype, int n_tokens, int ff, float limit, cudaStream_t st) {
@@ -305,8 +312,8 @@ int launch_clamped_glu(const float * gu, void * y, int otype, int n_tokens, int 
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
     return ck_launch([&] {
-        if (otype == T_BF16) k_clamped_glu<__nv_bfloat16><<<grid, 256, 0, st>>>(gu, (__nv_bfloat16 *) y, n_tokens, ff, limit);
-        else k_clamped_glu<float><<<grid, 256, 0, st>>>(gu, (float *) y, n_tokens, ff, limit);
+        if (otype == T_BF16) launch_dep(k_clamped_glu<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, gu, (__nv_bfloat16 *) y, n_tokens, ff, limit);
+        else launch_dep(k_clamped_glu<float>, dim3(grid), dim3(256), 0, st, gu, (float *) y, n_tokens, ff, limit);
     });
 }
 

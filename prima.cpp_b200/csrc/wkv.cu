@@ -63,6 +63,7 @@ constexpr int LR_SPLIT = 8;
 template <int TT>
 __global__ void __cluster_dims__(1, 1, LR_SPLIT) __launch_bounds__(256) k_lowrank_down(const float * __restrict__ m, const float * __restrict__ w1,
                                                                                     float * __restrict__ tmp, int T, int rank, int width) {
+    pdl_enter();
     __shared__ __align__(16) float As[TT][LR_S];
     __shared__ __align__(16) float Bs[LR_COLS][LR_S];
     cg::cluster_group cl = cg::this_cluster();
@@ -106,6 +107,7 @@ __global__ void __cluster_dims__(1, 1, LR_SPLIT) __launch_bounds__(256) k_lowran
 template <int TT, bool RAW>
 __global__ void __launch_bounds__(256) k_lowrank_up(const float * __restrict__ tmp, const float * __restrict__ w2, const float * __restrict__ w0,
                                                     float * __restrict__ decay, int T, int N, int rank) {
+    pdl_enter();
     __shared__ __align__(16) float As[TT][LR_S];
     __shared__ __align__(16) float Bs[LR_COLS][LR_S];
     const int t0 = blockIdx.y * TT, n0 = blockIdx.x * LR_COLS;
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(256) k_lowrank_up(const float * __restrict__ t
 // two maps side by side (LowrankMaps): column tiles of the decay first, then those of the gate
 template <int TT>
 __global__ void __launch_bounds__(256) k_lowrank_maps(LowrankMaps mp, int T, int a_tiles) {
+    pdl_enter();
     __shared__ __align__(16) float As[TT][LR_S];
     __shared__ __align__(16) float Bs[LR_COLS][LR_S];
     const bool is_a = (int) blockIdx.x < a_tiles;
@@ -202,6 +205,7 @@ template <int N> constexpr int ws_stage_floats() { return WS_CHUNK * (3 * N + WS
 template <int N>
 __global__ void __launch_bounds__(WS_COLS / 2 * (N / WS_NREG)) k_wkv_scan(GatedLinIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                                       GatedLinParams p, float * __restrict__ state, int64_t slot_stride, float * __restrict__ y) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];   // [stages][ r [16][N] | k [16][N] | w [16][N] | v [16][16] ], then the bonus products [16]
     constexpr int LN = N / WS_NREG, NT = WS_COLS / 2 * LN, STAGE = ws_stage_floats<N>();
     const int P = p.vdim, inner = p.heads * P, ptiles = (P + WS_COLS - 1) / WS_COLS;
@@ -313,7 +317,7 @@ int wkv_scan_launch(const GatedLinIO & io, const BatchView & b, const GatedLinPa
     const int rc = raise_smem(k_wkv_scan<N>, smem);
     if (rc) return rc;
     const dim3 grid((unsigned) (p.heads * ((p.vdim + WS_COLS - 1) / WS_COLS)), (unsigned) b.n_entries);
-    return ck_launch([&] { k_wkv_scan<N><<<grid, WS_COLS / 2 * (N / WS_NREG), smem, st>>>(io, b.slot, b.off, p, state, slot_stride, y); });
+    return ck_launch([&] { launch_dep(k_wkv_scan<N>, dim3(grid), dim3(WS_COLS / 2 * (N / WS_NREG)), smem, st, io, b.slot, b.off, p, state, slot_stride, y); });
 }
 
 }  // namespace
@@ -340,8 +344,8 @@ int launch_lowrank_maps(const LowrankMaps & mp, int n_tokens, cudaStream_t st) {
     const int at = (mp.heads * mp.dim + LR_COLS - 1) / LR_COLS;
     const unsigned tiles = (unsigned) (at + (mp.gate_cols + LR_COLS - 1) / LR_COLS);
     return ck_launch([&] {
-        if (n_tokens > 64) k_lowrank_maps<64><<<dim3(tiles, (unsigned) ((n_tokens + 63) / 64)), 256, 0, st>>>(mp, n_tokens, at);
-        else k_lowrank_maps<16><<<dim3(tiles, (unsigned) ((n_tokens + 15) / 16)), 256, 0, st>>>(mp, n_tokens, at);
+        if (n_tokens > 64) launch_dep(k_lowrank_maps<64>, dim3(tiles, (unsigned) ((n_tokens + 63) / 64)), dim3(256), 0, st, mp, n_tokens, at);
+        else launch_dep(k_lowrank_maps<16>, dim3(tiles, (unsigned) ((n_tokens + 15) / 16)), dim3(256), 0, st, mp, n_tokens, at);
     });
 }
 
@@ -353,16 +357,16 @@ int launch_lowrank_decay(const float * m, const float * w1, const float * w2, co
     if (n_tokens <= 4) {   // one or a few tokens: the weight-streaming product, the tanh at its reader
         const int rc = launch_dense(0 /* T_F32 */, m, width, w1, width, tmp, rank, n_tokens, rank, width, nullptr, nullptr, 0, 1.f, st);
         if (rc) return rc;
-        return ck_launch([&] { k_lowrank_up<16, true><<<dim3(ct, 1), 256, 0, st>>>(tmp, w2, w0, decay, n_tokens, channels, rank); });
+        return ck_launch([&] { launch_dep(k_lowrank_up<16, true>, dim3(ct, 1), dim3(256), 0, st, tmp, w2, w0, decay, n_tokens, channels, rank); });
     }
     int rc = ck_launch([&] {
-        if (n_tokens >= 1024) k_lowrank_down<64><<<dim3(rt, (unsigned) ((n_tokens + 63) / 64), LR_SPLIT), 256, 0, st>>>(m, w1, tmp, n_tokens, rank, width);
-        else k_lowrank_down<16><<<dim3(rt, (unsigned) ((n_tokens + 15) / 16), LR_SPLIT), 256, 0, st>>>(m, w1, tmp, n_tokens, rank, width);
+        if (n_tokens >= 1024) launch_dep(k_lowrank_down<64>, dim3(rt, (unsigned) ((n_tokens + 63) / 64), LR_SPLIT), dim3(256), 0, st, m, w1, tmp, n_tokens, rank, width);
+        else launch_dep(k_lowrank_down<16>, dim3(rt, (unsigned) ((n_tokens + 15) / 16), LR_SPLIT), dim3(256), 0, st, m, w1, tmp, n_tokens, rank, width);
     });
     if (rc) return rc;
     return ck_launch([&] {
-        if (n_tokens > 64) k_lowrank_up<64, false><<<dim3(ct, (unsigned) ((n_tokens + 63) / 64)), 256, 0, st>>>(tmp, w2, w0, decay, n_tokens, channels, rank);
-        else k_lowrank_up<16, false><<<dim3(ct, (unsigned) ((n_tokens + 15) / 16)), 256, 0, st>>>(tmp, w2, w0, decay, n_tokens, channels, rank);
+        if (n_tokens > 64) launch_dep(k_lowrank_up<64, false>, dim3(ct, (unsigned) ((n_tokens + 63) / 64)), dim3(256), 0, st, tmp, w2, w0, decay, n_tokens, channels, rank);
+        else launch_dep(k_lowrank_up<16, false>, dim3(ct, (unsigned) ((n_tokens + 15) / 16)), dim3(256), 0, st, tmp, w2, w0, decay, n_tokens, channels, rank);
     });
 }
 
