@@ -18,15 +18,15 @@
 // number of 64-element MMA steps whatever N, K and T are: round 1's one-tile-per-CTA grid left 84 of 148 SMs idle on an 8192-row matrix
 // at 512 tokens and 2/3 of the last wave idle on ffn_gate/up.  A CTA walks its range segment by segment (segment = its part of one
 // tile); a segment that covers the tile's whole K stores its result, a partial one adds it into the pre-zeroed dst with fp32 atomics
-// (two or three addends per element: the order of fp32 adds is the only non-determinism, below the kernel's own fp16 rounding).
+// (one addend per CTA of the tile: the order of fp32 adds is the only non-determinism, below the kernel's own fp16 rounding).
 // Inside a CTA the pipeline never drains between segments (raw-block ring, A and B stages and their barriers run on CTA-wide counters):
 //   warp 0      owns TMEM; one lane issues 4 x tcgen05.mma (M=128, N=BN, K=16, kind::f16) per step and accumulator, one commit per step
 //   warp 1      activation producer: one cp.async.bulk per step and accumulator of the pre-tiled fp16 chunk (BN x 128 B, already in the
 //               UMMA swizzle-128B image), 2-4 stages deep
 //   warps 2..17 (16 expansion warps, 4 threads per weight row) fetch their rows' raw quantized blocks (16-byte cp.async pieces, 3 K groups
 //               deep, completion through cp.async.mbarrier.arrive) and expand 128 x 64 weights per step to fp16 straight into the swizzled A
-//               stage (generic-proxy stores + fence.proxy.async), 2 stages (4 with CTA pairs); at the end of a segment warps 2..9 read the
-//               accumulators out of TMEM (tcgen05.ld 32x32b: quadrant = warp % 4, accumulator = (warp - 2) / 4) and store / add into dst
+//               stage (generic-proxy stores + fence.proxy.async), 2 stages (4 with CTA pairs); at the end of a segment all 16 read the
+//               accumulators out of TMEM (tcgen05.ld 32x32b: quadrant = warp % 4, every fourth chunk of 16 columns) and store / add into dst
 // CG = 2 (opt-in): the CTA pair of a cluster shares one M = 256 MMA (cta_group::2), see launch_mmq.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -69,7 +69,7 @@ struct MmqCtl {
     uint64_t raw_full[3], raw_empty[3];
     uint64_t a_ready[MMQ_A_MAX], b_full[MMQ_B_NST];
     uint64_t step_done[MMQ_B_NST];   // one tcgen05.commit per step: step u arrives on step_done[u % 4]; frees A stage u % 2 and B stage u % b_nst
-    uint64_t acc_ready, acc_free;    // per segment: accumulators complete (tcgen05.commit) / read out by the 4 epilogue warps (of both CTAs of a pair)
+    uint64_t acc_ready, acc_free;    // per segment: accumulators complete (tcgen05.commit) / read out by the 16 expansion warps (of both CTAs of a pair)
     uint64_t peer_ready[MMQ_B_NST];  // CTA pairs: step g's A and B stages of the peer CTA are filled (forwarded by the peer's otherwise idle warp 0)
     uint32_t tmem_base;
     volatile int abort;
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         for (int i = 0; i < MMQ_A_MAX; i++) mbar_init(&ctl->a_ready[i], MMQ_DQ_WARPS);
         for (int i = 0; i < MMQ_B_NST; i++) { mbar_init(&ctl->b_full[i], 1); mbar_init(&ctl->step_done[i], 1); }
         mbar_init(&ctl->acc_ready, 1);
-        mbar_init(&ctl->acc_free, 8 * CG);
+        mbar_init(&ctl->acc_free, MMQ_DQ_WARPS * CG);
         for (int i = 0; i < MMQ_B_NST; i++) mbar_init(&ctl->peer_ready[i], 1);
         ctl->abort = 0;
         mbar_fence_init();
@@ -481,64 +481,65 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 if (++rs == P.nraw) { rs = 0; rph ^= 1; }
             }
             // ================= epilogue of the segment: four consecutive warps cover the four 32-lane quadrants of TMEM =================
-            if (warp < MMQ_DQ_WARP0 + 8) {
-                // 8 epilogue warps: quadrant warp % 4 of the TMEM lanes (a warp may only read its own quadrant), accumulator (warp - 2) / 4
-                const int ehalf = (warp - MMQ_DQ_WARP0) >> 2;
+            // All 16 expansion warps read out: a warp may only read quadrant warp % 4, its group (warp - 2) / 4 takes every fourth chunk of 16
+            // columns.  Chunk ch holds tokens tt0 * BN + 16 ch ..: two accumulators lie 256 columns apart and are only used with BN = 256.
+            // What bounds it is instruction issue (128 x 512 values; 8 warps with a 64-bit index product, two tests and a select per value
+            // took 20 of the 26 us that a segment cost beyond its MMA steps), hence the walking pointers and the paths without residual tests.
+            {
                 const bool acc_ok = ok && mmq_wait(ctl, &ctl->acc_ready, seg & 1);
                 tc_fence_after();
                 const int tt0 = (tile / P.rtiles) * P.nacc;
-                const int nacc = min(P.nacc, P.ttiles - tt0);
+                const int nch = min(P.nacc, P.ttiles - tt0) * (BN >> 4);
                 const bool first = sbb == 0, whole = first && sbe == P.ngrp;   // bias / residual ride on the K group 0 segment
                 const int quad = warp & 3;
                 const int n = row0 + quad * 32 + lane;
-                const float bias = (P.bias && n < P.N && first) ? P.bias[n] : 0.f;
-                // The residual rows are fetched one 16-token chunk AHEAD, all 16 loads in flight at once: written as "load, add, store" per
-                // element the loads serialise behind the stores / atomics (dst and resid may alias as far as the compiler knows), which cost
-                // 220-260 us per launch with a residual (wo, ffn_down: profiles/r2_prefill_launches_streamk_before_resid_fix.csv)
-                const float * __restrict__ rp = (P.resid && first && n < P.N) ? P.resid + n : nullptr;
-                float rcur[16], rnext[16];
-                auto load_resid = [&](float (&rv)[16], int a, int c0) {
+                const bool live = acc_ok && n < P.N;
+                const float bias = (P.bias && live && first) ? P.bias[n] : 0.f;
+                const float * __restrict__ rp = (P.resid && first && live) ? P.resid + n : nullptr;
+                const size_t ldd = (size_t) P.N;
+                for (int ch = (warp - MMQ_DQ_WARP0) >> 2; ch < nch; ch += 4) {
+                    const int t0 = tt0 * BN + ch * 16;
+                    const int nt = min(16, P.T - t0);            // tokens of the chunk (<= 0: padding only)
+                    if (nt <= 0) break;
+                    float y[16];
+                    // all 16 residual loads in flight at once, ahead of the stores they could alias as far as the compiler knows
+                    if (rp) {
+                        const float * q = rp + (size_t) t0 * ldd;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int t = (tt0 + a) * BN + c0 + i;
-                        rv[i] = (rp && t < P.T) ? __ldg(rp + (size_t) t * P.N) : 0.f;
+                        for (int i = 0; i < 16; i++) y[i] = i < nt ? __ldg(q + i * ldd) : 0.f;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) y[i] = 0.f;
                     }
-                };
-                // two accumulators: one per warp group; one accumulator: its column halves (when they split into whole 16-column chunks)
-                const bool csplit = nacc == 1 && BN % 32 == 0;
-                const int a_lo = nacc == 2 ? ehalf : 0, a_hi = nacc == 2 ? ehalf + 1 : ((csplit || ehalf == 0) ? 1 : 0);
-                const int c_lo = csplit ? ehalf * (BN / 2) : 0, c_hi = csplit ? c_lo + BN / 2 : BN;
-                if (a_lo < a_hi) load_resid(rcur, a_lo, c_lo);
-                for (int a = a_lo; a < a_hi; a++) {
-                    for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
-                        {   // next chunk's residual
-                            int a2 = a, c2 = c0 + 16;
-                            if (c2 >= c_hi) { a2++; c2 = c_lo; }
-                            if (a2 < a_hi) load_resid(rnext, a2, c2);
-                        }
-                        uint32_t v[16];
-                        const uint32_t taddr = tmem + ((uint32_t) (quad * 32) << 16) + (uint32_t) (a * 256 + c0);
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                            : "r"(taddr)
-                            : "memory");
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (acc_ok && n < P.N) {
+                    __syncwarp();
+                    uint32_t v[16];
+                    const uint32_t taddr = tmem + ((uint32_t) (quad * 32) << 16) + (uint32_t) (ch * 16);
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                        : "r"(taddr)
+                        : "memory");
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (live) {
+                        float * d = P.dst + (size_t) t0 * ldd + n;
 #pragma unroll
-                            for (int i = 0; i < 16; i++) {
-                                const int t = (tt0 + a) * BN + c0 + i;
-                                if (t < P.T) {
-                                    const float y = __fadd_rn(__fadd_rn(__uint_as_float(v[i]), bias), rcur[i]);
-                                    if (whole) P.dst[(size_t) t * P.N + n] = y;
-                                    else atomicAdd(&P.dst[(size_t) t * P.N + n], y);   // <= 3 addends onto 0
-                                }
-                            }
-                        }
+                        for (int i = 0; i < 16; i++) y[i] = __fadd_rn(__fadd_rn(__uint_as_float(v[i]), bias), y[i]);
+                        if (whole && nt == 16) {
 #pragma unroll
-                        for (int i = 0; i < 16; i++) rcur[i] = rnext[i];
+                            for (int i = 0; i < 16; i++, d += ldd) *d = y[i];
+                        } else if (whole) {
+#pragma unroll
+                            for (int i = 0; i < 16; i++, d += ldd) if (i < nt) *d = y[i];
+                        } else if (nt == 16) {
+#pragma unroll
+                            for (int i = 0; i < 16; i++, d += ldd) atomicAdd(d, y[i]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 16; i++, d += ldd) if (i < nt) atomicAdd(d, y[i]);
+                        }
                     }
+                    __syncwarp();
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -695,6 +696,27 @@ static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size
     return cg == 2 ? mmq_launch_typed2<TYPE, 2>(P, grid, smem, st) : mmq_launch_typed2<TYPE, 1>(P, grid, smem, st);
 }
 
+// Units per CTA.  The least share that fits one wave is ceil(total / SMs); a longer one is better when it makes the CTAs' ranges end where
+// tiles end: a share that divides the tile's groups is one segment, one that is a multiple of them needs no adding and no cleared output,
+// any other can touch a tile more.  Costs in us on B200, Q4_K: a unit 3.05 (512 tokens: two accumulators, 8 x 171 clk of MMA a step; half of
+// it with one), a segment's fill and read-out 8, the clearing pass 3 + bytes / 6.2 TB/s.  At 512 tokens, us per launch (K = 4096): 512 and
+// 4096 rows as shares of at least 8 units 35.8 and 34.8, at least 1 unit 24.2 and 14.1; 14336 rows in shares of 13 units 64.1 and 7.8 for the
+// clearing, as whole tiles 63.5.
+static int mmq_pick_share(int64_t total, int ngrp, int nsm, int nacc, double out_bytes) {
+    const int base = (int) ((total + nsm - 1) / nsm);
+    const double unit = nacc == 2 ? 3.05 : 1.55, seg = nacc == 2 ? 8.0 : 5.0, clear = 3.0 + out_bytes / 6.2e6;
+    int best = base;
+    double best_us = 1e30;
+    for (int upc = base; upc <= base + ngrp; upc++) {
+        const bool whole = upc % ngrp == 0, divides = ngrp % upc == 0;
+        if (upc != base && !whole && !divides) continue;
+        const int segs = whole ? upc / ngrp : divides ? 1 : (upc + ngrp - 2) / ngrp + 1;
+        const double us = upc * unit + segs * seg + (whole ? 0.0 : clear);
+        if (us < best_us) { best_us = us; best = upc; }
+    }
+    return best;
+}
+
 cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const float * x, int64_t ldx, int64_t T, float * dst, const float * bias,
                        const float * resid, void * ws, cudaStream_t st, bool reuse_prep, const MmqPre * pre) {
     if (pre && pre->kind != 0 && (!pre->aux || K % 256 != 0 || pre->kind < 0 || pre->kind > 2)) return cudaErrorInvalidValue;
@@ -734,16 +756,15 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     if (P.nacc == 2 && 1024 + (size_t) 2 * MMQ_A_BYTES + (size_t) 2 * 2 * (BN / cg) * 128 + (size_t) 2 * MMQ_BM * P.slot + MMQ_CTL_BYTES > 232448) P.nacc = 1;
     const int tgroups = (P.ttiles + P.nacc - 1) / P.nacc;
     P.ngrp = (int) ((K / MMQ_BK + 3) / 4);
-    // stream-K: the tiles' K groups, tile after tile, in equal contiguous shares; a share is at least MMQ_MIN_UNITS groups (a segment's
-    // pipeline fill + 128 x 512 epilogue must stay small against its MMA steps) unless the whole launch is smaller than that
-    static const int min_units = getenv("PB200_MMQ_MIN_UNITS") ? std::max(1, atoi(getenv("PB200_MMQ_MIN_UNITS"))) : 8;
+    // stream-K: the tiles' K groups, tile after tile, in equal contiguous shares (mmq_pick_share)
+    static const int min_units = getenv("PB200_MMQ_MIN_UNITS") ? std::max(1, atoi(getenv("PB200_MMQ_MIN_UNITS"))) : 0;   // A/B: a fixed least share
     static const bool whole_tiles = getenv("PB200_MMQ_WHOLE_TILES") != nullptr;   // A/B: round 1's one tile per CTA (no split, no atomics)
     const int64_t total = (int64_t) P.rtiles * tgroups * P.ngrp;
     if (total > 0x7fffffff) return cudaErrorInvalidValue;
     P.total_units = (int) total;
     const int nsm = sm_count() / cg;           // CTAs (pairs) that can be resident: one CTA per SM
-    int upc = (int) ((total + nsm - 1) / nsm);
-    upc = std::max(upc, std::min(min_units, P.ngrp));
+    int upc = mmq_pick_share(total, P.ngrp, nsm, P.nacc, (double) T * (double) N * 4.0);
+    if (min_units) upc = std::max((int) ((total + nsm - 1) / nsm), std::min(min_units, P.ngrp));
     if (whole_tiles) upc = P.ngrp;
     P.upc = upc;
     const int grid_x = (int) ((total + upc - 1) / upc);
