@@ -776,7 +776,7 @@ def main():
                               "roofline": {"bound": "tensor", "achieved": (mm + att + head) / best / 1e12, "peak": tpeak, "unit": "TFLOP/s",
                                            "frac": (mm + att + head) / best / 1e12 / tpeak, "peak_source": tsrc,
                                            "algorithmic_flops": {"matmul": mm, "attention_causal": att, "lm_head_last_token": head},
-                                           "kernel": "k_mmq_tc (tcgen05 k-quant mat-mul); attention on CUDA cores (k_attn_prefill_tiled: K/V tiles shared by the GQA group x 4 tokens)"}}
+                                           "kernel": "k_mmq_tc (tcgen05 k-quant mat-mul); attention k_attn_prefill_tc (tcgen05 over the f16 cache)"}}
         except Exception as ex:   # the extra measurement must never take the headline line down
             out["prefill"] = {"value": None, "unit": "tokens/s", "error": repr(ex)}
 

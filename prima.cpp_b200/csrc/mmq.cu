@@ -12,10 +12,10 @@
 // Also the 32-element block types Q8_0 / Q5_1 (K % 64 == 0; activations quantized per 32 values like their CPU dot): Qwen2.5-72B's
 // ffn_down, whose K = 29 568 rules the k-quants out (src/llama.cpp:19516-19551).
 //
-// Work decomposition (round 2: stream-K, persistent).  A work UNIT = one 256-element K group of one output tile (128 weight rows x 1 or 2
+// Work decomposition (stream-K, persistent).  A work UNIT = one 256-element K group of one output tile (128 weight rows x 1 or 2
 // token tiles of BN <= 256 columns: two accumulators = all 512 TMEM columns share every expanded weight stage when T is large enough).
 // The units of a launch, ordered tile by tile, are cut into one contiguous range per CTA (at most one CTA per SM), so every SM gets the same
-// number of 64-element MMA steps whatever N, K and T are: round 1's one-tile-per-CTA grid left 84 of 148 SMs idle on an 8192-row matrix
+// number of 64-element MMA steps whatever N, K and T are: a one-tile-per-CTA grid left 84 of 148 SMs idle on an 8192-row matrix
 // at 512 tokens and 2/3 of the last wave idle on ffn_gate/up.  A CTA walks its range segment by segment (segment = its part of one
 // tile); a segment that covers the tile's whole K stores its result, a partial one adds it into the pre-zeroed dst with fp32 atomics
 // (one addend per CTA of the tile: the order of fp32 adds is the only non-determinism, below the kernel's own fp16 rounding).
@@ -758,7 +758,7 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     P.ngrp = (int) ((K / MMQ_BK + 3) / 4);
     // stream-K: the tiles' K groups, tile after tile, in equal contiguous shares (mmq_pick_share)
     static const int min_units = getenv("PB200_MMQ_MIN_UNITS") ? std::max(1, atoi(getenv("PB200_MMQ_MIN_UNITS"))) : 0;   // A/B: a fixed least share
-    static const bool whole_tiles = getenv("PB200_MMQ_WHOLE_TILES") != nullptr;   // A/B: round 1's one tile per CTA (no split, no atomics)
+    static const bool whole_tiles = getenv("PB200_MMQ_WHOLE_TILES") != nullptr;   // A/B: one tile per CTA (no split, no atomics)
     const int64_t total = (int64_t) P.rtiles * tgroups * P.ngrp;
     if (total > 0x7fffffff) return cudaErrorInvalidValue;
     P.total_units = (int) total;
