@@ -701,9 +701,10 @@ static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size
 // any other can touch a tile more.  Costs in us on B200, Q4_K: a unit 3.05 (512 tokens: two accumulators, 8 x 171 clk of MMA a step; half of
 // it with one), a segment's fill and read-out 8, the clearing pass 3 + bytes / 6.2 TB/s.  At 512 tokens, us per launch (K = 4096): 512 and
 // 4096 rows as shares of at least 8 units 35.8 and 34.8, at least 1 unit 24.2 and 14.1; 14336 rows in shares of 13 units 64.1 and 7.8 for the
-// clearing, as whole tiles 63.5.
+// clearing, as whole tiles 63.5.  Rows of up to 8 groups (K <= 2048) are not cut for idle SMs: there a tile costs at most 24 us, and uncut its
+// sums do not depend on the number of tokens, so a prompt's result does not depend on the slices it came in.
 static int mmq_pick_share(int64_t total, int ngrp, int nsm, int nacc, double out_bytes) {
-    const int base = (int) ((total + nsm - 1) / nsm);
+    const int fit = (int) ((total + nsm - 1) / nsm), base = ngrp <= 8 ? std::max(fit, ngrp) : fit;
     const double unit = nacc == 2 ? 3.05 : 1.55, seg = nacc == 2 ? 8.0 : 5.0, clear = 3.0 + out_bytes / 6.2e6;
     int best = base;
     double best_us = 1e30;

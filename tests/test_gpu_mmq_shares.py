@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 # (rows, K, tokens): on 148 SMs a share of one group of several, two tiles, a share that ends inside tiles, one whole tile, and the edges of
 # the 16-token chunks that the 16 reading warps take (1, 15, 17 tokens; a second accumulator with one token; rows that end inside a tile)
-@pytest.mark.parametrize("N,K,T", [(200, 2048, 1), (130, 1024, 15), (128, 4096, 17), (20480, 512, 17), (3840, 1792, 257), (14336, 256, 31), (129, 1024, 513)])
+@pytest.mark.parametrize("N,K,T", [(200, 2048, 1), (130, 3072, 15), (128, 4096, 17), (20480, 512, 17), (3840, 2816, 257), (14336, 256, 31), (129, 1024, 513)])
 @pytest.mark.parametrize("extra", [False, True], ids=["plain", "bias_residual"])
 def test_mmq_shares(cuda, lib, port, N, K, T, extra):
     rng = np.random.default_rng(N + K + T)
