@@ -1,15 +1,17 @@
 // prima.cpp_b200/csrc/attn_split.cu — prompt attention of the layer-list models (windows, kept first tokens, chunks, soft-cap, sinks, gates, grouped
 // heads, keys with a shared tail, another layer's cache) on the 5th-generation tensor cores, with fp32 inputs kept to 22 bits and more:
 // every fp32 operand x is two f16 numbers, hi = f16(x s) and lo = f16(x s - hi) with s a power of two per row that puts the row's largest
-// entry between 2^13 and 2^14, and a product is hi hi + hi lo + lo hi with fp32 accumulation.  What is dropped (lo lo and the rounding of lo) is
-// 2^-22 of the row's entries and less.  Scores, softmax, its running maximum and sum and the weighted sum across key tiles stay in fp32
-// registers; the weights are split like the other operands.
+// entry between 2^13 and 2^14, and a product is lo hi + hi lo + hi hi with fp32 accumulation, the small products first.  What is dropped (lo lo and
+// the rounding of lo) is 2^-22 of the row's entries and less.  A softmax weight takes its value row's power of two along: the largest such product
+// that a query has in a key tile comes to 2^14, or, in a tile that every query of the CTA sees and whose values lie within 2^12 of one another,
+// the tile's largest value does.  So what a query does not see, however large, or no number at all, does not touch its row.  Scores, softmax, its
+// running maximum and sum and the weighted sum across key tiles stay in fp32 registers.
 // Two launches: k_split_kv writes keys and values once, split and laid out as the operands' shared-memory images; k_attn_split walks them.
 // Only models that compute in bf16 come here (the result is rounded to 2^-9 next); float32 models keep the fp32 FMA kernels of mixers.cu.
-// Against float64 in models where nothing else rounds below fp32, over windows, chunks, sinks and 40 .. 700 keys: 2.9e-7 .. 5.8e-7 off, the FMA
-// kernel, whose sums round once a term, 2.9e-7 .. 5.8e-7 (at most 6 % less or more case by case; tests/test_gpu_attn_split.py).
-// Measured with the split pass: 2048 tokens, 16 heads of 128 over 4, causal 1516 -> 105 us; 512 tokens 176 -> 44; latent heads, prompts of 1111,
-// 300 and 77 tokens 522 -> 94.
+// Against float64 in models where nothing else rounds below fp32, six kinds of attention (windows, chunks, sinks, caps, gates, shared key tails), head
+// sizes 64 and 128, 40 to 300 keys, three seeds: 2.8e-7 .. 5.6e-7 off, 0.96 to 1.02 times the FMA kernel, 0.99 over all.
+// Measured with the split pass: 2048 tokens, 16 heads of 128 over 4, causal 1516 -> 114 us; 512 tokens 176 -> 48; latent heads, prompts of 1111,
+// 300 and 77 tokens 522 -> 102.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -27,7 +29,9 @@ namespace {
 constexpr int SP_KEYS = 128;                   // positions of a key tile
 constexpr int SP_K_UNIT = 2 * SP_KEYS * 128;   // 64 head entries of a tile's keys: hi, lo, each 128 rows of 128 bytes
 constexpr int SP_MAX_ND = 3, SP_MAX_NV = 2;    // head sizes up to 192, value sizes up to 128
-constexpr int SP_SCALES = 1040;                // key scales [128], value ratios [128], value factor [4] of a tile
+// of a tile: key scales [128], value scales relative to the tile's largest [128], value exponents [128], [4]: some value is no number; exponents
+// are far apart; the largest value scale
+constexpr int SP_SCALES = 1552, SP_SPREAD = 12;
 constexpr int SP_THREADS = 320, SP_SM_THREADS = 256;
 
 __host__ __device__ inline int sp_v_unit(int nv) { return 2 * nv * 64 * 128; }   // 64 positions of a tile's values: hi, lo, each nv blocks of 64 rows of 128 bytes
@@ -44,6 +48,19 @@ struct SplitParams {
     int * abort_flag;
 };
 
+constexpr uint32_t NO_NUMBER = 0x7f800000u;   // bits of a magnitude from here on: an infinity or a NaN
+__device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+// largest magnitude of the numbers in a warp's row, for rows whose plain maximum is none
+template <int N>
+__device__ __forceinline__ uint32_t max_number(const float (&x)[N][2]) {
+    uint32_t m = 0u;
+#pragma unroll
+    for (int c = 0; c < N; c++)
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            if (magnitude(x[c][i]) < NO_NUMBER) m = max(m, magnitude(x[c][i]));
+    return __reduce_max_sync(0xffffffffu, m);
+}
 // power of two that puts the largest entry (bits of its magnitude) in [2^13, 2^14); e: the clamped exponent it follows from
 __device__ __forceinline__ float split_scale(uint32_t max_bits, int lowest, int & e) {
     e = min(max((int) (max_bits >> 23), lowest), 254);
@@ -58,8 +75,8 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t & hi, uint32_t
 }
 
 // One CTA: a tile of 128 positions of one kv head and entry; a warp takes a position at a time, a lane two neighbouring entries of every 64.
-__global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitParams P) {
-    __shared__ int ev[SP_KEYS];
+__global__ void __launch_bounds__(256, 2) k_split_kv(const __grid_constant__ SplitParams P) {
+    __shared__ int ev[SP_KEYS];        // exponents, -: the row holds something that is no number, 0: nothing but zeros
     pdl_enter();
     const int e = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x;
     const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
@@ -76,6 +93,7 @@ __global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitP
     float * sc = reinterpret_cast<float *>(dv + 2 * sp_v_unit(P.nv));
     const int blk_b = sp_v_unit(P.nv) / 2;                         // the lo half of a unit of values
     constexpr int ROWS = 4;
+    int bad = 0;
     for (int r0 = warp * 16; r0 < warp * 16 + 16; r0 += ROWS) {
         float k[ROWS][SP_MAX_ND][2], v[ROWS][SP_MAX_NV][2];
 #pragma unroll
@@ -97,22 +115,44 @@ __global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitP
                     v[j][c][i] = live && d < DV ? vb[p * io.ldv + d] : 0.f;
                 }
         }
+        uint32_t mk[ROWS], mv[ROWS], worst = 0u;
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
-            const int r = r0 + j;
-            uint32_t mk = 0u, mv = 0u;
+            mk[j] = mv[j] = 0u;
 #pragma unroll
             for (int c = 0; c < SP_MAX_ND; c++)
 #pragma unroll
-                for (int i = 0; i < 2; i++) mk = max(mk, __float_as_uint(k[j][c][i]) & 0x7fffffffu);
+                for (int i = 0; i < 2; i++) mk[j] = max(mk[j], magnitude(k[j][c][i]));
 #pragma unroll
             for (int c = 0; c < SP_MAX_NV; c++)
 #pragma unroll
-                for (int i = 0; i < 2; i++) mv = max(mv, __float_as_uint(v[j][c][i]) & 0x7fffffffu);
-            mk = __reduce_max_sync(0xffffffffu, mk);
-            mv = __reduce_max_sync(0xffffffffu, mv);
+                for (int i = 0; i < 2; i++) mv[j] = max(mv[j], magnitude(v[j][c][i]));
+            mk[j] = __reduce_max_sync(0xffffffffu, mk[j]);
+            mv[j] = __reduce_max_sync(0xffffffffu, mv[j]);
+            worst = max(worst, max(mk[j], mv[j]));
+        }
+        uint32_t odd = 0u;   // bit j: a key of row j is no number, bit ROWS + j: a value
+        if (worst >= NO_NUMBER) {
+#pragma unroll
+            for (int j = 0; j < ROWS; j++) {
+                if (mk[j] >= NO_NUMBER) { mk[j] = max_number(k[j]); odd |= 1u << j; }
+                if (mv[j] >= NO_NUMBER) {   // such values stay out of the products (a weight of zero does not silence them): k_attn_split puts them in
+                    mv[j] = max_number(v[j]);
+                    odd |= 1u << (ROWS + j);
+                    bad = 1;
+#pragma unroll
+                    for (int c = 0; c < SP_MAX_NV; c++)
+#pragma unroll
+                        for (int i = 0; i < 2; i++)
+                            if (magnitude(v[j][c][i]) >= NO_NUMBER) v[j][c][i] = 0.f;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; j++) {
+            const int r = r0 + j;
             int ek, e_v;
-            const float sk = split_scale(mk, 14, ek), sv = split_scale(mv, 28, e_v);
+            const float sk = split_scale(mk[j], 14, ek), sv = split_scale(mv[j], 28, e_v);
             const uint32_t in_row = (uint32_t) ((((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
 #pragma unroll
             for (int c = 0; c < SP_MAX_ND; c++)
@@ -135,18 +175,42 @@ __global__ void __launch_bounds__(256) k_split_kv(const __grid_constant__ SplitP
                 }
             if (lane == 0) {
                 sc[r] = __uint_as_float((uint32_t) (ek - 13) << 23);
-                ev[r] = e_v;
+                sc[2 * SP_KEYS + r] = (float) (e_v - 127);
+                ev[r] = (odd >> (ROWS + j)) & 1u ? -e_v : mv[j] ? e_v : 0;
+            }
+            if ((odd >> j) & 1u) {   // an infinity or a NaN goes into lo alone: a score is then what its sign makes of it
+#pragma unroll
+                for (int c = 0; c < SP_MAX_ND; c++)
+                    if (c < P.nd) {
+                        const float x = k[j][c][0] * sk, y = k[j][c][1] * sk, fx = fabsf(x) < INFINITY ? x : 0.f, fy = fabsf(y) < INFINITY ? y : 0.f;
+                        uint32_t hi, lo;
+                        split2(fx, fy, hi, lo);
+                        const __half2 l = __floats2half2_rn(x, y);
+                        const uint32_t raw = *reinterpret_cast<const uint32_t *>(&l);
+                        if (fx != x) lo = (lo & 0xffff0000u) | (raw & 0xffffu);
+                        if (fy != y) lo = (lo & 0xffffu) | (raw & 0xffff0000u);
+                        uint8_t * o = dst + c * SP_K_UNIT + (r >> 3) * 1024 + (r & 7) * 128 + in_row;
+                        *reinterpret_cast<uint32_t *>(o) = hi;
+                        *reinterpret_cast<uint32_t *>(o + SP_K_UNIT / 2) = lo;
+                    }
             }
         }
     }
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     // the values' powers of two meet the weights: relative to the tile's largest one, times 2^14 (weights are at most 1, f16 reaches 2^16)
     if (warp < 4) {
-        int top = max(max(ev[lane], ev[lane + 32]), max(ev[lane + 64], ev[lane + 96]));
+        int top = 28, low = 254;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e_v = abs(ev[32 * i + lane]);
+            top = max(top, e_v);
+            low = min(low, e_v ? e_v : 254);
+        }
         top = __reduce_max_sync(0xffffffffu, top);
-        const int r = warp * 32 + lane, f = 141 + ev[r] - top;
-        sc[SP_KEYS + r] = f >= 1 ? __uint_as_float((uint32_t) f << 23) : 0.f;
-        if (r < 4) sc[2 * SP_KEYS + r] = __uint_as_float((uint32_t) (top - 27) << 23);
+        low = __reduce_min_sync(0xffffffffu, low);
+        const int r = warp * 32 + lane, f = 141 + max(abs(ev[r]), 28) - top;
+        sc[SP_KEYS + r] = __uint_as_float((f >= 1 ? (uint32_t) f << 23 : 0u) | (ev[r] < 0 ? 0x80000000u : 0u));   // sign: something that is no number
+        if (r < 4) sc[3 * SP_KEYS + r] = r == 0 ? (bad ? 1.f : 0.f) : r == 1 ? (top - low > SP_SPREAD ? 1.f : 0.f) : __uint_as_float((uint32_t) (top - 27) << 23);
     }
 }
 
@@ -154,14 +218,37 @@ struct SpCtl {
     uint64_t full[4], empty[4], sc_full[2], sc_empty[2], s_full[2], p_full[2], o_full[2], o_free[2];
     uint32_t tmem_base;
     int abort;
-    float row_max[2][2][128];      // [tile parity][half of the keys][row]
+    float2 row_max[2][2][128];     // [tile parity][half of the keys][row]: largest score, largest exponent of weight x value scale
     float q_scale[128];
     float row_l[2][128];
+    alignas(16) float ones[64];
 };
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// what column d of the values a query sees holds besides numbers, added up (0: nothing).  tiles: the entry's and kv head's first split tile
+__device__ __noinline__ float not_numbers(const SplitParams & P, const uint8_t * tiles, int e, int kvh, int qi, int d) {
+    const AttnIO & io = P.io;
+    const int64_t tile_bytes = sp_tile_bytes(P.nd, P.nv), row0 = io.kv_slot ? 0 : P.off[e];
+    const float * vb = io.v + (io.kv_slot ? (int64_t) io.kv_slot[e] * io.kv_slot_stride : row0 * io.ldv) + (int64_t) kvh * P.a.vdim + d;
+    const int lo = attn_first_visible(P.a, qi);
+    float sum = 0.f;
+    for (int tile = 0; tile * SP_KEYS <= qi; tile++) {
+        const float * sc = reinterpret_cast<const float *>(tiles + tile * tile_bytes + P.nd * SP_K_UNIT + 2 * sp_v_unit(P.nv));
+        if (sc[3 * SP_KEYS] == 0.f) continue;
+        for (int r = 0; r < SP_KEYS; r++) {
+            const int j = tile * SP_KEYS + r;
+            if (j <= qi && (j >= lo || j < P.a.keep_first) && (__float_as_uint(sc[SP_KEYS + r]) >> 31)) {
+                const float v = vb[(int64_t) j * io.ldv];
+                if (!(fabsf(v) < INFINITY)) sum += v;
+            }
+        }
+    }
+    return sum;
+}
+// 2^d for an integer d <= 0 (0 from 2^-127 on, and for what is no number)
+__device__ __forceinline__ float pow2_down(float d) { return d > -126.5f ? __uint_as_float((uint32_t) (127 + (int) d) << 23) : 0.f; }
 __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int h, int d, int DV) {
     if (io.gate_mode == 1) return sigmoid_f(io.gate[row * io.ldg + h]);
     if (io.gate_mode == 2) return sigmoid_f(io.gate[row * io.ldg + (int64_t) h * DV + d]);
@@ -174,7 +261,8 @@ __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int
 //   warp 1       MMA issuer, owner of the tensor memory; S(j + 1) goes before P(j) V(j)
 //   warps 2 - 9  softmax: thread = (row, half of the tile's keys); the weighted sum [row][half of the value columns] in registers
 // Bound: 24 MMAs of 107 clocks for S (operand A from shared memory) and 24 of 74 for P V a 128 x 128 tile of 128-wide heads, 4300 clocks; the
-// softmax warps take about half of that. 
+// softmax warps take about half of that.  Their 64 scores and 64 sums a thread do not fit 168 registers (ten warps to an SM): 170 to 180
+// bytes of them go through local memory once a tile.
 template <typename OT, bool CAP>
 __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_constant__ SplitParams P) {
     pdl_enter();
@@ -208,6 +296,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         ctl->abort = 0;
         mbar_fence_init();
     }
+    if (threadIdx.x < 64) ctl->ones[threadIdx.x] = 1.f;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -234,7 +323,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
 #pragma unroll
                 for (int c = 0; c < SP_MAX_ND; c++)
 #pragma unroll
-                    for (int i = 0; i < 2; i++) m = max(m, __float_as_uint(x[j][c][i]) & 0x7fffffffu);
+                    for (int i = 0; i < 2; i++) m = max(m, magnitude(x[j][c][i]));
                 m = __reduce_max_sync(0xffffffffu, m);
                 int eq;
                 const float s = split_scale(m, 14, eq);
@@ -296,26 +385,30 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         const uint64_t dq = desc_sw128(smem_u32(q_s));
         const uint32_t q_lo = (uint32_t) (q_piece >> 4);
         int u = 0;
+        // the small products of all units go first: what the tensor cores cut off at each step is a share of the sum so far
         auto scores = [&](int j) {
             const uint32_t d = tmem + (uint32_t) ((j & 1) * 128);
-            for (int c = 0; c < nd; c++, u++) {
-                const int s = u % stages;
-                mbar_wait(&ctl->full[s], (uint32_t) ((u / stages) & 1), cta_abort, P.abort_flag);
-                __syncwarp();
-                fence_after();
-                const uint64_t hk = desc_sw128(smem_u32(ring + s * SP_K_UNIT)), lk = hk + (SP_K_UNIT / 2 >> 4), hq = dq + c * (16384 >> 4), lq = hq + q_lo;
-                if (elect_one()) {
+            for (int c = 0; c < nd; c++) mbar_wait(&ctl->full[(u + c) % stages], (uint32_t) (((u + c) / stages) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            if (elect_one()) {
+                for (int c = 0; c < nd; c++) {
+                    const uint64_t hk = desc_sw128(smem_u32(ring + (u + c) % stages * SP_K_UNIT)), lk = hk + (SP_K_UNIT / 2 >> 4), hq = dq + c * (16384 >> 4), lq = hq + q_lo;
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16<1>(d, lq + 2 * k, hk + 2 * k, idesc, (uint32_t) ((c | k) != 0));
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, lk + 2 * k, idesc, 1u);
+                }
+                for (int c = 0; c < nd; c++) {
+                    const uint64_t hk = desc_sw128(smem_u32(ring + (u + c) % stages * SP_K_UNIT)), hq = dq + c * (16384 >> 4);
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, hk + 2 * k, idesc, 1u);
-                    mma_commit(&ctl->empty[s]);
-                    if (c == nd - 1) mma_commit(&ctl->s_full[j & 1]);
+                    mma_commit(&ctl->empty[(u + c) % stages]);
                 }
-                __syncwarp();
+                mma_commit(&ctl->s_full[j & 1]);
             }
+            __syncwarp();
+            u += nd;
         };
         scores(0);
         for (int j = 0; j < nt && !*cta_abort; j++) {
@@ -325,25 +418,31 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
             if (j >= 2) mbar_wait(&ctl->o_free[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
             __syncwarp();
             const uint32_t d = tmem + O0 + (uint32_t) (buf * 128);
-            for (int h = 0; h < 2; h++, u++) {
-                const int s = u % stages;
-                mbar_wait(&ctl->full[s], (uint32_t) ((u / stages) & 1), cta_abort, P.abort_flag);
-                __syncwarp();
-                fence_after();
-                const uint64_t hv = desc_sw128_mn(smem_u32(ring + s * SP_K_UNIT), 8192), lv = hv + (v_unit / 2 >> 4);
-                const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);          // 16 columns hi, 16 columns lo of 32 keys, then the next 32
-                if (elect_one()) {
+            for (int h = 0; h < 2; h++) mbar_wait(&ctl->full[(u + h) % stages], (uint32_t) (((u + h) / stages) & 1), cta_abort, P.abort_flag);
+            __syncwarp();
+            fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint64_t hv = desc_sw128_mn(smem_u32(ring + (u + h) % stages * SP_K_UNIT), 8192), lv = hv + (v_unit / 2 >> 4);
+                    const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);      // 16 columns hi, 16 columns lo of 32 keys, then the next 32
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + 16 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, (uint32_t) ((h | k) != 0));
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, lv + k * (2048 >> 4), idesc_v, 1u);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint64_t hv = desc_sw128_mn(smem_u32(ring + (u + h) % stages * SP_K_UNIT), 8192);
+                    const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, 1u);
-                    mma_commit(&ctl->empty[s]);
-                    if (h == 1) mma_commit(&ctl->o_full[buf]);
+                    mma_commit(&ctl->empty[(u + h) % stages]);
                 }
-                __syncwarp();
+                mma_commit(&ctl->o_full[buf]);
             }
+            __syncwarp();
+            u += 2;
         }
         __syncwarp();
     } else {
@@ -353,9 +452,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         const int h = kvh * P.gqa + (row < rows ? row % P.gqa : 0);
         const uint32_t mine = tmem + ((uint32_t) (quad * 32) << 16);
         constexpr float LOG2E = 1.4426950408889634f;
-        const float qs = CAP ? ctl->q_scale[row] * a.scale / a.softcap : ctl->q_scale[row] * a.scale * LOG2E, cap = a.softcap * LOG2E;
+        const float qs = CAP ? ctl->q_scale[row] * a.scale / a.softcap : ctl->q_scale[row] * a.scale, cap = a.softcap;
         const int all_from = attn_first_visible(a, q0 + toks - 1), all_to = q0;   // positions in [all_from, all_to] are visible to every row
         float o[64], m = -INFINITY, l = 0.f, corr1 = 0.f, f1 = 0.f;
+        bool bad = false;
 #pragma unroll
         for (int i = 0; i < 64; i++) o[i] = 0.f;
         auto add_tile = [&](int j, float corr, float f) {                        // o = o * corr + f * (tile j's weighted sum)
@@ -390,8 +490,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
             TMEM_LD32(at, v);
             TMEM_LD32(at + 32, v + 32);
             tmem_wait_ld();
-            const bool every = k0 >= all_from && k0 + 63 <= all_to;
-            float tm = -INFINITY;
+            // every row sees the whole tile, and its values lie within 2^12 of one another: their scales relative to the tile's largest go into the
+            // weights as they are.  Else a row's scales follow the largest product weight x power of two among the positions that it sees
+            const float * tail = scales + buf * (SP_SCALES / 4) + 3 * SP_KEYS;
+            const int tile0 = tile_of(j) * SP_KEYS;
+            const bool whole = tile0 >= all_from && tile0 + SP_KEYS - 1 <= all_to, plain = whole && tail[1] == 0.f;
+            float tm = -INFINITY, tw = -INFINITY;
 #pragma unroll
             for (int i = 0; i < 64; i += 4) {
                 const float4 s4 = *reinterpret_cast<const float4 *>(sc + i);
@@ -400,7 +504,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
                 for (int q = 0; q < 4; q++) {
                     float x = t[i + q] * f[q] * qs;
                     if constexpr (CAP) x = cap * tanhf(x);
-                    if (!every) {
+                    if (!whole) {
                         const int kj = k0 + i + q;
                         if (!(kj <= qi && (kj >= lo_q || kj < a.keep_first))) x = -INFINITY;
                     }
@@ -408,25 +512,52 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
                     tm = fmaxf(tm, x);
                 }
             }
-            ctl->row_max[buf][part][row] = tm;
+            if (!plain) {
+#pragma unroll
+                for (int i = 0; i < 64; i += 4) {
+                    const float4 w4 = *reinterpret_cast<const float4 *>(sc + 2 * SP_KEYS + i);
+                    tw = fmaxf(fmaxf(fmaxf(tw, fmaf(t[i], LOG2E, w4.x)), fmaxf(fmaf(t[i + 1], LOG2E, w4.y), fmaf(t[i + 2], LOG2E, w4.z))), fmaf(t[i + 3], LOG2E, w4.w));
+                }
+            }
+            ctl->row_max[buf][part][row] = make_float2(tm, tw);
             asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
-            const float mn = fmaxf(m, fmaxf(tm, ctl->row_max[buf][part ^ 1][row]));
-            const float ref = mn == -INFINITY ? 0.f : mn;
-            const float corr = m == -INFINITY ? 0.f : ex2(m - ref);
-            float e4[4] = {0.f, 0.f, 0.f, 0.f};
+            const float2 other = ctl->row_max[buf][part ^ 1][row];
+            // the exponentials are powers of two, references whole numbers: what joins tiles is exact
+            const float here = ceilf(fmaxf(tm, other.x) * LOG2E), mn = fmaxf(m, here), ref = here == -INFINITY ? 0.f : here;
+            const float corr = pow2_down(m - mn), part_f = pow2_down(here - mn);
+            int top = 0;
+            float e4[4] = {0.f, 0.f, 0.f, 0.f}, sum = 0.f;
+            if (!plain) {   // the exponents of the weights' own sum, then those of the products weight x power of two in their place
+                top = max(__float2int_ru(fmaxf(tw, other.y) - ref), -99);
+                const float lift = (float) (14 - top);
+#pragma unroll
+                for (int i = 0; i < 64; i += 4) {
+                    const float4 w4 = *reinterpret_cast<const float4 *>(sc + 2 * SP_KEYS + i);
+                    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const float y = fmaf(t[i + q], LOG2E, -ref);
+                        e4[q] += ex2(y);
+                        t[i + q] = y + (w[q] + lift);
+                    }
+                }
+                sum = (e4[0] + e4[1]) + (e4[2] + e4[3]);
+            }
+            const float * ratio = plain ? sc + SP_KEYS : ctl->ones;
+            const float slope = plain ? LOG2E : 1.f, offset = plain ? -ref : 0.f;
 #pragma unroll
             for (int c = 0; c < 64; c += 32) {
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                    const float4 r4 = *reinterpret_cast<const float4 *>(sc + SP_KEYS + c + i);
+                    const float4 r4 = *reinterpret_cast<const float4 *>(ratio + c + i);
                     const float r[4] = {r4.x, r4.y, r4.z, r4.w};
                     float p[4];
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        p[q] = ex2(t[c + i + q] - ref);
+                        p[q] = ex2(fmaf(t[c + i + q], slope, offset));
                         e4[q] += p[q];
-                        p[q] *= r[q];
+                        p[q] *= fabsf(r[q]);
                     }
                     split2(p[0], p[1], hi[i / 2], lo[i / 2]);
                     split2(p[2], p[3], hi[i / 2 + 1], lo[i / 2 + 1]);
@@ -434,12 +565,14 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
                 TMEM_ST16(at + c, hi);
                 TMEM_ST16(at + c + 16, lo);
             }
+            if (plain) sum = (e4[0] + e4[1]) + (e4[2] + e4[3]);
             tmem_wait_st();
-            const float f = scales[buf * (SP_SCALES / 4) + 2 * SP_KEYS];
+            const float f = (plain ? tail[2] : __uint_as_float((uint32_t) (top + 100) << 23)) * part_f;   // of the sums: 2^(top - 14 - 13)
+            bad = bad || tail[0] != 0.f;
             fence_before();
             __syncwarp();
             if (lane == 0) { mbar_arrive(&ctl->p_full[buf]); mbar_arrive(&ctl->sc_empty[buf]); }
-            l = l * corr + ((e4[0] + e4[1]) + (e4[2] + e4[3]));
+            l = l * corr + sum * part_f;
             m = mn;
             if (j > 0) add_tile(j - 1, corr1, f1);
             corr1 = corr;
@@ -449,7 +582,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         ctl->row_l[part][row] = l;
         asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
         l = ctl->row_l[0][row] + ctl->row_l[1][row];
-        if (a.sink && m != -INFINITY) l += ex2((io.sink ? io.sink[h] : 0.f) * LOG2E - m);
+        if (a.sink && m != -INFINITY) l += ex2(fmaf(io.sink ? io.sink[h] : 0.f, LOG2E, -m));
         const float inv = l > 0.f ? 1.f / l : 0.f;
         // through the ring's memory (every unit has been used; a row's 16-byte pieces rotated by the row), so that a warp stores whole rows
         float * os = reinterpret_cast<float *>(ring);
@@ -467,6 +600,19 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
             for (int c = 0; c < 128; c += 32) {
                 const int d = c + lane;
                 if (d < DV) put((OT *) P.out, tok * ((int64_t) a.heads * DV) + (int64_t) hh * DV + d, os[r * 128 + (((d >> 2) + r) & 31) * 4 + (d & 3)] * gate_factor(io, tok, hh, d, DV));
+            }
+        }
+        if (bad) {   // what is no number among the values that a row sees is its result
+            __syncwarp();   // over what other lanes have stored
+            const uint8_t * tiles = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
+#pragma unroll 1
+            for (int i = lane; i < 16 * DV; i += 32) {
+                const int r = w * 16 + i / DV, d = i % DV;
+                if (r >= rows) break;
+                const int64_t tok = t_begin + q0 + r / P.gqa;
+                const int hh = kvh * P.gqa + r % P.gqa;
+                const float y = not_numbers(P, tiles, e, kvh, q0 + r / P.gqa, d);
+                if (!(fabsf(y) < INFINITY)) put((OT *) P.out, tok * ((int64_t) a.heads * DV) + (int64_t) hh * DV + d, y * gate_factor(io, tok, hh, d, DV));
             }
         }
     }

@@ -107,3 +107,65 @@ def test_bfloat16_models_take_it_by_default(pkg, cuda, monkeypatch):
     out = m.batch_step([(m.seq_alloc(), t, list(range(len(t)))) for t in prompts])[0]
     m.close()
     assert np.array_equal(out, got.astype(np.float32))
+
+
+def loud_prompt(kind, power, tokens=128):
+    """Tokens of which only the one at position 100 has something in the first width entry, which the value product (power of two, or an overflow into one
+    infinite value) alone reads.  NaN: that token's embedding, hence its query, key and value, is no number."""
+    R, cfg = ludusun(dict(att(4, 2, 64), scale=1.0))
+    bits, W = R.random_weights(cfg, seed=11)
+    emb, v = W["embed"].copy(), W["l0.mix.v"].copy()
+    emb[:, 0] = 0.0
+    emb[5, 0] = 8.0 * 128 ** -0.5
+    v[:, 0] = 2.0 ** power * np.sign(v[:, 0]) if kind == "loud" else 0.0
+    if kind == "inf":
+        v[70, 0] = 3e38
+    for n, w in (("embed", emb), ("l0.mix.v", v)) + tuple(("l0.mix." + n, np.where(np.arange(128) == 0, 0.0, W["l0.mix." + n])) for n in "qk"):
+        R.set_weight(bits, W, n, w)
+    if kind == "nan":
+        bits["embed"] = bits["embed"].copy()
+        bits["embed"].reshape(64, 128)[5] = 0x7fc0
+    toks = np.random.default_rng(6).integers(6, 64, tokens)
+    return R, cfg, bits, W, toks
+
+
+def scored(pkg, cfg, bits, toks, dtype):
+    m = pkg.Model.from_config(cfg, dtype=dtype, n_ctx=len(toks), n_seq=1)
+    for k, b in bits.items():
+        m.set_tensor(k, 30, b)
+    m.finalize()
+    out = m.batch_step([(m.seq_alloc(), toks.tolist(), list(range(len(toks))))])[0]
+    m.close()
+    return np.delete(out, 5, axis=1)   # token 5's own logit reads its embedding
+
+
+@pytest.mark.parametrize("kind,power", [("loud", 12), ("loud", 24), ("loud", 40), ("loud", 100), ("inf", 0), ("nan", 0)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_value_that_a_query_does_not_see_does_not_touch_its_row(pkg, cuda, monkeypatch, kind, power, dtype):
+    monkeypatch.setenv("PB200_ATTN_SPLIT", "1")
+    R, cfg, bits, W, toks = loud_prompt(kind, power)
+    clean = scored(pkg, cfg, bits, toks, dtype)
+    toks[100] = 5
+    got = scored(pkg, cfg, bits, toks, dtype)
+    assert np.array_equal(got[:100], clean[:100])
+    assert not np.array_equal(got[100:], clean[100:])
+    if dtype == "float32":
+        want = np.delete(R.forward(cfg, W, toks[:100])[0], 5, axis=1)
+        assert np.linalg.norm(got[:100] - want) <= 2e-6 * np.linalg.norm(want)
+    if kind != "loud":   # one column of one kv head; the product behind it spreads it over the whole row
+        assert not np.isfinite(got[100:]).any()
+
+
+@pytest.mark.parametrize("power", [6, 12, 20, 28, 36])
+def test_a_loud_value_of_small_weight(pkg, cuda, monkeypatch, power):
+    """Scores spread over tens of binades: whatever weight the loud value has, a row is as close to float64 as with the FMA kernel, in the tile with
+    rows that do not see it and behind."""
+    R, cfg, bits, W, toks = loud_prompt("loud", power, 300)
+    toks[100] = 5
+    want = np.delete(R.forward(cfg, W, toks)[0], 5, axis=1)
+    off = {}
+    for split in "01":
+        monkeypatch.setenv("PB200_ATTN_SPLIT", split)
+        got = scored(pkg, cfg, bits, toks, "float32").astype(np.float64)
+        off[split] = np.sqrt(np.mean(np.sum((got - want) ** 2, axis=1) / np.sum(want ** 2, axis=1)))
+    assert off["1"] <= 1.2 * off["0"] + 5e-8, off
