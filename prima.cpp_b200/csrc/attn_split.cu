@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "launch.h"
@@ -42,7 +43,7 @@ struct SplitParams {
     AttnParams a;
     const int32_t * off;
     uint8_t * ws;              // [kv head][tile slot][sp_tile_bytes]; entry e's first slot: off[e] / 128 + e
-    int slots;
+    int slots, kv_first;       // kv heads go through the scratch in groups: this launch's first one
     void * out;
     int nd, nv, gqa, tok_per_cta, stages;
     int * abort_flag;
@@ -78,7 +79,7 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t & hi, uint32_t
 __global__ void __launch_bounds__(256, 2) k_split_kv(const __grid_constant__ SplitParams P) {
     __shared__ int ev[SP_KEYS];        // exponents, -: the row holds something that is no number, 0: nothing but zeros
     pdl_enter();
-    const int e = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x;
+    const int e = blockIdx.z, kvh = P.kv_first + blockIdx.y, tile = blockIdx.x;
     const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
     if (tile * SP_KEYS >= n) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(256, 2) k_split_kv(const __grid_constant__ Spl
     const float * kb = io.k + (io.kv_slot ? at : (int64_t) t_begin * io.ldk) + (int64_t) kvh * DN;
     const float * vb = io.v + (io.kv_slot ? at : (int64_t) t_begin * io.ldv) + (int64_t) kvh * DV;
     const float * ks = io.ks ? io.ks + (int64_t) t_begin * io.ldks : nullptr;
-    uint8_t * dst = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e + tile) * sp_tile_bytes(P.nd, P.nv);
+    uint8_t * dst = P.ws + ((int64_t) blockIdx.y * P.slots + t_begin / SP_KEYS + e + tile) * sp_tile_bytes(P.nd, P.nv);
     uint8_t * dv = dst + P.nd * SP_K_UNIT;
     float * sc = reinterpret_cast<float *>(dv + 2 * sp_v_unit(P.nv));
     const int blk_b = sp_v_unit(P.nv) / 2;                         // the lo half of a unit of values
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
     extern __shared__ uint8_t smem_raw[];
     const AttnIO & io = P.io;
     const AttnParams & a = P.a;
-    const int e = blockIdx.z, kvh = blockIdx.x;
+    const int e = blockIdx.z, kvh = P.kv_first + blockIdx.x;
     const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
     const int q0 = ((int) gridDim.y - 1 - (int) blockIdx.y) * P.tok_per_cta;      // long rows first
     if (q0 >= n) return;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
     constexpr uint32_t O0 = 256;
 
     if (warp == 0) {
-        const uint8_t * src0 = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
+        const uint8_t * src0 = P.ws + ((int64_t) blockIdx.x * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
         int u = 0;
         auto load = [&](const uint8_t * src, uint32_t bytes) {
             const int s = u % stages;
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         }
         if (bad) {   // what is no number among the values that a row sees is its result
             __syncwarp();   // over what other lanes have stored
-            const uint8_t * tiles = P.ws + ((int64_t) kvh * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
+            const uint8_t * tiles = P.ws + ((int64_t) blockIdx.x * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
 #pragma unroll 1
             for (int i = lane; i < 16 * DV; i += 32) {
                 const int r = w * 16 + i / DV, d = i % DV;
@@ -635,15 +636,23 @@ int split_slots(int n_tokens, int n_entries) { return n_tokens / SP_KEYS + n_ent
 
 }  // namespace
 
-// scratch that a batch of n_tokens prompt tokens in up to n_tokens / 128 + 16 entries needs
-size_t attn_split_bytes(const AttnParams & a, int n_tokens) {
-    if (a.dim > 64 * SP_MAX_ND || a.vdim > 64 * SP_MAX_NV || a.dim <= 0 || a.vdim <= 0 || a.kv_heads <= 0) return 0;
-    return (size_t) a.kv_heads * (size_t) split_slots(n_tokens, n_tokens / SP_KEYS + 16) * (size_t) sp_tile_bytes((a.dim + 63) / 64, (a.vdim + 63) / 64);
+// Scratch of one kv head; all heads at once up to SP_SCRATCH bytes (2000 tiles of 128-wide heads: far more CTAs than SMs), beyond that in groups.
+constexpr size_t SP_SCRATCH = (size_t) 256 << 20;
+static bool split_shape(const AttnParams & a) {
+    return a.dim > 0 && a.dim <= 64 * SP_MAX_ND && a.vdim > 0 && a.vdim <= 64 * SP_MAX_NV && a.kv_heads > 0 && a.heads % a.kv_heads == 0 && a.heads / a.kv_heads <= 128;
+}
+static size_t split_head_bytes(const AttnParams & a, int n_tokens, int n_entries) {
+    return (size_t) split_slots(n_tokens, n_entries) * (size_t) sp_tile_bytes((a.dim + 63) / 64, (a.vdim + 63) / 64);
+}
+size_t attn_split_bytes(const AttnParams & a, int n_tokens, int n_entries) {
+    if (!split_shape(a)) return 0;
+    const size_t head = split_head_bytes(a, n_tokens, n_entries);
+    return head * std::min<size_t>((size_t) a.kv_heads, std::max<size_t>(1, SP_SCRATCH / head));
 }
 bool attn_split_ok(const AttnIO & io, const BatchView & b, const AttnParams & a) {
-    if (!io.split_ws || a.dim > 64 * SP_MAX_ND || a.vdim > 64 * SP_MAX_NV || a.heads / a.kv_heads > 128 || b.n_entries > 65535) return false;
-    const size_t need = (size_t) a.kv_heads * (size_t) split_slots(b.n_tokens, b.n_entries) * (size_t) sp_tile_bytes((a.dim + 63) / 64, (a.vdim + 63) / 64);
-    return need <= io.split_bytes;
+    if (!io.split_ws || !split_shape(a) || b.n_entries > 65535) return false;
+    const int tok_per_cta = 128 / (a.heads / a.kv_heads);
+    return (b.max_n - 1) / tok_per_cta < 65535 && attn_split_bytes(a, b.n_tokens, b.n_entries) <= io.split_bytes;   // a grid's second dimension
 }
 int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t st) {
     SplitParams P{};
@@ -656,13 +665,19 @@ int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams &
     P.tok_per_cta = 128 / P.gqa;
     P.stages = P.nd == 3 ? 3 : 4;
     P.abort_flag = abort_flag();
-    g_launches += 2;
-    const int rc = launch_dep(k_split_kv, dim3((unsigned) ((b.max_n + SP_KEYS - 1) / SP_KEYS), (unsigned) a.kv_heads, (unsigned) b.n_entries), dim3(256), 0, st, P);
-    if (rc) return rc;
+    const int group = (int) (attn_split_bytes(a, b.n_tokens, b.n_entries) / split_head_bytes(a, b.n_tokens, b.n_entries));
     const size_t smem = 1024 + (size_t) P.nd * 32768 + (size_t) P.stages * SP_K_UNIT + 2 * SP_SCALES + sizeof(SpCtl);
-    const dim3 grid((unsigned) a.kv_heads, (unsigned) ((b.max_n + P.tok_per_cta - 1) / P.tok_per_cta), (unsigned) b.n_entries);
-    if (otype == T_BF16) return a.softcap > 0.f ? launch_typed<__nv_bfloat16, true>(P, grid, smem, st) : launch_typed<__nv_bfloat16, false>(P, grid, smem, st);
-    return a.softcap > 0.f ? launch_typed<float, true>(P, grid, smem, st) : launch_typed<float, false>(P, grid, smem, st);
+    for (P.kv_first = 0; P.kv_first < a.kv_heads; P.kv_first += group) {
+        const unsigned heads = (unsigned) std::min(group, a.kv_heads - P.kv_first);
+        g_launches += 2;
+        int rc = launch_dep(k_split_kv, dim3((unsigned) ((b.max_n + SP_KEYS - 1) / SP_KEYS), heads, (unsigned) b.n_entries), dim3(256), 0, st, P);
+        if (rc) return rc;
+        const dim3 grid(heads, (unsigned) ((b.max_n + P.tok_per_cta - 1) / P.tok_per_cta), (unsigned) b.n_entries);
+        if (otype == T_BF16) rc = a.softcap > 0.f ? launch_typed<__nv_bfloat16, true>(P, grid, smem, st) : launch_typed<__nv_bfloat16, false>(P, grid, smem, st);
+        else rc = a.softcap > 0.f ? launch_typed<float, true>(P, grid, smem, st) : launch_typed<float, false>(P, grid, smem, st);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 }  // namespace pb

@@ -218,8 +218,8 @@ struct LayerList {
     float *x = nullptr, *x0 = nullptr, *xalt = nullptr, *big = nullptr, *msub = nullptr, *xbc = nullptr, *yssm = nullptr, *logits = nullptr;
     void *act = nullptr, *act2 = nullptr, *actw = nullptr;
     // FRAME_PRENORM and its mixers: results of all layers [layers + 1][capT][width]; further fp32 and operand-type scratch
-    void * split_ws = nullptr;      // split keys and values of a prompt (attn_split.cu); bf16 models with an attention layer that fits
-    size_t split_bytes = 0;
+    void * split_ws = nullptr;      // split keys and values of a prompt (attn_split.cu); bf16 models with an attention layer that fits, none where
+    size_t split_bytes = 0;         // memory does not suffice (prompts then keep the fp32 FMA attention)
     float *hist = nullptr, *big2 = nullptr, *big3 = nullptr, *big4 = nullptr, *krb = nullptr;
     float * lat_part = nullptr;     // partial results of the split decode attention kernels: latent [entries][splits][heads][kv_rank + 2], windowed [entries][heads][splits][vdim + 2]
     size_t lat_part_cap = 0;
@@ -1816,6 +1816,7 @@ void ll_free(pb200_model * m) {
     if (ll->logits_host) cudaFreeHost(ll->logits_host);
     if (ll->moe_count_host) cudaFreeHost(ll->moe_count_host);
     if (ll->lat_part) cudaFree(ll->lat_part);
+    if (ll->split_ws) cudaFree(ll->split_ws);
     if (ll->tap) cudaFree(ll->tap);
     for (cudaEvent_t e : ll->prof_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ll->ev_rows) if (e) cudaEventDestroy(e);
@@ -1859,7 +1860,8 @@ static void ll_drop_graphs(LayerList & ll) {
         if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     ll.graphs.clear();
 }
-static int ll_reserve(pb200_model * m, int T, int nW, int nE) {
+// long_prompt: a prompt batch with an entry beyond 16 tokens
+static int ll_reserve(pb200_model * m, int T, int nW, int nE, bool long_prompt) {
     LayerList & ll = *m->ll;
     const bool grow = T > ll.capT || nW > ll.capW || (size_t) 2 * T + 4 * (size_t) nE + 1 + (size_t) nW + 64 > ll.meta_cap;
     if (grow) ll_drop_graphs(ll);   // captured steps hold the addresses of buffers that are about to move
@@ -1867,6 +1869,8 @@ static int ll_reserve(pb200_model * m, int T, int nW, int nE) {
         CK(cudaStreamSynchronize(m->stream));
         for (void * p : ll.scratch) cudaFree(p);
         ll.scratch.clear();
+        if (ll.split_ws) cudaFree(ll.split_ws);   // what a pass can do without is taken last
+        ll.split_ws = nullptr; ll.split_bytes = 0;
         const int cT = std::max(T, ll.capT), cW = std::max(nW, ll.capW);
         ll.capT = ll.capW = 0;
         int64_t maxact = ll.width, maxact2 = ll.width, maxbig = ll.width, maxch = 1, maxinner = 1, maxb2 = 0, maxb3 = 0, maxb4 = 0, maxkr = 0;
@@ -1957,21 +1961,6 @@ static int ll_reserve(pb200_model * m, int T, int nW, int nE) {
             if (!ll.moe_count_host) CK(cudaMallocHost((void **) &ll.moe_count_host, (size_t) 2 * 4096 * 4));
         }
         CK(grab(&ll.actw, (size_t) cW * W * es));
-        ll.split_ws = nullptr; ll.split_bytes = 0;
-        // PB200_ATTN_SPLIT: 0 = prompts keep the fp32 FMA attention, 1 = float32 models take the split kernel as well (A/B runs, tests)
-        const char * sp = getenv("PB200_ATTN_SPLIT");
-        if (cT > 16 && (sp ? atoi(sp) != 0 : ll.ctype == T_BF16)) {
-            size_t need = 0;
-            for (const LLayer & L : ll.layers) {
-                AttnParams ap = L.att;
-                if (L.weights_of >= 0) continue;
-                if (L.kind == MIX_LATENT) { ap.kv_heads = L.lat.heads; ap.dim = L.lat.dim + L.lat.rot_dim; ap.vdim = L.lat.vdim; }
-                else if (L.kind != MIX_ATTENTION && L.kind != MIX_DUAL) continue;
-                need = std::max(need, attn_split_bytes(ap, cT));
-            }
-            if (need) CK(grab(&ll.split_ws, need));
-            ll.split_bytes = need;
-        }
         CK(grab((void **) &ll.logits, (size_t) cW * (size_t) ll.vocab * 4));
         CK(grab((void **) &ll.greedy_dev, (size_t) cW * 4));
         if (ll.greedy_host) cudaFreeHost(ll.greedy_host);
@@ -2012,6 +2001,25 @@ static int ll_reserve(pb200_model * m, int T, int nW, int nE) {
         ll.logits_host = nullptr; ll.logits_host_cap = 0;
         CK(cudaMallocHost((void **) &ll.logits_host, need_lh * 4));
         ll.logits_host_cap = need_lh;
+    }
+    // scratch of the split prompt attention by this call's own tokens and entries: which kernel runs does not depend on what ran before.
+    // PB200_ATTN_SPLIT: 0 = prompts keep the fp32 FMA attention, 1 = float32 models take the split kernel as well (A/B runs, tests)
+    const char * sp = getenv("PB200_ATTN_SPLIT");
+    if (long_prompt && (sp ? atoi(sp) != 0 : ll.ctype == T_BF16)) {
+        size_t need = 0;
+        for (const LLayer & L : ll.layers) {
+            AttnParams ap = L.att;
+            if (L.weights_of >= 0) continue;
+            if (L.kind == MIX_LATENT) { ap.kv_heads = L.lat.heads; ap.dim = L.lat.dim + L.lat.rot_dim; ap.vdim = L.lat.vdim; }
+            else if (L.kind != MIX_ATTENTION && L.kind != MIX_DUAL) continue;
+            need = std::max(need, attn_split_bytes(ap, T, nE));
+        }
+        if (need > ll.split_bytes) {
+            CK(cudaStreamSynchronize(m->stream));
+            if (ll.split_ws) cudaFree(ll.split_ws);
+            ll.split_bytes = cudaMalloc(&ll.split_ws, need) == cudaSuccess ? need : 0;
+            if (!ll.split_bytes) { ll.split_ws = nullptr; cudaGetLastError(); }
+        }
     }
     return 0;
 }
@@ -2756,7 +2764,7 @@ static int ll_run_sub(pb200_model * m, std::vector<SubEntry> & es, bool prefill,
     if (!nE) return 0;
     int T = 0, nW = 0, max_n = 0;
     for (const SubEntry & e : es) { T += e.n; nW += (int) e.want.size(); max_n = std::max(max_n, e.n); }
-    CK(ll_reserve(m, T, nW, nE));
+    CK(ll_reserve(m, T, nW, nE, prefill && max_n > 16));
     // meta layout: tokens[T] | entry_of[T] | slot[nE] | off[nE+1] | pos0[nE] | want[nW] | prev[nE]
     int32_t * h = ll.meta_host;
     int32_t *h_tok = h, *h_ent = h + T, *h_slot = h + 2 * T, *h_off = h_slot + nE, *h_pos = h_off + nE + 1, *h_want = h_pos + nE;

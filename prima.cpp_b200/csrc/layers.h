@@ -189,7 +189,7 @@ int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnPara
                           void * out, int otype, cudaStream_t stream, float * part = nullptr);
 
 // prompt attention with every operand as two f16 numbers on the tensor cores (attn_split.cu): head sizes up to 192, value sizes up to 128
-size_t attn_split_bytes(const AttnParams & a, int n_tokens);   // scratch for prompt batches of up to n_tokens tokens (0: the shape is not taken)
+size_t attn_split_bytes(const AttnParams & a, int n_tokens, int n_entries);   // scratch for a prompt batch (0: the shape is not taken)
 bool attn_split_ok(const AttnIO & io, const BatchView & b, const AttnParams & a);
 int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t stream);
 

@@ -169,3 +169,40 @@ def test_a_loud_value_of_small_weight(pkg, cuda, monkeypatch, power):
         got = scored(pkg, cfg, bits, toks, "float32").astype(np.float64)
         off[split] = np.sqrt(np.mean(np.sum((got - want) ** 2, axis=1) / np.sum(want ** 2, axis=1)))
     assert off["1"] <= 1.2 * off["0"] + 5e-8, off
+
+
+def test_equal_calls_give_equal_bits_whatever_ran_before(pkg, cuda, monkeypatch):
+    """Many short prompts in one batch, before and after a larger batch has grown the model's work space; and the kernel that runs is the split one."""
+    R, cfg = CASES["sink, rotation, group of 3"]
+    rng = np.random.default_rng(8)
+    short = [rng.integers(0, 64, 30).tolist() for _ in range(40)]
+    bits, W = R.random_weights(cfg, seed=7)
+    outs = []
+    for split in ("1", "0"):
+        monkeypatch.setenv("PB200_ATTN_SPLIT", split)
+        m = pkg.Model.from_config(cfg, dtype="float32", n_ctx=900, n_seq=41)
+        for k, b in bits.items():
+            m.set_tensor(k, 30, b)
+        m.finalize()
+        for again in range(2):
+            slots = [m.seq_alloc() for _ in short]
+            outs.append(m.batch_step([(s, t, [29]) for s, t in zip(slots, short)])[0])
+            for s in slots:
+                m.seq_free(s)
+            if not again:
+                s = m.seq_alloc()
+                m.batch_step([(s, rng.integers(0, 64, 900).tolist(), [0])])
+                m.seq_free(s)
+        m.close()
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[2], outs[3])
+    assert not np.array_equal(outs[0], outs[2])
+
+
+def test_more_heads_than_the_scratch_holds(pkg, cuda, monkeypatch):
+    """128 key heads of 17 tiles each are 290 MB of split keys and values: they go through the scratch in two groups."""
+    R, cfg = ludusun({"heads": 128, "dim": 128, "vdim": 128, "kv_rank": 32, "q_rank": 32, "scale": 0.1, "mask": {"size": 600}}, "latent_attention")
+    prompts = [np.random.default_rng(9).integers(0, 64, 2100).tolist()]
+    fma, _ = run(pkg, monkeypatch, R, cfg, prompts, "0")
+    split, _ = run(pkg, monkeypatch, R, cfg, prompts, "1")
+    assert not np.array_equal(split, fma)
+    assert np.abs(split - fma).max() < 2e-5 * np.abs(fma).max()
