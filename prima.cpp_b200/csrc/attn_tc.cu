@@ -315,6 +315,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2)
             mbar_wait(&ctl->o_full, 0u, cta_abort, P.abort_flag);
             softmax_barrier();   // every warp has looked through its values
             fence_after();
+        } else {
+            mbar_wait(&ctl->full[0], 0u, cta_abort, P.abort_flag);   // key tile 0 is on its way into the ring all the same
         }
         // the result goes through the ring's memory (every tile has been used; row r's 16-byte pieces rotated by r) so that a warp stores whole rows
         float * os = reinterpret_cast<float *>(ring);

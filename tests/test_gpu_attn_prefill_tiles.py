@@ -91,3 +91,15 @@ def test_a_value_that_is_no_number_stays_with_the_rows_that_see_it(cuda, lib, ba
     assert not bool(torch.isfinite(out[30:, 1, 77]).any())
     out[30:, 1, 77] = clean[30:, 1, 77]
     assert torch.equal(out, clean)
+
+
+def test_tokens_that_see_nothing(cuda, lib):
+    """Whole tiles of queries before the first position: their first key tile is loaded all the same and must not reach the result."""
+    import torch
+    q, k, v = inputs(90, 8, 2, 300, seed=8)
+    pos = torch.arange(200, 290, dtype=torch.int32, device="cuda")
+    pos[32:64] = -1                   # 32 tokens x 4 heads: one CTA's rows
+    for _ in range(20):
+        out = check(lib, q, k, v, pos, 0.1)
+        assert bool((out[32:64] == 0).all())
+        assert bool((run(lib, q, k, v, torch.full_like(pos, -1), 0.1) == 0).all())
