@@ -345,7 +345,8 @@ __global__ void __launch_bounds__(256) k_attn_decode(const float * __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Tiled prompt-processing attention for arrays that the tensor-core kernel (attn_tc.cu) does not take (queries at 4-byte boundaries): one CTA per (kv head, ATT_TQ consecutive tokens; 4, or 2 / 1 for long contexts).  Warp w =
+// Tiled prompt-processing attention for queries at 4-byte boundaries, which the tensor-core kernel (attn_tc.cu) does not take (it reads them by 16
+// bytes); cache and result lie at 16-byte boundaries.  One CTA per (kv head, ATT_TQ consecutive tokens; 4, or 2 / 1 for long contexts).  Warp w =
 // q head w of the GQA group (loops when gqa > 8) for those tokens; K and V stream through shared memory in 32-position tiles and every tile is used by all
 // gqa x 4 query rows (a per-(head, token) grid re-reads K/V for every row: measured L2-bound at 7 TB/s, 0.6 ms per 70B layer at T = 512).  Numerics are the CPU
 // graph's (FA off): q and the probabilities rounded to f16, softmax sum in double; scores of all rows live in shared memory,
@@ -1314,7 +1315,8 @@ int launch_attn_batch(const float * q, const __half * kcache, const __half * vca
     // one kernel for every length, so that a row's bits do not depend on how a prompt is cut (prompts of 32 tokens and less lose 1 to 3 us of 6 by it)
     if (attn_mode == 0 && attn_prefill_tc_ok(q, kcache, vcache, out, n_head, n_head_kv, D, n_kv_max))
         return launch_attn_prefill_tc(q, kcache, vcache, out, n_head, n_head_kv, pos_dev, n_tok, n_kv_max, scale, stream);
-    if ((attn_mode == 0 || attn_mode == 2) && n_head % n_head_kv == 0) {   // tiled kernel: all score rows of gqa x TQ queries in shared memory
+    const uintptr_t at = (uintptr_t) kcache | (uintptr_t) vcache;
+    if ((attn_mode == 0 || attn_mode == 2) && n_head % n_head_kv == 0 && ((at | (uintptr_t) out) & 15) == 0) {   // tiled kernel: all score rows of gqa x TQ queries in shared memory
         const int gqa = n_head / n_head_kv;
         const int n_kv_pad = (n_kv_max + 31) & ~31;
         auto smem_for = [&](int tq) { return (size_t) gqa * tq * n_kv_pad * 4 + (size_t) gqa * tq * D * 4 + (size_t) ATT_TK * ATT_KSTRIDE * 2; };
@@ -1334,6 +1336,8 @@ int launch_attn_batch(const float * q, const __half * kcache, const __half * vca
             return (int) cudaGetLastError();
         }
     }
+    // the per-(head, token) kernel reads queries by 16 bytes and the cache by 8: what is laid out otherwise no kernel here takes
+    if (((uintptr_t) q & 15) != 0 || (at & 7) != 0) return (int) cudaErrorInvalidValue;
     const size_t smem = ((size_t) ((n_kv_max + 31) & ~31) + 8 * 128) * sizeof(float);
     {
         cudaError_t e = ensure_dyn_smem(g_attn_attr, (const void *) k_attn_decode, smem, false);

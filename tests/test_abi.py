@@ -50,6 +50,14 @@ def test_argument_validation_no_gpu(lib, pkg):
     assert c.pb200_attn_prefill(None, None, None, None, 8, 2, 128, None, 4, 4, 0.1, None) == -1
 
 
+def test_attn_prefill_refuses_what_no_kernel_reads(lib):
+    """Queries at 4-byte boundaries: up to what the tiled kernel's shared memory holds.  A cache at less than 8 bytes: never.  Refused before any launch."""
+    base = 1 << 20
+    args = lambda q, k, v, n_kv: (base + q, base + k, base + v, base, 16, 2, 128, base, 4, n_kv, 0.1, None)   # noqa: E731
+    for a in [(4, 0, 0, 50000), (4, 8, 0, 64), (0, 2, 0, 64), (0, 0, 4, 64), (8, 0, 8, 64)]:
+        assert lib.c.pb200_attn_prefill(*args(*a)) == 1, a   # cudaErrorInvalidValue
+
+
 def test_hparams_layout_matches_header(pkg):
     assert C.sizeof(pkg.HParams) == 10 * 4 + 3 * 4
 

@@ -103,3 +103,16 @@ def test_tokens_that_see_nothing(cuda, lib):
         out = check(lib, q, k, v, pos, 0.1)
         assert bool((out[32:64] == 0).all())
         assert bool((run(lib, q, k, v, torch.full_like(pos, -1), 0.1) == 0).all())
+
+
+@pytest.mark.parametrize("H,G,T,pos0", [(8, 2, 21, 5), (16, 2, 6, 1790), (64, 8, 9, 120)])
+@pytest.mark.parametrize("q_off,kv_off", [(1, 0), (0, 4)], ids=["queries at 4 bytes: tiled kernel", "cache at 8 bytes: one CTA per head and token"])
+def test_other_alignments(cuda, lib, H, G, T, pos0, q_off, kv_off):
+    import torch
+    q, k, v = inputs(T, H, G, pos0 + T)
+
+    def shifted(t, by):
+        flat = torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")
+        flat[by:by + t.numel()] = t.reshape(-1)
+        return flat[by:by + t.numel()].view(t.shape)
+    check(lib, shifted(q, q_off), shifted(k, kv_off), shifted(v, kv_off), torch.arange(pos0, pos0 + T, dtype=torch.int32, device="cuda"), 128 ** -0.5)

@@ -211,10 +211,10 @@ def test_attn_decode(cuda, lib, port, n_kv):
 
 
 @pytest.mark.parametrize("H,HK,n_tok,pos0", [(8, 2, 21, 5), (64, 8, 9, 120), (16, 2, 6, 1790), (16, 2, 3, 6390)],
-                         ids=["tiled-gqa4-ragged", "tiled-gqa8-70B-heads", "tiled-2-tokens-per-cta-long-context", "per-head-fallback-very-long"])
+                         ids=["gqa4-ragged", "gqa8-70B-heads", "gqa8-long-context", "gqa8-very-long"])
 def test_attn_prefill_vs_oracle(cuda, lib, port, H, HK, n_tok, pos0):
     """Prompt-processing attention: every (token, head) row against the oracle's decode attention at that token's causal length.
-    Covers the tiled kernel (K/V tiles shared by the GQA group x 4 / 2 tokens) and the per-(head, token) fallback."""
+    Aligned arrays: the tensor-core kernel (the other kernels: test_gpu_attn_prefill_tiles.py)."""
     rng = np.random.default_rng(H + n_tok)
     D = 128
     n_ctx = pos0 + n_tok
