@@ -12,26 +12,29 @@
 // Also the 32-element block types Q8_0 / Q5_1 (K % 64 == 0; activations quantized per 32 values like their CPU dot): Qwen2.5-72B's
 // ffn_down, whose K = 29 568 rules the k-quants out (src/llama.cpp:19516-19551).
 //
-// Work decomposition (stream-K, persistent).  A work UNIT = one 256-element K group of one output tile (128 weight rows x 1 or 2
-// token tiles of BN <= 256 columns: two accumulators = all 512 TMEM columns share every expanded weight stage when T is large enough).
-// The units of a launch, ordered tile by tile, are cut into one contiguous range per CTA (at most one CTA per SM), so every SM gets the same
-// number of 64-element MMA steps whatever N, K and T are: a one-tile-per-CTA grid left 84 of 148 SMs idle on an 8192-row matrix
-// at 512 tokens and 2/3 of the last wave idle on ffn_gate/up.  A CTA walks its range segment by segment (segment = its part of one
-// tile); a segment that covers the tile's whole K stores its result, a partial one adds it into the pre-zeroed dst with fp32 atomics
-// (one addend per CTA of the tile: the order of fp32 adds is the only non-determinism, below the kernel's own fp16 rounding).
+// Work decomposition.  A work UNIT = one 256-element K group of one output tile (128 weight rows x 1 or 2 token tiles of BN <= 256 columns: two
+// accumulators = all 512 TMEM columns share every expanded weight stage when T is large enough).  Two forms, chosen by mmq_pick_cut:
+//   shares   the units of a launch, ordered tile by tile, are cut into one contiguous range per CTA (at most one CTA per SM), so that few SMs are
+//            idle in a last wave.  A CTA walks its range segment by segment (segment = its part of one tile); a segment that covers the
+//            tile's whole K stores its result, a partial one adds it into the pre-zeroed dst with fp32 atomics; a tile has two such
+//            segments at most
+//   cut      few tiles: a cluster of up to 8 CTAs shares one tile, each takes a part of its K, and the parts' sums are added in order through
+//            distributed shared memory
+// Either way an element's sum has one order: equal calls give equal bits.
 // Inside a CTA the pipeline never drains between segments (raw-block ring, A and B stages and their barriers run on CTA-wide counters):
 //   warp 0      owns TMEM; one lane issues 4 x tcgen05.mma (M=128, N=BN, K=16, kind::f16) per step and accumulator, one commit per step
 //   warp 1      activation producer: one cp.async.bulk per step and accumulator of the pre-tiled fp16 chunk (BN x 128 B, already in the
 //               UMMA swizzle-128B image), 2-4 stages deep
 //   warps 2..17 (16 expansion warps, 4 threads per weight row) fetch their rows' raw quantized blocks (16-byte cp.async pieces, 3 K groups
 //               deep, completion through cp.async.mbarrier.arrive) and expand 128 x 64 weights per step to fp16 straight into the swizzled A
-//               stage (generic-proxy stores + fence.proxy.async), 2 stages (4 with CTA pairs); at the end of a segment all 16 read the
+//               stage (generic-proxy stores + fence.proxy.async), 2 stages (4 with CTA pairs); at the end of a segment or part all 16 read the
 //               accumulators out of TMEM (tcgen05.ld 32x32b: quadrant = warp % 4, every fourth chunk of 16 columns) and store / add into dst
 // CG = 2 (opt-in): the CTA pair of a cluster shares one M = 256 MMA (cta_group::2), see launch_mmq.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -48,6 +51,7 @@ constexpr int MMQ_DQ_WARP0 = 2;   // warps 0,1 = MMA issuer (owns TMEM), activat
 constexpr int MMQ_THREADS = (MMQ_DQ_WARP0 + MMQ_DQ_WARPS) * 32;
 constexpr int MMQ_A_BYTES = MMQ_BM * 128;   // one A stage: 128 rows x 64 fp16
 constexpr int MMQ_CTL_BYTES = 320;
+constexpr int MMQ_MAX_PARTS = 8;  // CTAs of a cluster that share a tile's K
 
 struct MmqParams {
     int * abort_flag;      // host-mapped, raised by the wait watchdog
@@ -60,7 +64,9 @@ struct MmqParams {
     int nraw, b_nst, a_nst;   // ring depths chosen at launch from the shared-memory budget (a_nst: 2 or 4)
     int nacc, ttiles;      // accumulators (token tiles) per output tile, number of token tiles
     int ngrp, rtiles;      // 256-K groups per row (the last one may be short: 32-element block types), row tiles
+    int parts;             // > 1: the CTAs of a cluster, one tile each cluster, share the tile's K groups; else
     int upc, total_units;  // work units per CTA (CTA c owns units [c * upc, min((c + 1) * upc, total_units)) ), units of the launch
+    int chain;             // > 0: instead, chains of that many tiles (the last one: what is left), each in equal shares for one CTA more than it has tiles
     int N, K, T, BN, bpb, slot;   // slot: bytes reserved per row in a raw stage (16-B aligned window around one block)
     uint32_t tmem_cols, idesc;
 };
@@ -157,6 +163,22 @@ __device__ __forceinline__ uint32_t mmq_cluster_rank() { uint32_t r; asm volatil
 __device__ __forceinline__ void mmq_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// what every thread of the cluster has loaded from the others' shared memory is in its registers: nothing is published
+__device__ __forceinline__ void mmq_cluster_read() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+// a shared-memory address of this CTA in CTA `rank` of the cluster, and the float there
+__device__ __forceinline__ uint32_t mmq_peer_addr(uint32_t saddr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(saddr), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ float mmq_peer_f32(uint32_t ra) {
+    float f;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(ra) : "memory");
+    return f;
 }
 // arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster
 __device__ __forceinline__ void mbar_arrive_cluster(uint64_t * bar, uint32_t rank) {
@@ -288,7 +310,7 @@ __device__ __forceinline__ void cp_async16(void * smem_dst, const void * gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
 
-template <int TYPE, int CG>
+template <int TYPE, int CG, bool CUT>
 __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant__ MmqParams P) {
     extern __shared__ uint8_t smem_raw[];
     // the swizzle-128B atoms (A and B stages) need 1024-byte alignment in the shared window
@@ -306,7 +328,16 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nstep_all = P.K / MMQ_BK;                          // 64-element steps of a whole row; group sb holds steps [4 sb, min(4 sb + 4, nstep_all))
-    const int w0 = (int) (blockIdx.x / CG) * P.upc, w1 = min(w0 + P.upc, P.total_units);   // this CTA's (pair's) units
+    // this CTA's (pair's) units; CUT: the part-th of a tile's equal consecutive parts, one segment
+    const int part = CUT ? (int) blockIdx.x % P.parts : 0, cut0 = CUT ? (int) blockIdx.x / P.parts * P.ngrp : 0;
+    int w0 = CUT ? cut0 + P.ngrp * part / P.parts : (int) (blockIdx.x / CG) * P.upc;
+    int w1 = CUT ? cut0 + P.ngrp * (part + 1) / P.parts : min(w0 + P.upc, P.total_units);
+    if (!CUT && P.chain > 0) {
+        const int b = (int) blockIdx.x / CG, c = b / (P.chain + 1), j = b - c * (P.chain + 1), u0 = c * P.chain * P.ngrp;
+        const int units = min(P.chain * P.ngrp, P.total_units - u0), shares = units / P.ngrp + 1;
+        w0 = u0 + (int) ((int64_t) units * min(j, shares) / shares);
+        w1 = u0 + (int) ((int64_t) units * min(j + 1, shares) / shares);
+    }
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 3; i++) { mbar_init(&ctl->raw_full[i], MMQ_DQ_WARPS * 32); mbar_init(&ctl->raw_empty[i], MMQ_DQ_WARPS); }
@@ -480,6 +511,64 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 prs = rs; pph = rph;
                 if (++rs == P.nraw) { rs = 0; rph ^= 1; }
             }
+            if constexpr (CUT) {
+                // ================= epilogue of a part: partial sums [token][row] go over the stages' memory (every load and MMA of this CTA is done),
+                // one accumulator after the other; token t is added up, in the parts' order, by CTA t % parts =================
+                const bool acc_ok = ok && mmq_wait(ctl, &ctl->acc_ready, 0);
+                tc_fence_after();
+                const int tt0 = (tile / P.rtiles) * P.nacc, nacc = min(P.nacc, P.ttiles - tt0);
+                const int quad = warp & 3, grp = (warp - MMQ_DQ_WARP0) >> 2, n = row0 + quad * 32 + lane;
+                float * red = reinterpret_cast<float *>(smem) + quad * 32 + lane;
+                const float bias = (P.bias && n < P.N) ? P.bias[n] : 0.f;
+                for (int a = 0; a < nacc; a++) {
+                    const int t0 = (tt0 + a) * BN, tn = min(BN, P.T - t0);
+                    for (int c0 = 16 * grp; c0 < tn && acc_ok; c0 += 64) {
+                        uint32_t v[16];
+                        const uint32_t taddr = tmem + ((uint32_t) (quad * 32) << 16) + (uint32_t) (a * 256 + c0);
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                            : "r"(taddr)
+                            : "memory");
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 16; i++) red[(c0 + i) * MMQ_BM] = __uint_as_float(v[i]);
+                    }
+                    __syncwarp();
+                    mmq_cluster_sync();
+                    if (n < P.N) {
+                        constexpr int U = 8;                     // tokens of a thread at once, two parts of them on their way: what takes time is the latency
+                        const int step = 4 * P.parts;
+                        for (int t = part + P.parts * grp; t < tn; t += U * step) {
+                            float sum[U], f[2][U];                // bias and residual ride on part 0
+#pragma unroll
+                            for (int i = 0; i < U; i++) sum[i] = P.resid && t + i * step < tn ? __ldg(P.resid + (size_t) (t0 + t + i * step) * (size_t) P.N + n) : 0.f;
+                            for (int c = 0; c < P.parts; c += 2) {
+#pragma unroll
+                                for (int h = 0; h < 2; h++)
+                                    if (c + h < P.parts) {
+                                        const uint32_t at = mmq_peer_addr(smem_u32(red + t * MMQ_BM), (uint32_t) (c + h));
+#pragma unroll
+                                        for (int i = 0; i < U; i++)
+                                            if (t + i * step < tn) f[h][i] = mmq_peer_f32(at + (uint32_t) (i * step * MMQ_BM * 4));
+                                    }
+#pragma unroll
+                                for (int h = 0; h < 2; h++)
+                                    if (c + h < P.parts) {
+#pragma unroll
+                                        for (int i = 0; i < U; i++) sum[i] = c + h == 0 ? __fadd_rn(__fadd_rn(f[h][i], bias), sum[i]) : __fadd_rn(sum[i], f[h][i]);
+                                    }
+                            }
+#pragma unroll
+                            for (int i = 0; i < U; i++)
+                                if (t + i * step < tn) P.dst[(size_t) (t0 + t + i * step) * (size_t) P.N + n] = sum[i];
+                        }
+                    }
+                    __syncwarp();
+                    mmq_cluster_read();   // read by every CTA: the next accumulator may go there, or the CTA leave
+                }
+            } else
             // ================= epilogue of the segment: four consecutive warps cover the four 32-lane quadrants of TMEM =================
             // All 16 expansion warps read out: a warp may only read quadrant warp % 4, its group (warp - 2) / 4 takes every fourth chunk of 16
             // columns.  Chunk ch holds tokens tt0 * BN + 16 ch ..: two accumulators lie 256 columns apart and are only used with BN = 256.
@@ -549,6 +638,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             }
             w += sbe - sbb;
         }
+    }
+    if (CUT && warp < MMQ_DQ_WARP0) {   // the cluster's barriers count every warp
+        const int rounds = min(P.nacc, P.ttiles - (w0 / P.ngrp / P.rtiles) * P.nacc);
+        for (int i = 0; i < rounds; i++) { mmq_cluster_sync(); mmq_cluster_read(); }
     }
     tc_fence_before();
     __syncthreads();
@@ -674,10 +767,14 @@ bool mmq_supported(int type, int64_t K) {
     return (type == T_Q8_0 || type == T_Q5_1) && K % 64 == 0 && K >= 256;   // 32-element blocks: two per 64-element step
 }
 
-template <int TYPE, int CG>
-static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st) {
+template <int TYPE, int CG, bool CUT>
+static cudaError_t mmq_allow_smem(size_t smem) {
     static FuncAttrCache attr_cache;
-    cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG>, smem, false);
+    return ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
+}
+template <int TYPE, int CG, bool CUT>
+static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st) {
+    cudaError_t e = mmq_allow_smem<TYPE, CG, CUT>(smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -686,34 +783,76 @@ static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = CUT ? (unsigned) P.parts : CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = CG > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG>, P);
+    cfg.numAttrs = CG > 1 || CUT ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT>, P);
 }
 template <int TYPE>
 static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size_t smem, cudaStream_t st) {
-    return cg == 2 ? mmq_launch_typed2<TYPE, 2>(P, grid, smem, st) : mmq_launch_typed2<TYPE, 1>(P, grid, smem, st);
+    if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, grid, smem, st);
+    return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, grid, smem, st) : mmq_launch_typed2<TYPE, 1, false>(P, grid, smem, st);
+}
+// clusters of `parts` CTAs of this kernel that run at the same time (a CTA takes an SM; a cluster stays within a group of SMs)
+static int mmq_clusters(int parts) {
+    static std::atomic<int> known[MMQ_MAX_PARTS + 1];
+    int n = known[parts].load(std::memory_order_relaxed);
+    if (n == 0) {
+        const size_t smem = 160 * 1024;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned) (parts * 148));
+        cfg.blockDim = dim3(MMQ_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned) parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (mmq_allow_smem<T_Q4_K, 1, true>(smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, (const void *) k_mmq_tc<T_Q4_K, 1, true>, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = -1;
+        }
+        known[parts].store(n, std::memory_order_relaxed);
+    }
+    return std::max(n, 0);
 }
 
-// Units per CTA.  The least share that fits one wave is ceil(total / SMs); a longer one is better when it makes the CTAs' ranges end where
-// tiles end: a share that divides the tile's groups is one segment, one that is a multiple of them needs no adding and no cleared output,
-// any other can touch a tile more.  Costs in us on B200, Q4_K: a unit 3.05 (512 tokens: two accumulators, 8 x 171 clk of MMA a step; half of
-// it with one), a segment's fill and read-out 8, the clearing pass 3 + bytes / 6.2 TB/s.  At 512 tokens, us per launch (K = 4096): 512 and
-// 4096 rows as shares of at least 8 units 35.8 and 34.8, at least 1 unit 24.2 and 14.1; 14336 rows in shares of 13 units 64.1 and 7.8 for the
-// clearing, as whole tiles 63.5.  Rows of up to 8 groups (K <= 2048) are not cut for idle SMs: there a tile costs at most 24 us, and uncut its
-// sums do not depend on the number of tokens, so a prompt's result does not depend on the slices it came in.
-static int mmq_pick_share(int64_t total, int ngrp, int nsm, int nacc, double out_bytes) {
-    const int fit = (int) ((total + nsm - 1) / nsm), base = ngrp <= 8 ? std::max(fit, ngrp) : fit;
-    const double unit = nacc == 2 ? 3.05 : 1.55, seg = nacc == 2 ? 8.0 : 5.0, clear = 3.0 + out_bytes / 6.2e6;
-    int best = base;
-    double best_us = 1e30;
-    for (int upc = base; upc <= base + ngrp; upc++) {
-        const bool whole = upc % ngrp == 0, divides = ngrp % upc == 0;
-        if (upc != base && !whole && !divides) continue;
-        const int segs = whole ? upc / ngrp : divides ? 1 : (upc + ngrp - 2) / ngrp + 1;
-        const double us = upc * unit + segs * seg + (whole ? 0.0 : clear);
-        if (us < best_us) { best_us = us; best = upc; }
+// How a launch's tiles are shared:
+//   parts > 1   the CTAs of a cluster cut one tile's K into equal consecutive parts and add their sums in the parts' order through distributed shared
+//               memory
+//   chain > 0   chains of tiles, each in equal contiguous shares for one CTA more than it has tiles: every tile is cut once
+//   else        contiguous shares of upc units: whole tiles, or at least a tile less one group, so that again no tile is cut twice
+// Where a tile is cut once its two sums meet on a cleared output: in either order they give the same bits.  An element's sum so has one order,
+// fixed by the launch's tiles and K groups, not by its tokens: the same call gives the same bits, and k-quant weights give a row the same
+// bits with 8 or 511 others beside it.
+// Costs in us on B200, Q4_K, 512 tokens: a unit 3.05 (2.7 with few tokens: the expansion of the weights), a segment's fill and read-out 8, the join of
+// p parts 7.5 + 1.25 p (what distributed shared memory gives: 256 KB a CTA; in proportion to the tokens), the clearing pass 3 + bytes /
+// 6.2 TB/s.  Measured with the activation pass, K = 4096, 512 tokens: 1024 rows whole 63.5, 2 parts 48.7, 4 parts 38.4, 8 parts 34.1; 4096 rows
+// whole 63.7, 4 parts 37.2; 64 tokens: 1024 rows 53.3, 31.9, 21.8, 16.6.  8192 x 8192 in halves: 79.1 by a cluster, 74 onto a cleared
+// output; 64 tokens 56 and 57.  20480 x 2048: whole tiles 71.4, shares of 9 units 58.4.
+// What the order costs: shares for every SM whose sums meet as they arrive took (512 / 64 tokens, then -> now) 20.0 / 11.9 -> 34.1 / 16.6 at
+// 1024 x 4096, 31.4 / 21.0 -> 37.2 / 21.9 at 4096 x 4096, 25.1 / 14.8 -> 32.4 / 18.8 at 3072 x 3072, 74.0 / 54.9 -> 78.3 / 55.1 at 4096 x 14336,
+// 229 / 169 -> 244 / 183 at 8192 x 28672, 175 / 126 -> 183 / 138 at 12800 x 14336; 37.8 / 29.7 -> 28.9 / 19.9 at 2048 x 2048, where tiles stayed whole.
+struct MmqCut { int parts, chain, upc; };
+static int64_t mmq_chain_ctas(int64_t tiles, int m) { return tiles / m * (m + 1) + (tiles % m ? tiles % m + 1 : 0); }
+static MmqCut mmq_pick_cut(int64_t tiles, int ngrp, int nsm, int max_parts, double tokens) {
+    const double unit = 3.05, seg = 8.0, tile_us = 128.0 * 512.0 * 4.0 / 6.2e6, clear = 3.0 + (double) tiles * tile_us;
+    const int rounds = (int) ((tiles + nsm - 1) / nsm);
+    MmqCut best{1, 0, rounds * ngrp};
+    double best_us = rounds * (ngrp * unit + seg);
+    auto consider = [&](const MmqCut & c, double us) { if (us < best_us) { best_us = us; best = c; } };
+    const int upc = std::max((int) ((tiles * ngrp + nsm - 1) / nsm), ngrp - 1);
+    if (upc % ngrp != 0) consider({1, 0, upc}, upc * unit + ((upc + ngrp - 2) / ngrp + 1) * seg + clear);
+    for (int m = 2; m <= 8; m++)
+        if (mmq_chain_ctas(tiles, m) <= nsm) consider({1, m, 0}, (m * ngrp + m) / (m + 1) * unit + 2 * seg + clear);
+    // two halves: by a cluster or a chain of one tile, whichever is the faster one for these tokens; the bits are the same
+    const bool pairs = max_parts >= 2 && tiles <= mmq_clusters(2);
+    if (tiles * 2 <= nsm && ngrp >= 2)
+        consider(pairs && 10.0 * tokens <= 3.0 * 512.0 + (double) tiles * tile_us * tokens ? MmqCut{2, 0, 0} : MmqCut{1, 1, 0}, (ngrp + 1) / 2 * unit + seg + std::min(10.0, clear));
+    for (int p = 3; p <= max_parts && p <= ngrp && tiles * p <= nsm; p++) {
+        const double us = (ngrp + p - 1) / p * unit + seg + 7.5 + 1.25 * p;
+        if (us < best_us && tiles <= mmq_clusters(p)) consider({p, 0, 0}, us);
     }
     return best;
 }
@@ -757,27 +896,14 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     if (P.nacc == 2 && 1024 + (size_t) 2 * MMQ_A_BYTES + (size_t) 2 * 2 * (BN / cg) * 128 + (size_t) 2 * MMQ_BM * P.slot + MMQ_CTL_BYTES > 232448) P.nacc = 1;
     const int tgroups = (P.ttiles + P.nacc - 1) / P.nacc;
     P.ngrp = (int) ((K / MMQ_BK + 3) / 4);
-    // stream-K: the tiles' K groups, tile after tile, in equal contiguous shares (mmq_pick_share)
-    static const int min_units = getenv("PB200_MMQ_MIN_UNITS") ? std::max(1, atoi(getenv("PB200_MMQ_MIN_UNITS"))) : 0;   // A/B: a fixed least share
     static const bool whole_tiles = getenv("PB200_MMQ_WHOLE_TILES") != nullptr;   // A/B: one tile per CTA (no split, no atomics)
-    const int64_t total = (int64_t) P.rtiles * tgroups * P.ngrp;
+    const int64_t tiles = (int64_t) P.rtiles * tgroups, total = tiles * P.ngrp;
     if (total > 0x7fffffff) return cudaErrorInvalidValue;
     P.total_units = (int) total;
-    const int nsm = sm_count() / cg;           // CTAs (pairs) that can be resident: one CTA per SM
-    int upc = mmq_pick_share(total, P.ngrp, nsm, P.nacc, (double) T * (double) N * 4.0);
-    if (min_units) upc = std::max((int) ((total + nsm - 1) / nsm), std::min(min_units, P.ngrp));
-    if (whole_tiles) upc = P.ngrp;
-    P.upc = upc;
-    const int grid_x = (int) ((total + upc - 1) / upc);
-    const bool split = upc % P.ngrp != 0;      // some tile is shared by two CTAs: partial results meet in dst by atomic add
     if (!reuse_prep) {
         k_mmq_prep<<<tpad, 256, 0, st>>>(x, ldx, (int) T, (int) K, BN, (uint8_t *) ws, is_kquant(type) ? 0 : 1, pre ? pre->kind : 0,
                                          pre ? pre->aux : nullptr, pre ? pre->ld_aux : 0, pre ? pre->eps : 0.f);
         cudaError_t e0 = cudaGetLastError();
-        if (e0 != cudaSuccess) return e0;
-    }
-    if (split) {
-        cudaError_t e0 = cudaMemsetAsync(dst, 0, (size_t) T * (size_t) N * sizeof(float), st);
         if (e0 != cudaSuccess) return e0;
     }
     uint32_t cols = 32;
@@ -800,7 +926,17 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     while (P.b_nst > 2 && smem_for(P.nraw, P.b_nst) > 232448) P.b_nst--;
     const size_t smem = smem_for(P.nraw, P.b_nst);
     if (smem > 232448) return cudaErrorInvalidConfiguration;
-    dim3 grid((unsigned) (grid_x * cg), 1, 1);
+    const int nsm = sm_count() / cg;           // CTAs (pairs) that can be resident: one CTA per SM
+    MmqCut cut = mmq_pick_cut(tiles, P.ngrp, nsm, cg == 1 && (size_t) MMQ_BM * BN * 4 <= smem - 1024 - MMQ_CTL_BYTES ? MMQ_MAX_PARTS : 1, (double) std::min<int64_t>(T, 512));
+    if (whole_tiles) cut = {1, 0, P.ngrp};
+    P.parts = cut.parts;
+    P.chain = cut.chain;
+    P.upc = cut.upc;
+    if (cut.chain > 0 || (cut.parts == 1 && cut.upc % P.ngrp != 0)) {   // some tile is shared by two CTAs: their sums meet in dst by atomic add
+        cudaError_t e0 = cudaMemsetAsync(dst, 0, (size_t) T * (size_t) N * sizeof(float), st);
+        if (e0 != cudaSuccess) return e0;
+    }
+    dim3 grid((unsigned) (cut.parts > 1 ? tiles * cut.parts : cg * (cut.chain > 0 ? mmq_chain_ctas(tiles, cut.chain) : (total + cut.upc - 1) / cut.upc)), 1, 1);
     if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, cg, grid, smem, st);
     if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, cg, grid, smem, st);
     if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, cg, grid, smem, st);
