@@ -256,8 +256,10 @@ PB200_API int          pb200_arch_family(const char * name);
 
 /* ---- layer-list family ----
  * config_json: the text of the model's configuration file; its "architecture" selects the design.  compute_type: PB200_TYPE_BF16 (dense
- * products on bf16 operands with fp32 accumulation; norms, attention scores and weights, the residual stream and all recurrent state stay
- * fp32) or PB200_TYPE_F32 (everything in true fp32).  n_ctx: the most positions one sequence can have where a layer has to keep all of
+ * products on bf16 operands with fp32 accumulation; norms, the residual stream and all recurrent state stay fp32; attention takes fp32
+ * queries, keys, values and softmax weights and accumulates in fp32, in prompts beyond 16 tokens with every operand as two f16 numbers,
+ * 22 bits and more) or PB200_TYPE_F32 (everything in true fp32).  A row of a batch does not depend on what the others hold; how many they
+ * are may change the order of its fp32 sums.  n_ctx: the most positions one sequence can have where a layer has to keep all of
  * them; a windowed attention layer keeps keep_first + window rows per sequence whatever its length.  n_seq: sequence slots
  * (<= 0: as many as 8 GiB of state hold, 4 .. 256).  Tensors arrive through pb200_model_set_tensor under their checkpoint names with
  * type PB200_TYPE_BF16 or PB200_TYPE_F32 (converted to what the model computes in); then pb200_model_finalize.  pb200_model_synth

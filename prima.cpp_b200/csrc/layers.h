@@ -39,7 +39,8 @@ struct BatchView {
 // ---- dense products ----
 // C[t][n] = alpha * sum_k A[t][k] * W[n][k] (+ bias[n]) (+ resid[t][n]);  A and W share `type` (T_F32: true fp32 multiply-add;
 // T_BF16: bf16 operands, fp32 accumulation), C / bias / resid are f32.  resid may alias C.  lda / ldw / ldc / ldr in elements.
-// The result of a row does not depend on the other rows of the call beyond the choice between the small-batch and the tiled kernel.
+// The result of a row does not depend on what the other rows of the call hold.  Their number chooses the kernel, and in the tensor-core kernel how K is cut
+// (plan_tc in dense_tc.cu): the order of the fp32 sum may change with it, its error bound does not.
 int launch_dense(int type, const void * A, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K,
                  const float * bias, const float * resid, int64_t ldr, float alpha, cudaStream_t stream);
 // Grouped product in one launch: rows [start[g], start[g] + count[g]) of A times the g-th matrix of W (w_stride elements apart, [N][K]
@@ -188,7 +189,8 @@ int launch_attn_prefill_io(const AttnIO & io, const BatchView & b, const AttnPar
 int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnParams & a, const float * kcache, const float * vcache, int64_t slot_stride,
                           void * out, int otype, cudaStream_t stream, float * part = nullptr);
 
-// prompt attention with every operand as two f16 numbers on the tensor cores (attn_split.cu): head sizes up to 192, value sizes up to 128
+// prompt attention with every operand as two f16 numbers on the tensor cores (attn_split.cu): head sizes up to 192, value sizes up to 128.  A prompt batch whose
+// longest entry is beyond 16 tokens takes it for all of its entries; shorter ones keep the fp32 FMA kernel
 size_t attn_split_bytes(const AttnParams & a, int n_tokens, int n_entries);   // scratch for a prompt batch (0: the shape is not taken)
 bool attn_split_ok(const AttnIO & io, const BatchView & b, const AttnParams & a);
 int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t stream);

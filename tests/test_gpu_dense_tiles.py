@@ -55,3 +55,24 @@ def test_residual_in_place_and_repeatable(lib, cuda, T, N, K):
         lib.check(lib.c.pb200_dense(30, ptr(A), K, ptr(W), K, ptr(out), N, T, N, K, None, ptr(resid), N, 1.0, None), "dense")
     torch.cuda.synchronize()
     assert torch.equal(apart, inplace)
+
+
+@pytest.mark.parametrize("N,K", [(2048, 8192), (4096, 2048)])
+def test_a_row_in_batches_of_other_sizes(lib, cuda, N, K):
+    """The cut of K, hence the order of a row's sum, follows the number of tokens: the row keeps within the bound of float64 in every batch, and its bits do
+    not follow what the other rows hold."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    A, W = torch.randn(700, K, generator=g, device="cuda").bfloat16(), torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    B = torch.randn(700, K, generator=g, device="cuda").bfloat16()
+    B[:5] = A[:5]
+    want, mass = A[:5].double() @ W.double().T, A[:5].double().abs() @ W.double().abs().T
+    for T in (5, 16, 17, 64, 129, 200, 300, 512, 700):
+        rows = []
+        for X in (A, B):
+            out = torch.empty(T, N, device="cuda")
+            lib.check(lib.c.pb200_dense(30, ptr(X), K, ptr(W), K, ptr(out), N, T, N, K, None, None, 0, 1.0, None), "dense")
+            rows.append(out[:5])
+        torch.cuda.synchronize()
+        assert torch.equal(rows[0], rows[1]), T
+        assert bool(((rows[0].double() - want).abs() <= (K / 16 + 16) * 2.0 ** -22 * mass).all()), T
