@@ -22,8 +22,9 @@ namespace {
 //   warps 2 - 9  softmax: thread = (row, half of the tile's keys, 32 at a time); row = TMEM lane
 // Bound: 2 exponentials per score on the MUFU (16 a clock: 2048 clocks a 128 x 128 tile) against 1536 clocks of MMA; two CTAs together take
 // 1100 clocks a tile in the first walk and 1550 in the second, a CTA's start and end 6500.  Measured at 2048 tokens, 32 heads over 8:
-// 2994 us with the scores in shared memory and fp32 FMA before, 80.6 us (427 TFLOP/s of visible pairs); one CTA to an SM with both
-// operands twice in tensor memory took 101 us.  512 tokens: 120 -> 17.5 us; 16 tokens behind 2000: 201 -> 47 us.
+// 2994 us with the scores in shared memory and fp32 FMA before, 80.6 us (427 TFLOP/s of visible pairs; 85 with launch and wait); one CTA to an SM with both
+// operands twice in tensor memory took 101 us.  512 tokens: 120 -> 17.5 us; 16 tokens behind 2000: 201 -> 47 us.  A first prompt of 16 / 32 / 64 tokens
+// (32 heads over 8), which is a start and an end and little between: 5.9 / 6.6 / 10.0 -> 7.4 / 8.1 / 8.7 us.
 constexpr int AT_STAGES = 2, AT_STAGE = 32768, AT_BLOCK = 16384;
 constexpr int AT_PARTS = 2, AT_COLS = 128 / AT_PARTS, AT_SM_THREADS = 128 * AT_PARTS, AT_THREADS = 64 + AT_SM_THREADS;
 

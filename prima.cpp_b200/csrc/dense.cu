@@ -252,9 +252,11 @@ __global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, i
 }
 
 constexpr int ROWS_MAX_T = 8;
-// Largest batch the weight-streaming kernel takes when the tensor-core kernel could run instead.  Measured on a B200 at 28672 x 4096 bf16:
-// 8 tokens stream at 1.9 TB/s through this kernel (one L1 read of the activations per token and weight chunk) and at 3.3 TB/s through
-// the tensor-core kernel's 64-token tile, so the hand-over is at 4.  PB200_DENSE_ROWS_MAX overrides for A/B runs.
+// Largest batch the weight-streaming kernel takes when the tensor-core kernel could run instead.  PB200_DENSE_ROWS_MAX overrides for A/B runs.  The line was
+// drawn when the tensor-core kernel had 64-token tiles.  With its 16-token tiles and K over a cluster, us on a B200 for 2 / 4 tokens (weights
+// from HBM): 28672 x 4096 51 / 67 here, 39 / 40 there; 4096 x 14336 27 / 36, 22 / 22; 4096 x 4096 11.3 / 14.1, 9.6 / 9.7; 2048 x 2048 5.9 / 7.2,
+// 6.2 / 6.3; 512 x 2048 5.2 / 6.7, 5.2 / 5.2.  One token: 44 here at 28672 x 4096 and 4.9 at 2048 x 2048.  So batches of 2 to 4 would gain by a
+// lower line, which changes the order of their sums.
 int rows_max_t() {
     static const int v = [] {
         const char * e = getenv("PB200_DENSE_ROWS_MAX");

@@ -10,7 +10,7 @@
 //                  partial sums in the parts' order through distributed shared memory
 // What bounds them: all SMs together take about 12.5 TB/s from L2, and a 64-k step of a tile loads (rows + tokens) * 128 bytes: 128 x 256 tiles
 // are held to 0.65 of the tensor rate by that, the pair's 256 x 256 to 0.87; small batches are bound by the weights' way from HBM.  Measured
-// (2048 x 28672 x 4096): 870 us with cp.async producers and 128 x 256 tiles before, 330 us with the pair.  No atomics: the sum of an
+// (2048 x 28672 x 4096): 870 us with cp.async producers and 128 x 256 tiles before, 345 us with the pair, 389 in calls one by one under the power limit.  No atomics: the sum of an
 // element has one order, fixed by (T, N, K).  Every wait is bounded (common.cuh).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -1312,7 +1312,9 @@ int launch_attn_batch(const float * q, const __half * kcache, const __half * vca
                       const int32_t * pos_dev, int n_tok, int n_kv_max, float scale, cudaStream_t stream) {
     if (D != 128 || n_tok <= 0 || n_tok > 65535) return (int) cudaErrorInvalidValue;
     static const int attn_mode = getenv("PB200_ATTN_MODE") ? atoi(getenv("PB200_ATTN_MODE")) : 0;   // A/B switch: 1 = the per-(head, token) grid of k_attn_decode, 2 = the tiled kernel of this file
-    // one kernel for every length, so that a row's bits do not depend on how a prompt is cut (prompts of 32 tokens and less lose 1 to 3 us of 6 by it)
+    // one kernel for every length, so that a row's bits do not depend on how a prompt is cut.  First prompts of 32 tokens and less lose by it (us, tiled
+    // kernel -> this one): 16 tokens 5.9 -> 7.4 and 32 tokens 6.6 -> 8.1 for 32 heads over 8, 4.7 -> 7.3 and 5.7 -> 7.4 for 4 over 4, 8.3 -> 8.1 and
+    // 9.3 -> 8.1 for 32 over 4; from 48 tokens on, or behind a context, it wins (16 tokens behind 112: 16.1 -> 8.1)
     if (attn_mode == 0 && attn_prefill_tc_ok(q, kcache, vcache, out, n_head, n_head_kv, D, n_kv_max))
         return launch_attn_prefill_tc(q, kcache, vcache, out, n_head, n_head_kv, pos_dev, n_tok, n_kv_max, scale, stream);
     const uintptr_t at = (uintptr_t) kcache | (uintptr_t) vcache;
