@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py — decode tokens/s of the quantized-decode hot path (BASELINE.json metric) on N B200s of one node.
+"""bench.py — decode tokens/s of the quantized-decode hot path on N B200s of one node.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--model llama3-70b] [--impl b200|reference]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P bench.py --gpus N ...
@@ -71,7 +71,7 @@ def tensor_peak():
 
 
 def prefill_flops(hp, T):
-    """Algorithmic FLOPs of one prompt batch (SURVEY 8d): 2 * sum(N*K) * T over the per-layer mat-muls, causal attention
+    """Algorithmic FLOPs of one prompt batch: 2 * sum(N*K) * T over the per-layer mat-muls, causal attention
     4 * T^2/2 * n_embd per layer, lm_head for the last token only."""
     E, F, D = hp["n_embd"], hp["n_ff"], 128
     QD, EK = hp["n_head"] * D, hp["n_head_kv"] * D
@@ -289,8 +289,8 @@ def boundary_leg(eng, cfg, hp, args, lib):
 
 # ------------------------------------------------------------------------------------------------ same-box GPU comparator
 def ggml_cuda_arm(args, cfg, hp, config):
-    """--impl ggml-cuda: the reference's OWN ggml-cuda backend (unmodified, built for sm_100 by oracle/Makefile.cudaref — BASELINE.md §3
-    "the existing kernel to beat") on the same box, same synthetic weights, same host graph (host/llama_graph_host.cpp), same protocol
+    """--impl ggml-cuda: the reference's OWN ggml-cuda backend (unmodified, built for sm_100 by oracle/Makefile.cudaref:
+    the existing kernel to beat) on the same box, same synthetic weights, same host graph (host/llama_graph_host.cpp), same protocol
     as the B200 arm's e2e leg: host token / position / mask in, logits out, every step.  Measurement infrastructure: none of the
     product's kernels run inside the timed region (the engine is used before it, to synthesise the weights, and is then freed)."""
     import numpy as np
@@ -730,7 +730,7 @@ def main():
                             f"matrices read) / their summed CUDA-event durations ({gemv_ms:.3f} ms, events on the launching stream, mean of 4 profiled steps)",
                      "whole_step": {"algorithmic_bytes_per_token": wb + kv_bytes, "achieved": (wb + kv_bytes) / (ms_step * 1e-3) / 1e9,
                                     "frac": (wb + kv_bytes) / (ms_step * 1e-3) / 1e9 / peak,
-                                    "frac_of_8TBs_north_star": (wb + kv_bytes) / (ms_step * 1e-3) / 8e12}},
+                                    "frac_of_8TBs": (wb + kv_bytes) / (ms_step * 1e-3) / 8e12}},
         "model_load_s": t_load,
     }
     if pp_result is not None:
@@ -755,7 +755,7 @@ def main():
     if stage_ms is not None:
         out["pipeline"] = {"stages": world, "hand_offs_per_token": world, "sum_of_stage_ms": stage_ms, "pipelined_ms_per_token": ms_step,
                            "exposed_handoff_ms": max(0.0, ms_step - stage_ms), "exposed_frac": max(0.0, ms_step - stage_ms) / ms_step,
-                           "note": "b=1 decode is serial across stages (SURVEY H7): N GPUs hold N x the model, they do not cut the token latency"}
+                           "note": "b=1 decode is serial across stages: N GPUs hold N x the model, they do not cut the token latency"}
     if world == 1 and args.pp > 0 and args.pp <= args.n_ctx:
         try:
             # prompt processing (prefill) of one ubatch through pb200_prefill: tensor-core mat-muls, batched attention

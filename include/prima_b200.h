@@ -5,7 +5,7 @@
  * CUDA failures or a negative PB200_E* code for argument errors; nothing throws or aborts across the ABI.
  * Device pointers are raw CUDA device addresses, `stream` is a cudaStream_t passed as void* (NULL = default stream).
  *
- * What each entry point replaces in the reference (paths under /root/reference):
+ * What each entry point replaces in the reference (paths within its project):
  *   pb200_mul_mat_vec*      ggml_cuda_mul_mat -> ggml_cuda_op_mul_mat_vec_q -> mul_mat_vec_q<type,1>
  *                           ggml/src/ggml-cuda.cu:1883-1948, ggml-cuda/mmvq.cu:55-202, vecdotq.cuh:357-787
  *                           (+ the per-call quantize_row_q8_1_cuda, quantize.cu:129-141); CPU semantics:
@@ -171,7 +171,7 @@ PB200_API int pb200_model_set_tensor(pb200_model * m, const char * name, int typ
 /* The same without the copy: reserves the tensor's device memory and returns its address in *dev_ptr (NULL with return 0: the tensor
  * belongs to another stage) for hosts that stream the bytes themselves (pb200_model_load_gguf does). */
 PB200_API int pb200_model_tensor_alloc(pb200_model * m, const char * name, int type, size_t nbytes, void ** dev_ptr);
-/* GGUF file -> finalized model shard (SURVEY N2; replaces gguf_init_from_file + llm_load_hparams + llm_load_tensors' per-tensor
+/* GGUF file -> finalized model shard (replaces gguf_init_from_file + llm_load_hparams + llm_load_tensors' per-tensor
  * synchronous set_tensor, ggml-cuda.cu:464-487, for this path): v2 / v3 containers, architectures "llama" and "qwen2", tensors kept in
  * their raw block layout; the file is streamed through two pinned 64-MiB buffers with cudaMemcpyAsync so reading chunk i+1 overlaps the
  * PCIe copy of chunk i.  layer_end < 0: to the last layer; with_embd / with_head < 0: derived from the window; n_ctx <= 0:

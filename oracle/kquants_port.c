@@ -7,11 +7,11 @@
  * prima.cpp_b200/ may link, import or call it.
  *
  * Parity pin: every function here is checked (tests/test_oracle_port.py) against
- *   (1) the real reference compiled from /root/reference into oracle/_ref/ (when present), and
+ *   (1) the real reference compiled into oracle/_ref/ (when present), and
  *   (2) committed golden vectors in tests/golden/*.npz generated from that same compiled
  *       reference by tests/golden/make_golden.py.
  *
- * Each function cites the reference file:line it follows (paths relative to /root/reference).
+ * Each function cites the reference file:line it follows (paths within its project).
  * Written from the algorithm description; scalar form only (SIMD paths of the reference are
  * integer-identical and differ only in fp32 summation order).
  */
@@ -514,7 +514,7 @@ void port_silu_mul(const float *gate, const float *up, float *y, int64_t n) {
     for (int64_t i = 0; i < n; i++) y[i] = silu_f32(gate[i]) * up[i];
 }
 
-/* Decode attention, FA-off numerics of the CPU backend (SURVEY §7.3 H1):
+/* Decode attention, FA-off numerics of the CPU backend:
  *   kq[p]  = dot_f32( f16(K[p]), f16(q) )              ggml.c:12445-12473 (src1 -> vec_dot_type F16)
  *   p      = softmax(kq*scale + mask)   in f32          ggml.c:13783
  *   out[d] = dot_f32( V^T[d,:], f16(p) )                second mul_mat, src1 = probs -> f16

@@ -1,5 +1,5 @@
 // prima.cpp_b200/csrc/engine.cu — the decode engine behind include/prima_b200.h: weights resident in HBM in raw GGUF
-// block layout, one fused launch sequence per token (10 kernels per layer instead of the reference's ~30, SURVEY App. A),
+// block layout, one fused launch sequence per token (10 kernels per layer instead of the reference's ~30),
 // all PDL-chained and replayed as ONE CUDA graph per token; token id and position live in device memory so the graph
 // never changes (the reference re-captures / patches cpy nodes, ggml-cuda.cu:2602-2617, 2741-2752).
 //
@@ -319,7 +319,7 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
     const int QD = H * D, EK = HK * D;
     cudaStream_t st = m->stream;
     static const bool pdl = getenv("PB200_NO_PDL") == nullptr;   // programmatic dependent launch on every kernel of the step
-    static const bool attn_v2 = getenv("PB200_ATTN_V1") == nullptr;   // A/B: round 1's attention kernel + quantize prologue in wo
+    static const bool attn_v2 = getenv("PB200_ATTN_V1") == nullptr;   // A/B: the one-launch attention kernel without clusters + quantize prologue in wo
     static const bool dist_env = getenv("PB200_NO_DIST") == nullptr;   // A/B: single-CTA rmsnorm / silu kernels in front of the GEMVs instead
     const bool dist = dist_env && gemv_dist_prologue_ok();
     uint64_t n = 0;

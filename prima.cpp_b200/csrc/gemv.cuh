@@ -10,7 +10,7 @@
 //     what lets consecutive kernels of the token overlap under programmatic dependent launch: when a CTA of launch A exits,
 //     a CTA of launch B becomes resident on that SM and streams its first weight tiles (they never depend on A) while the
 //     rest of A drains; a small kernel between two GEMVs (attention, silu-quant) runs while the next GEMV's rings fill.
-//     Round 1's single 512-thread / 227-KB CTA per SM serialised every launch boundary: 9.25 us fixed cost per launch
+//     A single 512-thread / 227-KB CTA per SM serialised every launch boundary: 9.25 us fixed cost per launch
 //     (profiles/r1_gemv_microbench.txt) x 321 launches = 3 ms of a 10-ms token;
 //   * row tiles of raw blocks stream HBM -> shared memory with cp.async.bulk (1-D TMA) into an nstage-deep ring
 //     (4-8 stages of ~16-24 KB chosen per launch; ~185 KB in flight per SM).  There is no producer warp: the consumer warp
@@ -59,9 +59,9 @@ struct GemvMat {
 //   PRO_SILU_DIST     act = q8_K( silu(in0) * in1 )         llm_build_ffn LLM_FFN_SILU / LLM_FFN_PAR -> ffn_down
 //   Distributed: CTA c quantizes super-block c into `act` (HBM/L2), ONE grid barrier (all CTAs of the persistent grid are
 //   co-resident), then every CTA stages the finished vector like PRO_NONE.  No tiny kernel + launch boundary in front of the GEMV
-//   (measured chain ~9.5 us from "previous GEMV done" to "first tile consumed", profiles/r2_token_trace_v2.txt), and 1/296 of the
-//   work per CTA instead of every CTA recomputing the whole vector from L2 (round 1: ~7 us and 19 MB of L2 reads per launch).
-//   Built, measured on the B200 and REMOVED in round 2 (profiles/r2_ab_sweeps.txt, ab14-ab16):
+//   (measured chain ~9.5 us from "previous GEMV done" to "first tile consumed", profiles/r2_token_trace_v2_attn_v2_single_cta_norm.txt), and 1/296 of the
+//   work per CTA instead of every CTA recomputing the whole vector from L2 (~7 us and 19 MB of L2 reads per launch).
+//   Built, measured on the B200 and removed (profiles/r2_ab_sweeps.txt, ab14-ab16):
 //   * L2 look-ahead — prefetching a launch's tiles beyond its ring, and the next launch's first weights from ring slots that have no tile
 //     left, to keep HBM busy during the dependency chain at a launch boundary: DRAM bytes unchanged (ncu), the launch that is fed from L2
 //     gains (ffn_down -4.6 us) but the prefetching launch loses more (gate|up +7 us), and the small latency-critical loads of the prologue

@@ -1,4 +1,4 @@
-// prima.cpp_b200/csrc/gguf.cu — GGUF file -> device loader (SURVEY §8 row N2).
+// prima.cpp_b200/csrc/gguf.cu — GGUF file -> device loader.
 //
 // Replaces, for the tensors of the decode path: gguf_init_from_file (ggml/src/ggml.c, GGUF v2/v3 container: header, KV pairs, tensor
 // infos, aligned data section) + llm_load_hparams' key lookups (src/llama.cpp "%s.block_count", "%s.embedding_length", ...) +

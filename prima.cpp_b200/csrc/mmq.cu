@@ -1,7 +1,7 @@
 // prima.cpp_b200/csrc/mmq.cu — batched (prefill) k-quant mat-mul on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
 // Replaces: ggml_cuda_op_mul_mat_q -> mul_mat_q<type,mmq_x,8,chk> (ggml-cuda/mmq.cu:3-98, mmq.cuh:2583-2650: int8 mma.sync
-// tiles with __syncthreads ping-pong) and quantize_mmq_q8_1_cuda (quantize.cu:143-169), SURVEY §8 row a-4.
+// tiles with __syncthreads ping-pong) and quantize_mmq_q8_1_cuda (quantize.cu:143-169).
 // Numerics follow the CPU backend the oracle restates: every activation row is quantized to q8_K exactly as
 // quantize_row_q8_K_ref does (ggml-quants.c:3785-3822) and the weights are expanded with the dequantize_row_q{4,5,6}_K
 // formulas (ggml-quants.c:2040-2065, 2390-2420, 2690-2725) evaluated in fp16 (exact integer q, fp16 sub-block scale and

@@ -1,6 +1,6 @@
 // prima.cpp_b200/csrc/quantize.cuh — activation quantization, bit-exact with the CPU backend's from_float.
 //
-// Replaces (different numerics on purpose, see SURVEY §0 trap #1): quantize_q8_1 ggml-cuda/quantize.cu:4-38.
+// Replaces (different numerics on purpose: the CPU backend's): quantize_q8_1 ggml-cuda/quantize.cu:4-38.
 // Follows: quantize_row_q8_K_ref ggml-quants.c:3785-3822 (Q8_K), quantize_row_q8_0 AVX2 branch ggml-quants.c:943-1010
 // (Q8_0), quantize_row_q8_1 AVX2 branch ggml-quants.c:1260-1330 (Q8_1).
 // One warp quantizes 256 consecutive values: lane l owns x[8l .. 8l+7].

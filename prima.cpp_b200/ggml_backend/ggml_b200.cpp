@@ -2,7 +2,7 @@
 // implemented on top of the C ABI of libprima_b200.so.  Written against the interface, not against ggml-cuda.cu: buffers are
 // plain cudaMalloc regions, there is one stream per backend instance, graph_compute maps each node to one or two pb200_* calls.
 //
-// supports_op is exact (SURVEY §7.3 H6): only what the Llama / Qwen2 decode graph needs (build_llama / build_qwen2,
+// supports_op is exact: only what the Llama / Qwen2 decode graph needs (build_llama / build_qwen2,
 // src/llama.cpp:11000-11216, 12736-12916, FA off); everything else returns false so the scheduler keeps it on the CPU.
 #include "ggml-backend-impl.h"
 #include "ggml-backend.h"

@@ -14,7 +14,7 @@ COMPUTE_TYPES = {"bfloat16": 30, "bf16": 30, "float32": 0, "f32": 0}
 
 def lib_path() -> Path:
     import os
-    alt = os.environ.get("PB200_LIB")   # development only: A/B of two builds of the library on one box (tools/runs/*.sh)
+    alt = os.environ.get("PB200_LIB")   # development only: A/B of two builds of the library
     return Path(alt) if alt else PKG / "libprima_b200.so"
 
 

@@ -1,6 +1,5 @@
-"""Generates tests/golden/*.npz from the UNMODIFIED reference compiled into oracle/_ref (run in the build container where
-/root/reference exists:  python tests/golden/make_golden.py).  The fixtures travel with the repo; the GPU box never needs
-/root/reference."""
+"""Generates tests/golden/*.npz from the UNMODIFIED reference compiled into oracle/_ref (run where the reference's sources are,
+/root/reference:  python tests/golden/make_golden.py).  The fixtures are part of the repository: the tests never need the sources."""
 import sys
 from pathlib import Path
 

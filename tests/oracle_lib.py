@@ -2,7 +2,7 @@
 
 * ``port``  : oracle/liboracle_port.so — our plain-C restatement (oracle/kquants_port.c).
 * ``ref``   : oracle/_ref/{v3,v4}/libggml_ref.so + libgraph_ref.so — the UNMODIFIED reference CPU ggml
-              compiled from /root/reference (oracle/Makefile); travels to the GPU box pre-built.
+              compiled from the reference's sources (oracle/Makefile).
 Also: synthetic GGUF-block generators shared by the tests and bench.py's cpu legs.
 """
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""GGUF -> device loader (SURVEY N2).  CPU: the container parser (pb200_gguf_probe) against files written by the upstream gguf-py writer
+"""GGUF -> device loader.  CPU: the container parser (pb200_gguf_probe) against files written by the upstream gguf-py writer
 and against malformed files.  -m gpu: a model loaded by pb200_model_load_gguf decodes bit-identically to the same bytes handed over
 tensor by tensor with pb200_model_set_tensor, whole and as a layer-window shard."""
 import ctypes as C

@@ -1,5 +1,5 @@
 """-m gpu: the whole decode step (CUDA-graph replay of the fused launch sequence) against the CPU oracles.
-Bar (north_star): logits within 1e-3 max-abs of the reference CPU backend on identical GGUF weights and prompts."""
+Bar: logits within 1e-3 max-abs of the reference CPU backend on identical GGUF weights and prompts."""
 from pathlib import Path
 
 import numpy as np
@@ -16,7 +16,7 @@ TOL = 1e-3
 def check_decode_parity(got, want):
     """Multi-token parity bar.  Until the first activation-quantization / f16 flip (see the comment above
     test_engine_vs_port_longer_decode) the logits agree to fp32 summation order; after it the deviation is the same noise the
-    reference's own AVX2 and AVX-512 CPU builds show against each other on these models (measured in DESIGN.md §parity:
+    reference's own AVX2 and AVX-512 CPU builds show against each other on these models (tests/test_reference_self_divergence.py:
     0.04-0.05 max-abs, onset at token 4-18).  So: first token exact, NMSE over the run below the reference's whole-block bar
     (2e-3, tests/test-backend-ops.cpp:3000), max-abs bounded, greedy tokens (argmax) agree on >= 90 % of the steps."""
     e = np.max(np.abs(got - want), axis=1)
@@ -81,7 +81,7 @@ def test_engine_vs_compiled_reference(cuda, pkg, ref):
 
 
 def test_engine_llama3_70b_layer_shapes_vs_compiled_reference(cuda, pkg, ref):
-    """Whole-engine parity at the BASELINE config's layer shapes: 2 full-size Llama-3-70B layers (n_embd 8192, 64/8 heads,
+    """Whole-engine parity at the benchmark's layer shapes: 2 full-size Llama-3-70B layers (n_embd 8192, 64/8 heads,
     n_ff 28672: the split-row ffn_down kernel, the 3-matrix q|k|v launch, the Q5_K / Q6_K v and down of the Q4_K_M mixture) + a
     small vocabulary, decoded token by token against the UNMODIFIED reference CPU backend (oracle/_ref) on the same quantized bytes."""
     tm = TinyModel(n_layer=2, n_embd=8192, n_head=64, n_head_kv=8, n_ff=28672, n_vocab=512, n_ctx=32, arch="llama", ftype="q4_K_M", seed=21,

@@ -46,5 +46,3 @@ def test_backend_perf_mode_mul_mat(cuda):
     assert rc == 0, out[-2000:]
     lines = [l for l in out.splitlines() if "q4_K" in l and "n=1," in l]
     assert lines, out[-2000:]
-    (ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / "test_backend_ops_perf.txt").write_text(out)

@@ -237,7 +237,7 @@ def test_attn_prefill_vs_oracle(cuda, lib, port, H, HK, n_tok, pos0):
 
 
 def test_full_size_gemv_properties(cuda, lib):
-    """BASELINE sizes (Llama-3-70B shapes): the fused TMA kernel must agree with an independent evaluation —
+    """Llama-3-70B shapes: the fused TMA kernel must agree with an independent evaluation —
     dequantized weights (get_rows kernel, bit-exact vs the oracle above) times the dequantized q8_K activation in fp64."""
     import gpu_util
     # N large enough that every CTA streams > 4 tiles: exercises the mbarrier ring wrap-around and both parities

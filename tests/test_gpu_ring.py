@@ -1,5 +1,5 @@
 """-m gpu: sequence slots of the engine, device-resident token / position / greedy argmax, and (with >= 2 GPUs) the ring of
-sequences across NCCL ranks against single-process decoding — bit for bit (same kernels, same order; SURVEY §8e)."""
+sequences across NCCL ranks against single-process decoding — bit for bit (same kernels, same order)."""
 import ctypes as C
 import os
 import socket
@@ -139,7 +139,7 @@ def _ring_rank(rank, world, port, rounds, q):
 def test_ring_across_nccl_ranks_bit_identical_to_single_process(cuda, pkg):
     world = 2
     if torch.cuda.device_count() < world:
-        pytest.skip("needs 2 GPUs (run with gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
     rounds = 5
     want = greedy_reference(_model(), pkg, [(5 + 9 * s, s) for s in range(world)], rounds)

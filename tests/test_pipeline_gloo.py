@@ -1,5 +1,5 @@
 """CPU: the N>1 host logic (layer windows + hidden-state hand-off + token ring) over gloo, world_size 2 and 3, against a
-single-process run of the same toy layers (bit-identical, like the N-rank == 1-rank requirement of SURVEY §8e)."""
+single-process run of the same toy layers (bit-identical: N ranks compute what one does)."""
 import os
 import socket
 

@@ -1,4 +1,4 @@
-"""CPU: how far the REFERENCE is from ITSELF.  north_star asks for <= 1e-3 max-abs on logits against the reference CPU backend.
+"""CPU: how far the REFERENCE is from ITSELF.  The single-token bar is <= 1e-3 max-abs on logits against the reference CPU backend.
 The reference's own AVX2 (x86-64-v3) and AVX-512 (x86-64-v4) builds of ggml-quants.c / ggml.c sum the same integer dot products in
 different fp32 orders; one ulp of difference in an activation flips `round(x * 127 / amax)` of a q8_K code now and then, the flip is
 a ~3e-4 relative kick to one mat-vec output and it stays in the KV cache.  This test measures that divergence on the model the GPU
