@@ -34,7 +34,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -768,13 +767,9 @@ bool mmq_supported(int type, int64_t K) {
 }
 
 template <int TYPE, int CG, bool CUT>
-static cudaError_t mmq_allow_smem(size_t smem) {
-    static FuncAttrCache attr_cache;
-    return ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
-}
-template <int TYPE, int CG, bool CUT>
 static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st) {
-    cudaError_t e = mmq_allow_smem<TYPE, CG, CUT>(smem);
+    static FuncAttrCache attr_cache;
+    cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -793,29 +788,12 @@ static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size
     if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, grid, smem, st);
     return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, grid, smem, st) : mmq_launch_typed2<TYPE, 1, false>(P, grid, smem, st);
 }
-// clusters of `parts` CTAs of this kernel that run at the same time (a CTA takes an SM; a cluster stays within a group of SMs)
-static int mmq_clusters(int parts) {
-    static std::atomic<int> known[MMQ_MAX_PARTS + 1];
-    int n = known[parts].load(std::memory_order_relaxed);
-    if (n == 0) {
-        const size_t smem = 160 * 1024;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned) (parts * 148));
-        cfg.blockDim = dim3(MMQ_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned) parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (mmq_allow_smem<T_Q4_K, 1, true>(smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, (const void *) k_mmq_tc<T_Q4_K, 1, true>, &cfg) != cudaSuccess || n <= 0) {
-            cudaGetLastError();
-            n = -1;
-        }
-        known[parts].store(n, std::memory_order_relaxed);
-    }
-    return std::max(n, 0);
+// Clusters of `parts` CTAs of this kernel that run at the same time (a CTA takes an SM; a cluster stays within a group of SMs): what
+// cudaOccupancyMaxActiveClusters says on a B200, 5 and 7 from below.  A table and no query, so that the order of a sum does not follow which SMs of a GPU
+// are there; where fewer clusters fit, the rest of them come after.
+static int mmq_clusters(int parts, int nsm) {
+    constexpr int of_148[MMQ_MAX_PARTS + 1] = {0, 148, 74, 45, 33, 24, 22, 16, 15};
+    return of_148[parts] * nsm / 148;
 }
 
 // How a launch's tiles are shared:
@@ -847,12 +825,12 @@ static MmqCut mmq_pick_cut(int64_t tiles, int ngrp, int nsm, int max_parts, doub
     for (int m = 2; m <= 8; m++)
         if (mmq_chain_ctas(tiles, m) <= nsm) consider({1, m, 0}, (m * ngrp + m) / (m + 1) * unit + 2 * seg + clear);
     // two halves: by a cluster or a chain of one tile, whichever is the faster one for these tokens; the bits are the same
-    const bool pairs = max_parts >= 2 && tiles <= mmq_clusters(2);
+    const bool pairs = max_parts >= 2 && tiles <= mmq_clusters(2, nsm);
     if (tiles * 2 <= nsm && ngrp >= 2)
         consider(pairs && 10.0 * tokens <= 3.0 * 512.0 + (double) tiles * tile_us * tokens ? MmqCut{2, 0, 0} : MmqCut{1, 1, 0}, (ngrp + 1) / 2 * unit + seg + std::min(10.0, clear));
     for (int p = 3; p <= max_parts && p <= ngrp && tiles * p <= nsm; p++) {
         const double us = (ngrp + p - 1) / p * unit + seg + 7.5 + 1.25 * p;
-        if (us < best_us && tiles <= mmq_clusters(p)) consider({p, 0, 0}, us);
+        if (us < best_us && tiles <= mmq_clusters(p, nsm)) consider({p, 0, 0}, us);
     }
     return best;
 }
