@@ -74,7 +74,16 @@ int pb200_mul_mat_vec_q(int type, const void * W, int64_t n, int64_t k, const vo
 }
 
 int pb200_mul_mat_vec(int type, const void * W, int64_t n, int64_t k, const float * x, float * y, void * act_ws, void * stream) {
-    int e = pb200_quantize_act(type, x, k, act_ws, stream);
+    if (!type_ok(type) || !W || !x || !act_ws || !y || n <= 0 || k <= 0 || k % block_elems(type) != 0) return PB200_EINVAL;
+    if (gemv_quant_prologue_ok(type, W, (int) n, (int) k, x)) {
+        const GemvDesc d = {W, y, nullptr, nullptr, type, (int) n};
+        GemvFused pro;
+        pro.kind = GEMV_PRO_QUANT;
+        pro.in0 = x;
+        g_launches++;
+        return launch_gemv_kquant_fused(&d, 1, (int) k, act_from_ws(act_ws, k), pro, (cudaStream_t) stream, true);
+    }
+    const int e = pb200_quantize_act(type, x, k, act_ws, stream);
     if (e) return e;
     return pb200_mul_mat_vec_q(type, W, n, k, act_ws, y, nullptr, nullptr, stream);
 }

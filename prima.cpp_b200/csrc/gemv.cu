@@ -22,6 +22,9 @@ static_assert(sizeof(GemvSmemCtl) <= GEMV_CTL_BYTES, "ctl block");
 
 __device__ __forceinline__ float silu_f(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }   // ggml.c:2560
 
+// instantiations of the kernel: plain; with time stamps; quantizing its own activation (PRO_QUANT, gemv.cuh)
+enum : int { GV_PLAIN = 0, GV_TRACE = 1, GV_QUANT = 2 };
+
 // TRACE instantiation only: slot k (0..5) of this CTA's 8-entry row = %globaltimer (ns) at stamp k; slots 6 / 7 = clock64 at
 // the first / last stamp (the SM clock during the launch follows from the two)
 template <bool TRACE>
@@ -81,14 +84,16 @@ __device__ __forceinline__ void release_stage(const GemvParams & P, GemvSmemCtl 
     }
 }
 
+// initial stages from `first` on, by one thread
+__device__ __forceinline__ void fill_from(const GemvParams & P, GemvSmemCtl * ctl, uint8_t * stages, uint64_t pol, int first) {
+    for (int it = first; it < P.nstage_init; it++) {
+        const int t = blockIdx.x + it * gridDim.x;
+        if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
+    }
+}
 // initial stages that were held back until the activation loads had been issued (P.prefill < P.nstage_init)
 __device__ __forceinline__ void fill_rest(const GemvParams & P, GemvSmemCtl * ctl, uint8_t * stages, uint64_t pol) {
-    if (threadIdx.x == 0) {
-        for (int it = P.prefill; it < P.nstage_init; it++) {
-            const int t = blockIdx.x + it * gridDim.x;
-            if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
-        }
-    }
+    if (threadIdx.x == 0) fill_from(P, ctl, stages, pol, P.prefill);
 }
 
 // TYPE = weight type of every matrix of the launch (one dot routine in the hot loop: the three unrolled routines together are
@@ -158,6 +163,26 @@ __device__ __forceinline__ void dist_prologue(const GemvParams & P, GemvSmemCtl 
         quantize_warp_q8K(bx, lane, b, P.act);
     }
 }
+// ---- PRO_QUANT: every CTA quantizes the whole activation in0 into its shared memory; super-block b also goes to P.act, from CTA b mod grid (what a
+// caller finds in its workspace is the same as behind a quantizing kernel).  The weights' first tiles travel meanwhile ----
+__device__ __forceinline__ void quant_prologue(const GemvParams & P, GemvSmemCtl * ctl, uint8_t * stages, const ActQ & sa, int warp, int lane, uint64_t pol) {
+    const int nblk = P.nblk;
+    for (int b0 = warp; b0 < nblk; b0 += GEMV_NW * PRO_B) {
+        float x[PRO_B][8];
+#pragma unroll
+        for (int j = 0; j < PRO_B; j++)
+            if (b0 + j * GEMV_NW < nblk) load8(P.in0 + (b0 + j * GEMV_NW) * 256 + lane * 8, x[j]);
+        if (b0 == GEMV_NW - 1 && lane == 0) fill_from(P, ctl, stages, pol, 0);   // the last warp has the fewest super-blocks
+#pragma unroll
+        for (int j = 0; j < PRO_B; j++) {
+            const int b = b0 + j * GEMV_NW;
+            if (b >= nblk) break;
+            quantize_warp_q8K(x[j], lane, b, sa);
+            if (b % (int) gridDim.x == (int) blockIdx.x) quantize_warp_q8K(x[j], lane, b, P.act);
+        }
+    }
+    if (nblk < GEMV_NW && warp == GEMV_NW - 1 && lane == 0) fill_from(P, ctl, stages, pol, 0);
+}
 // All CTAs of the launch meet once.  Safe because the persistent grid is co-resident by construction (launcher: grid <= 2 x SMs,
 // gemv_dist_prologue_ok()); bounded like every other wait.  State = {arrivals, departures}; the last CTA to leave re-arms both.
 __device__ __forceinline__ void grid_barrier(const GemvParams & P, GemvSmemCtl * ctl) {
@@ -197,8 +222,9 @@ __device__ __forceinline__ void finish_split_row(const GemvParams & P, GemvSmemC
     }
 }
 
-template <int TYPE, bool SPLIT, bool TRACE>
+template <int TYPE, bool SPLIT, int VAR>
 __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(const __grid_constant__ GemvParams P) {
+    constexpr bool TRACE = VAR == GV_TRACE;
     extern __shared__ __align__(128) uint8_t smem[];
     GemvSmemCtl * ctl = reinterpret_cast<GemvSmemCtl *>(smem);
     uint8_t * stages = smem + GEMV_CTL_BYTES;
@@ -226,7 +252,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
     pdl_trigger();   // the next kernel's CTAs may take this SM's free slots as soon as CTAs of this grid exit
     // Weights never depend on the previous kernel: start streaming BEFORE griddepcontrol.wait.  Under PDL this CTA is resident
     // while the tail of the previous GEMV (or a whole small kernel: attention, silu-quant) still runs on other SMs.
-    if (threadIdx.x == 0) {
+    // (GV_QUANT serves callers whose weights may be the previous kernel's result: nothing is read before the wait.)
+    if (VAR != GV_QUANT && threadIdx.x == 0) {
         for (int it = 0; it < P.prefill; it++) {
             const int t = blockIdx.x + it * gridDim.x;
             if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
@@ -287,6 +314,11 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
 #pragma unroll
             for (int j = 0; j < 8; j++) { r.d8[j] = sd[blk * 8 + j]; r.s8[j] = TYPE == T_Q5_1 ? ss[blk * 8 + j] : 0.f; }
         }
+    } else if (VAR == GV_QUANT) {
+        quant_prologue(P, ctl, stages, sa, warp, lane, pol);
+        __syncthreads();
+        load_act_regs(r, sa, blk, valid);
+        finish_act_regs(r);
     } else {
         // ONE coalesced copy of the quantized activation per CTA (qs | bsums | d), staged with the padded strides
         constexpr int NQ_MAX = (GEMV_ACT_MAX_NBLK * 16 + GEMV_THREADS - 1) / GEMV_THREADS;   // int4 of qs per thread (7)
@@ -797,13 +829,21 @@ bool gemv_dist_prologue_ok() {
     if (!cache[dev]) {
         int per_sm = 0;
         static FuncAttrCache tmp;
-        bool ok = ensure_dyn_smem(tmp, (const void *) k_gemv_kquant<T_Q4_K, false, false>, GEMV_SMEM_LIMIT, true) == cudaSuccess &&
-                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemv_kquant<T_Q4_K, false, false>, GEMV_THREADS, GEMV_SMEM_LIMIT) == cudaSuccess &&
+        bool ok = ensure_dyn_smem(tmp, (const void *) k_gemv_kquant<T_Q4_K, false, GV_PLAIN>, GEMV_SMEM_LIMIT, true) == cudaSuccess &&
+                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemv_kquant<T_Q4_K, false, GV_PLAIN>, GEMV_THREADS, GEMV_SMEM_LIMIT) == cudaSuccess &&
                   per_sm >= GEMV_CTAS_PER_SM;
         if (!ok) cudaGetLastError();
         cache[dev] = ok ? 1 : 2;
     }
     return cache[dev] == 1;
+}
+// Up to this length every CTA quantizes the activation for itself; above it a kernel in front does.  us per call, two launches / one: Q4_K 1000 x 2048
+// 9.1 / 4.6, 4096 x 4096 12.1 / 6.4, 14336 x 4096 14.8 / 9.3, 4096 x 14336 16.5 / 15.2, 28672 x 14336 47.2 / 44.5, Q6_K 1000 x 14336 12.4 / 11.2; but
+// Q5_K 301 x 28672 12.3 / 15.8: there 14 super-blocks a warp, one after the other, are what the call waits for.
+constexpr int GEMV_QUANT_MAX_K = 16384;
+bool gemv_quant_prologue_ok(int type, const void * W, int N, int K, const float * x) {
+    GemvPlan pl;
+    return is_kquant(type) && K <= GEMV_QUANT_MAX_K && (((uintptr_t) W | (uintptr_t) x) & 15) == 0 && gemv_plan(&type, &N, 1, K, pl);
 }
 int gemv_smem_bytes(int type, int K, int N) {
     GemvPlan pl;
@@ -879,19 +919,26 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     int ty = types[0];
     for (int i = 1; i < nmat; i++) if (types[i] != ty) ty = 0;
     const int ti = ty == T_Q4_K ? 1 : ty == T_Q5_K ? 2 : ty == T_Q6_K ? 3 : ty == T_Q8_0 ? 4 : ty == T_Q5_1 ? 5 : 0;
-    const bool tr = g_trace_buf != nullptr;
+    const int var = pro.kind == PRO_QUANT ? GV_QUANT : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
     typedef void (*kern_t)(const GemvParams);
-    static const kern_t table[6][2][2] = {
-        {{k_gemv_kquant<0, false, false>, k_gemv_kquant<0, false, true>}, {k_gemv_kquant<0, true, false>, k_gemv_kquant<0, true, true>}},
-        {{k_gemv_kquant<T_Q4_K, false, false>, k_gemv_kquant<T_Q4_K, false, true>}, {k_gemv_kquant<T_Q4_K, true, false>, k_gemv_kquant<T_Q4_K, true, true>}},
-        {{k_gemv_kquant<T_Q5_K, false, false>, k_gemv_kquant<T_Q5_K, false, true>}, {k_gemv_kquant<T_Q5_K, true, false>, k_gemv_kquant<T_Q5_K, true, true>}},
-        {{k_gemv_kquant<T_Q6_K, false, false>, k_gemv_kquant<T_Q6_K, false, true>}, {k_gemv_kquant<T_Q6_K, true, false>, k_gemv_kquant<T_Q6_K, true, true>}},
-        {{k_gemv_kquant<T_Q8_0, false, false>, k_gemv_kquant<T_Q8_0, false, true>}, {k_gemv_kquant<T_Q8_0, true, false>, k_gemv_kquant<T_Q8_0, true, true>}},
-        {{k_gemv_kquant<T_Q5_1, false, false>, k_gemv_kquant<T_Q5_1, false, true>}, {k_gemv_kquant<T_Q5_1, true, false>, k_gemv_kquant<T_Q5_1, true, true>}}};
-    static FuncAttrCache attr_cache[6][2][2];
+    static const kern_t table[6][2][3] = {
+        {{k_gemv_kquant<0, false, GV_PLAIN>, k_gemv_kquant<0, false, GV_TRACE>, nullptr},
+         {k_gemv_kquant<0, true, GV_PLAIN>, k_gemv_kquant<0, true, GV_TRACE>, nullptr}},
+        {{k_gemv_kquant<T_Q4_K, false, GV_PLAIN>, k_gemv_kquant<T_Q4_K, false, GV_TRACE>, k_gemv_kquant<T_Q4_K, false, GV_QUANT>},
+         {k_gemv_kquant<T_Q4_K, true, GV_PLAIN>, k_gemv_kquant<T_Q4_K, true, GV_TRACE>, k_gemv_kquant<T_Q4_K, true, GV_QUANT>}},
+        {{k_gemv_kquant<T_Q5_K, false, GV_PLAIN>, k_gemv_kquant<T_Q5_K, false, GV_TRACE>, k_gemv_kquant<T_Q5_K, false, GV_QUANT>},
+         {k_gemv_kquant<T_Q5_K, true, GV_PLAIN>, k_gemv_kquant<T_Q5_K, true, GV_TRACE>, k_gemv_kquant<T_Q5_K, true, GV_QUANT>}},
+        {{k_gemv_kquant<T_Q6_K, false, GV_PLAIN>, k_gemv_kquant<T_Q6_K, false, GV_TRACE>, k_gemv_kquant<T_Q6_K, false, GV_QUANT>},
+         {k_gemv_kquant<T_Q6_K, true, GV_PLAIN>, k_gemv_kquant<T_Q6_K, true, GV_TRACE>, k_gemv_kquant<T_Q6_K, true, GV_QUANT>}},
+        {{k_gemv_kquant<T_Q8_0, false, GV_PLAIN>, k_gemv_kquant<T_Q8_0, false, GV_TRACE>, nullptr},
+         {k_gemv_kquant<T_Q8_0, true, GV_PLAIN>, k_gemv_kquant<T_Q8_0, true, GV_TRACE>, nullptr}},
+        {{k_gemv_kquant<T_Q5_1, false, GV_PLAIN>, k_gemv_kquant<T_Q5_1, false, GV_TRACE>, nullptr},
+         {k_gemv_kquant<T_Q5_1, true, GV_PLAIN>, k_gemv_kquant<T_Q5_1, true, GV_TRACE>, nullptr}}};
+    static FuncAttrCache attr_cache[6][2][3];
     const int si = pl.wpr > 1 ? 1 : 0;
-    const kern_t fn = table[ti][si][tr ? 1 : 0];
-    cudaError_t e = ensure_dyn_smem(attr_cache[ti][si][tr ? 1 : 0], (const void *) fn, GEMV_SMEM_LIMIT, true);
+    if (pro.kind == PRO_QUANT && ti == 0) return (int) cudaErrorInvalidValue;
+    const kern_t fn = table[ti][si][var];
+    cudaError_t e = ensure_dyn_smem(attr_cache[ti][si][var], (const void *) fn, GEMV_SMEM_LIMIT, true);
     if (e != cudaSuccess) return (int) e;
     int grid = sm_count() * GEMV_CTAS_PER_SM;
     if (grid > P.ntiles) grid = P.ntiles;

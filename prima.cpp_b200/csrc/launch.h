@@ -17,8 +17,9 @@ struct GemvDesc {
     int N;
 };
 
+constexpr int GEMV_PRO_QUANT = 6;
 struct GemvFused {       // fused activation prologue of the k-quant GEMV (PRO_* in gemv.cuh)
-    int kind = 0;        // 0 none (activation already quantized), 4 rms_norm(in0)*in1, 5 silu(in0)*in1 — distributed over the grid (PRO_* in gemv.cuh)
+    int kind = 0;        // 0 none (activation already quantized), 4 rms_norm(in0)*in1, 5 silu(in0)*in1 — distributed over the grid; 6 in0 itself (PRO_* in gemv.cuh)
     const float * in0 = nullptr;
     const float * in1 = nullptr;
     float eps = 0.f;
@@ -44,6 +45,7 @@ int gemv_smem_bytes(int type, int K, int N);        // dynamic shared memory of 
 int launch_gemv_kquant(const GemvDesc * d, int nmat, int K, const ActQ & act, cudaStream_t stream, bool pdl);
 int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & act, const GemvFused & pro, cudaStream_t stream, bool pdl);
 bool gemv_fused_prologue_ok(int K);
+bool gemv_quant_prologue_ok(int type, const void * W, int N, int K, const float * x);   // kind 6 takes this product and is the faster way
 bool gemv_dist_prologue_ok();   // the full persistent grid is co-resident on the current device (needed by the in-kernel grid barrier)
 // any supported type / any K, one warp per row, direct global loads
 int launch_gemv_generic(const GemvDesc & d, int K, const ActQ & act, cudaStream_t stream, bool pdl);
