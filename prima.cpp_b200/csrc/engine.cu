@@ -371,7 +371,9 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
         const bool wo_k = is_kquant(L.wo.type) && gemv_fused_prologue_ok(QD);
         bool att_quantized = false;
         if (wo_k && attn_v2) {   // clustered attention writes the q8_K activation of wo itself
-            const int rc = launch_attn_fused2(m->q, m->k, m->v, kc, vc, m->att, m->actQD.q, H, HK, D, pos_dev, hp.n_ctx, m->rp, m->rope_ff, kq_scale, st, pdl);
+            int rc = launch_attn_group(m->q, m->k, m->v, kc, vc, m->att, m->actQD.q, H, HK, D, pos_dev, hp.n_ctx, m->rp, m->rope_ff, kq_scale, st, pdl);
+            if (rc == (int) cudaErrorNotSupported)
+                rc = launch_attn_fused2(m->q, m->k, m->v, kc, vc, m->att, m->actQD.q, H, HK, D, pos_dev, hp.n_ctx, m->rp, m->rope_ff, kq_scale, st, pdl);
             if (rc == 0) { att_quantized = true; n++; }
             else if (rc != (int) cudaErrorNotSupported) return rc;
         }

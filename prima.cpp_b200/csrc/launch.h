@@ -102,7 +102,12 @@ int launch_attn_fused2(const float * q, const float * k, const float * v, __half
                        int n_head_kv, int D, const int32_t * pos_dev, int n_ctx, const RopeParams & rp, const float * freq_factors, float scale,
                        cudaStream_t stream, bool pdl);
 
-// the same kernel on the reference graph's tensors (FA off, one token): K cache [cell][n_head_kv*128] f16, V cache TRANSPOSED
+// the same for groups of 2, 4 or 8 query heads to a kv head (attn_group.cu): the cells over a cluster of CTAs, each of which serves the whole group;
+// cudaErrorNotSupported otherwise
+int launch_attn_group(const float * q, const float * k, const float * v, __half * kcache, __half * vcache, float * out, const ActQ & outq, int n_head, int n_head_kv, int D,
+                      const int32_t * pos_dev, int n_ctx, const RopeParams & rp, const float * freq_factors, float scale, cudaStream_t stream, bool pdl);
+
+// launch_attn_fused2's kernel on the reference graph's tensors (FA off, one token): K cache [cell][n_head_kv*128] f16, V cache TRANSPOSED
 // [n_head_kv*128][vt_stride] f16, additive f32 mask row over n_cells (multiple of 32) cells, this token stored in cell kv_head
 int launch_attn_ggml(const float * q, const float * k, const float * v, __half * kcache, __half * vcache_t, int64_t vt_stride, float * out, const ActQ & outq,
                      int n_head, int n_head_kv, int D, const int32_t * pos_dev, int n_cells, int kv_head, const int32_t * kv_head_dev, const float * mask,

@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256) k_attn_fused(const float * __restrict__ q
 }
 
 // ------------------------------------------------------------------------------------------------
-// Decode attention v2 (the engine's per-token path): same arithmetic as k_attn_fused, restructured for LATENCY — under PDL this
+// Decode attention v2 (the ggml plugin's per-token path, and the engine's where attn_group.cu has no kernel for the group of heads): same arithmetic as k_attn_fused, restructured for LATENCY — under PDL this
 // kernel sits between the q|k|v GEMV and the wo GEMV, and every microsecond of it is a bubble in the weight stream:
 //   * one CTA of 16 warps per q head, launched as CLUSTERS OF 2 (heads 2j, 2j+1 = one 256-value q8_K super-block of the output):
 //     the pair agrees on the block's arg-max through distributed shared memory and writes the QUANTIZED activation itself,
