@@ -116,3 +116,44 @@ def test_other_alignments(cuda, lib, H, G, T, pos0, q_off, kv_off):
         flat[by:by + t.numel()] = t.reshape(-1)
         return flat[by:by + t.numel()].view(t.shape)
     check(lib, shifted(q, q_off), shifted(k, kv_off), shifted(v, kv_off), torch.arange(pos0, pos0 + T, dtype=torch.int32, device="cuda"), 128 ** -0.5)
+
+
+def test_more_tiles_than_the_machine_holds(cuda, lib):
+    """A CTA takes several items in a row: 8 tokens of 16 heads each, 51 x 8 items over at most two CTAs an SM, ragged at the end."""
+    q, k, v = inputs(405, 128, 8, 405, seed=9)
+    import torch
+    pos = torch.arange(0, 405, dtype=torch.int32, device="cuda")
+    full = check(lib, q, k, v, pos, 128 ** -0.5)
+    pos[40:56] = -1                   # two items' tokens see nothing: one is its CTA's first item, one its second
+    pos[392:400] = -1
+    out = check(lib, q, k, v, pos, 128 ** -0.5)
+    live = pos >= 0
+    assert bool((out[~live] == 0).all()) and torch.equal(out[live], full[live])
+
+
+def test_scores_that_grow_and_fall(cuda, lib):
+    """A row's reference moves on when a tile's score is beyond it by more than 2^8: in every tile, in none behind the first, in some rows of a warp only."""
+    import torch
+    q, k, v = inputs(64, 8, 2, 900, seed=10)
+    pos = torch.arange(836, 900, dtype=torch.int32, device="cuda")
+    at = torch.arange(900, device="cuda")[:, None, None]
+    for grow in (0.3 + at / 60.0, 8.0 - at / 130.0, torch.where(at // 128 % 2 == 0, 0.1, 6.0)):
+        kk = (k.float() * grow).half()
+        kk[:, 1] = k[:, 1]            # the second group's rows stay as they are
+        check(lib, q, kk, v, pos, 128 ** -0.5)
+    some = q.clone()
+    some[::3] *= 0.01
+    check(lib, some, (k.float() * (0.3 + at / 60.0)).half(), v, pos, 128 ** -0.5)
+
+
+def test_a_score_that_is_no_number_takes_its_rows(cuda, lib):
+    import torch
+    q, k, v = inputs(64, 4, 4, 264, seed=11)
+    pos = torch.arange(200, 264, dtype=torch.int32, device="cuda")
+    clean = run(lib, q, k, v, pos, 0.1)
+    for bad in (float("nan"), float("inf")):
+        kb = k.clone()
+        kb[230, 1] = bad              # an infinite key: products of both signs meet
+        out = run(lib, q, kb, v, pos, 0.1)
+        assert torch.equal(out[:30], clean[:30]) and torch.equal(out[:, [0, 2, 3]], clean[:, [0, 2, 3]])
+        assert not bool(torch.isfinite(out[30:, 1]).any())
