@@ -288,6 +288,11 @@ typedef struct pb200_batch_entry {
     int32_t n_want;
     const int32_t * want;
 } pb200_batch_entry;
+/* Page-locked host memory for logits_host, out of a pool of fixed size that a layer-list model holds from pb200_model_finalize on: the rows arrive in it without a
+ * copy through a staging buffer (as in any page-locked memory of the caller's).  NULL: the pool has no room, use any other memory.  A block stays valid until it is
+ * given back, also beyond the model's end.  Both calls may come from any thread. */
+PB200_API void * pb200_result_take(pb200_model * m, size_t bytes);
+PB200_API int    pb200_result_give(void * block);
 PB200_API int pb200_batch_step(pb200_model * m, int n_entries, const pb200_batch_entry * entries, float * logits_host, int32_t * greedy_host);
 /* white-box tests: on != 0 keeps the residual stream after every layer run of the next batches; read it with
  * pb200_debug_read(m, "layers", host, runs * tokens * n_embd) */

@@ -228,9 +228,11 @@ struct LayerList {
     float *moe_wt = nullptr, *moe_gu = nullptr, *moe_ds = nullptr, *moe_sg = nullptr;
     void *moe_y = nullptr, *moe_hs = nullptr;
     int32_t *meta_dev = nullptr, *meta_host = nullptr, *greedy_dev = nullptr, *greedy_host = nullptr;
-    float * logits_host = nullptr;
+    float * logits_host = nullptr;   // staging of wanted rows on their way to ordinary memory
+    ResultPool * results = nullptr;
     size_t meta_cap = 0, logits_host_cap = 0;
-    static constexpr int ROW_PARTS = 4;
+    static constexpr int ROW_PARTS = 4, DIRECT_RUNS = 16;
+    static constexpr size_t RESULT_BYTES = 32u << 20;   // the logits of 32 steps of eight requests over 32 000 tokens
     cudaEvent_t ev_rows[ROW_PARTS] = {};   // a part of the wanted logits has arrived in logits_host
     std::vector<void *> scratch;
     // white-box tap: residual stream after every layer run of the last batch
@@ -1800,6 +1802,7 @@ int ll_finalize(pb200_model * m) {
     ll.seq_prev.assign((size_t) ll.n_seq, -1);
     m->n_seq = ll.n_seq;
     m->weight_bytes = ll.weight_bytes;
+    ll.results = result_pool_create(LayerList::RESULT_BYTES);   // none: every step's logits go through the staging buffer
     m->finalized = true;
     return 0;
 }
@@ -1814,6 +1817,7 @@ void ll_free(pb200_model * m) {
     if (ll->meta_host) cudaFreeHost(ll->meta_host);
     if (ll->greedy_host) cudaFreeHost(ll->greedy_host);
     if (ll->logits_host) cudaFreeHost(ll->logits_host);
+    result_pool_release(ll->results);
     if (ll->moe_count_host) cudaFreeHost(ll->moe_count_host);
     if (ll->lat_part) cudaFree(ll->lat_part);
     if (ll->split_ws) cudaFree(ll->split_ws);
@@ -1993,14 +1997,6 @@ static int ll_reserve(pb200_model * m, int T, int nW, int nE, bool long_prompt) 
         CK(cudaMalloc((void **) &ll.meta_dev, cap * 4));
         CK(cudaMallocHost((void **) &ll.meta_host, cap * 4));
         ll.meta_cap = cap;
-    }
-    const size_t need_lh = (size_t) std::max(nW, 1) * (size_t) ll.vocab;
-    if (need_lh > ll.logits_host_cap) {
-        CK(cudaStreamSynchronize(m->stream));
-        if (ll.logits_host) cudaFreeHost(ll.logits_host);
-        ll.logits_host = nullptr; ll.logits_host_cap = 0;
-        CK(cudaMallocHost((void **) &ll.logits_host, need_lh * 4));
-        ll.logits_host_cap = need_lh;
     }
     // scratch of the split prompt attention by this call's own tokens and entries: which kernel runs does not depend on what ran before.
     // PB200_ATTN_SPLIT: 0 = prompts keep the fp32 FMA attention, 1 = float32 models take the split kernel as well (A/B runs, tests)
@@ -2756,7 +2752,18 @@ static void for_row_runs(const std::vector<int> & lrows, size_t k0, size_t k1, F
     }
 }
 
-// dst (may be null): the caller's logits.  While the device works the host touches the pages the rows will go to (a fresh buffer has none yet), and the rows
+static int ll_reserve_staging(pb200_model * m, int nW) {
+    LayerList & ll = *m->ll;
+    const size_t need = (size_t) nW * (size_t) ll.vocab;
+    if (need <= ll.logits_host_cap) return 0;
+    if (ll.logits_host) cudaFreeHost(ll.logits_host);   // a step returns with everything it copies in place
+    ll.logits_host = nullptr; ll.logits_host_cap = 0;
+    CK(cudaMallocHost((void **) &ll.logits_host, need * 4));
+    ll.logits_host_cap = need;
+    return 0;
+}
+
+// dst (may be null): the caller's logits.  Rows for page-locked memory go there at once, run by run.  Otherwise, while the device works, the host touches the pages the rows will go to (a fresh buffer has none yet), and the rows
 // come over in up to four parts, one being handed to the caller while the next is on its way: eight rows of 32 000 logits, a decode step of eight requests: 636 -> 540 us
 static int ll_run_sub(pb200_model * m, std::vector<SubEntry> & es, bool prefill, float * dst) {
     LayerList & ll = *m->ll;
@@ -2783,6 +2790,14 @@ static int ll_run_sub(pb200_model * m, std::vector<SubEntry> & es, bool prefill,
         for (const auto & pr : es[(size_t) i].want) { h_want[w++] = h_off[i] + pr.first; lrows.push_back(pr.second); }
     int32_t * h_prev = h_want + nW;   // the token before each entry's first one (-1: none)
     for (int i = 0; i < nE; i++) h_prev[i] = es[(size_t) i].pos0 > 0 ? ll.seq_prev[(size_t) es[(size_t) i].slot] : -1;
+    // where the wanted rows go: at once to the caller (few runs of neighbours, all page-locked), through the staging buffer, or nowhere
+    const size_t V = (size_t) ll.vocab;
+    int runs = 0;
+    bool direct = dst != nullptr;
+    if (dst) for_row_runs(lrows, 0, (size_t) nW, [&](size_t, int row, size_t n) { direct = direct && ++runs <= LayerList::DIRECT_RUNS && result_direct(dst + (size_t) row * V, n * V * 4); });
+    direct = direct && runs > 0;
+    const bool staged = dst && !direct;
+    if (staged) CK(ll_reserve_staging(m, nW));
     const size_t total = (size_t) (h_prev + nE - h);
     int32_t * d = ll.meta_dev;
     CK(cudaMemcpyAsync(d, h, total * 4, cudaMemcpyHostToDevice, m->stream));
@@ -2814,8 +2829,14 @@ static int ll_run_sub(pb200_model * m, std::vector<SubEntry> & es, bool prefill,
         }
     }
     if (!ran) CK(ll_forward(m, b, prefill, d, d + (h_want - h), nW, 0));
-    const size_t V = (size_t) ll.vocab;
-    const int parts = (int) std::min<size_t>(LayerList::ROW_PARTS, std::min<size_t>((size_t) nW, 1 + (size_t) nW * V * 4 / (256 << 10)));
+    if (direct) {
+        int rc = 0;
+        for_row_runs(lrows, 0, (size_t) nW, [&](size_t k, int row, size_t n) {
+            if (!rc) rc = (int) cudaMemcpyAsync(dst + (size_t) row * V, ll.logits + k * V, n * V * 4, cudaMemcpyDeviceToHost, m->stream);
+        });
+        CK(rc);
+    }
+    const int parts = !staged ? 0 : (int) std::min<size_t>(LayerList::ROW_PARTS, std::min<size_t>((size_t) nW, 1 + (size_t) nW * V * 4 / (256 << 10)));
     auto part_row = [&](int c) { return (size_t) nW * (size_t) c / (size_t) std::max(parts, 1); };
     for (int c = 0; c < parts; c++) {
         const size_t k0 = part_row(c), k1 = part_row(c + 1);
@@ -2823,12 +2844,12 @@ static int ll_run_sub(pb200_model * m, std::vector<SubEntry> & es, bool prefill,
         if (!ll.ev_rows[c]) CK(cudaEventCreateWithFlags(&ll.ev_rows[c], cudaEventDisableTiming));
         CK(cudaEventRecord(ll.ev_rows[c], m->stream));
     }
-    if (dst)
+    if (parts)
         for_row_runs(lrows, 0, (size_t) nW, [&](size_t, int row, size_t n) {
             volatile char * q = (volatile char *) (dst + (size_t) row * V);
             for (size_t i = 0; i < n * V * 4; i += 4096) q[i] = q[i];
         });
-    for (int c = 0; c < parts && dst; c++) {
+    for (int c = 0; c < parts; c++) {
         CK(cudaEventSynchronize(ll.ev_rows[c]));
         for_row_runs(lrows, part_row(c), part_row(c + 1), [&](size_t k, int row, size_t n) { memcpy(dst + (size_t) row * V, ll.logits_host + k * V, n * V * 4); });
     }
@@ -3061,6 +3082,7 @@ int pb200_seq_length(pb200_model * m, int slot) {
     if (!m->ll) return PB200_ENOTSUP;
     return ll_seq_length(m, slot);
 }
+void * pb200_result_take(pb200_model * m, size_t bytes) { return m && m->ll ? result_take(m->ll->results, bytes) : nullptr; }
 int pb200_batch_step(pb200_model * m, int n_entries, const pb200_batch_entry * entries, float * logits_host, int32_t * greedy_host) {
     if (!m) return PB200_EINVAL;
     if (!m->ll) return PB200_ENOTSUP;

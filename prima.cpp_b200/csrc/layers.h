@@ -445,4 +445,11 @@ int launch_stream_add_rmsnorm(float * x, const float * x0, const float * vec, co
 int launch_rmsnorm_pair_residual(const float * a, int64_t lda, const float * bb, int64_t ldb, const float * wa, const float * wb, float mult, float eps,
                                  float * x, const float * wn, void * y, int otype, int n_rows, int width, cudaStream_t stream);
 
+// page-locked memory for the logits of batch steps (results.cu)
+struct ResultPool;
+ResultPool * result_pool_create(size_t bytes);              // NULL: no memory that can be page-locked
+void result_pool_release(ResultPool * p);                   // the model's share; blocks that are out keep the pool
+void * result_take(ResultPool * p, size_t bytes);
+bool result_direct(const void * p, size_t bytes);           // the device can write [p, p + bytes) itself
+
 }  // namespace pb

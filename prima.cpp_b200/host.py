@@ -124,6 +124,9 @@ class Lib:
         c.pb200_seq_alloc.argtypes = [vp]
         c.pb200_seq_free.argtypes = [vp, C.c_int]
         c.pb200_seq_length.argtypes = [vp, C.c_int]
+        c.pb200_result_take.restype = vp
+        c.pb200_result_take.argtypes = [vp, C.c_size_t]
+        c.pb200_result_give.argtypes = [vp]
         c.pb200_batch_step.argtypes = [vp, C.c_int, C.POINTER(BatchEntry), vp, vp]
         c.pb200_debug_tap_layers.argtypes = [vp, C.c_int]
         c.pb200_debug_profile.argtypes = [vp, C.c_int]
@@ -138,6 +141,17 @@ class Lib:
     def check(self, rc: int, what: str = "") -> None:
         if rc != 0:
             raise Pb200Error(f"{what}: {self.c.pb200_error_string(rc).decode()} ({rc})")
+
+
+class _Result:
+    """A block of a model's result pool as the base of a numpy array."""
+
+    def __init__(self, lib: Lib, ptr: int, rows: int, cols: int):
+        self._give, self._ptr = lib.c.pb200_result_give, ptr
+        self.__array_interface__ = {"data": (ptr, False), "shape": (rows, cols), "typestr": "<f4", "version": 3}
+
+    def __del__(self):
+        self._give(self._ptr)
 
 
 class Model:
@@ -216,6 +230,13 @@ class Model:
     def seq_length(self, slot: int) -> int:
         return self.lib.c.pb200_seq_length(self.h, slot)
 
+    def _result(self, rows: int, cols: int):
+        """float32 [rows, cols] for the device to write: page-locked memory of the model's pool while it has room, which returns when the last view of the
+        array is gone; ordinary memory otherwise."""
+        import numpy as np
+        ptr = self.lib.c.pb200_result_take(self.h, rows * cols * 4) if rows else None
+        return np.asarray(_Result(self.lib, ptr, rows, cols)) if ptr else np.empty((rows, cols), dtype=np.float32)
+
     def batch_step(self, entries, greedy: bool = False):
         """entries: [(slot, tokens, want)] with want = indices into tokens whose logits are asked for.  Returns (logits [rows, n_vocab]
         float32 in the order of the entries and of want, greedy tokens per entry or None)."""
@@ -234,7 +255,7 @@ class Model:
             arr[i].n_want = int(w.size)
             arr[i].want = w.ctypes.data_as(C.POINTER(C.c_int32)) if w.size else None
             rows += int(w.size)
-        logits = np.empty((rows, self.hp.n_vocab), dtype=np.float32)
+        logits = self._result(rows, self.hp.n_vocab)
         g = np.zeros(n, dtype=np.int32) if greedy else None
         self.lib.check(self.lib.c.pb200_batch_step(self.h, n, arr, logits.ctypes.data_as(C.c_void_p) if rows else None,
                                                    g.ctypes.data_as(C.c_void_p) if greedy else None), "batch_step")
