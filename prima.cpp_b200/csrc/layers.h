@@ -445,6 +445,14 @@ int launch_stream_add_rmsnorm(float * x, const float * x0, const float * vec, co
 int launch_rmsnorm_pair_residual(const float * a, int64_t lda, const float * bb, int64_t ldb, const float * wa, const float * wb, float mult, float eps,
                                  float * x, const float * wn, void * y, int otype, int n_rows, int width, cudaStream_t stream);
 
+// norms and embeddings with the row in registers (rows.cu); cudaErrorNotSupported: not a row they take
+int launch_rms_rows(const float * x, const int32_t * rows, const float * w, float eps, void * y, int otype, int n_rows, int width, cudaStream_t stream);
+int launch_embed_rms_rows(const void * table, int type, int width, const int32_t * tokens, int n_tokens, const float * w, float scale, float eps, float * x, const float * wn,
+                          void * y, cudaStream_t stream);
+// x given: x += mult * (layernorm(m) * w + bias) and, where y is given, y = x; else y = layernorm(m[rows]) * w + bias
+int launch_layernorm_rows(const float * m, const int32_t * rows, const float * w, const float * bias, float mult, float eps, float * x, void * y, int otype, int n_rows, int width,
+                          cudaStream_t stream);
+
 // page-locked memory for the logits of batch steps (results.cu)
 struct ResultPool;
 ResultPool * result_pool_create(size_t bytes);              // NULL: no memory that can be page-locked

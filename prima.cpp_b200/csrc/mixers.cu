@@ -930,6 +930,8 @@ int launch_embed_rmsnorm(const void * table, int type, int width, const int32_t 
                          const float * wn, void * y, int otype, cudaStream_t st) {
     if (n_tokens <= 0) return 0;
     if (y && (!wn || otype != type)) return (int) cudaErrorInvalidValue;
+    const int rc = launch_embed_rms_rows(table, type, width, tokens, n_tokens, w, scale, eps, x, wn, y, st);
+    if (rc != (int) cudaErrorNotSupported) return rc;
     return ck_launch([&] {
         if (type == T_BF16)
             k_embed_rmsnorm<__nv_bfloat16, __nv_bfloat16><<<n_tokens, row_threads(n_tokens, width), 0, st>>>((const __nv_bfloat16 *) table, width, tokens, w, scale, eps, x, wn, (__nv_bfloat16 *) y);
@@ -946,6 +948,8 @@ int launch_cast(const float * x, void * y, int otype, int64_t n, cudaStream_t st
 }
 int launch_layernorm(const float * x, const int32_t * rows, const float * w, float eps, void * y, int otype, int n_rows, int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
+    const int rc = launch_layernorm_rows(x, rows, w, nullptr, 1.f, eps, nullptr, y, otype, n_rows, width, st);
+    if (rc != (int) cudaErrorNotSupported) return rc;
     return ck_launch([&] {
         if (otype == T_BF16) launch_dep(k_layernorm<__nv_bfloat16, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, nullptr, eps, (__nv_bfloat16 *) y, nullptr, width);
         else launch_dep(k_layernorm<float, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, nullptr, eps, (float *) y, nullptr, width);
@@ -954,6 +958,8 @@ int launch_layernorm(const float * x, const int32_t * rows, const float * w, flo
 int launch_layernorm_affine(const float * x, const int32_t * rows, const float * w, const float * bias, float eps, void * y, int otype, int n_rows, int width,
                             cudaStream_t st) {
     if (n_rows <= 0) return 0;
+    const int rc = launch_layernorm_rows(x, rows, w, bias, 1.f, eps, nullptr, y, otype, n_rows, width, st);
+    if (rc != (int) cudaErrorNotSupported) return rc;
     return ck_launch([&] {
         if (otype == T_BF16) launch_dep(k_layernorm<__nv_bfloat16, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, bias, eps, (__nv_bfloat16 *) y, nullptr, width);
         else launch_dep(k_layernorm<float, false>, dim3(n_rows), dim3(256), 0, st, x, rows, w, bias, eps, (float *) y, nullptr, width);
@@ -962,6 +968,8 @@ int launch_layernorm_affine(const float * x, const int32_t * rows, const float *
 int launch_layernorm_affine_residual(const float * m, const float * w, const float * bias, float mult, float eps, float * x, void * xa, int otype, int n_rows,
                                      int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
+    const int rc = launch_layernorm_rows(m, nullptr, w, bias, mult, eps, x, xa, otype, n_rows, width, st);
+    if (rc != (int) cudaErrorNotSupported) return rc;
     return ck_launch([&] {
         if (otype == T_BF16) launch_dep(k_layernorm_affine_residual<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, st, m, w, bias, mult, eps, x, (__nv_bfloat16 *) xa, width);
         else launch_dep(k_layernorm_affine_residual<float>, dim3(n_rows), dim3(256), 0, st, m, w, bias, mult, eps, x, (float *) xa, width);
@@ -1003,6 +1011,8 @@ int launch_embed_pos(const void * table, const void * pos_table, int type, int w
 }
 int launch_layernorm_residual(const float * m, const float * w, float eps, float * x, int n_rows, int width, cudaStream_t st) {
     if (n_rows <= 0) return 0;
+    const int rc = launch_layernorm_rows(m, nullptr, w, nullptr, 1.f, eps, x, nullptr, T_F32, n_rows, width, st);
+    if (rc != (int) cudaErrorNotSupported) return rc;
     return ck_launch([&] { launch_dep(k_layernorm<float, true>, dim3(n_rows), dim3(256), 0, st, m, nullptr, w, nullptr, eps, nullptr, x, width); });
 }
 int launch_layernorm_residual_next(const float * m, const float * wa, const float * wb, float eps, float * x, void * y, int otype, int n_rows, int width,

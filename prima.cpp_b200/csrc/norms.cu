@@ -234,6 +234,10 @@ int launch_group_rmsnorm(const float * x, const int32_t * rows, const float * w,
                          cudaStream_t st) {
     if (n_rows <= 0) return 0;
     if (groups <= 0 || groups > MAX_NORM_GROUPS || width % groups != 0) return (int) cudaErrorInvalidValue;
+    if (groups == 1) {
+        const int rc = launch_rms_rows(x, rows, w, eps, y, otype, n_rows, width, st);
+        if (rc != (int) cudaErrorNotSupported) return rc;
+    }
     return ck_launch([&] {
         if (otype == T_BF16) launch_dep(k_group_rmsnorm<__nv_bfloat16>, dim3(n_rows), dim3(row_threads(n_rows, width)), 0, st, x, rows, w, groups, eps, (__nv_bfloat16 *) y, width);
         else launch_dep(k_group_rmsnorm<float>, dim3(n_rows), dim3(row_threads(n_rows, width)), 0, st, x, rows, w, groups, eps, (float *) y, width);
