@@ -18,7 +18,7 @@ namespace {
 
 // y[r] = x[rows[r]] / rms * w
 template <int V, typename OT>
-__global__ void __launch_bounds__(512) k_rms_rows(const float * __restrict__ x, const int32_t * __restrict__ rows, const float * __restrict__ w, float eps, OT * __restrict__ y,
+__global__ void __launch_bounds__(512) k_rms_rows(const float * x, const int32_t * rows, const float * __restrict__ w, float eps, OT * y,
                                                   int width, int n_rows, int wpr) {
     __shared__ float red[32];
     const RowPlace at(wpr);
@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(512) k_embed_rms_rows(const WT * __restrict__ 
 
 // RESID: x[r] += mult * (layernorm(m[r]) * w + bias), y[r] = x[r] in the operand type where y is given; else y[r] = layernorm(m[rows[r]]) * w + bias
 template <int V, typename OT, bool RESID>
-__global__ void __launch_bounds__(512) k_layernorm_rows(const float * __restrict__ m, const int32_t * __restrict__ rows, const float * __restrict__ w, const float * __restrict__ bias,
-                                                        float mult, float eps, float * __restrict__ x, OT * __restrict__ y, int width, int n_rows, int wpr) {
+__global__ void __launch_bounds__(512) k_layernorm_rows(const float * m, const int32_t * rows, const float * __restrict__ w, const float * __restrict__ bias,
+                                                        float mult, float eps, float * x, OT * y, int width, int n_rows, int wpr) {
     __shared__ float red[2][32];
     const RowPlace at(wpr);
     const int r = blockIdx.x * (blockDim.x / (32 * wpr)) + at.row, n4 = width / 4;
