@@ -70,6 +70,7 @@ __global__ void k_causal_conv(const float * __restrict__ u, int64_t ldu, const i
 }
 __global__ void k_causal_conv_state(const float * __restrict__ u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, int channels,
                                     int taps, float * __restrict__ conv_state, int64_t slot_stride) {
+    pdl_enter();
     const int e = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
@@ -693,13 +694,14 @@ int launch_causal_conv(const float * u, int64_t ldu, const BatchView & b, int ch
     if (taps < 1 || !w || (taps > 1 && !conv_state)) return (int) cudaErrorInvalidValue;
     const int tiles = b.n_tokens >= 512 ? 1 : std::min((channels + 127) / 128, 32);   // few tokens: a token's channels spread over CTAs
     const int advance = b.max_n == 1 && taps > 1;   // one-token entries: the same kernel moves the state on
-    int rc = ck_launch([&] {
+    int rc = taps == 4 ? launch_conv4(u, ldu, b, channels, w, silu_from, conv_state, slot_stride, out, ldo, advance, st) : (int) cudaErrorNotSupported;
+    if (rc == (int) cudaErrorNotSupported) rc = ck_launch([&] {
         launch_dep(k_causal_conv, dim3((unsigned) b.n_tokens, (unsigned) tiles), dim3(128), 0, st, u, ldu, b.slot, b.off, b.entry_of, channels, taps, w, silu_from, conv_state,
                                                                                      slot_stride, out, ldo, advance);
     });
     if (rc || taps == 1 || advance) return rc;
     return ck_launch([&] {
-        k_causal_conv_state<<<dim3((unsigned) ((channels + 127) / 128), (unsigned) b.n_entries), 128, 0, st>>>(u, ldu, b.slot, b.off, channels, taps, conv_state, slot_stride);
+        launch_dep(k_causal_conv_state, dim3((unsigned) ((channels + 127) / 128), (unsigned) b.n_entries), dim3(128), 0, st, u, ldu, b.slot, b.off, channels, taps, conv_state, slot_stride);
     });
 }
 
@@ -711,6 +713,12 @@ static int dual_prep_launch(const RecPrep & rc, float * q, int64_t ldq, float * 
     if (a.heads <= 0 || a.dim <= 0 || a.vdim <= 0 || pr.rot_dims < 0 || pr.rot_dims > a.dim || (pr.rot_dims & 1) ||
         (pr.rot_dims > 0 && !pr.rot_freq) || (pr.v_rot && !pr.v_freq) || (pr.norm == QKN_WHOLE_WEIGHT && (!pr.wq || !pr.wk)))
         return (int) cudaErrorInvalidValue;
+    if (rc.kind <= 0) {
+        const bool rec = rc.kind == 0;
+        const int r = launch_head_prep(rec ? rc.q : nullptr, rc.ldq, rc.k, rc.ldk, rc.beta, rc.ldb, rc.a, rc.lda, rc.p0, rc.p1, rc.qk_heads, rc.heads, rc.dim, q, ldq, k, ldk, v, ldv, b, a, pr,
+                                       kcache, vcache, slot_stride, st);
+        if (r != (int) cudaErrorNotSupported) return r;
+    }
     // the token's rows in shared memory when they fit
     const size_t floats = (size_t) a.heads * a.dim + (size_t) a.kv_heads * a.dim + (size_t) attn_v_row(a) + (rc.kind >= 0 ? 2 * (size_t) rc.qk_heads * rc.dim : 0);
     const size_t table = (size_t) ((pr.rot_dims + a.vdim + 3) & ~3);   // cosines and sines of the token's position
@@ -829,6 +837,10 @@ int launch_dual_post(const float * o, const BatchView & b, int heads, int vdim, 
     if (b.n_tokens <= 0) return 0;
     if (heads <= 0 || vdim <= 0 || r_heads <= 0 || r_vdim <= 0 || (gate_mode != 0 && !gate) || !o || !y) return (int) cudaErrorInvalidValue;
     if (!r_gate) r_gate_act = -1;
+    if (!v_freq) {
+        const int rc = launch_join_heads(o, b.n_tokens, heads, vdim, gate, ldg, gate_mode, left_scale, y, r_heads, r_vdim, r_gate, ldrg, r_w, r_gate_act, eps, right_scale, out, ldo, otype, st);
+        if (rc != (int) cudaErrorNotSupported) return rc;
+    }
     const dim3 grid((unsigned) b.n_tokens, (unsigned) (heads + r_heads));
     return ck_launch([&] {
         if (otype == T_BF16)

@@ -453,6 +453,16 @@ int launch_embed_rms_rows(const void * table, int type, int width, const int32_t
 int launch_layernorm_rows(const float * m, const int32_t * rows, const float * w, const float * bias, float mult, float eps, float * x, void * y, int otype, int n_rows, int width,
                           cudaStream_t stream);
 
+// a warp to a head (heads.cu): launch_dual_prep_store with a delta rule or none (rq null), launch_dual_post over values that do not turn, launch_causal_conv with four
+// taps (without the state's move behind entries of several tokens); cudaErrorNotSupported: not heads or rows they take
+int launch_head_prep(float * rq, int64_t ldrq, float * rk, int64_t ldrk, float * beta, int64_t ldb, float * ra, int64_t lda, const float * A_log, const float * dt_bias, int r_qk,
+                     int r_heads, int r_dim, float * q, int64_t ldq, float * k, int64_t ldk, const float * v, int64_t ldv, const BatchView & b, const AttnParams & a, const AttnPrep & pr,
+                     float * kcache, float * vcache, int64_t slot_stride, cudaStream_t stream);
+int launch_join_heads(const float * o, int n_tokens, int heads, int vdim, const float * gate, int64_t ldg, int gate_mode, float left_scale, const float * y, int r_heads, int r_vdim,
+                      const float * r_gate, int64_t ldrg, const float * r_w, int r_gate_act, float eps, float right_scale, void * out, int64_t ldo, int otype, cudaStream_t stream);
+int launch_conv4(const float * u, int64_t ldu, const BatchView & b, int channels, const float * w, int silu_from, float * conv_state, int64_t slot_stride, float * out, int64_t ldo,
+                 int advance, cudaStream_t stream);
+
 // page-locked memory for the logits of batch steps (results.cu)
 struct ResultPool;
 ResultPool * result_pool_create(size_t bytes);              // NULL: no memory that can be page-locked

@@ -38,3 +38,33 @@ def test_layer_norm_and_residual(pkg, cuda, width):
         m.seq_free(s)
         assert RS.rel_err(np.asarray(got, dtype=np.float64), want).max() < S.F32_TOL
     m.close()
+
+
+# a lane has four entries of a head: full warps, part of one, heads and rotations that go to the kernels with an element a thread
+@pytest.mark.parametrize("dim,vdim,rot,r_dim,r_vdim,taps", [(128, 128, 128, 128, 128, 4), (64, 32, 64, 32, 64, 4), (4, 8, 0, 4, 4, 4), (24, 20, 8, 12, 20, 3), (128, 96, 40, 100, 36, 4),
+                                                            (128, 128, 4, 64, 16, 4), (132, 132, 8, 132, 132, 4), (10, 6, 2, 6, 10, 4)])
+def test_heads_of_every_size(pkg, cuda, dim, vdim, rot, r_dim, r_vdim, taps):
+    cfg = L.config([L.att(heads=3, kv_heads=1, dim=dim, vdim=vdim, rot=rot, ff=0), L.par(heads=4, kv_heads=2, dim=dim, r_heads=4, r_kv=2, r_dim=r_dim, r_vdim=r_vdim, taps=taps, ff=0),
+                    L.att(heads=3, kv_heads=1, dim=dim, vdim=vdim, rot=rot, ff=0, of=0)], width=64, vocab=37)
+    bits, W = RL.random_weights(cfg, seed=dim + taps)
+    m = L.load(pkg, cfg, bits, n_ctx=256)
+    for n in (1, 3, 9, 130):
+        t = L.tokens_for(cfg, n, n)
+        want = RL.forward(cfg, W, t)[0]
+        L.check(L.run_whole(m, t), want, L.F32_TOL)
+        L.check(L.run_decoded(m, t, max(1, n - 6)), want, L.F32_TOL)
+    m.close()
+
+
+@pytest.mark.parametrize("dtype,tol", [("float32", L.F32_TOL), ("bfloat16", L.BF16_TOL)])
+@pytest.mark.parametrize("kv_rank,q_rank", [(4, 4), (64, 64), (256, 260), (512, 1024), (508, 40), (30, 20), (20, 30)])
+def test_latents_of_every_size(pkg, cuda, kv_rank, q_rank, dtype, tol):
+    cfg = L.config([L.lat(heads=4, dim=16, vdim=16, kv_rank=kv_rank, q_rank=q_rank, window=24, ff=0)], width=64, vocab=37)
+    bits, W = RL.random_weights(cfg, seed=kv_rank)
+    m = L.load(pkg, cfg, bits, dtype=dtype, n_ctx=256)
+    for n in (1, 17, 45, 130):
+        t = L.tokens_for(cfg, n, n)
+        want = RL.forward(cfg, W, t)[0]
+        L.check(L.run_whole(m, t), want, tol)
+        L.check(L.run_decoded(m, t, max(1, n // 2)), want, tol)
+    m.close()
