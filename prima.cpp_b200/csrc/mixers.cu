@@ -11,6 +11,7 @@
 
 #include "layers.h"
 #include "mixers.cuh"
+#include "rows.cuh"
 
 namespace pb {
 thread_local bool g_pdl = false;
@@ -144,6 +145,15 @@ __global__ void k_relu2(const float * __restrict__ u, OT * __restrict__ y, int64
     const float v = fmaxf(u[i], 0.f);
     put(y, i, v * v);
 }
+template <typename OT>   // four elements a thread
+__global__ void k_relu2_4(const float * __restrict__ u, OT * __restrict__ y, int64_t n) {
+    pdl_enter();
+    const int64_t i = 4 * ((int64_t) blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    float4 v = ld4(u, i);
+    v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    put4(y, i, make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w));
+}
 template <typename OT>
 __global__ void k_xielu(const float * __restrict__ u, const float * __restrict__ pq, OT * __restrict__ y, int64_t n) {
     pdl_enter();
@@ -161,12 +171,20 @@ __global__ void k_softcap(float * __restrict__ x, int64_t n, float cap) {
 template <typename WT, typename OT>
 __global__ void k_embed_pos(const WT * __restrict__ table, const WT * __restrict__ ptab, int width, const int32_t * __restrict__ tokens,
                             const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, float * __restrict__ x,
-                            OT * __restrict__ xa) {
+                            OT * __restrict__ xa, int wide) {
     const int t = blockIdx.x;
     const int e = entry_of[t];
     const int64_t p = pos0[e] + (t - off[e]);
     const WT * row = table + (int64_t) tokens[t] * width;
     const WT * prow = ptab + p * width;
+    if (wide) {
+        for (int i = 4 * threadIdx.x; i < width; i += 4 * blockDim.x) {
+            const float4 a = ld4(row, i), b = ld4(prow, i), v = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+            put4(x, (int64_t) t * width + i, v);
+            if (xa) put4(xa, (int64_t) t * width + i, v);
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < width; i += blockDim.x) {
         const float v = ld_f(row, i) + ld_f(prow, i);
         x[(int64_t) t * width + i] = v;
@@ -978,6 +996,11 @@ int launch_layernorm_affine_residual(const float * m, const float * w, const flo
 int launch_relu2(const float * u, void * y, int otype, int64_t n, cudaStream_t st) {
     if (n <= 0) return 0;
     const unsigned grid = (unsigned) ((n + 255) / 256);
+    if (n % 4 == 0 && at16(u) && at16(y))   // 2048 x 2048 elements, us: 14.8 with an element a thread, 5.6 with four
+        return ck_launch([&] {
+            if (otype == T_BF16) launch_dep(k_relu2_4<__nv_bfloat16>, dim3((unsigned) ((n / 4 + 255) / 256)), dim3(256), 0, st, u, (__nv_bfloat16 *) y, n);
+            else launch_dep(k_relu2_4<float>, dim3((unsigned) ((n / 4 + 255) / 256)), dim3(256), 0, st, u, (float *) y, n);
+        });
     return ck_launch([&] {
         if (otype == T_BF16) launch_dep(k_relu2<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, u, (__nv_bfloat16 *) y, n);
         else launch_dep(k_relu2<float>, dim3(grid), dim3(256), 0, st, u, (float *) y, n);
@@ -1000,13 +1023,14 @@ int launch_embed_pos(const void * table, const void * pos_table, int type, int w
                      int otype, cudaStream_t st) {
     if (b.n_tokens <= 0) return 0;
     if ((xa && otype != type) || !pos_table) return (int) cudaErrorInvalidValue;
+    const int wide = width % 4 == 0 && at16(table) && at16(pos_table) && at16(x) && at16(xa);   // four elements a load
     return ck_launch([&] {
         if (type == T_BF16)
             k_embed_pos<__nv_bfloat16, __nv_bfloat16><<<b.n_tokens, 128, 0, st>>>((const __nv_bfloat16 *) table, (const __nv_bfloat16 *) pos_table, width, tokens,
-                                                                                   b.off, b.pos0, b.entry_of, x, (__nv_bfloat16 *) xa);
+                                                                                   b.off, b.pos0, b.entry_of, x, (__nv_bfloat16 *) xa, wide);
         else
             k_embed_pos<float, float><<<b.n_tokens, 128, 0, st>>>((const float *) table, (const float *) pos_table, width, tokens, b.off, b.pos0, b.entry_of, x,
-                                                                   (float *) xa);
+                                                                   (float *) xa, wide);
     });
 }
 int launch_layernorm_residual(const float * m, const float * w, float eps, float * x, int n_rows, int width, cudaStream_t st) {

@@ -15,6 +15,7 @@
 
 #include "layers.h"
 #include "mixers.cuh"
+#include "rows.cuh"
 
 namespace pb {
 namespace {
@@ -108,33 +109,9 @@ __device__ __forceinline__ void warp_argmax(const float * v, int n, int lane, fl
     }
 }
 
-// one CTA per token: sigmoid scores, choice with the correction among the experts of the best groups, weights from the plain scores
-template <typename HT>
-__global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p,
-                                                           int width, const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt,
-                                                           float * __restrict__ sg_out) {
-    pdl_enter();
-    extern __shared__ float sm[];
-    float * hs = sm;                 // [width]
-    float * sc = hs + width;         // [experts] sigmoid scores
-    float * ch = sc + p.experts;     // [experts] choice scores, -inf once taken or not eligible
-    float * gs = ch + p.experts;     // [groups] group scores
-    float * kp = gs + p.groups;      // [groups] 1: the group stays eligible
-    const int t = blockIdx.x;
-    for (int i = threadIdx.x; i < width; i += blockDim.x) hs[i] = ld_f(h, (int64_t) t * width + i);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int e = warp; e < p.experts + (sgw ? 1 : 0); e += nw) {
-        if (e == p.experts) {        // the shared expert's gate rides along as one more row
-            const float acc = wsum(dot_lane8(sgw, hs, width, lane));
-            if (lane == 0) sg_out[t] = sigmoid_f(acc);
-        } else {
-            const float acc = wsum(dot_lane8(wr + (int64_t) e * width, hs, width, lane));
-            if (lane == 0) { const float s = sigmoid_f(acc); sc[e] = s; ch[e] = corr ? s + corr[e] : s; }
-        }
-    }
-    __syncthreads();
-    if (warp != 0) return;
+// a warp picks a token's experts: the best groups by their two largest choice scores, then the `top` best of their experts.  sc: scores, ch: choice scores (overwritten),
+// gs and kp: [groups] of scratch
+__device__ __forceinline__ void pick_experts(const MoeParams & p, const float * sc, float * ch, float * gs, float * kp, int lane, int32_t * idx, float * wt) {
     const int per = p.experts / p.groups;
     if (p.groups > 1 && p.keep_groups < p.groups) {
         for (int g = lane; g < p.groups; g += 32) {   // the two largest choice scores of the group, summed
@@ -166,11 +143,97 @@ __global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restric
         warp_argmax(ch, p.experts, lane, best, bi);
         if (bi == 0x7fffffff) bi = 0;             // only with non-finite scores
         if (lane == k) mine = sc[bi];
-        if (lane == 0) { idx[(int64_t) t * p.top + k] = bi; ch[bi] = -INFINITY; }
+        if (lane == 0) { idx[k] = bi; ch[bi] = -INFINITY; }
         __syncwarp();
     }
     const float sum = wsum(lane < p.top ? mine : 0.f);
-    if (lane < p.top) wt[(int64_t) t * p.top + lane] = (p.norm_weights ? mine / (sum + 1e-20f) : mine) * p.route_scale;
+    if (lane < p.top) wt[lane] = (p.norm_weights ? mine / (sum + 1e-20f) : mine) * p.route_scale;
+}
+
+// one CTA per token: sigmoid scores, choice with the correction among the experts of the best groups, weights from the plain scores
+template <typename HT>
+__global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p,
+                                                           int width, const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt,
+                                                           float * __restrict__ sg_out) {
+    pdl_enter();
+    extern __shared__ float sm[];
+    float * hs = sm;                 // [width]
+    float * sc = hs + width;         // [experts] sigmoid scores
+    float * ch = sc + p.experts;     // [experts] choice scores, -inf once taken or not eligible
+    float * gs = ch + p.experts;     // [groups] group scores
+    float * kp = gs + p.groups;      // [groups] 1: the group stays eligible
+    const int t = blockIdx.x;
+    for (int i = threadIdx.x; i < width; i += blockDim.x) hs[i] = ld_f(h, (int64_t) t * width + i);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int e = warp; e < p.experts + (sgw ? 1 : 0); e += nw) {
+        if (e == p.experts) {        // the shared expert's gate rides along as one more row
+            const float acc = wsum(dot_lane8(sgw, hs, width, lane));
+            if (lane == 0) sg_out[t] = sigmoid_f(acc);
+        } else {
+            const float acc = wsum(dot_lane8(wr + (int64_t) e * width, hs, width, lane));
+            if (lane == 0) { const float s = sigmoid_f(acc); sc[e] = s; ch[e] = corr ? s + corr[e] : s; }
+        }
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    pick_experts(p, sc, ch, gs, kp, lane, idx + (int64_t) t * p.top, wt + (int64_t) t * p.top);
+}
+
+// the same for a prompt: a CTA takes ROUTE_TOKENS tokens, so that a router row is read once for all of them (a token's sums in the same order), and a warp picks a token's
+// experts
+constexpr int ROUTE_TOKENS = 8;
+template <typename HT>
+__global__ void __launch_bounds__(1024) k_moe_route_sigmoid_many(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p, int width,
+                                                                const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt, float * __restrict__ sg_out,
+                                                                int n_tokens) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    float * hs = sm;                                     // [ROUTE_TOKENS][width]
+    float * per_token = hs + ROUTE_TOKENS * width;       // scores, choice scores, group scores, groups that stay
+    const int each = 2 * p.experts + 2 * p.groups, t0 = blockIdx.x * ROUTE_TOKENS, nt = min(ROUTE_TOKENS, n_tokens - t0);
+#pragma unroll
+    for (int j = 0; j < ROUTE_TOKENS; j++) {
+        const HT * src = h + (int64_t) (t0 + min(j, nt - 1)) * width;
+        for (int k = 4 * threadIdx.x; k < width; k += 4 * blockDim.x) put4(hs, (int64_t) j * width + k, ld4(src, k));
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int e = warp; e < p.experts + (sgw ? 1 : 0); e += nw) {
+        const float * w = e == p.experts ? sgw : wr + (int64_t) e * width;   // the shared expert's gate rides along as one more row
+        float acc[ROUTE_TOKENS];
+#pragma unroll
+        for (int j = 0; j < ROUTE_TOKENS; j++) acc[j] = 0.f;
+        auto step = [&](float f, int k) {
+#pragma unroll
+            for (int j = 0; j < ROUTE_TOKENS; j++) acc[j] = fmaf(f, hs[j * width + k], acc[j]);
+        };
+        int k = lane;
+        for (; k + 7 * 32 < width; k += 8 * 32) {
+            float f[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) f[u] = w[k + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 8; u++) step(f[u], k + 32 * u);
+        }
+        for (; k < width; k += 32) step(w[k], k);
+#pragma unroll
+        for (int j = 0; j < ROUTE_TOKENS; j++) {
+            const float s = sigmoid_f(wsum(acc[j]));
+            if (lane != 0 || j >= nt) continue;
+            if (e == p.experts) sg_out[t0 + j] = s;
+            else {
+                float * sc = per_token + j * each;
+                sc[e] = s;
+                sc[p.experts + e] = corr ? s + corr[e] : s;
+            }
+        }
+    }
+    __syncthreads();
+    for (int j = warp; j < nt; j += nw) {
+        float * sc = per_token + j * each;
+        pick_experts(p, sc, sc + p.experts, sc + 2 * p.experts, sc + 2 * p.experts + p.groups, lane, idx + (int64_t) (t0 + j) * p.top, wt + (int64_t) (t0 + j) * p.top);
+    }
 }
 
 // grid (ceil(ff / 8), pairs): warp -> row j of gate and of up of the pair's expert
@@ -229,6 +292,7 @@ __global__ void __launch_bounds__(256) k_moe_down_rows(const WT * __restrict__ y
 
 // ---- sort by expert ----
 __global__ void __launch_bounds__(256) k_moe_count(const int32_t * __restrict__ idx, int n_pairs, int32_t * __restrict__ count) {
+    pdl_enter();
     __shared__ float red[33];
     const int e = blockIdx.x;
     int c = 0;
@@ -239,6 +303,7 @@ __global__ void __launch_bounds__(256) k_moe_count(const int32_t * __restrict__ 
 // one CTA per expert: walks the pairs in order, 256 at a time, and places its own at start[e] + rank (stable)
 __global__ void __launch_bounds__(256) k_moe_place(const int32_t * __restrict__ idx, int n_pairs, const int32_t * __restrict__ count, int32_t * __restrict__ start,
                                                    int32_t * __restrict__ perm) {
+    pdl_enter();
     __shared__ int wbase[9];
     const int e = blockIdx.x;
     int s0 = 0;
@@ -264,18 +329,42 @@ __global__ void __launch_bounds__(256) k_moe_place(const int32_t * __restrict__ 
     }
 }
 template <typename WT>
-__global__ void k_moe_gather(const WT * __restrict__ h, const int32_t * __restrict__ perm, int top, int width, WT * __restrict__ hs) {
+__global__ void k_moe_gather(const WT * __restrict__ h, const int32_t * __restrict__ perm, int top, int width, WT * __restrict__ hs, int wide) {
+    pdl_enter();
     const int r = blockIdx.x;
     const WT * src = h + (int64_t) (perm[r] / top) * width;
+    if (wide) {
+        constexpr int V = Pack<WT>::n;
+        for (int i = V * threadIdx.x; i < width; i += V * blockDim.x) *reinterpret_cast<uint4 *>(hs + (int64_t) r * width + i) = *reinterpret_cast<const uint4 *>(src + i);
+        return;
+    }
     for (int i = threadIdx.x; i < width; i += blockDim.x) hs[(int64_t) r * width + i] = src[i];
 }
 __global__ void k_moe_invert(const int32_t * __restrict__ perm, int32_t * __restrict__ row_of, int n_pairs) {
+    pdl_enter();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < n_pairs) row_of[perm[r]] = r;
 }
 __global__ void k_moe_combine(const float * __restrict__ ds, const int32_t * __restrict__ row_of, const float * __restrict__ wt, int top, int width,
-                              float * __restrict__ x, int base, const float * __restrict__ xscale, float out_scale) {
+                              float * __restrict__ x, int base, const float * __restrict__ xscale, float out_scale, int wide) {
+    pdl_enter();
     const int t = blockIdx.x;
+    if (wide) {
+        for (int n = 4 * threadIdx.x; n < width; n += 4 * blockDim.x) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < top; k++) {
+                const float4 d = ld4(ds + (int64_t) row_of[(int64_t) t * top + k] * width, n);
+                const float f = wt ? wt[(int64_t) t * top + k] : 1.f;
+                acc = make_float4(fmaf(f, d.x, acc.x), fmaf(f, d.y, acc.y), fmaf(f, d.z, acc.z), fmaf(f, d.w, acc.w));
+            }
+            float * xo = x + (int64_t) t * width + n;
+            const float s = base == MOE_SCALE ? xscale[t] : 1.f;
+            float4 b = base == MOE_SET ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(xo, 0);
+            b = make_float4(b.x * s, b.y * s, b.z * s, b.w * s);
+            put4(xo, 0, make_float4(b.x + acc.x * out_scale, b.y + acc.y * out_scale, b.z + acc.z * out_scale, b.w + acc.w * out_scale));
+        }
+        return;
+    }
     for (int n = threadIdx.x; n < width; n += blockDim.x) {
         float acc = 0.f;
         for (int k = 0; k < top; k++) {
@@ -331,6 +420,17 @@ int launch_moe_route_sigmoid(const void * h, int htype, const float * wr, const 
     // one warp per router row (the shared gate included) up to 32 warps, so that all rows stream at once
     const int rows = p.experts + (shared_gate ? 1 : 0);
     const int threads = rows <= 8 ? 256 : rows >= 32 ? 1024 : 32 * rows;
+    // prompts: the router's rows, which every CTA reads in whole, are what the time goes into: 1024 tokens, 17 rows of 2048, us: 26.6 with a token a CTA, 17.7 with eight
+    const size_t many = ROUTE_TOKENS * ((size_t) width + 2 * (size_t) p.experts + 2 * (size_t) p.groups) * sizeof(float);
+    if (n_tokens >= 64 && many <= 200 * 1024 && width % 4 == 0 && at16(h)) {
+        const dim3 grid((unsigned) ((n_tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS));
+        auto go = [&](auto kernel, auto * x) {
+            const int rc = raise_smem(kernel, many);
+            if (rc) return rc;
+            return ck_launch([&] { launch_dep(kernel, grid, dim3(threads), many, st, x, wr, correction, p, width, shared_gate, idx, wt, sg_out, n_tokens); });
+        };
+        return htype == T_BF16 ? go(k_moe_route_sigmoid_many<__nv_bfloat16>, (const __nv_bfloat16 *) h) : go(k_moe_route_sigmoid_many<float>, (const float *) h);
+    }
     if (htype == T_BF16) {
         int rc = raise_smem(k_moe_route_sigmoid<__nv_bfloat16>, smem);
         if (rc) return rc;
@@ -388,15 +488,16 @@ int launch_moe_sort(const int32_t * idx, const MoeParams & p, int n_tokens, int3
     if (n_tokens <= 0) return 0;
     if (!moe_ok(p) || (int64_t) n_tokens * p.top >= (1 << 24)) return (int) cudaErrorInvalidValue;
     const int n_pairs = n_tokens * p.top;
-    int rc = ck_launch([&] { k_moe_count<<<p.experts, 256, 0, st>>>(idx, n_pairs, count); });
+    int rc = ck_launch([&] { launch_dep(k_moe_count, dim3((unsigned) p.experts), dim3(256), 0, st, idx, n_pairs, count); });
     if (rc) return rc;
-    return ck_launch([&] { k_moe_place<<<p.experts, 256, 0, st>>>(idx, n_pairs, count, start, perm); });
+    return ck_launch([&] { launch_dep(k_moe_place, dim3((unsigned) p.experts), dim3(256), 0, st, idx, n_pairs, count, start, perm); });
 }
 int launch_moe_gather(const void * h, int type, const int32_t * perm, int top, int width, void * hs, int n_rows, cudaStream_t st) {
     if (n_rows <= 0) return 0;
+    const int wide = type == T_BF16 ? vec_ok<__nv_bfloat16>(h, hs, width) : vec_ok<float>(h, hs, width);
     return ck_launch([&] {
-        if (type == T_BF16) k_moe_gather<__nv_bfloat16><<<n_rows, 128, 0, st>>>((const __nv_bfloat16 *) h, perm, top, width, (__nv_bfloat16 *) hs);
-        else k_moe_gather<float><<<n_rows, 128, 0, st>>>((const float *) h, perm, top, width, (float *) hs);
+        if (type == T_BF16) launch_dep(k_moe_gather<__nv_bfloat16>, dim3((unsigned) n_rows), dim3(128), 0, st, (const __nv_bfloat16 *) h, perm, top, width, (__nv_bfloat16 *) hs, wide);
+        else launch_dep(k_moe_gather<float>, dim3((unsigned) n_rows), dim3(128), 0, st, (const float *) h, perm, top, width, (float *) hs, wide);
     });
 }
 int launch_moe_combine(const float * ds, const int32_t * perm, int32_t * row_of, const float * wt, int top, int width, float * x, int n_tokens,
@@ -404,9 +505,10 @@ int launch_moe_combine(const float * ds, const int32_t * perm, int32_t * row_of,
     if (n_tokens <= 0) return 0;
     if (base == MOE_SCALE && !xscale) return (int) cudaErrorInvalidValue;
     const int n_pairs = n_tokens * top;
-    int rc = ck_launch([&] { k_moe_invert<<<(unsigned) ((n_pairs + 255) / 256), 256, 0, st>>>(perm, row_of, n_pairs); });
+    int rc = ck_launch([&] { launch_dep(k_moe_invert, dim3((unsigned) ((n_pairs + 255) / 256)), dim3(256), 0, st, perm, row_of, n_pairs); });
     if (rc) return rc;
-    return ck_launch([&] { k_moe_combine<<<n_tokens, 256, 0, st>>>(ds, row_of, wt, top, width, x, base, xscale, out_scale); });
+    const int wide = vec_ok<float>(ds, x, width);
+    return ck_launch([&] { launch_dep(k_moe_combine, dim3((unsigned) n_tokens), dim3(256), 0, st, ds, row_of, wt, top, width, x, base, xscale, out_scale, wide); });
 }
 
 }  // namespace pb
