@@ -86,6 +86,11 @@ PB200_API int pb200_rms_norm(const float * x, float * y, int64_t n, int64_t nrow
 PB200_API int pb200_rope(const float * x, float * y, int64_t n_tokens, int n_head, int head_dim, int n_dims, int mode, const int32_t * pos,
                          float freq_base, float freq_scale, float ext_factor, float attn_factor, float beta_fast, float beta_slow,
                          int n_ctx_orig, const float * freq_factors, void * stream);
+/* The tokens of a prompt with heads of 128: q [T][n_head][128] rotated in place, rope(k) and v as f16 to rows pos[t] of caches [.][n_head_kv][128].
+ * PB200_ENOTSUP for rotated sizes that are no multiple of 8 and arrays that are not 16-byte aligned. */
+PB200_API int pb200_rope_kv_prompt(float * q, const float * k, const float * v, void * kcache, void * vcache, int64_t n_tokens, int n_head, int n_head_kv, int n_dims,
+                                   int mode, const int32_t * pos, float freq_base, float freq_scale, float ext_factor, float attn_factor, float beta_fast,
+                                   float beta_slow, int n_ctx_orig, const float * freq_factors, void * stream);
 PB200_API int pb200_soft_max(const float * x, const float * mask, float * y, int64_t ncols, int64_t nrows, int64_t mask_rows, float scale, void * stream);
 PB200_API int pb200_silu_mul(const float * gate, const float * up, float * y, int64_t n, void * stream);
 /* element-wise glue of the graph (binbcast.cu / unary.cu / cpy.cu): y = a (+|*) b[i % nb]  (op 0 add, 1 mul); y = silu(x);

@@ -155,6 +155,18 @@ int pb200_rope(const float * x, float * y, int64_t n_tokens, int n_head, int hea
     return launch_rope(x, y, n_tokens, n_head, head_dim, (int64_t) n_head * head_dim, head_dim, pos, rp, freq_factors, (cudaStream_t) stream);
 }
 
+int pb200_rope_kv_prompt(float * q, const float * k, const float * v, void * kcache, void * vcache, int64_t n_tokens, int n_head, int n_head_kv, int n_dims, int mode,
+                         const int32_t * pos, float freq_base, float freq_scale, float ext_factor, float attn_factor, float beta_fast, float beta_slow, int n_ctx_orig,
+                         const float * freq_factors, void * stream) {
+    if (!q || !k || !v || !kcache || !vcache || !pos || n_tokens <= 0 || n_tokens > 0x7fffffff || n_head <= 0 || n_head_kv <= 0 || n_dims <= 0 || n_dims > 128) return PB200_EINVAL;
+    RopeParams rp;
+    rope_params_init(rp, n_dims, mode, n_ctx_orig, freq_base, freq_scale, ext_factor, attn_factor, beta_fast, beta_slow);
+    const int e = launch_rope_kvstore_batch(q, k, v, (__half *) kcache, (__half *) vcache, (int) n_tokens, n_head, n_head_kv, 128, pos, rp, freq_factors, (cudaStream_t) stream, false);
+    if (e == (int) cudaErrorNotSupported) return PB200_ENOTSUP;
+    g_launches++;
+    return e;
+}
+
 int pb200_soft_max(const float * x, const float * mask, float * y, int64_t ncols, int64_t nrows, int64_t mask_rows, float scale, void * stream) {
     if (!x || !y || ncols <= 0 || nrows <= 0) return PB200_EINVAL;
     g_launches++;

@@ -74,7 +74,6 @@ __global__ void __launch_bounds__(AT_THREADS, 2)
     uint8_t * q_s = smem, * ring = smem + AT_STAGE;                        // queries: two blocks of 128 rows x 64 entries
     AtCtl * ctl = reinterpret_cast<AtCtl *>(ring + AT_STAGES * AT_STAGE);
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
-    pdl_trigger();
     volatile int * cta_abort = &ctl->abort;
     int u = 0;                                                             // tiles loaded (warp 0) or used (warp 1)
     if (warp == 0 && lane == 0) {
@@ -92,6 +91,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2)
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
     }
     pdl_wait();                                                            // queries, positions, keys and values may be the kernel in front's
     uint32_t tmem = 0, tiles = 0, looks = 0, loads = 0, o_phase = 0;       // of the items in front: key tiles, tiles looked at, loads

@@ -126,7 +126,6 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     constexpr int B_BYTES = BN * 128, STAGE = TC_A_BYTES + B_BYTES, COLS = BN < 32 ? 32 : BN;
     float * Cm = P.C;
     int Tn = P.T, tile_y = blockIdx.y, grp = 0, a_row0 = 0;
-    pdl_trigger();
     if (P.grp_count) {
         pdl_wait();                    // the counts come from the kernels in front
         for (; grp < P.groups; grp++) {
@@ -159,6 +158,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
     }
     fence_before();
     __syncthreads();
@@ -272,7 +272,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles = P.row_tiles * P.tok_tiles;
     const int nk = (P.K + TC_BK - 1) / TC_BK;
-    pdl_trigger();
 
     if (threadIdx.x == 0) {
         prefetch_map(&map_w);
@@ -285,6 +284,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) __cluster_dims__(2, 1, 1)
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
     }
     fence_before();
     __syncthreads();

@@ -585,6 +585,10 @@ static int pf_reserve(pb200_model * m, int T) {
 // y[t][:] = W . x[t][:] (+ bias): tensor-core path when the type / K allow it, otherwise the decode GEMV row by row
 // same_x_as: the matrix of the previous pf_matmul call when it read the same x (q -> k -> v, gate -> up): its tiled fp16 activation image
 // in the workspace is reused if both went down the tensor-core path with the same activation format
+static bool no_pdl() {   // A/B: every kernel of a prompt waits for the one in front before it is launched
+    static const bool v = getenv("PB200_NO_PDL") != nullptr;
+    return v;
+}
 static bool pf_tc(const Tensor & W, int T) { return mmq_supported(W.type, W.K) && T >= 8; }
 static int pf_matmul(pb200_model * m, const Tensor & W, const float * x, int T, float * y, const float * bias, const float * resid, uint64_t & n,
                      const Tensor * same_x_as = nullptr, const MmqPre * pre = nullptr) {
@@ -592,7 +596,7 @@ static int pf_matmul(pb200_model * m, const Tensor & W, const float * x, int T, 
     if (pf_tc(W, T)) {
         const bool reuse = same_x_as && pf_tc(*same_x_as, T) && same_x_as->K == W.K && is_kquant(same_x_as->type) == is_kquant(W.type);
         n += reuse ? 1 : 2;
-        return (int) launch_mmq(W.type, W.data, W.N, W.K, x, W.K, T, y, bias, resid, m->pf.ws, st, reuse, reuse ? nullptr : pre);
+        return (int) launch_mmq(W.type, W.data, W.N, W.K, x, W.K, T, y, bias, resid, m->pf.ws, st, reuse, reuse ? nullptr : pre, !no_pdl());
     }
     if (pre) return (int) cudaErrorInvalidValue;   // callers fuse a producer only when pf_tc(W, T) && is_kquant(W.type)
     ActQ act = act_from_ws(m->actF.base, W.K);
@@ -683,10 +687,13 @@ static int prefill_ubatch(pb200_model * m, const int32_t * tokens_host, const fl
             CK(pf_matmul(m, L.wk, P.xn, T, P.k, L.bk, nullptr, n, &L.wq));
             CK(pf_matmul(m, L.wv, P.xn, T, P.v, L.bv, nullptr, n, &L.wk));
         }
-        CK(launch_rope(P.q, P.q, T, H, D, QD, D, P.pos, m->rp, m->rope_ff, st)); n++;
-        CK(launch_rope(P.k, P.k, T, HK, D, EK, D, P.pos, m->rp, m->rope_ff, st)); n++;
-        CK(launch_cpy_f32_f16(P.k, kc + (size_t) pos0 * EK, (int64_t) T * EK, st)); n++;
-        CK(launch_cpy_f32_f16(P.v, vc + (size_t) pos0 * EK, (int64_t) T * EK, st)); n++;
+        const int rs = launch_rope_kvstore_batch(P.q, P.k, P.v, kc, vc, T, H, HK, D, P.pos, m->rp, m->rope_ff, st, !no_pdl());
+        if (rs == (int) cudaErrorNotSupported) {
+            CK(launch_rope(P.q, P.q, T, H, D, QD, D, P.pos, m->rp, m->rope_ff, st)); n++;
+            CK(launch_rope(P.k, P.k, T, HK, D, EK, D, P.pos, m->rp, m->rope_ff, st)); n++;
+            CK(launch_cpy_f32_f16(P.k, kc + (size_t) pos0 * EK, (int64_t) T * EK, st)); n++;
+            CK(launch_cpy_f32_f16(P.v, vc + (size_t) pos0 * EK, (int64_t) T * EK, st)); n++;
+        } else { CK(rs); n++; }
         CK(launch_attn_batch(P.q, kc, vc, P.att, H, HK, D, P.pos, T, pos0 + T, kq_scale, st)); n++;
         CK(pf_matmul(m, L.wo, P.att, T, y, nullptr, x, n));                  // ffn_inp = wo.att + inpSA (residual in the epilogue)
         // --- FFN block ---

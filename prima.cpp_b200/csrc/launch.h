@@ -74,6 +74,10 @@ void rope_params_init(RopeParams & rp, int n_dims, int mode, int n_ctx_orig, flo
 // (rope.cu:188-271 + cpy_f32_f16 cpy.cu:34 + llm_build_kv_store src/llama.cpp:9673-9718).  pos is read from device memory.
 int launch_rope_kvstore(float * q, const float * k, const float * v, __half * kcache, __half * vcache, int n_head, int n_head_kv, int D,
                         const int32_t * pos_dev, const RopeParams & rp, const float * freq_factors, cudaStream_t stream, bool pdl);
+// the same for the tokens of a prompt, with a warp to a head: q in place, rope(k) and v to rows pos[t] of the caches; cudaErrorNotSupported: head size other than 128,
+// rotated entries not a multiple of 8, arrays not at 16 bytes
+int launch_rope_kvstore_batch(float * q, const float * k, const float * v, __half * kcache, __half * vcache, int n_tok, int n_head, int n_head_kv, int D, const int32_t * pos_dev,
+                              const RopeParams & rp, const float * freq_factors, cudaStream_t stream, bool pdl);
 // generic rope for the plugin: x [ntok][n_head][D] -> y, positions pos[ntok]
 int launch_rope(const float * x, float * y, int64_t ntok, int n_head, int D, int64_t tok_stride, int64_t head_stride, const int32_t * pos,
                 const RopeParams & rp, const float * freq_factors, cudaStream_t stream);
@@ -133,7 +137,8 @@ struct MmqPre {            // producer fused into the activation pass: 1: x <- s
     float eps = 0.f;
 };
 cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const float * x, int64_t ldx, int64_t T, float * dst, const float * bias,
-                       const float * resid, void * ws, cudaStream_t st, bool reuse_prep = false, const MmqPre * pre = nullptr);
+                       const float * resid, void * ws, cudaStream_t st, bool reuse_prep = false, const MmqPre * pre = nullptr, bool pdl = false);
+// pdl: the kernel in front may be programmatic; the weights, which are then fetched before it ends, must not be its result.
 // resid: [T][N] added in the epilogue (must not alias dst).  reuse_prep: ws already holds this x (same K, T) from the previous launch_mmq
 // on the stream (q|k|v and gate|up share one activation: the q8_K -> fp16 tiling pass runs once)
 int launch_get_rows(const void * table, int type, int K, const int32_t * ids, int n_ids, float * y, cudaStream_t stream, bool pdl);

@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(P.tmem_cols) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
     }
     tc_fence_before();
     __syncthreads();
@@ -420,6 +421,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ================= activation producer: runs up to b_nst steps ahead of the tensor core =================
+        pdl_wait();                // activations are the kernel in front's; weights are fetched and expanded meanwhile
         if (lane == 0) {
             const size_t tile_stride = (size_t) nstep_all * b1;
             int g = 0;
@@ -510,6 +512,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 prs = rs; pph = rph;
                 if (++rs == P.nraw) { rs = 0; rph ^= 1; }
             }
+            pdl_wait();            // residuals are read and results written behind it
             if constexpr (CUT) {
                 // ================= epilogue of a part: partial sums [token][row] go over the stages' memory (every load and MMA of this CTA is done),
                 // one accumulator after the other; token t is added up, in the parts' order, by CTA t % parts =================
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                         for (int t = part + P.parts * grp; t < tn; t += U * step) {
                             float sum[U], f[2][U];                // bias and residual ride on part 0
 #pragma unroll
-                            for (int i = 0; i < U; i++) sum[i] = P.resid && t + i * step < tn ? __ldg(P.resid + (size_t) (t0 + t + i * step) * (size_t) P.N + n) : 0.f;
+                            for (int i = 0; i < U; i++) sum[i] = P.resid && t + i * step < tn ? P.resid[(size_t) (t0 + t + i * step) * (size_t) P.N + n] : 0.f;
                             for (int c = 0; c < P.parts; c += 2) {
 #pragma unroll
                                 for (int h = 0; h < 2; h++)
@@ -583,7 +586,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 const int n = row0 + quad * 32 + lane;
                 const bool live = acc_ok && n < P.N;
                 const float bias = (P.bias && live && first) ? P.bias[n] : 0.f;
-                const float * __restrict__ rp = (P.resid && first && live) ? P.resid + n : nullptr;
+                const float * rp = (P.resid && first && live) ? P.resid + n : nullptr;
                 const size_t ldd = (size_t) P.N;
                 for (int ch = (warp - MMQ_DQ_WARP0) >> 2; ch < nch; ch += 4) {
                     const int t0 = tt0 * BN + ch * 16;
@@ -594,7 +597,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     if (rp) {
                         const float * q = rp + (size_t) t0 * ldd;
 #pragma unroll
-                        for (int i = 0; i < 16; i++) y[i] = i < nt ? __ldg(q + i * ldd) : 0.f;
+                        for (int i = 0; i < 16; i++) y[i] = i < nt ? q[i * ldd] : 0.f;
                     } else {
 #pragma unroll
                         for (int i = 0; i < 16; i++) y[i] = 0.f;
@@ -658,19 +661,39 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
 // Fused producers of the activation (pre_kind): 1 = silu(x) * aux[t][k] (llm_build_ffn's SILU + MUL in front of ffn_down, the f32 product never
 // goes to HBM), 2 = rms_norm(x) * aux[k] (llm_build_norm in front of q|k|v and gate|up): the same arithmetic, rounding for rounding, as
 // k_silu_mul / k_rms_norm_rows followed by the plain pass.
+// Bound by the latency of its loads: a warp's first two blocks are fetched ahead of the norm's sum, which loads eight at a time, and long rows go over two CTAs
+// (a prompt of 512 tokens and 4 layers of 4096 / 14336: 1632 -> 1561 us with it).
 __device__ __forceinline__ float mmq_silu(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }   // ggml.c:2560
-__global__ void __launch_bounds__(256) k_mmq_prep(const float * __restrict__ x, int64_t ldx, int T, int K, int BN, uint8_t * __restrict__ out,
-                                                  int blk32, int pre_kind, const float * __restrict__ aux, int64_t ld_aux, float eps) {
+__global__ void __launch_bounds__(256) k_mmq_prep(const float * x, int64_t ldx, int T, int K, int BN, uint8_t * out,
+                                                  int blk32, int pre_kind, const float * aux, int64_t ld_aux, float eps) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nblk = (K + 255) / 256;
     const int t = blockIdx.x;                       // 0 .. Tpad-1
     const int b_bytes = BN * 128;
     float nscale = 1.f;
+    pdl_trigger();
+    pdl_wait();
+    // a warp's blocks two at a time, eight warps and gridDim.y CTAs apart; the first two are on their way while the row's norm is taken
+    const int step = 8 * (int) gridDim.y;
+    float4 xa[2], xb[2];
+    auto fetch = [&](int b0) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int b = b0 + j * step;
+            const float4 * p = reinterpret_cast<const float4 *>(x + (size_t) t * ldx + (size_t) b * 256 + lane * 8);
+            const bool live = t < T && b < nblk && b * 256 + lane * 8 < K;   // K % 32 == 0: a 4-lane group (one 32-block) is live or dead as a whole
+            xa[j] = live ? p[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+            xb[j] = live ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    const int first = warp + 8 * (int) blockIdx.y;
+    fetch(first);
     if (pre_kind == 2 && t < T) {                   // k_rms_norm_rows' sum, in its order (ggml.c:11950-11996: double-precision sum of squares)
         __shared__ double red[8];
         __shared__ float s_scale;
         const float * xr = x + (size_t) t * ldx;
         double sum = 0.0;
+#pragma unroll 8
         for (int i = threadIdx.x; i < K; i += 256) sum += (double) __fmul_rn(xr[i], xr[i]);
         sum = warp_sum_d(sum);
         if (lane == 0) red[warp] = sum;
@@ -684,70 +707,68 @@ __global__ void __launch_bounds__(256) k_mmq_prep(const float * __restrict__ x, 
         __syncthreads();
         nscale = s_scale;
     }
-    for (int b = warp; b < nblk; b += 8) {
-        float v[8];
-        const bool live = b * 256 + lane * 8 < K;   // K % 32 == 0: a 4-lane group (one 32-block) is live or dead as a whole
-        if (t < T && live) {
-            const float4 * p = reinterpret_cast<const float4 *>(x + (size_t) t * ldx + (size_t) b * 256 + lane * 8);
-            const float4 a = p[0], c = p[1];
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
-            if (pre_kind) {
+    for (int b0 = first; b0 < nblk; b0 += 2 * step) {
+        if (b0 != first) fetch(b0);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int b = b0 + u * step;
+            if (b >= nblk) break;
+            const bool live = b * 256 + lane * 8 < K;
+            float v[8] = {xa[u].x, xa[u].y, xa[u].z, xa[u].w, xb[u].x, xb[u].y, xb[u].z, xb[u].w};
+            if (pre_kind && t < T && live) {
                 const float4 * q = reinterpret_cast<const float4 *>(aux + (pre_kind == 1 ? (size_t) t * ld_aux : (size_t) 0) + (size_t) b * 256 + lane * 8);
                 const float4 e = q[0], f = q[1];
                 const float w[8] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
 #pragma unroll
                 for (int i = 0; i < 8; i++) v[i] = pre_kind == 1 ? __fmul_rn(mmq_silu(v[i]), w[i]) : __fmul_rn(__fmul_rn(v[i], nscale), w[i]);
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = 0.f;
-        }
-        float amax = 0.f, vmax = 0.f;
-        int idx = 0x7fffffff;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float ax = fabsf(v[i]);
-            if (ax > amax) { amax = ax; vmax = v[i]; idx = lane * 8 + i; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-            const float ov = __shfl_xor_sync(0xffffffffu, vmax, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (oa > amax || (oa == amax && oi < idx)) { amax = oa; vmax = ov; idx = oi; }
-        }
-        uint32_t h[4] = {0u, 0u, 0u, 0u};
-        if (blk32) {
-            float am = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) am = fmaxf(am, fabsf(v[i]));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-            const float d = __half2float(__float2half_rn(__fdiv_rn(am, 127.f)));
-            const float id = am != 0.f ? __fdiv_rn(127.f, am) : 0.f;
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = __fmul_rn(d, (float) __float2int_rn(__fmul_rn(v[i], id)));
-            h[0] = pack_h2(f[0], f[2]); h[1] = pack_h2(f[1], f[3]); h[2] = pack_h2(f[4], f[6]); h[3] = pack_h2(f[5], f[7]);
-        } else if (amax != 0.f) {
-            const float iscale = __fdiv_rn(-127.f, vmax);
-            const float d = __fdiv_rn(1.f, iscale);
-            float f[8];
+            float amax = 0.f, vmax = 0.f;
+            int idx = 0x7fffffff;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
-                int q = nearest_int_magic(__fmul_rn(iscale, v[i]));
-                q = q < 127 ? q : 127;
-                f[i] = __fmul_rn(d, (float) q);
+                const float ax = fabsf(v[i]);
+                if (ax > amax) { amax = ax; vmax = v[i]; idx = lane * 8 + i; }
             }
 #pragma unroll
-            // within every 4 consecutive k the order is (0,2,1,3): the weight expansion produces its half2 pairs that way
-            h[0] = pack_h2(f[0], f[2]); h[1] = pack_h2(f[1], f[3]); h[2] = pack_h2(f[4], f[6]); h[3] = pack_h2(f[5], f[7]);
+            for (int o = 16; o > 0; o >>= 1) {
+                const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
+                const float ov = __shfl_xor_sync(0xffffffffu, vmax, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+                if (oa > amax || (oa == amax && oi < idx)) { amax = oa; vmax = ov; idx = oi; }
+            }
+            uint32_t h[4] = {0u, 0u, 0u, 0u};
+            if (blk32) {
+                float am = 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; i++) am = fmaxf(am, fabsf(v[i]));
+                am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
+                am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+                const float d = __half2float(__float2half_rn(__fdiv_rn(am, 127.f)));
+                const float id = am != 0.f ? __fdiv_rn(127.f, am) : 0.f;
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) f[i] = __fmul_rn(d, (float) __float2int_rn(__fmul_rn(v[i], id)));
+                h[0] = pack_h2(f[0], f[2]); h[1] = pack_h2(f[1], f[3]); h[2] = pack_h2(f[4], f[6]); h[3] = pack_h2(f[5], f[7]);
+            } else if (amax != 0.f) {
+                const float iscale = __fdiv_rn(-127.f, vmax);
+                const float d = __fdiv_rn(1.f, iscale);
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    int q = nearest_int_magic(__fmul_rn(iscale, v[i]));
+                    q = q < 127 ? q : 127;
+                    f[i] = __fmul_rn(d, (float) q);
+                }
+#pragma unroll
+                // within every 4 consecutive k the order is (0,2,1,3): the weight expansion produces its half2 pairs that way
+                h[0] = pack_h2(f[0], f[2]); h[1] = pack_h2(f[1], f[3]); h[2] = pack_h2(f[4], f[6]); h[3] = pack_h2(f[5], f[7]);
+            }
+            const int k = b * 256 + lane * 8;
+            const int kc = k >> 6, j = (k & 63) >> 3;
+            const int tt = t / BN, tl = t % BN;
+            uint8_t * dstp = out + ((size_t) tt * (K / 64) + kc) * b_bytes + (size_t) tl * 128 + (size_t) ((j ^ (tl & 7)) << 4);
+            if (live) *reinterpret_cast<uint4 *>(dstp) = make_uint4(h[0], h[1], h[2], h[3]);
         }
-        const int k = b * 256 + lane * 8;
-        const int kc = k >> 6, j = (k & 63) >> 3;
-        const int tt = t / BN, tl = t % BN;
-        uint8_t * dstp = out + ((size_t) tt * (K / 64) + kc) * b_bytes + (size_t) tl * 128 + (size_t) ((j ^ (tl & 7)) << 4);
-        if (live) *reinterpret_cast<uint4 *>(dstp) = make_uint4(h[0], h[1], h[2], h[3]);
     }
 }
 
@@ -767,7 +788,7 @@ bool mmq_supported(int type, int64_t K) {
 }
 
 template <int TYPE, int CG, bool CUT>
-static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st) {
+static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
     static FuncAttrCache attr_cache;
     cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
     if (e != cudaSuccess) return e;
@@ -776,17 +797,19 @@ static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem
     cfg.blockDim = dim3(MMQ_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CUT ? (unsigned) P.parts : CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = CUT ? (unsigned) P.parts : CG; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = CG > 1 || CUT ? 1 : 0;
+    cfg.numAttrs = CG > 1 || CUT ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT>, P);
 }
 template <int TYPE>
-static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size_t smem, cudaStream_t st) {
-    if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, grid, smem, st);
-    return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, grid, smem, st) : mmq_launch_typed2<TYPE, 1, false>(P, grid, smem, st);
+static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
+    if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, grid, smem, st, pdl);
+    return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, grid, smem, st, pdl) : mmq_launch_typed2<TYPE, 1, false>(P, grid, smem, st, pdl);
 }
 // Clusters of `parts` CTAs of this kernel that run at the same time (a CTA takes an SM; a cluster stays within a group of SMs): what
 // cudaOccupancyMaxActiveClusters says on a B200, 5 and 7 from below.  A table and no query, so that the order of a sum does not follow which SMs of a GPU
@@ -836,7 +859,7 @@ static MmqCut mmq_pick_cut(int64_t tiles, int ngrp, int nsm, int max_parts, doub
 }
 
 cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const float * x, int64_t ldx, int64_t T, float * dst, const float * bias,
-                       const float * resid, void * ws, cudaStream_t st, bool reuse_prep, const MmqPre * pre) {
+                       const float * resid, void * ws, cudaStream_t st, bool reuse_prep, const MmqPre * pre, bool pdl) {
     if (pre && pre->kind != 0 && (!pre->aux || K % 256 != 0 || pre->kind < 0 || pre->kind > 2)) return cudaErrorInvalidValue;
     if (!mmq_supported(type, K) || N <= 0 || T <= 0) return cudaErrorInvalidValue;
     const int BN = mmq_pick_bn((int) T);
@@ -879,9 +902,18 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     if (total > 0x7fffffff) return cudaErrorInvalidValue;
     P.total_units = (int) total;
     if (!reuse_prep) {
-        k_mmq_prep<<<tpad, 256, 0, st>>>(x, ldx, (int) T, (int) K, BN, (uint8_t *) ws, is_kquant(type) ? 0 : 1, pre ? pre->kind : 0,
-                                         pre ? pre->aux : nullptr, pre ? pre->ld_aux : 0, pre ? pre->eps : 0.f);
-        cudaError_t e0 = cudaGetLastError();
+        const int kind = pre ? pre->kind : 0;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned) tpad, kind != 2 && K >= 32 * 256 ? 2 : 1);   // long rows over two CTAs (a norm wants the whole row)
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e0 = cudaLaunchKernelEx(&cfg, k_mmq_prep, x, ldx, (int) T, (int) K, BN, (uint8_t *) ws, is_kquant(type) ? 0 : 1, kind, pre ? pre->aux : (const float *) nullptr,
+                                                  pre ? pre->ld_aux : (int64_t) 0, pre ? pre->eps : 0.f);
         if (e0 != cudaSuccess) return e0;
     }
     uint32_t cols = 32;
@@ -915,11 +947,11 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
         if (e0 != cudaSuccess) return e0;
     }
     dim3 grid((unsigned) (cut.parts > 1 ? tiles * cut.parts : cg * (cut.chain > 0 ? mmq_chain_ctas(tiles, cut.chain) : (total + cut.upc - 1) / cut.upc)), 1, 1);
-    if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, cg, grid, smem, st);
-    if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, cg, grid, smem, st);
-    if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, cg, grid, smem, st);
-    if (type == T_Q8_0) return mmq_launch_typed<T_Q8_0>(P, cg, grid, smem, st);
-    return mmq_launch_typed<T_Q5_1>(P, cg, grid, smem, st);
+    if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, cg, grid, smem, st, pdl);
+    if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, cg, grid, smem, st, pdl);
+    if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, cg, grid, smem, st, pdl);
+    if (type == T_Q8_0) return mmq_launch_typed<T_Q8_0>(P, cg, grid, smem, st, pdl);
+    return mmq_launch_typed<T_Q5_1>(P, cg, grid, smem, st, pdl);
 }
 
 }  // namespace pb

@@ -239,6 +239,57 @@ __global__ void k_rope_kvstore(float * __restrict__ q, const float * __restrict_
     }
 }
 
+// A prompt's tokens: one CTA per token takes its angles once; a warp takes a head, a lane four neighbouring entries.  512 tokens, 32 heads over 8: rotation of q and of k
+// and two conversions into the cache, with a CTA and its angles per head and token, 13.9 + 5.8 + 3.7 + 3.7 us; this 8.1 (20 MB).
+__global__ void __launch_bounds__(256) k_rope_kvstore_batch(float * q, const float * k, const float * v, __half * kc, __half * vc, int n_head, int n_head_kv, const int32_t * pos_dev,
+                                                            RopeParams rp, const float * __restrict__ freq_factors) {
+    constexpr int D = 128;
+    __shared__ __align__(16) float cs[64][2];
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half_dims = rp.n_dims / 2;
+    const bool neox = rp.mode & 2;
+    pdl_trigger();
+    pdl_wait();
+    const int32_t pos = pos_dev[t];
+    if ((int) threadIdx.x < half_dims) rope_cos_sin(rp, pos, threadIdx.x, freq_factors, cs[threadIdx.x][0], cs[threadIdx.x][1]);
+    __syncthreads();
+    const int64_t row = (int64_t) pos * n_head_kv * D;
+    for (int task = warp; task < n_head + 2 * n_head_kv; task += 8) {
+        const bool is_q = task < n_head, is_v = task >= n_head + n_head_kv;
+        const int h = is_q ? task : is_v ? task - n_head - n_head_kv : task - n_head;
+        const float * src = is_q ? q + ((int64_t) t * n_head + h) * D : (is_v ? v : k) + ((int64_t) t * n_head_kv + h) * D;
+        float4 x = *reinterpret_cast<const float4 *>(src + 4 * lane);
+        if (!is_v && !neox && 4 * lane < rp.n_dims) {
+            const float4 f = *reinterpret_cast<const float4 *>(&cs[2 * lane][0]);   // pairs 2 lane and 2 lane + 1
+            float4 r;
+            rope_rotate(x.x, x.y, f.x, f.y, r.x, r.y);
+            rope_rotate(x.z, x.w, f.z, f.w, r.z, r.w);
+            x = r;
+        } else if (!is_v && neox) {                       // entry i meets entry i + n_dims / 2
+            const bool low = 4 * lane < half_dims, high = !low && 4 * lane < rp.n_dims;
+            const int other = low ? lane + rp.n_dims / 8 : high ? lane - rp.n_dims / 8 : lane;
+            const float mine[4] = {x.x, x.y, x.z, x.w};
+            float r[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float o = __shfl_sync(0xffffffffu, mine[i], other);
+                r[i] = mine[i];
+                if (low || high) {
+                    const float * f = cs[4 * (low ? lane : other) + i];
+                    float a, b;
+                    rope_rotate(low ? mine[i] : o, low ? o : mine[i], f[0], f[1], a, b);
+                    r[i] = low ? a : b;
+                }
+            }
+            x = make_float4(r[0], r[1], r[2], r[3]);
+        }
+        if (is_q) *reinterpret_cast<float4 *>(q + ((int64_t) t * n_head + h) * D + 4 * lane) = x;
+        else {
+            const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+            *reinterpret_cast<uint2 *>((is_v ? vc : kc) + row + h * D + 4 * lane) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        }
+    }
+}
+
 // generic rope for the plugin: one CTA per (token, head)
 __global__ void k_rope(const float * __restrict__ x, float * __restrict__ y, int n_head, int D, int64_t tok_stride, int64_t head_stride,
                        const int32_t * __restrict__ pos, RopeParams rp, const float * __restrict__ freq_factors) {
@@ -1286,6 +1337,14 @@ int launch_rope_kvstore(float * q, const float * k, const float * v, __half * kc
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
     launch_cfg(cfg, attr, dim3(n_head + n_head_kv), dim3(D / 2), 0, stream, pdl);
     return (int) cudaLaunchKernelEx(&cfg, k_rope_kvstore, q, k, v, kcache, vcache, n_head, n_head_kv, D, pos_dev, rp, freq_factors);
+}
+int launch_rope_kvstore_batch(float * q, const float * k, const float * v, __half * kcache, __half * vcache, int n_tok, int n_head, int n_head_kv, int D, const int32_t * pos_dev,
+                              const RopeParams & rp, const float * freq_factors, cudaStream_t stream, bool pdl) {
+    const uintptr_t a = (uintptr_t) q | (uintptr_t) k | (uintptr_t) v | (uintptr_t) kcache | (uintptr_t) vcache;
+    if (D != 128 || n_tok <= 0 || rp.n_dims <= 0 || rp.n_dims > 128 || rp.n_dims % 8 != 0 || (a & 15) != 0) return (int) cudaErrorNotSupported;
+    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+    launch_cfg(cfg, attr, dim3((unsigned) n_tok), dim3(256), 0, stream, pdl);
+    return (int) cudaLaunchKernelEx(&cfg, k_rope_kvstore_batch, q, k, v, kcache, vcache, n_head, n_head_kv, pos_dev, rp, freq_factors);
 }
 int launch_rope(const float * x, float * y, int64_t ntok, int n_head, int D, int64_t tok_stride, int64_t head_stride, const int32_t * pos,
                 const RopeParams & rp, const float * freq_factors, cudaStream_t stream) {

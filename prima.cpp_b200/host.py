@@ -68,6 +68,7 @@ class Lib:
         c.pb200_mul_mat_vec_host.argtypes = [C.c_int, vp, i64, i64, vp, vp]
         c.pb200_rms_norm.argtypes = [vp, vp, i64, i64, f32, vp]
         c.pb200_rope.argtypes = [vp, vp, i64, C.c_int, C.c_int, C.c_int, C.c_int, vp, f32, f32, f32, f32, f32, f32, C.c_int, vp, vp]
+        c.pb200_rope_kv_prompt.argtypes = [vp] * 5 + [i64, C.c_int, C.c_int, C.c_int, C.c_int, vp, f32, f32, f32, f32, f32, f32, C.c_int, vp, vp]
         c.pb200_soft_max.argtypes = [vp, vp, vp, i64, i64, i64, f32, vp]
         c.pb200_silu_mul.argtypes = [vp, vp, vp, i64, vp]
         c.pb200_get_rows.argtypes = [C.c_int, vp, i64, vp, i64, vp, vp]
