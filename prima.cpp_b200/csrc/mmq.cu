@@ -25,10 +25,14 @@
 //   warp 0      owns TMEM; one lane issues 4 x tcgen05.mma (M=128, N=BN, K=16, kind::f16) per step and accumulator, one commit per step
 //   warp 1      activation producer: one cp.async.bulk per step and accumulator of the pre-tiled fp16 chunk (BN x 128 B, already in the
 //               UMMA swizzle-128B image), 2-4 stages deep
-//   warps 2..17 (16 expansion warps, 4 threads per weight row) fetch their rows' raw quantized blocks (16-byte cp.async pieces, 3 K groups
-//               deep, completion through cp.async.mbarrier.arrive) and expand 128 x 64 weights per step to fp16 straight into the swizzled A
+//   warp 18     fetches the rows' raw quantized blocks, a K group of the tile as one TMA box, 3 groups deep (rows that do not lie at multiples of 16
+//               bytes: the expansion warps fetch them in 16-byte cp.async pieces)
+//   warps 2..17 (16 expansion warps, 4 threads per weight row) take a group's blocks into registers (Q4_K, Q5_K: header and quants at once) and expand 128 x 64 weights per step to fp16 straight into the swizzled A
 //               stage (generic-proxy stores + fence.proxy.async), 2 stages (4 with CTA pairs); at the end of a segment or part all 16 read the
 //               accumulators out of TMEM (tcgen05.ld 32x32b: quadrant = warp % 4, every fourth chunk of 16 columns) and store / add into dst
+// What bounds it: with two accumulators the tensor pipe (a step takes 1424 clocks, its eight M = 128, N = 256 MMAs 1368); with one, the chain of waits, fence
+// and commit of a step (1050 clocks at 64 tokens).  14336 x 4096 at 512 tokens, Q4_K, raw blocks and scales by every thread -> by boxes and groups: 173 -> 126
+// instructions a warp and step, 69.5 -> 67 us; Q6_K 4096 x 14336 73.5 -> 71; a group with few tokens 2.7 -> 2.3 us.
 // CG = 2 (opt-in): the CTA pair of a cluster shares one M = 256 MMA (cta_group::2), see launch_mmq.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -38,6 +42,7 @@
 
 #include "common.cuh"
 #include "launch.h"
+#include "tc.cuh"
 
 namespace pb {
 
@@ -47,7 +52,8 @@ constexpr int MMQ_A_MAX = 4;      // expanded-weight stages: P.a_nst = 2 or 4 (a
 constexpr int MMQ_B_NST = 4;      // activation stages (L2 loads: the deep ring)
 constexpr int MMQ_DQ_WARPS = 16;  // expansion warps: 4 threads per weight row, 16 weights per thread and step (8 warps were the latency-bound bottleneck: 45 % tensor pipe)
 constexpr int MMQ_DQ_WARP0 = 2;   // warps 0,1 = MMA issuer (owns TMEM), activation producer
-constexpr int MMQ_THREADS = (MMQ_DQ_WARP0 + MMQ_DQ_WARPS) * 32;
+constexpr int MMQ_RAW_WARP = MMQ_DQ_WARP0 + MMQ_DQ_WARPS;   // fetches the raw blocks by tiled TMA
+constexpr int MMQ_THREADS = (MMQ_RAW_WARP + 1) * 32;
 constexpr int MMQ_A_BYTES = MMQ_BM * 128;   // one A stage: 128 rows x 64 fp16
 constexpr int MMQ_CTL_BYTES = 320;
 constexpr int MMQ_MAX_PARTS = 8;  // CTAs of a cluster that share a tile's K
@@ -65,6 +71,7 @@ struct MmqParams {
     int ngrp, rtiles;      // 256-K groups per row (the last one may be short: 32-element block types), row tiles
     int parts;             // > 1: the CTAs of a cluster, one tile each cluster, share the tile's K groups; else
     int upc, total_units;  // work units per CTA (CTA c owns units [c * upc, min((c + 1) * upc, total_units)) ), units of the launch
+    int tma;               // the raw blocks come by tiled TMA; 0: rows that do not lie at multiples of 16 bytes, fetched by the expansion warps
     int chain;             // > 0: instead, chains of that many tiles (the last one: what is left), each in equal shares for one CTA more than it has tiles
     int N, K, T, BN, bpb, slot;   // slot: bytes reserved per row in a raw stage (16-B aligned window around one block)
     uint32_t tmem_cols, idesc;
@@ -218,14 +225,6 @@ __device__ __forceinline__ void expand_word(uint32_t t, __half2 bias, __half2 sc
     o02 = h2_bits(__hfma2(__hadd2(bits_h2(p02), bias), scale, off));
     o13 = h2_bits(__hfma2(__hadd2(bits_h2(p13), bias), scale, off));
 }
-__device__ __forceinline__ void scale_min_k4(const uint8_t * sc, int j, int & s, int & m) {   // get_scale_min_k4, ggml-quants.c:1950-1958
-    // branch-free: both packings are computed, j selects
-    const int lo_s = sc[j & 3], lo_m = sc[(j & 3) + 4], hi = sc[(j & 3) + 8];
-    const int s0 = lo_s & 63, m0 = lo_m & 63;
-    const int s1 = (hi & 0xF) | ((lo_s >> 6) << 4), m1 = (hi >> 4) | ((lo_m >> 6) << 4);
-    s = j < 4 ? s0 : s1;
-    m = j < 4 ? m0 : m1;
-}
 // thread (row, h, hh) produces K elements [64c + 32h + 16hh, 64c + 32h + 16hh + 16) of its row as 8 half2 (two 16-byte pieces of the A stage)
 template <int TYPE>
 __device__ __forceinline__ void expand(const uint8_t * blk, int c, int h, int hh, uint32_t (&out)[8]) {
@@ -260,27 +259,6 @@ __device__ __forceinline__ void expand(const uint8_t * blk, int c, int h, int hh
             const uint32_t hb = ((((qh >> (4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
             expand_word<0x001F001Fu>(((w[i] >> (4 * hh)) & 0x0F0F0F0Fu) | hb, bias, scale, off, out[2 * i], out[2 * i + 1]);
         }
-    } else if (TYPE == T_Q4_K || TYPE == T_Q5_K) {
-        const float d = __half2float(*reinterpret_cast<const __half *>(blk));
-        const float dmin = __half2float(*reinterpret_cast<const __half *>(blk + 2));
-        const int j = 2 * c + h;
-        int s, m;
-        scale_min_k4(blk + 4, j, s, m);
-        const __half2 scale = __float2half2_rn(__fmul_rn(d, (float) s)), off = __float2half2_rn(-__fmul_rn(dmin, (float) m));
-        const __half2 bias = __float2half2_rn(-1024.f);
-        const uint4 qa = *reinterpret_cast<const uint4 *>(blk + (TYPE == T_Q4_K ? 16 : 48) + 32 * c + 16 * hh);
-        const uint32_t w[4] = {qa.x, qa.y, qa.z, qa.w};
-        if (TYPE == T_Q4_K) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) expand_word<0x000F000Fu>(w[i] >> (4 * h), bias, scale, off, out[2 * i], out[2 * i + 1]);
-        } else {
-            const uint4 ha = *reinterpret_cast<const uint4 *>(blk + 16 + 16 * hh);
-            const uint32_t hq[4] = {ha.x, ha.y, ha.z, ha.w};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                expand_word<0x001F001Fu>(((w[i] >> (4 * h)) & 0x0F0F0F0Fu) | (((hq[i] >> j) << 4) & 0x10101010u), bias, scale, off, out[2 * i],
-                                         out[2 * i + 1]);
-        }
     } else {
         // Q6_K: blk is 2-byte aligned only (210-byte blocks): words are fetched as aligned pairs and funnel-shifted
         const float d = __half2float(*reinterpret_cast<const __half *>(blk + 208));
@@ -305,12 +283,63 @@ __device__ __forceinline__ void expand(const uint8_t * blk, int c, int h, int hh
     }
 }
 
+// Q4_K / Q5_K: what a thread takes of its row's block, all four steps of it: scales and offsets of the sub-blocks 2c + h (get_scale_min_k4, ggml-quants.c:1950-1958, for
+// four bytes at a time; byte 2 (c & 1) of word c / 2 is step c's), the quants' words and for Q5_K the words of the fifth bits.  The header so is one load of a group and not five a step.
+template <int TYPE>
+struct KGroup {
+    float d, dmin;
+    uint32_t s[2], m[2], hb[4];
+    uint4 q[4];
+    __device__ __forceinline__ void load(const uint8_t * blk, int h, int hh) {
+        const uint4 hd = *reinterpret_cast<const uint4 *>(blk);
+#pragma unroll
+        for (int c = 0; c < 4; c++) q[c] = *reinterpret_cast<const uint4 *>(blk + (TYPE == T_Q4_K ? 16 : 48) + 32 * c + 16 * hh);
+        if (TYPE == T_Q5_K) {
+            const uint4 b = *reinterpret_cast<const uint4 *>(blk + 16 + 16 * hh);
+            hb[0] = b.x >> h; hb[1] = b.y >> h; hb[2] = b.z >> h; hb[3] = b.w >> h;
+        }
+        const __half2 dm = bits_h2(hd.x);
+        d = __low2float(dm);
+        dmin = __high2float(dm);
+        s[0] = (hd.y & 0x3f3f3f3fu) >> (8 * h);
+        m[0] = (hd.z & 0x3f3f3f3fu) >> (8 * h);
+        s[1] = ((hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u)) >> (8 * h);
+        m[1] = (((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u)) >> (8 * h);
+    }
+    static __device__ __forceinline__ float byte_f(uint32_t w, int c) {   // exact: 2^23 + byte less 2^23
+        return __fadd_rn(__uint_as_float(and_or((c & 1) ? w >> 16 : w, 0xffu, 0x4b000000u)), -8388608.f);
+    }
+    __device__ __forceinline__ void expand(int c, int h, uint32_t (&out)[8]) const {
+        const __half2 so = __floats2half2_rn(__fmul_rn(d, byte_f(s[c >> 1], c)), -__fmul_rn(dmin, byte_f(m[c >> 1], c)));
+        const __half2 scale = __low2half2(so), off = __high2half2(so);
+        const uint32_t w[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
+        // a nibble in the low place makes 1024 + q, one in the high place 64 + q (0x5400 = 64, steps of 1 / 16)
+        const uint32_t mask = h ? 0x00F000F0u : 0x000F000Fu, magic = h ? 0x54005400u : 0x64006400u;
+        const __half2 bias = TYPE == T_Q5_K ? __float2half2_rn(-1024.f) : bits_h2(h ? 0xD400D400u : 0xE400E400u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (TYPE == T_Q4_K) {
+                const uint32_t p02 = (w[i] & mask) | magic, p13 = ((w[i] >> 8) & mask) | magic;
+                out[2 * i] = h2_bits(__hfma2(__hadd2(bits_h2(p02), bias), scale, off));
+                out[2 * i + 1] = h2_bits(__hfma2(__hadd2(bits_h2(p13), bias), scale, off));
+            } else {
+                const uint32_t fifth = c < 2 ? hb[i] << (4 - 2 * c) : hb[i] >> (2 * c - 4);
+                expand_word<0x001F001Fu>(((w[i] >> (4 * h)) & 0x0F0F0F0Fu) | (fifth & 0x10101010u), bias, scale, off, out[2 * i], out[2 * i + 1]);
+            }
+        }
+    }
+};
+
+__device__ __forceinline__ void tma_raw(uint32_t dst, const CUtensorMap * m, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(m), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async16(void * smem_dst, const void * gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
 
 template <int TYPE, int CG, bool CUT>
-__global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant__ MmqParams P) {
+__global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant__ MmqParams P, const __grid_constant__ CUtensorMap map_w) {
     extern __shared__ uint8_t smem_raw[];
     // the swizzle-128B atoms (A and B stages) need 1024-byte alignment in the shared window
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -325,7 +354,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
     uint8_t * raw = b_st + P.b_nst * b_bytes;                    // [nraw][128 * slot]
     MmqCtl * ctl = reinterpret_cast<MmqCtl *>(raw + P.nraw * MMQ_BM * P.slot);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nstep_all = P.K / MMQ_BK;                          // 64-element steps of a whole row; group sb holds steps [4 sb, min(4 sb + 4, nstep_all))
     // this CTA's (pair's) units; CUT: the part-th of a tile's equal consecutive parts, one segment
     const int part = CUT ? (int) blockIdx.x % P.parts : 0, cut0 = CUT ? (int) blockIdx.x / P.parts * P.ngrp : 0;
@@ -339,7 +368,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
     }
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 3; i++) { mbar_init(&ctl->raw_full[i], MMQ_DQ_WARPS * 32); mbar_init(&ctl->raw_empty[i], MMQ_DQ_WARPS); }
+        for (int i = 0; i < 3; i++) { mbar_init(&ctl->raw_full[i], P.tma ? 1 : MMQ_DQ_WARPS * 32); mbar_init(&ctl->raw_empty[i], MMQ_DQ_WARPS); }
         for (int i = 0; i < MMQ_A_MAX; i++) mbar_init(&ctl->a_ready[i], MMQ_DQ_WARPS);
         for (int i = 0; i < MMQ_B_NST; i++) { mbar_init(&ctl->b_full[i], 1); mbar_init(&ctl->step_done[i], 1); }
         mbar_init(&ctl->acc_ready, 1);
@@ -383,25 +412,25 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         }
         __syncwarp();
     } else if (warp == 0) {
-        // ================= MMA issuer =================
-        if (lane == 0) {
-            int g = 0, seg = 0;                                  // CTA-wide step and segment counters (barrier phases follow them)
-            bool ok = true;
-            for (int w = w0; w < w1 && ok; seg++) {
-                const int tile = w / P.ngrp, sbb = w - tile * P.ngrp, sbe = min(P.ngrp, sbb + (w1 - w));
-                const int nacc = min(P.nacc, P.ttiles - (tile / P.rtiles) * P.nacc);
-                const int nsteps = min(4 * sbe, nstep_all) - 4 * sbb;
-                if (seg > 0 && !mmq_wait(ctl, &ctl->acc_free, (seg - 1) & 1)) break;   // the previous segment's accumulators have been read out
+        // ================= MMA issuer (the whole warp walks, an elected lane issues) =================
+        int g = 0, seg = 0;                                      // CTA-wide step and segment counters (barrier phases follow them)
+        bool ok = true;
+        for (int w = w0; w < w1 && ok; seg++) {
+            const int tile = w / P.ngrp, sbb = w - tile * P.ngrp, sbe = min(P.ngrp, sbb + (w1 - w));
+            const int nacc = min(P.nacc, P.ttiles - (tile / P.rtiles) * P.nacc);
+            const int nsteps = min(4 * sbe, nstep_all) - 4 * sbb;
+            if (seg > 0 && !mmq_wait(ctl, &ctl->acc_free, (seg - 1) & 1)) break;   // the previous segment's accumulators have been read out
+            tc_fence_after();
+            for (int u = 0; u < nsteps; u++, g++) {
+                const int sa = g & amask, sb = g % P.b_nst;
+                if (!mmq_wait(ctl, &ctl->b_full[sb], (g / P.b_nst) & 1)) { ok = false; break; }
+                if (!mmq_wait(ctl, &ctl->a_ready[sa], (g >> ashift) & 1)) { ok = false; break; }
+                if (CG == 2 && !mmq_wait(ctl, &ctl->peer_ready[g % MMQ_B_NST], (g / MMQ_B_NST) & 1)) { ok = false; break; }
                 tc_fence_after();
-                for (int u = 0; u < nsteps; u++, g++) {
-                    const int sa = g & amask, sb = g % P.b_nst;
-                    if (!mmq_wait(ctl, &ctl->b_full[sb], (g / P.b_nst) & 1)) { ok = false; break; }
-                    if (!mmq_wait(ctl, &ctl->a_ready[sa], (g >> ashift) & 1)) { ok = false; break; }
-                    if (CG == 2 && !mmq_wait(ctl, &ctl->peer_ready[g % MMQ_B_NST], (g / MMQ_B_NST) & 1)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t da = umma_desc_sw128(smem_u32(a_st + (size_t) sa * MMQ_A_BYTES));
-                    const uint64_t db = umma_desc_sw128(smem_u32(b_st + (size_t) sb * b_bytes));
-                    const uint64_t db2 = umma_desc_sw128(smem_u32(b_st + (size_t) sb * b_bytes + b1c));
+                const uint64_t da = umma_desc_sw128(smem_u32(a_st + (size_t) sa * MMQ_A_BYTES));
+                const uint64_t db = umma_desc_sw128(smem_u32(b_st + (size_t) sb * b_bytes));
+                const uint64_t db2 = umma_desc_sw128(smem_u32(b_st + (size_t) sb * b_bytes + b1c));
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < MMQ_BK / 16; k++) {
                         if (CG == 2) {
@@ -414,39 +443,57 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     }
                     if (CG == 2) umma_commit_cg2(&ctl->step_done[g % MMQ_B_NST]); else umma_commit(&ctl->step_done[g % MMQ_B_NST]);
                 }
-                if (CG == 2) umma_commit_cg2(&ctl->acc_ready); else umma_commit(&ctl->acc_ready);
-                w += sbe - sbb;
+                __syncwarp();
             }
+            if (elect_one()) {
+                if (CG == 2) umma_commit_cg2(&ctl->acc_ready); else umma_commit(&ctl->acc_ready);
+            }
+            __syncwarp();
+            w += sbe - sbb;
         }
-        __syncwarp();
     } else if (warp == 1) {
         // ================= activation producer: runs up to b_nst steps ahead of the tensor core =================
         pdl_wait();                // activations are the kernel in front's; weights are fetched and expanded meanwhile
-        if (lane == 0) {
-            const size_t tile_stride = (size_t) nstep_all * b1;
-            int g = 0;
-            bool ok = true;
-            for (int w = w0; w < w1 && ok;) {
-                const int tile = w / P.ngrp, sbb = w - tile * P.ngrp, sbe = min(P.ngrp, sbb + (w1 - w));
-                const int tt0 = (tile / P.rtiles) * P.nacc;
-                const int nacc = min(P.nacc, P.ttiles - tt0);
-                const int nsteps = min(4 * sbe, nstep_all) - 4 * sbb;
-                const uint8_t * Bt = P.B + (size_t) tt0 * tile_stride + (size_t) sbb * 4 * b1 + (size_t) rank * b1c;
-                for (int u = 0; u < nsteps; u++, g++) {
-                    const int sb = g % P.b_nst;
-                    if (g >= P.b_nst) {   // step g - b_nst consumed this stage
-                        const int f = g - P.b_nst;
-                        if (!mmq_wait(ctl, &ctl->step_done[f % MMQ_B_NST], (f / MMQ_B_NST) & 1)) { ok = false; break; }
-                    }
+        const size_t tile_stride = (size_t) nstep_all * b1;
+        int g = 0;
+        bool ok = true;
+        for (int w = w0; w < w1 && ok;) {
+            const int tile = w / P.ngrp, sbb = w - tile * P.ngrp, sbe = min(P.ngrp, sbb + (w1 - w));
+            const int tt0 = (tile / P.rtiles) * P.nacc;
+            const int nacc = min(P.nacc, P.ttiles - tt0);
+            const int nsteps = min(4 * sbe, nstep_all) - 4 * sbb;
+            const uint8_t * Bt = P.B + (size_t) tt0 * tile_stride + (size_t) sbb * 4 * b1 + (size_t) rank * b1c;
+            for (int u = 0; u < nsteps; u++, g++) {
+                const int sb = g % P.b_nst;
+                if (g >= P.b_nst) {   // step g - b_nst consumed this stage
+                    const int f = g - P.b_nst;
+                    if (!mmq_wait(ctl, &ctl->step_done[f % MMQ_B_NST], (f / MMQ_B_NST) & 1)) { ok = false; break; }
+                }
+                if (elect_one()) {
                     mbar_arrive_expect_tx(&ctl->b_full[sb], (uint32_t) (nacc * b1c));
                     for (int a = 0; a < nacc; a++)
-                        bulk_g2s_plain(b_st + (size_t) sb * b_bytes + (size_t) a * b1c, Bt + (size_t) a * tile_stride + (size_t) u * b1, (uint32_t) b1c,
-                                       &ctl->b_full[sb]);
+                        bulk_g2s_plain(b_st + (size_t) sb * b_bytes + (size_t) a * b1c, Bt + (size_t) a * tile_stride + (size_t) u * b1, (uint32_t) b1c, &ctl->b_full[sb]);
                 }
-                w += sbe - sbb;
+                __syncwarp();
+            }
+            w += sbe - sbb;
+        }
+    } else if (warp == MMQ_RAW_WARP) {
+        // ================= raw blocks: a K group of the tile's rows is one box, up to nraw groups ahead =================
+        if (P.tma) {
+            const int nx = w1 - w0;
+            int sb = w0 % P.ngrp, rt = w0 / P.ngrp % P.rtiles, slot = 0, ph = 1;
+            for (int x = 0; x < nx; x++) {
+                if (x >= P.nraw && !mmq_wait(ctl, &ctl->raw_empty[slot], ph)) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&ctl->raw_full[slot], (uint32_t) (MMQ_BM * P.slot));
+                    tma_raw(smem_u32(raw + (size_t) slot * MMQ_BM * P.slot), &map_w, (sb * P.bpb & ~15) >> 1, (rt * CG + (int) rank) * MMQ_BM, smem_u32(&ctl->raw_full[slot]));
+                }
+                __syncwarp();
+                if (++slot == P.nraw) { slot = 0; ph ^= 1; }
+                if (++sb == P.ngrp) { sb = 0; if (++rt == P.rtiles) rt = 0; }
             }
         }
-        __syncwarp();
     } else {
         // ================= weight expansion =================
         const int dt = threadIdx.x - MMQ_DQ_WARP0 * 32;        // 0..511
@@ -469,7 +516,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             f_x++;
             if (++f_sb == P.ngrp) { f_sb = 0; if (++f_rt == P.rtiles) f_rt = 0; }
         };
-        for (int i = 0; i < P.nraw - 1 && i < nx; i++) fetch_next(i);
+        if (!P.tma) for (int i = 0; i < P.nraw - 1 && i < nx; i++) fetch_next(i);
         // the four 16-byte pieces this thread writes per step, already swizzled
         const uint32_t arow = r * 128;
         const uint32_t o0 = arow + (((4 * h + 2 * hh + 0) ^ (r & 7)) << 4), o1 = arow + (((4 * h + 2 * hh + 1) ^ (r & 7)) << 4);
@@ -482,7 +529,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             const int gr = min(row0 + r, P.N - 1);
             for (int sb = sbb; sb < sbe && ok; sb++) {
                 // refill the slot the previous group used, once every expansion warp has left it
-                if (f_x < nx) {
+                if (!P.tma && f_x < nx) {
                     if (f_x >= P.nraw && !mmq_wait(ctl, &ctl->raw_empty[prs], pph)) { ok = false; break; }
                     fetch_next(prs);
                 }
@@ -490,11 +537,19 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 const int64_t g0 = (int64_t) gr * P.row_bytes + (int64_t) sb * P.bpb;
                 const uint8_t * blk = raw + (size_t) (rs * MMQ_BM + r) * P.slot + (g0 & 15);
                 const int nst = min(4, nstep_all - 4 * sb);      // the last group of a K % 256 != 0 row (32-element block types) is short
+                constexpr bool K45 = TYPE == T_Q4_K || TYPE == T_Q5_K;
+                KGroup<TYPE> kg;
+                if constexpr (K45) {
+                    kg.load(blk, h, hh);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
+                }
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     if (c >= nst) break;
                     uint32_t v[8];
-                    expand<TYPE>(blk, c, h, hh, v);
+                    if constexpr (K45) kg.expand(c, h, v);
+                    else expand<TYPE>(blk, c, h, hh, v);
                     if (g >= P.a_nst) {     // step g - a_nst has consumed this A stage
                         const int f = g - P.a_nst;
                         if (!mmq_wait(ctl, &ctl->step_done[f % MMQ_B_NST], (f / MMQ_B_NST) & 1)) { ok = false; break; }
@@ -507,8 +562,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     if (lane == 0) mbar_arrive(&ctl->a_ready[g & amask]);
                     g++;
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
+                if (!K45) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
+                }
                 prs = rs; pph = rph;
                 if (++rs == P.nraw) { rs = 0; rph ^= 1; }
             }
@@ -641,7 +698,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             w += sbe - sbb;
         }
     }
-    if (CUT && warp < MMQ_DQ_WARP0) {   // the cluster's barriers count every warp
+    if (CUT && (warp < MMQ_DQ_WARP0 || warp == MMQ_RAW_WARP)) {   // the cluster's barriers count every warp
         const int rounds = min(P.nacc, P.ttiles - (w0 / P.ngrp / P.rtiles) * P.nacc);
         for (int i = 0; i < rounds; i++) { mmq_cluster_sync(); mmq_cluster_read(); }
     }
@@ -788,7 +845,7 @@ bool mmq_supported(int type, int64_t K) {
 }
 
 template <int TYPE, int CG, bool CUT>
-static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
+static cudaError_t mmq_launch_typed2(const MmqParams & P, const CUtensorMap & map_w, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
     static FuncAttrCache attr_cache;
     cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
     if (e != cudaSuccess) return e;
@@ -804,12 +861,12 @@ static cudaError_t mmq_launch_typed2(const MmqParams & P, dim3 grid, size_t smem
     attr[1].val.clusterDim.x = CUT ? (unsigned) P.parts : CG; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = CG > 1 || CUT ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT>, P);
+    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT>, P, map_w);
 }
 template <int TYPE>
-static cudaError_t mmq_launch_typed(const MmqParams & P, int cg, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
-    if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, grid, smem, st, pdl);
-    return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, grid, smem, st, pdl) : mmq_launch_typed2<TYPE, 1, false>(P, grid, smem, st, pdl);
+static cudaError_t mmq_launch_typed(const MmqParams & P, const CUtensorMap & map_w, int cg, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
+    if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, map_w, grid, smem, st, pdl);
+    return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, map_w, grid, smem, st, pdl) : mmq_launch_typed2<TYPE, 1, false>(P, map_w, grid, smem, st, pdl);
 }
 // Clusters of `parts` CTAs of this kernel that run at the same time (a CTA takes an SM; a cluster stays within a group of SMs): what
 // cudaOccupancyMaxActiveClusters says on a B200, 5 and 7 from below.  A table and no query, so that the order of a sum does not follow which SMs of a GPU
@@ -946,12 +1003,20 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
         cudaError_t e0 = cudaMemsetAsync(dst, 0, (size_t) T * (size_t) N * sizeof(float), st);
         if (e0 != cudaSuccess) return e0;
     }
+    CUtensorMap map_w{};
+    if (P.row_bytes % 16 == 0 && ((uintptr_t) W & 15) == 0) {   // 16-bit entries: a box is at most 256 of them wide
+        const EncodeTiled fn = encode_tiled();
+        const cuuint64_t dims[2] = {(cuuint64_t) P.row_bytes / 2, (cuuint64_t) N}, strides[1] = {(cuuint64_t) P.row_bytes};
+        const cuuint32_t box[2] = {(cuuint32_t) P.slot / 2, MMQ_BM}, one[2] = {1, 1};
+        P.tma = fn && fn(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void *) W, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
     dim3 grid((unsigned) (cut.parts > 1 ? tiles * cut.parts : cg * (cut.chain > 0 ? mmq_chain_ctas(tiles, cut.chain) : (total + cut.upc - 1) / cut.upc)), 1, 1);
-    if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, cg, grid, smem, st, pdl);
-    if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, cg, grid, smem, st, pdl);
-    if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, cg, grid, smem, st, pdl);
-    if (type == T_Q8_0) return mmq_launch_typed<T_Q8_0>(P, cg, grid, smem, st, pdl);
-    return mmq_launch_typed<T_Q5_1>(P, cg, grid, smem, st, pdl);
+    if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, map_w, cg, grid, smem, st, pdl);
+    if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, map_w, cg, grid, smem, st, pdl);
+    if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, map_w, cg, grid, smem, st, pdl);
+    if (type == T_Q8_0) return mmq_launch_typed<T_Q8_0>(P, map_w, cg, grid, smem, st, pdl);
+    return mmq_launch_typed<T_Q5_1>(P, map_w, cg, grid, smem, st, pdl);
 }
 
 }  // namespace pb
