@@ -884,7 +884,7 @@ static int mmq_clusters(int parts, int nsm) {
 // Where a tile is cut once its two sums meet on a cleared output: in either order they give the same bits.  An element's sum so has one order,
 // fixed by the launch's tiles and K groups, not by its tokens: the same call gives the same bits, and k-quant weights give a row the same
 // bits with 8 or 511 others beside it.
-// Costs in us on B200, Q4_K, 512 tokens: a unit 3.05 (2.7 with few tokens: the expansion of the weights), a segment's fill and read-out 8, the join of
+// Costs in us on B200, Q4_K, 512 tokens: a unit 3.05 (2.3 with few tokens: the chain of a step), a segment's fill and read-out 8, the join of
 // p parts 7.5 + 1.25 p (what distributed shared memory gives: 256 KB a CTA; in proportion to the tokens), the clearing pass 3 + bytes /
 // 6.2 TB/s.  Measured with the activation pass, K = 4096, 512 tokens: 1024 rows whole 63.5, 2 parts 48.7, 4 parts 38.4, 8 parts 34.1; 4096 rows
 // whole 63.7, 4 parts 37.2; 64 tokens: 1024 rows 53.3, 31.9, 21.8, 16.6.  8192 x 8192 in halves: 79.1 by a cluster, 74 onto a cleared
