@@ -63,7 +63,7 @@ PB200_API int pb200_quantize_act(int wtype, const float * x, int64_t k, void * a
  * plugin and pb200_model_set_tensor pad for you. */
 PB200_API int pb200_mul_mat_vec_q(int type, const void * W, int64_t n, int64_t k, const void * act_ws, float * y,
                                   const float * bias, const float * resid, void * stream);
-/* convenience: quantize + mul_mat_vec in one call (what ggml_cuda_mul_mat does for ne11 == 1) */
+/* convenience: quantize + mul_mat_vec in one call (what ggml_cuda_mul_mat does for ne11 == 1).  y may lie over x. */
 PB200_API int pb200_mul_mat_vec(int type, const void * W, int64_t n, int64_t k, const float * x, float * y, void * act_ws, void * stream);
 /* up to 3 matrices sharing one activation, one fused launch (q|k|v, gate|up) */
 PB200_API int pb200_mul_mat_vec_fused(int nmat, const int * types, const void * const * W, const int64_t * n, int64_t k,

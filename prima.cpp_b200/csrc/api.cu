@@ -26,6 +26,7 @@ ActQ act_from_ws(void * ws, int64_t k) {
     return a;
 }
 bool type_ok(int t) { return t == T_Q4_K || t == T_Q5_K || t == T_Q6_K || t == T_Q8_0 || t == T_Q5_1; }
+bool overlap(const float * a, int64_t na, const float * b, int64_t nb) { return (uintptr_t) a < (uintptr_t) (b + nb) && (uintptr_t) b < (uintptr_t) (a + na); }
 }  // namespace
 
 extern "C" {
@@ -75,7 +76,8 @@ int pb200_mul_mat_vec_q(int type, const void * W, int64_t n, int64_t k, const vo
 
 int pb200_mul_mat_vec(int type, const void * W, int64_t n, int64_t k, const float * x, float * y, void * act_ws, void * stream) {
     if (!type_ok(type) || !W || !x || !act_ws || !y || n <= 0 || k <= 0 || k % block_elems(type) != 0) return PB200_EINVAL;
-    if (gemv_quant_prologue_ok(type, W, (int) n, (int) k, x)) {
+    // one launch reads x in every CTA while others may already store rows of y: a y that lies over x takes the two launches, the first of which ends with x
+    if (!overlap(x, k, y, n) && gemv_quant_prologue_ok(type, W, (int) n, (int) k, x)) {
         const GemvDesc d = {W, y, nullptr, nullptr, type, (int) n};
         GemvFused pro;
         pro.kind = GEMV_PRO_QUANT;

@@ -27,3 +27,19 @@ def test_one_launch_equals_two(cuda, lib, t, N, K, launches):
     sync()
     assert torch.equal(y, want)
     assert torch.equal(ws, ws2)
+
+
+# y over x: in place, over x's end, over its start; the last ones only touch and take one launch
+@pytest.mark.parametrize("N,at,launches", [(4096, 0, 2), (300, 0, 2), (4096, 4092, 2), (4096, -4092, 2), (5000, -600, 2), (4096, 4096, 1), (4096, -4096, 1)])
+def test_result_over_the_activation(cuda, lib, N, at, launches):
+    K, x0 = 4096, 8192
+    buf = torch.zeros(5 * 4096, device="cuda")
+    buf[x0:x0 + K] = torch.from_numpy(np.random.default_rng(N).standard_normal(K).astype(np.float32))
+    x, y = buf[x0:x0 + K], buf[x0 + at:x0 + at + N]
+    Wd, apart, ws = dev_u8(O.synth_blocks(O.Q4_K, N, K, seed=N)), torch.empty(N, device="cuda"), act_ws(lib, K)
+    lib.check(lib.c.pb200_mul_mat_vec(O.Q4_K, ptr(Wd), N, K, ptr(x), ptr(apart), ptr(ws), None), "mul_mat_vec")
+    before = lib.c.pb200_kernel_launches()
+    lib.check(lib.c.pb200_mul_mat_vec(O.Q4_K, ptr(Wd), N, K, ptr(x), ptr(y), ptr(ws), None), "mul_mat_vec")
+    assert lib.c.pb200_kernel_launches() - before == launches
+    sync()
+    assert torch.equal(y, apart)
