@@ -327,9 +327,13 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
     const size_t nl_ = m->layers.size();
     float * x = m->x_in;
     if (m->with_embd) {
-        CK(launch_get_rows(m->tok_embd.data, m->tok_embd.type, E, tok_dev, 1, m->x_a, st, pdl)); n++; CK(dbg_sync(st, "get_rows"));
+        CK(launch_get_rows(m->tok_embd.data, m->tok_embd.type, E, tok_dev, 1, m->x_a, st, false)); n++; CK(dbg_sync(st, "get_rows"));
         x = m->x_a;
     }
+    // The first kernel of a step waits for all work in front of it: the attention kernels read the position and the cells of earlier tokens ahead of their
+    // own wait, and nothing else orders that behind the kernels of the step before (pb200_step_seq_dev without graphs)
+    bool first = !m->with_embd;
+    auto dep = [&] { const bool d = pdl && !first; first = false; return d; };
     const float kq_scale = 1.0f / sqrtf((float) D);
     // three rotating hidden-state buffers so that a residual source is never overwritten by its consumer
     float * bufs[3] = {m->x_a, m->x_b, m->xn};
@@ -351,14 +355,14 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
             if (dist) {   // rms_norm * attn_norm -> q8_K inside the GEMV: CTA c produces super-block c, one grid barrier
                 pro.kind = 4; pro.in0 = x; pro.in1 = L.attn_norm; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
             } else {      // ... or once by a single-CTA kernel in front of it
-                CK(launch_rmsnorm_quant(x, L.attn_norm, E, hp.rms_eps, ACT_Q8_K, m->actE.q, nullptr, st, pdl)); n++;
+                CK(launch_rmsnorm_quant(x, L.attn_norm, E, hp.rms_eps, ACT_Q8_K, m->actE.q, nullptr, st, dep())); n++;
             }
             CK(prof_begin(m, tbytes(L.wq) + tbytes(L.wk) + tbytes(L.wv)));
-            CK(launch_gemv_kquant_fused(d, 3, E, m->actE.q, pro, st, pdl)); n++; CK(dbg_sync(st, "gemv qkv"));
+            CK(launch_gemv_kquant_fused(d, 3, E, m->actE.q, pro, st, dep())); n++; CK(dbg_sync(st, "gemv qkv"));
             CK(prof_end(m));
         } else {
             ActQ none{};
-            CK(launch_rmsnorm_quant(x, L.attn_norm, E, hp.rms_eps, ACT_Q8_K, none, m->g, st, pdl)); n++;   // f32 normalized -> g (scratch)
+            CK(launch_rmsnorm_quant(x, L.attn_norm, E, hp.rms_eps, ACT_Q8_K, none, m->g, st, dep())); n++;   // f32 normalized -> g (scratch)
             Tensor * ws[3] = {&L.wq, &L.wk, &L.wv};
             float * ys[3] = {m->q, m->k, m->v};
             const float * bs[3] = {L.bq, L.bk, L.bv};
@@ -783,7 +787,7 @@ __global__ void __launch_bounds__(1024) k_argmax(const float * __restrict__ x, i
         if (lane == 0) { *out = bi; if (out2) *out2 = bi; }
     }
 }
-__global__ void k_advance_pos(int32_t * tp) { pdl_trigger(); pdl_wait(); tp[1] += 1; }
+__global__ void k_advance_pos(int32_t * tp) { tp[1] += 1; }
 
 int pb200_decode_async(pb200_model * m, int32_t token, int32_t pos) {
     NOT_FOR_LAYER_LIST(m);
