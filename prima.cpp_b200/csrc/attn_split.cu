@@ -266,12 +266,11 @@ __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int
 // bytes of them go through local memory once a tile.
 template <typename OT, bool CAP>
 __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_constant__ SplitParams P) {
-    pdl_enter();
     extern __shared__ uint8_t smem_raw[];
     const AttnIO & io = P.io;
     const AttnParams & a = P.a;
     const int e = blockIdx.z, kvh = P.kv_first + blockIdx.x;
-    const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;
+    const int t_begin = P.off[e], n = P.off[e + 1] - t_begin;                     // of the batch's description, copied in front of the pass
     const int q0 = ((int) gridDim.y - 1 - (int) blockIdx.y) * P.tok_per_cta;      // long rows first
     if (q0 >= n) return;
     const int toks = min(P.tok_per_cta, n - q0), rows = toks * P.gqa;
@@ -301,7 +300,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    } else if (warp >= 2) {
+        pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
+    }
+    pdl_wait();          // queries and the split images are the kernels' in front
+    if (warp >= 2) {
         const int w = warp - 2, D = a.dim;
         for (int r0 = w * 16; r0 < w * 16 + 16; r0 += 4) {
             float x[4][SP_MAX_ND][2];
