@@ -34,7 +34,7 @@ __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float
 constexpr int TM = 64, TN = 64, TK = 16;
 
 template <typename WT>
-__global__ void __launch_bounds__(256) k_dense_tile(const WT * __restrict__ A, int64_t lda, const WT * __restrict__ W, int64_t ldw, float * C, int64_t ldc,
+__global__ void __launch_bounds__(256) k_dense_tile(const WT * A, int64_t lda, const WT * __restrict__ W, int64_t ldw, float * C, int64_t ldc,
                                                     int T, int N, int K, const float * __restrict__ bias, const float * resid, int64_t ldr, float alpha,
                                                     DenseAct act) {
     pdl_enter();
@@ -120,7 +120,7 @@ template <int N> __device__ __forceinline__ void unpack(const uint4 & raw, float
 // through shared memory): matrices with few, long rows keep more loads in flight that way.  KS comes from (N, K) alone.
 // GLU (DenseAct::silu_glu): n counts pairs of rows, a warp streams both rows of its pair.
 template <typename WT, int TB, bool VEC, bool GLU>
-__global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, int64_t lda, const WT * __restrict__ W, int64_t ldw, float * C, int64_t ldc,
+__global__ void __launch_bounds__(256) k_dense_rows(const WT * A, int64_t lda, const WT * __restrict__ W, int64_t ldw, float * C, int64_t ldc,
                                                     int T, int N, int K, const float * __restrict__ bias, const float * resid, int64_t ldr, float alpha,
                                                     int KS, int plane_rows, int64_t a_plane, DenseAct act) {
     constexpr int R = GLU ? 2 : 1;
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) k_dense_rows(const WT * __restrict__ A, i
                 for (int t = 0; t < TB; t++) {
                     if (t < T) {
                         float af[V];
-                        unpack<V>(__ldg(reinterpret_cast<const uint4 *>(A + (int64_t) t * lda + k)), af, WT());
+                        unpack<V>(*reinterpret_cast<const uint4 *>(A + (int64_t) t * lda + k), af, WT());
 #pragma unroll
                         for (int r = 0; r < R; r++)
 #pragma unroll

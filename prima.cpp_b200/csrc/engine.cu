@@ -756,7 +756,7 @@ static int step(pb200_model * m, int seq = 0) {
 }
 
 // greedy sampling on the device (ggml_cuda_argmax, ggml-cuda/argmax.cu:7; first index of the maximum like ggml_compute_forward_argmax)
-__global__ void __launch_bounds__(1024) k_argmax(const float * __restrict__ x, int n, int32_t * __restrict__ out, int32_t * __restrict__ out2) {
+__global__ void __launch_bounds__(1024) k_argmax(const float * x, int n, int32_t * __restrict__ out, int32_t * __restrict__ out2) {
     __shared__ float sv[32];
     __shared__ int si[32];
     pdl_trigger();

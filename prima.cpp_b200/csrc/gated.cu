@@ -46,7 +46,7 @@ __global__ void k_embed_bigram(const WT * __restrict__ table, const WT * __restr
 
 // ---------------------------------------------------------------------------------------------------------------
 // grid (tokens, channel tiles): a thread owns one channel of one token
-__global__ void k_causal_conv(const float * __restrict__ u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+__global__ void k_causal_conv(const float * u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                               const int32_t * __restrict__ entry_of, int channels, int taps, const float * __restrict__ w, int silu_from,
                               float * __restrict__ conv_state, int64_t slot_stride, float * __restrict__ out, int64_t ldo, int advance) {
     pdl_enter();
@@ -68,7 +68,7 @@ __global__ void k_causal_conv(const float * __restrict__ u, int64_t ldu, const i
         }
     }
 }
-__global__ void k_causal_conv_state(const float * __restrict__ u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, int channels,
+__global__ void k_causal_conv_state(const float * u, int64_t ldu, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, int channels,
                                     int taps, float * __restrict__ conv_state, int64_t slot_stride) {
     pdl_enter();
     const int e = blockIdx.y;
@@ -254,9 +254,9 @@ __global__ void __launch_bounds__(1024) k_dual_prep_store(RecPrep rc, float * __
 
 // grid (tokens, heads): one thread per pair of the head's result
 template <typename OT>
-__global__ void k_attn_unrotate_gate(const float * __restrict__ o, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
+__global__ void k_attn_unrotate_gate(const float * o, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
                                      const int32_t * __restrict__ entry_of, int heads, int vdim, int v_layout, const float * __restrict__ v_freq,
-                                     const float * __restrict__ gate, int64_t ldg, int gate_mode, float out_scale, OT * __restrict__ out, int64_t ldo) {
+                                     const float * gate, int64_t ldg, int gate_mode, float out_scale, OT * __restrict__ out, int64_t ldo) {
     pdl_enter();
     const int t = blockIdx.x, h = blockIdx.y;
     const int e = entry_of[t];
@@ -304,10 +304,10 @@ __global__ void k_hgrn2_prep(float * __restrict__ q, int64_t ldq, float * __rest
 // kind turns an attention head back and gates it; one of the second kind divides a recurrence head by its root mean square, applies the
 // weight and the gate ----
 template <typename OT>
-__global__ void __launch_bounds__(128) k_dual_post(const float * __restrict__ o, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
+__global__ void __launch_bounds__(128) k_dual_post(const float * o, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
                                                    const int32_t * __restrict__ entry_of, int heads, int vdim, int v_layout, const float * __restrict__ v_freq,
-                                                   const float * __restrict__ gate, int64_t ldg, int gate_mode, float left_scale, const float * __restrict__ y,
-                                                   int r_heads, int r_vdim, const float * __restrict__ r_gate, int64_t ldrg, const float * __restrict__ r_w,
+                                                   const float * gate, int64_t ldg, int gate_mode, float left_scale, const float * y,
+                                                   int r_heads, int r_vdim, const float * r_gate, int64_t ldrg, const float * __restrict__ r_w,
                                                    int r_gate_act, float eps, float right_scale, OT * __restrict__ out, int64_t ldo) {
     pdl_enter();
     __shared__ float red[33];
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(256) k_gated_linattn_smem(GatedLinIO io, const
 // ---------------------------------------------------------------------------------------------------------------
 // one CTA per token: both rows are normed, joined onto the stream, and the new stream row is normed for the next sublayer
 template <typename OT>
-__global__ void __launch_bounds__(256) k_rmsnorm_pair_residual(const float * __restrict__ a, int64_t lda, const float * __restrict__ bb, int64_t ldb,
+__global__ void __launch_bounds__(256) k_rmsnorm_pair_residual(const float * a, int64_t lda, const float * bb, int64_t ldb,
                                                                const float * __restrict__ wa, const float * __restrict__ wb, float mult, float eps,
                                                                float * __restrict__ x, const float * __restrict__ wn, OT * __restrict__ y, int width) {
     pdl_enter();
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_pair_residual(const float * __r
 }
 
 template <typename OT>
-__global__ void __launch_bounds__(256) k_stream_add_rmsnorm(float * __restrict__ x, const float * __restrict__ x0, const float * __restrict__ vec,
+__global__ void __launch_bounds__(256) k_stream_add_rmsnorm(float * __restrict__ x, const float * x0, const float * __restrict__ vec,
                                                             const float * __restrict__ w, float eps, OT * __restrict__ y, int width) {
     pdl_enter();
     __shared__ float red[33];

@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(1024) k_head_prep(const __grid_constant__ Head
 
 // One CTA per token: a warp gates an attention head, or divides a recurrence head by its root mean square and applies its weight and gate
 template <typename OT>
-__global__ void __launch_bounds__(1024) k_join_heads(const float * __restrict__ o, int heads, int vdim, const float * __restrict__ gate, int64_t ldg, int gate_mode, float left_scale,
-                                                    const float * __restrict__ y, int r_heads, int r_vdim, const float * __restrict__ r_gate, int64_t ldrg,
+__global__ void __launch_bounds__(1024) k_join_heads(const float * o, int heads, int vdim, const float * gate, int64_t ldg, int gate_mode, float left_scale,
+                                                    const float * y, int r_heads, int r_vdim, const float * r_gate, int64_t ldrg,
                                                     const float * __restrict__ r_w, int r_gate_act, float eps, float right_scale, OT * __restrict__ out, int64_t ldo) {
     pdl_enter();
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, i = 4 * lane;

@@ -32,7 +32,7 @@ __device__ __forceinline__ void turn(float u, float v, int pos, float f, float m
 }
 
 // factor on output element (head h, entry dv): sigmoid of the head's gate logit, of the element's, or none
-__device__ __forceinline__ float latent_gate(const LatentParams & p, const float * __restrict__ gate, int64_t at, int h, int dv) {
+__device__ __forceinline__ float latent_gate(const LatentParams & p, const float * gate, int64_t at, int h, int dv) {
     return gate ? sigmoid_f(gate[at + (p.gate_mode == 1 ? h : h * p.vdim + dv)]) : 1.f;
 }
 // turns the rotated part of every query head of one token
@@ -182,7 +182,7 @@ __global__ void k_latent_gather(const float * __restrict__ cache, int64_t slot_s
 // CTA (head, token, 128 latent entries): qa[r] = sum_d W_uk[h * dim + d][r] q[d]; four groups of 128 threads walk a quarter of the head's rows
 // each (coalesced over r, eight loads in flight); the quarters are summed in order
 template <typename WT>
-__global__ void __launch_bounds__(512) k_latent_absorb_q(const float * __restrict__ q, int64_t ldq, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
+__global__ void __launch_bounds__(512) k_latent_absorb_q(const float * q, int64_t ldq, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0,
                                                          const int32_t * __restrict__ entry_of, const WT * __restrict__ wuk, LatentParams p,
                                                          const float * __restrict__ freq, float * __restrict__ qa) {
     pdl_enter();
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(512) k_latent_absorb_q(const float * __restric
 
 // one CTA per (head, token): a warp per output row of the head's block of W_uv, lanes split the latent
 template <typename WT, typename OT>
-__global__ void __launch_bounds__(256) k_latent_up_v(const float * __restrict__ olat, const WT * __restrict__ wuv, LatentParams p,
-                                                     const float * __restrict__ gate, int64_t ldg, OT * __restrict__ out) {
+__global__ void __launch_bounds__(256) k_latent_up_v(const float * olat, const WT * __restrict__ wuv, LatentParams p,
+                                                     const float * gate, int64_t ldg, OT * __restrict__ out) {
     pdl_enter();
     extern __shared__ float os[];   // [kv_rank]
     const int h = blockIdx.x, t = blockIdx.y;
@@ -263,8 +263,8 @@ __host__ __device__ inline int latent_row_stride(const LatentParams & p) {
 }
 __device__ __forceinline__ int latent_rows_per_split(int rows_used, int splits) { return ((rows_used + splits - 1) / splits + LT_ROWS - 1) / LT_ROWS * LT_ROWS; }
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_latent_decode_split(const float * __restrict__ qa, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
-                                                             const int32_t * __restrict__ pos0, LatentParams p, const float * __restrict__ cache,
+__global__ void __launch_bounds__(256) k_latent_decode_split(const float * qa, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+                                                             const int32_t * __restrict__ pos0, LatentParams p, const float * cache,
                                                              int64_t slot_stride, int splits, float * __restrict__ part) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
@@ -400,9 +400,9 @@ __global__ void __launch_bounds__(256) k_latent_decode_split(const float * __res
 // a warp per output row of the head's block of W_uv (lanes split the latent) and the output gate.  Up to 64 splits: a lane of warp 0
 // weighs splits lane and lane + 32.
 template <typename WT, typename OT>
-__global__ void __launch_bounds__(256) k_latent_merge_up_v(const float * __restrict__ part, int all_splits, const int32_t * __restrict__ off,
+__global__ void __launch_bounds__(256) k_latent_merge_up_v(const float * part, int all_splits, const int32_t * __restrict__ off,
                                                            const int32_t * __restrict__ pos0, const WT * __restrict__ wuv,
-                                                           LatentParams p, const float * __restrict__ sink, const float * __restrict__ gate, int64_t ldg,
+                                                           LatentParams p, const float * __restrict__ sink, const float * gate, int64_t ldg,
                                                            OT * __restrict__ out) {
     pdl_enter();
     extern __shared__ float os[];   // [kv_rank], then [64] weights of the splits

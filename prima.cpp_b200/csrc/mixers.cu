@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(1024) k_embed_rmsnorm(const WT * __restrict__ 
 }
 
 template <typename OT>
-__global__ void k_cast(const float * __restrict__ x, OT * __restrict__ y, int64_t n) {
+__global__ void k_cast(const float * x, OT * __restrict__ y, int64_t n) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) put(y, i, x[i]);
@@ -65,7 +65,7 @@ __global__ void k_cast(const float * __restrict__ x, OT * __restrict__ y, int64_
 
 // layer norm with a weight and an optional bias; two passes over the row (mean, then the mean of squared deviations)
 template <typename OT, bool RESID>
-__global__ void __launch_bounds__(256) k_layernorm(const float * __restrict__ x, const int32_t * __restrict__ rows, const float * __restrict__ w,
+__global__ void __launch_bounds__(256) k_layernorm(const float * x, const int32_t * rows, const float * __restrict__ w,
                                                    const float * __restrict__ bias, float eps, OT * __restrict__ y, float * __restrict__ xres, int width) {
     pdl_enter();
     __shared__ float red[33];
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256) k_layernorm(const float * __restrict__ x,
 // x[t] += layernorm(m[t]) * wa, then y[t] = layernorm(x[t]) * wb: the post-norm + residual of one sublayer and the pre-norm of the next in
 // one pass over the token (every thread re-reads only the elements of x it has written itself)
 template <typename OT>
-__global__ void __launch_bounds__(256) k_layernorm_residual_next(const float * __restrict__ m, const float * __restrict__ wa, const float * __restrict__ wb,
+__global__ void __launch_bounds__(256) k_layernorm_residual_next(const float * m, const float * __restrict__ wa, const float * __restrict__ wb,
                                                                  float eps, float * __restrict__ x, OT * __restrict__ y, int width) {
     pdl_enter();
     __shared__ float red[33];
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) k_layernorm_residual_next(const float * _
 // x[t] += mult * (layernorm(m[t]) * w + bias); xa[t] = x[t] in the operand type.  The row of m is kept in registers (width <= 256 * LNR)
 // or re-read; x is read and written once.
 template <typename OT>
-__global__ void __launch_bounds__(256) k_layernorm_affine_residual(const float * __restrict__ m, const float * __restrict__ w, const float * __restrict__ bias,
+__global__ void __launch_bounds__(256) k_layernorm_affine_residual(const float * m, const float * __restrict__ w, const float * __restrict__ bias,
                                                                    float mult, float eps, float * __restrict__ x, OT * __restrict__ xa, int width) {
     pdl_enter();
     __shared__ float red[33];
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) k_layernorm_affine_residual(const float *
 }
 
 template <typename OT>
-__global__ void k_relu2(const float * __restrict__ u, OT * __restrict__ y, int64_t n) {
+__global__ void k_relu2(const float * u, OT * __restrict__ y, int64_t n) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -146,7 +146,7 @@ __global__ void k_relu2(const float * __restrict__ u, OT * __restrict__ y, int64
     put(y, i, v * v);
 }
 template <typename OT>   // four elements a thread
-__global__ void k_relu2_4(const float * __restrict__ u, OT * __restrict__ y, int64_t n) {
+__global__ void k_relu2_4(const float * u, OT * __restrict__ y, int64_t n) {
     pdl_enter();
     const int64_t i = 4 * ((int64_t) blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
@@ -155,7 +155,7 @@ __global__ void k_relu2_4(const float * __restrict__ u, OT * __restrict__ y, int
     put4(y, i, make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w));
 }
 template <typename OT>
-__global__ void k_xielu(const float * __restrict__ u, const float * __restrict__ pq, OT * __restrict__ y, int64_t n) {
+__global__ void k_xielu(const float * u, const float * __restrict__ pq, OT * __restrict__ y, int64_t n) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -193,7 +193,7 @@ __global__ void k_embed_pos(const WT * __restrict__ table, const WT * __restrict
 }
 
 template <typename OT>
-__global__ void k_gelu_mul(const float * __restrict__ gu, OT * __restrict__ y, int n_tokens, int ff) {
+__global__ void k_gelu_mul(const float * gu, OT * __restrict__ y, int n_tokens, int ff) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t) n_tokens * ff) return;
@@ -268,7 +268,7 @@ __device__ __forceinline__ float attn_gate(const AttnIO & io, int64_t row, int h
     return 1.f;
 }
 
-__global__ void k_attn_kv_store(const float * __restrict__ qkvg, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+__global__ void k_attn_kv_store(const float * qkvg, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                 const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, AttnParams a, float * __restrict__ kcache,
                                 float * __restrict__ vcache, int64_t slot_stride) {
     pdl_enter();
@@ -580,7 +580,7 @@ __device__ __forceinline__ int dec_rows_used(const AttnParams & a, int pi) { ret
 template <typename OT, int NV, bool TIED>
 __global__ void __launch_bounds__(DEC_WARPS * 32) k_attn_window_decode(const AttnIO io, const int32_t * __restrict__ slot,
                                                                        const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, AttnParams a,
-                                                                       const float * __restrict__ kcache, const float * __restrict__ vcache,
+                                                                       const float * kcache, const float * vcache,
                                                                        int64_t slot_stride, OT * __restrict__ out, float * __restrict__ part, int chunk) {
     pdl_enter();
     extern __shared__ float sm[];
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) k_attn_window_decode(const Att
 // most), then one thread per value dimension sums the splits that hold rows, eight loads in flight.
 template <typename OT>
 __global__ void __launch_bounds__(128) k_attn_decode_merge(const AttnIO io, const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, AttnParams a,
-                                                           const float * __restrict__ part, int all_splits, int chunk, OT * __restrict__ out) {
+                                                           const float * part, int all_splits, int chunk, OT * __restrict__ out) {
     pdl_enter();
     __shared__ float w[64];
     const int e = blockIdx.y, h = blockIdx.x, DV = a.vdim;
@@ -754,9 +754,9 @@ __global__ void __launch_bounds__(128) k_attn_decode_merge(const AttnIO io, cons
 
 // ---------------------------------------------------------------------------------------------------------------
 // Mamba-2
-__global__ void k_mamba2_conv(const float * __restrict__ u, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+__global__ void k_mamba2_conv(const float * u, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                               const int32_t * __restrict__ entry_of, Mamba2Params p, const float * __restrict__ w, const float * __restrict__ bias,
-                              const float * __restrict__ conv_state, int64_t slot_stride, float * __restrict__ xbc) {
+                              const float * conv_state, int64_t slot_stride, float * __restrict__ xbc) {
     pdl_enter();
     const int t = blockIdx.x;
     const int e = entry_of[t];
@@ -788,7 +788,7 @@ __global__ void k_mamba2_conv_state(const float * __restrict__ u, const int32_t 
 }
 
 // one CTA per (head, entry); the state S [N][P] lives in shared memory for the whole entry, tokens are walked in order
-__global__ void __launch_bounds__(256) k_mamba2_scan(const float * __restrict__ u, const float * __restrict__ xbc, const int32_t * __restrict__ slot,
+__global__ void __launch_bounds__(256) k_mamba2_scan(const float * u, const float * xbc, const int32_t * __restrict__ slot,
                                                      const int32_t * __restrict__ off, Mamba2Params p, const float * __restrict__ dt_bias,
                                                      const float * __restrict__ A_log, const float * __restrict__ Dp, float * __restrict__ ssm_state,
                                                      int64_t slot_stride, float * __restrict__ y) {
@@ -839,7 +839,7 @@ __global__ void __launch_bounds__(256) k_mamba2_scan(const float * __restrict__ 
 // shuffle reduction per token.  Used for state sizes up to 128; larger states take k_mamba2_scan.
 constexpr int SCAN_CHUNK = 16, SCAN_COLS = 32;
 template <int NREG>
-__global__ void __launch_bounds__(128) k_mamba2_scan_reg(const float * __restrict__ u, const float * __restrict__ xbc, const int32_t * __restrict__ slot,
+__global__ void __launch_bounds__(128) k_mamba2_scan_reg(const float * u, const float * xbc, const int32_t * __restrict__ slot,
                                                          const int32_t * __restrict__ off, Mamba2Params p, const float * __restrict__ dt_bias,
                                                          const float * __restrict__ A_log, const float * __restrict__ Dp, float * __restrict__ ssm_state,
                                                          int64_t slot_stride, float * __restrict__ y) {
@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(128) k_mamba2_scan_reg(const float * __restric
 }
 
 template <typename OT>
-__global__ void __launch_bounds__(256) k_mamba2_gate_norm(const float * __restrict__ y, const float * __restrict__ u, Mamba2Params p, const float * __restrict__ w,
+__global__ void __launch_bounds__(256) k_mamba2_gate_norm(const float * y, const float * u, Mamba2Params p, const float * __restrict__ w,
                                                           float eps, OT * __restrict__ out) {
     pdl_enter();
     __shared__ float red[33];

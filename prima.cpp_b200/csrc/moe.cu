@@ -33,7 +33,7 @@ __device__ __forceinline__ void unpack16(const uint4 & r, float (&f)[8], __nv_bf
 }
 // lane's share of sum_k w[k] a[k]; VEC: 16-byte loads (K a multiple of the pack, both rows 16-byte aligned)
 template <typename WT, bool VEC>
-__device__ __forceinline__ float dot_part(const WT * __restrict__ w, const WT * __restrict__ a, int K, int lane) {
+__device__ __forceinline__ float dot_part(const WT * __restrict__ w, const WT * a, int K, int lane) {
     float acc = 0.f;
     if constexpr (VEC) {
         constexpr int V = Pack<WT>::n;
@@ -52,7 +52,7 @@ __device__ __forceinline__ float dot_part(const WT * __restrict__ w, const WT * 
 
 // one CTA per token: the activations in shared memory as fp32, warps split the experts, warp 0 picks
 template <typename HT>
-__global__ void __launch_bounds__(256) k_moe_route(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ bias, MoeParams p,
+__global__ void __launch_bounds__(256) k_moe_route(const HT * h, const float * __restrict__ wr, const float * __restrict__ bias, MoeParams p,
                                                    int width, int32_t * __restrict__ idx, float * __restrict__ wt) {
     pdl_enter();
     extern __shared__ float sm[];
@@ -152,7 +152,7 @@ __device__ __forceinline__ void pick_experts(const MoeParams & p, const float * 
 
 // one CTA per token: sigmoid scores, choice with the correction among the experts of the best groups, weights from the plain scores
 template <typename HT>
-__global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p,
+__global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p,
                                                            int width, const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt,
                                                            float * __restrict__ sg_out) {
     pdl_enter();
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(1024) k_moe_route_sigmoid(const HT * __restric
 // experts
 constexpr int ROUTE_TOKENS = 8;
 template <typename HT>
-__global__ void __launch_bounds__(1024) k_moe_route_sigmoid_many(const HT * __restrict__ h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p, int width,
+__global__ void __launch_bounds__(1024) k_moe_route_sigmoid_many(const HT * h, const float * __restrict__ wr, const float * __restrict__ corr, MoeParams p, int width,
                                                                 const float * __restrict__ sgw, int32_t * __restrict__ idx, float * __restrict__ wt, float * __restrict__ sg_out,
                                                                 int n_tokens) {
     pdl_enter();
@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(1024) k_moe_route_sigmoid_many(const HT * __re
 
 // grid (ceil(ff / 8), pairs): warp -> row j of gate and of up of the pair's expert
 template <typename WT, bool VEC>
-__global__ void __launch_bounds__(256) k_moe_gateup_rows(const WT * __restrict__ h, const WT * __restrict__ gateup, const int32_t * __restrict__ idx, MoeParams p,
-                                                         int width, WT * __restrict__ y, const float * __restrict__ in_wt) {
+__global__ void __launch_bounds__(256) k_moe_gateup_rows(const WT * h, const WT * __restrict__ gateup, const int32_t * idx, MoeParams p,
+                                                         int width, WT * __restrict__ y, const float * in_wt) {
     pdl_enter();
     const int pair = blockIdx.y, t = pair / p.top;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -269,9 +269,9 @@ __global__ void __launch_bounds__(256) k_moe_gateup_rows(const WT * __restrict__
 }
 // grid (ceil(width / 8), tokens): warp -> output n of the token, summed over its experts in the order of the choice
 template <typename WT, bool VEC>
-__global__ void __launch_bounds__(256) k_moe_down_rows(const WT * __restrict__ y, const WT * __restrict__ down, const int32_t * __restrict__ idx,
-                                                       const float * __restrict__ wt, MoeParams p, int width, float * __restrict__ x, int base,
-                                                       const float * __restrict__ xscale, float out_scale) {
+__global__ void __launch_bounds__(256) k_moe_down_rows(const WT * y, const WT * __restrict__ down, const int32_t * idx,
+                                                       const float * wt, MoeParams p, int width, float * __restrict__ x, int base,
+                                                       const float * xscale, float out_scale) {
     pdl_enter();
     const int t = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256) k_moe_down_rows(const WT * __restrict__ y
 }
 
 // ---- sort by expert ----
-__global__ void __launch_bounds__(256) k_moe_count(const int32_t * __restrict__ idx, int n_pairs, int32_t * __restrict__ count) {
+__global__ void __launch_bounds__(256) k_moe_count(const int32_t * idx, int n_pairs, int32_t * __restrict__ count) {
     pdl_enter();
     __shared__ float red[33];
     const int e = blockIdx.x;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) k_moe_count(const int32_t * __restrict__ 
     if (threadIdx.x == 0) count[e] = (int32_t) s;
 }
 // one CTA per expert: walks the pairs in order, 256 at a time, and places its own at start[e] + rank (stable)
-__global__ void __launch_bounds__(256) k_moe_place(const int32_t * __restrict__ idx, int n_pairs, const int32_t * __restrict__ count, int32_t * __restrict__ start,
+__global__ void __launch_bounds__(256) k_moe_place(const int32_t * idx, int n_pairs, const int32_t * count, int32_t * __restrict__ start,
                                                    int32_t * __restrict__ perm) {
     pdl_enter();
     __shared__ int wbase[9];
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) k_moe_place(const int32_t * __restrict__ 
     }
 }
 template <typename WT>
-__global__ void k_moe_gather(const WT * __restrict__ h, const int32_t * __restrict__ perm, int top, int width, WT * __restrict__ hs, int wide) {
+__global__ void k_moe_gather(const WT * h, const int32_t * perm, int top, int width, WT * __restrict__ hs, int wide) {
     pdl_enter();
     const int r = blockIdx.x;
     const WT * src = h + (int64_t) (perm[r] / top) * width;
@@ -340,13 +340,13 @@ __global__ void k_moe_gather(const WT * __restrict__ h, const int32_t * __restri
     }
     for (int i = threadIdx.x; i < width; i += blockDim.x) hs[(int64_t) r * width + i] = src[i];
 }
-__global__ void k_moe_invert(const int32_t * __restrict__ perm, int32_t * __restrict__ row_of, int n_pairs) {
+__global__ void k_moe_invert(const int32_t * perm, int32_t * __restrict__ row_of, int n_pairs) {
     pdl_enter();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < n_pairs) row_of[perm[r]] = r;
 }
-__global__ void k_moe_combine(const float * __restrict__ ds, const int32_t * __restrict__ row_of, const float * __restrict__ wt, int top, int width,
-                              float * __restrict__ x, int base, const float * __restrict__ xscale, float out_scale, int wide) {
+__global__ void k_moe_combine(const float * ds, const int32_t * row_of, const float * wt, int top, int width,
+                              float * __restrict__ x, int base, const float * xscale, float out_scale, int wide) {
     pdl_enter();
     const int t = blockIdx.x;
     if (wide) {
@@ -377,7 +377,7 @@ __global__ void k_moe_combine(const float * __restrict__ ds, const int32_t * __r
 }
 
 template <typename OT>
-__global__ void k_silu_mul(const float * __restrict__ gu, OT * __restrict__ y, int n_rows, int ff, const float * __restrict__ in_wt, const int32_t * __restrict__ perm,
+__global__ void k_silu_mul(const float * gu, OT * __restrict__ y, int n_rows, int ff, const float * in_wt, const int32_t * perm,
                            int interleaved) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;

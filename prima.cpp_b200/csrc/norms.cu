@@ -18,7 +18,7 @@ constexpr int MAX_NORM_GROUPS = 64;
 
 // 1 / sqrt(mean(part^2) + eps) of every group of a row -> inv[0..groups) in shared memory; all threads of the CTA take part.
 // Several groups: a warp sums a whole group (no CTA-wide reduction, one barrier); one group: the CTA sums it together.
-__device__ __forceinline__ void group_inv_rms(const float * __restrict__ row, int width, int groups, float eps, float * inv, float * red) {
+__device__ __forceinline__ void group_inv_rms(const float * row, int width, int groups, float eps, float * inv, float * red) {
     const int part = width / groups;
     if (groups == 1) {
         float q = 0.f;
@@ -40,7 +40,7 @@ __device__ __forceinline__ void group_inv_rms(const float * __restrict__ row, in
 }
 
 template <typename OT>
-__global__ void __launch_bounds__(1024) k_group_rmsnorm(const float * __restrict__ x, const int32_t * __restrict__ rows, const float * __restrict__ w, int groups,
+__global__ void __launch_bounds__(1024) k_group_rmsnorm(const float * x, const int32_t * rows, const float * __restrict__ w, int groups,
                                                        float eps, OT * __restrict__ y, int width) {
     pdl_enter();
     __shared__ float red[33];
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(1024) k_group_rmsnorm(const float * __restrict
 
 // one CTA per token: the norm of the token and of the one before it (recomputed: a second read of a row that is in L2), then the blend
 template <typename OT>
-__global__ void __launch_bounds__(256) k_group_rmsnorm_shift(const float * __restrict__ x, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+__global__ void __launch_bounds__(256) k_group_rmsnorm_shift(const float * x, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                              const int32_t * __restrict__ entry_of, const float * __restrict__ w, int groups, float eps,
                                                              const float * __restrict__ mu, float * __restrict__ shift_state, int64_t slot_stride,
                                                              OT * __restrict__ y, int width) {
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(256) k_shift_state(const float * __restrict__ 
 
 // one CTA per token: the norm of the token and of the one before it, then one blend per plane (operand type) and one more in fp32
 template <typename OT>
-__global__ void __launch_bounds__(1024) k_rmsnorm_token_mix(const float * __restrict__ x, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
+__global__ void __launch_bounds__(1024) k_rmsnorm_token_mix(const float * x, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                                             const int32_t * __restrict__ entry_of, const float * __restrict__ w, float eps,
                                                             const float * __restrict__ mu, int n_planes, float * __restrict__ shift_state, int64_t slot_stride,
                                                             OT * __restrict__ y, int64_t plane, float * __restrict__ yf, int width) {
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(1024) k_rmsnorm_token_mix(const float * __rest
 }
 
 // sum_j coef[j] * planes[j * plane_stride + i], eight planes' loads in flight
-__device__ __forceinline__ float depth_sum(const float * __restrict__ planes, int64_t plane_stride, const float * __restrict__ coef, int n, int64_t i) {
+__device__ __forceinline__ float depth_sum(const float * planes, int64_t plane_stride, const float * __restrict__ coef, int n, int64_t i) {
     float acc = 0.f;
     int j = 0;
     for (; j + 7 < n; j += 8) {
@@ -131,7 +131,7 @@ __device__ __forceinline__ float depth_sum(const float * __restrict__ planes, in
     for (; j < n; j++) acc = fmaf(coef[j], planes[(int64_t) j * plane_stride + i], acc);
     return acc;
 }
-__global__ void k_depth_average(const float * __restrict__ planes, int64_t plane_stride, const float * __restrict__ coef, int n, float * __restrict__ out,
+__global__ void k_depth_average(const float * planes, int64_t plane_stride, const float * __restrict__ coef, int n, float * __restrict__ out,
                                 int64_t count) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,7 +141,7 @@ __global__ void k_depth_average(const float * __restrict__ planes, int64_t plane
 // batches of one-token entries: the depth average that closes a layer, and the next layer's norm and token shift with its state update, on
 // one row held in shared memory
 template <typename OT>
-__global__ void __launch_bounds__(256) k_depth_average_norm_shift(const float * __restrict__ planes, int64_t plane_stride, const float * __restrict__ coef, int n,
+__global__ void __launch_bounds__(256) k_depth_average_norm_shift(const float * planes, int64_t plane_stride, const float * __restrict__ coef, int n,
                                                                   float * __restrict__ x, const int32_t * __restrict__ slot, const float * __restrict__ w,
                                                                   int groups, float eps, const float * __restrict__ mu, float * __restrict__ shift_state,
                                                                   int64_t slot_stride, OT * __restrict__ y, int width) {
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) k_depth_average_norm_shift(const float * 
 }
 
 template <typename OT>
-__global__ void __launch_bounds__(256) k_norm_gate(const float * __restrict__ y, const float * __restrict__ gate, int64_t ldg, int part,
+__global__ void __launch_bounds__(256) k_norm_gate(const float * y, const float * gate, int64_t ldg, int part,
                                                    const float * __restrict__ w, int gate_act, float eps, OT * __restrict__ out, int inner, int64_t ldo,
                                                    float out_scale) {
     pdl_enter();
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_norm_gate(const float * __restrict__ y,
 }
 
 template <typename OT>
-__global__ void k_clamped_glu(const float * __restrict__ gu, OT * __restrict__ y, int n_tokens, int ff, float limit) {
+__global__ void k_clamped_glu(const float * gu, OT * __restrict__ y, int n_tokens, int ff, float limit) {
     pdl_enter();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t) n_tokens * ff) return;

@@ -28,7 +28,7 @@ static inline int launch_cfg(cudaLaunchConfig_t & cfg, cudaLaunchAttribute * att
 
 // ------------------------------------------------------------------------------------------------
 // activation quantization: one warp per 256 values
-__global__ void __launch_bounds__(256) k_quantize_act(const float * __restrict__ x, int K, int mode, ActQ out) {
+__global__ void __launch_bounds__(256) k_quantize_act(const float * x, int K, int mode, ActQ out) {
     pdl_trigger();   // dependents may launch now; they still wait for this grid's completion in their own pdl_wait()
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_quantize_act(const float * __restrict__
 
 __device__ __forceinline__ float silu_f32(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }   // ggml.c:2560
 
-__global__ void __launch_bounds__(256) k_silu_mul_quant(const float * __restrict__ g, const float * __restrict__ u, int K, int mode, ActQ out,
+__global__ void __launch_bounds__(256) k_silu_mul_quant(const float * g, const float * u, int K, int mode, ActQ out,
                                                         float * __restrict__ f32_out) {
     pdl_trigger();   // dependents may launch now; they still wait for this grid's completion in their own pdl_wait()
     pdl_wait();
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) k_silu_mul_quant(const float * __restrict
 
 // ------------------------------------------------------------------------------------------------
 // y = rms_norm(x) * w, then quantize; single CTA (n <= 32 K), double-precision sum of squares like ggml.c:11976-11984
-__global__ void __launch_bounds__(1024) k_rmsnorm_quant(const float * __restrict__ x, const float * __restrict__ w, int n, float eps, int mode,
+__global__ void __launch_bounds__(1024) k_rmsnorm_quant(const float * x, const float * __restrict__ w, int n, float eps, int mode,
                                                         ActQ out, float * __restrict__ f32_out) {
     __shared__ double red[32];
     __shared__ float s_scale;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(1024) k_rmsnorm_quant(const float * __restrict
 // of each of its 296 CTAs cost ~7 us per launch (profiles/r2_token_trace_v1_first_coresident_build.txt: 19 MB of redundant L2 reads).
 constexpr int RQ_WARPS = 16;   // RQ_B super-blocks per warp in registers: 2 (n <= 8192, ~64 registers: fits beside a resident GEMV CTA) or 4
 template <int RQ_B>
-__global__ void __launch_bounds__(RQ_WARPS * 32) k_rmsnorm_q8K(const float * __restrict__ x, const float * __restrict__ w, int n, float eps, ActQ out) {
+__global__ void __launch_bounds__(RQ_WARPS * 32) k_rmsnorm_q8K(const float * x, const float * __restrict__ w, int n, float eps, ActQ out) {
     __shared__ double red[RQ_WARPS];
     pdl_trigger();
     pdl_wait();
@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(256) k_rms_norm_rows(const float * __restrict_
 // like ggml_rope_cache_init's running product, so the angle is bit-identical to the CPU's.
 // grid = n_head + n_head_kv CTAs of D/2 threads: q heads rotate in place; k heads rotate into the f16 K cache and carry
 // the matching v head into the f16 V cache.
-__global__ void k_rope_kvstore(float * __restrict__ q, const float * __restrict__ k, const float * __restrict__ v, __half * __restrict__ kc,
-                               __half * __restrict__ vc, int n_head, int n_head_kv, int D, const int32_t * __restrict__ pos_dev, RopeParams rp,
+__global__ void k_rope_kvstore(float * __restrict__ q, const float * k, const float * v, __half * __restrict__ kc,
+                               __half * __restrict__ vc, int n_head, int n_head_kv, int D, const int32_t * pos_dev, RopeParams rp,
                                const float * __restrict__ freq_factors) {
     pdl_trigger();   // dependents may launch now; they still wait for this grid's completion in their own pdl_wait()
     pdl_wait();
@@ -314,8 +314,8 @@ __global__ void k_rope(const float * __restrict__ x, float * __restrict__ y, int
 //   s[p] = sum_d f32(K16[p][d]) * f32(f16(q[d]))            (CPU: mul_mat with f16 src0 rounds src1 to f16, ggml.c:12445)
 //   w    = softmax(s * scale)                               (ggml.c:13783; double sum, p = e * float(1/sum))
 //   o[d] = sum_p f32(V16[p][d]) * f32(f16(w[p]))            (second mul_mat, probabilities rounded to f16)
-__global__ void __launch_bounds__(256) k_attn_decode(const float * __restrict__ q, const __half * __restrict__ kc, const __half * __restrict__ vc,
-                                                     float * __restrict__ out, int n_head, int n_head_kv, int D, const int32_t * __restrict__ pos_dev,
+__global__ void __launch_bounds__(256) k_attn_decode(const float * q, const __half * kc, const __half * vc,
+                                                     float * __restrict__ out, int n_head, int n_head_kv, int D, const int32_t * pos_dev,
                                                      float scale, int64_t q_tok_stride, int64_t out_tok_stride) {
     extern __shared__ float sm[];   // S[n_kv_pad] | red[8][128]
     pdl_trigger();   // dependents may launch now; they still wait for this grid's completion in their own pdl_wait()
@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(256) k_attn_prefill_tiled(const float * __rest
 // engine's per-token loop (same arithmetic, one launch): the CTA rotates its q head and its kv head's k in shared memory,
 // rounds k / v to f16 exactly like the cache store does, attends over cache rows [0, pos) plus the fresh row from shared
 // memory, and the first q head of each GQA group writes the fresh K/V row to the cache for later tokens.
-__global__ void __launch_bounds__(256) k_attn_fused(const float * __restrict__ q, const float * __restrict__ k, const float * __restrict__ v,
+__global__ void __launch_bounds__(256) k_attn_fused(const float * q, const float * k, const float * v,
                                                     __half * __restrict__ kc, __half * __restrict__ vc, float * __restrict__ out, int n_head,
-                                                    int n_head_kv, const int32_t * __restrict__ pos_dev, RopeParams rp,
+                                                    int n_head_kv, const int32_t * pos_dev, RopeParams rp,
                                                     const float * __restrict__ freq_factors, float scale) {
     constexpr int D = 128;
     extern __shared__ float sm[];   // S[n_kv_pad] | red[8][128]
@@ -1123,7 +1123,7 @@ __device__ float dequant_elem(int type, const uint8_t * row, int e) {
 }
 
 __global__ void __launch_bounds__(256) k_get_rows(const uint8_t * __restrict__ table, int type, int K, int64_t row_bytes_,
-                                                  const int32_t * __restrict__ ids, float * __restrict__ y) {
+                                                  const int32_t * ids, float * __restrict__ y) {
     pdl_trigger();   // dependents may launch now; they still wait for this grid's completion in their own pdl_wait()
     pdl_wait();
     const int64_t id = ids[blockIdx.y];

@@ -11,6 +11,8 @@ namespace pb {
 // what it does in front of the wait (weights never depend on the kernel before) lie beside the other's work.  Each such kernel waits in all of
 // its threads before it touches anything another kernel writes, so the end of a kernel means the end of all before it; kernels launched the
 // plain way (the first of a pass, behind a copy; behind an event of another stream) keep their full dependency.
+// What such a kernel reads of an earlier kernel's results it takes by pointers without __restrict__ and by ordinary loads: data that is constant to the
+// compiler may be loaded ahead of the wait, wherever the load stands.  Weights and the batch's description (copied in front of the pass) may be.
 extern thread_local bool g_pdl;
 struct PdlScope {
     bool was;

@@ -1,8 +1,7 @@
 // prima.cpp_b200/csrc/rows.cuh — rows of floats in the registers of a few warps: loads, stores and sums for the row-wise steps of the layer-list engine.
 // A row of width floats (a multiple of four, 16-byte aligned) is held by `wpr` warps, a thread having the float4s tl, tl + 32 wpr, ... (V at most),
 // so that a row is read once, all its loads are in flight together, and a sum costs one barrier (none for a row of one warp).
-// Kernels that load weights in front of pdl_wait take what the kernel in front writes by pointers without __restrict__: a load that may be taken for a constant's
-// may be moved in front of the wait.
+// What the kernel in front writes comes by pointers without __restrict__ (pdl.h).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -44,7 +44,7 @@ template <int ROWS>
 struct LowrankFetch {
     static constexpr int NV = ROWS * LR_K / 256;
     float v[NV];
-    __device__ __forceinline__ void load(const float * __restrict__ M, int64_t ld, int r0, int rows, int k0, int K) {
+    __device__ __forceinline__ void load(const float * M, int64_t ld, int r0, int rows, int k0, int K) {
 #pragma unroll
         for (int u = 0; u < NV; u++) {
             const int i = threadIdx.x + 256 * u, r = r0 + i / LR_K, k = k0 + i % LR_K;
@@ -61,7 +61,7 @@ struct LowrankFetch {
 // distributed shared memory, summed in the order of the CTAs (a token's result depends on the width alone, not on the batch)
 constexpr int LR_SPLIT = 8;
 template <int TT>
-__global__ void __cluster_dims__(1, 1, LR_SPLIT) __launch_bounds__(256) k_lowrank_down(const float * __restrict__ m, const float * __restrict__ w1,
+__global__ void __cluster_dims__(1, 1, LR_SPLIT) __launch_bounds__(256) k_lowrank_down(const float * m, const float * __restrict__ w1,
                                                                                     float * __restrict__ tmp, int T, int rank, int width) {
     pdl_enter();
     __shared__ __align__(16) float As[TT][LR_S];
@@ -105,7 +105,7 @@ __global__ void __cluster_dims__(1, 1, LR_SPLIT) __launch_bounds__(256) k_lowran
 }
 // decay[t][n] = exp(-exp(w0[n] + sum_j tmp[t][j] w2[n][j]));  RAW: tmp holds the sums before their tanh
 template <int TT, bool RAW>
-__global__ void __launch_bounds__(256) k_lowrank_up(const float * __restrict__ tmp, const float * __restrict__ w2, const float * __restrict__ w0,
+__global__ void __launch_bounds__(256) k_lowrank_up(const float * tmp, const float * __restrict__ w2, const float * __restrict__ w0,
                                                     float * __restrict__ decay, int T, int N, int rank) {
     pdl_enter();
     __shared__ __align__(16) float As[TT][LR_S];

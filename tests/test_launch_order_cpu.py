@@ -25,11 +25,15 @@ def kernels():
 
 
 KERNELS = list(kernels())
+WAITING = [k for k in KERNELS if re.search(r"pdl_(enter|wait)\(\)", k[3])]
+# weights and tables of the model, and the batch's description, which is copied in front of the pass: no kernel of the pass writes them
+CONSTANT = set("""W w wa wb wn wq wk wkv wr wuk wuv w0 w1 w2 r_w bias corr sgw gateup down sink freq v_freq freq_factors A_log dt_bias Dp decay pq f_bias lower vec mu coef
+                  table slot off pos0 entry_of""".split())
 ALLOC = [k for k in KERNELS if "tcgen05.alloc" in k[3]]
 
 
 def test_every_kernel_is_found():
-    assert len(KERNELS) > 100 and len(ALLOC) == 5
+    assert len(KERNELS) > 100 and len(WAITING) > 60 and len(ALLOC) == 5
 
 
 @pytest.mark.parametrize("kernel", ALLOC, ids=lambda k: k[1])
@@ -37,3 +41,11 @@ def test_successor_starts_behind_the_allocation_of_tensor_memory(kernel):
     """A successor that takes columns an SM's older CTA has yet to allocate waits for that CTA, and that CTA for the columns."""
     body = kernel[3]
     assert body.rindex("tcgen05.alloc") < body.index("pdl_trigger()") and "pdl_enter()" not in body
+
+
+@pytest.mark.parametrize("kernel", WAITING, ids=lambda k: k[1])
+def test_results_of_earlier_kernels_are_no_constants(kernel):
+    """const __restrict__ and __ldg tell the compiler that nobody writes the data while the kernel runs; it may then load ahead of the wait."""
+    taken = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", kernel[2]))
+    assert taken <= CONSTANT, taken - CONSTANT
+    assert "__ldg(" not in kernel[3] and "ld.global.nc" not in kernel[3]
