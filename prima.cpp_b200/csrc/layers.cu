@@ -3086,7 +3086,9 @@ void * pb200_result_take(pb200_model * m, size_t bytes) { return m && m->ll ? re
 int pb200_batch_step(pb200_model * m, int n_entries, const pb200_batch_entry * entries, float * logits_host, int32_t * greedy_host) {
     if (!m) return PB200_EINVAL;
     if (!m->ll) return PB200_ENOTSUP;
-    return ll_batch_step(m, n_entries, entries, logits_host, greedy_host);
+    const int rc = ll_batch_step(m, n_entries, entries, logits_host, greedy_host);
+    if (rc) cudaStreamSynchronize(m->stream);   // a step that fails half way leaves no copy on its way to the caller's memory
+    return rc;
 }
 int pb200_dense(int type, const void * A, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
                 const float * resid, int64_t ldr, float alpha, void * stream) {

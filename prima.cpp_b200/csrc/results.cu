@@ -4,6 +4,7 @@
 //
 // One pool per model, of a fixed size, taken when the model is finalized.  Blocks may outlive the model: the pool goes with the last of both.  All calls are
 // safe from any thread.  The memory is the process's own (registered, not allocated by the driver), in huge pages where the system gives them.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdlib.h>
 #include <sys/mman.h>
@@ -86,13 +87,47 @@ void * result_take(ResultPool * p, size_t bytes) {
         }
     return nullptr;
 }
-bool result_direct(const void * p, size_t bytes) {
-    cudaPointerAttributes a{}, b{};
-    if (!p || bytes == 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, (const uint8_t *) p + bytes - 1) != cudaSuccess) {
+namespace {
+// the driver's page-locked range that holds p (the entry point comes from the driver at run time, nothing links against it)
+bool locked_range(const void * p, uintptr_t & start, size_t & size) {
+    using Get = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Get get = [] {
+        void * f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
+        return (Get) f;
+    }();
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeHost && b.type == cudaMemoryTypeHost;
+    CUdeviceptr at = 0;
+    if (a.type != cudaMemoryTypeHost || !get || get(&at, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr) p) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr) p) != CUDA_SUCCESS)
+        return false;
+    start = (uintptr_t) at;
+    return true;
+}
+}  // namespace
+// One copy takes the whole of [p, p + bytes), so it has to lie in one allocation or registration: two of them side by side, or with ordinary pages between
+// them, have page-locked ends as well
+bool result_direct(const void * p, size_t bytes) {
+    uintptr_t start = 0;
+    size_t size = 0;
+    if (!p || bytes == 0) return false;
+    {
+        Pools & ps = pools();
+        std::lock_guard<std::mutex> g(ps.lock);
+        auto it = ps.by_base.upper_bound((uintptr_t) p);
+        if (it != ps.by_base.begin()) {
+            --it;
+            start = it->first;
+            size = it->second->bytes;
+        }
+    }
+    auto holds = [&] { return (uintptr_t) p >= start && bytes <= size && (uintptr_t) p - start <= size - bytes; };
+    return holds() || (locked_range(p, start, size) && holds());
 }
 
 }  // namespace pb
