@@ -28,7 +28,7 @@ namespace {
 // Bound: a tile's chain of about 3500 clocks (S after P 1300, weights 1450 .. 1700, agreement on the row's score 230, stores and barriers 200), of which two CTAs hide
 // half of each other's, and 5 us per item for queries, last P V and output.  1024 clocks a tile are the MUFU's, 1450 the MMAs'.
 // us in a row of calls, two walks (all scores twice, for maximum and sum first) and an item a CTA / this: 32 heads over 8, 2048 tokens 80.4 / 52.5 (654 TFLOP/s of
-// visible pairs), 700 23.9 / 19, 512 17.8 / 14.4, 300 13.9 / 12.7, 250 11.8 / 12.4, 128 9.6 / 9.4, 16 7.8 / 7.7, 16 behind 2000 49 / 35; 8 heads over 4, 1500 behind
+// visible pairs), 700 23.9 / 19, 512 17.8 / 13.6, 300 13.9 / 11.6, 250 11.8 / 11.4, 128 9.6 / 9.0, 16 7.8 / 7.1, 16 behind 2000 49 / 35; 8 heads over 4, 1500 behind
 // 548 51 / 37.  One walk with an item a CTA took 58.6 at 2048; the maximum in a pass of its own over S in every tile 50.9, but 37 for 16 behind 2000 and 39 for 1500
 // behind 548; weights as two f16 numbers, which need no look at short rows and are within 1.4e-6 of 64 bits, 61.5.  Error against 64 bits at 2048 tokens 2.02e-4 / 1.99e-4.
 constexpr int AT_STAGES = 2, AT_STAGE = 32768, AT_BLOCK = 16384;
@@ -449,10 +449,10 @@ bool attn_prefill_tc_ok(const float * q, const __half * kcache, const __half * v
 
 int launch_attn_prefill_tc(const float * q, const __half * kcache, const __half * vcache, float * out, int n_head, int n_head_kv, const int32_t * pos_dev, int n_tok,
                            int n_kv_max, float scale, cudaStream_t st) {
-    constexpr size_t smem = 1024 + (size_t) (AT_STAGES + 1) * AT_STAGE + sizeof(AtCtl);
-    static_assert(smem <= 232448, "shared memory of an SM");
+    constexpr size_t smem = 1024 + (size_t) (AT_STAGES + 1) * AT_STAGE + sizeof(AtCtl), alone = 116 * 1024;   // alone: more than half of an SM's
+    static_assert(smem <= alone && 2 * alone > 232448, "shared memory of an SM");
     static FuncAttrCache cache;
-    const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_attn_prefill_tc, smem, true);
+    const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_attn_prefill_tc, alone, true);
     if (e != cudaSuccess) return (int) e;
     const int gqa = n_head / n_head_kv;
     const float c = scale == 0.f ? FLT_MIN : fabsf(scale) * 1.4426950408889634f;   // a masked score stays -inf
@@ -465,18 +465,21 @@ int launch_attn_prefill_tc(const float * q, const __half * kcache, const __half 
     if (!rc) rc = make_map(mv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, vcache, ld, n_kv_max, 1, ld, 0, 128);
     if (rc) return rc;
     const int64_t slots = 2 * (int64_t) sm_count();
+    const bool spread = items <= sm_count();   // an SM for every item
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned) (items < slots ? items : slots));
     cfg.blockDim = dim3(AT_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = spread ? alone : smem;
     cfg.stream = st;
     // Barriers and tensor memory are set up while the kernel in front ends (the kernel waits before it reads anything), unless that could put two items on one SM while
-    // others are idle, because the kernel in front is still there: 512 tokens, 32 heads over 8, 14.4 us in calls one after the other without, 15.9 with; 16 tokens 8.5 / 7.7
+    // others are idle, because the kernel in front is still there.  Where every item can have an SM of its own, shared memory for one CTA to an SM keeps them apart.
+    // us in calls one after the other, 150 tokens / 250 / 512, waiting for the end of the kernel in front / this: 64 heads over 8 14.3 / 11.6, 14.4 / 11.8, - ; 32 over 8 12.0 / 11.0,
+    // 12.8 / 11.4, 14.4 / 13.6 (two walks over the keys 12.3, 12.3, 17.8)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2 * items <= sm_count() || items >= slots ? 1 : 0;
+    cfg.numAttrs = spread || items >= slots ? 1 : 0;
     return (int) cudaLaunchKernelEx(&cfg, k_attn_prefill_tc, mk, mv, P);
 }
 
