@@ -37,9 +37,14 @@ Pools & pools() {   // never destroyed: blocks may come back while the process e
     static Pools * p = new Pools;
     return *p;
 }
-void drop_user(Pools & ps, ResultPool * p) {
-    if (--p->users > 0) return;
+// the pool, if that was its last user: for unmake, without the lock, which other models' calls share
+ResultPool * drop_user(Pools & ps, ResultPool * p) {
+    if (--p->users > 0) return nullptr;
     ps.by_base.erase((uintptr_t) p->base);
+    return p;
+}
+void unmake(ResultPool * p) {
+    if (!p) return;
     if (cudaHostUnregister(p->base) != cudaSuccess) cudaGetLastError();   // at the process's end the driver may be gone
     free(p->base);
     delete p;
@@ -69,8 +74,11 @@ ResultPool * result_pool_create(size_t bytes) {
 void result_pool_release(ResultPool * p) {
     if (!p) return;
     Pools & ps = pools();
-    std::lock_guard<std::mutex> g(ps.lock);
-    drop_user(ps, p);
+    {
+        std::lock_guard<std::mutex> g(ps.lock);
+        p = drop_user(ps, p);
+    }
+    unmake(p);
 }
 void * result_take(ResultPool * p, size_t bytes) {
     if (!p || bytes == 0 || bytes > p->bytes) return nullptr;
@@ -135,7 +143,7 @@ bool result_direct(const void * p, size_t bytes) {
 extern "C" int pb200_result_give(void * block) {
     using namespace pb;
     Pools & ps = pools();
-    std::lock_guard<std::mutex> g(ps.lock);
+    std::unique_lock<std::mutex> g(ps.lock);
     auto it = ps.by_base.upper_bound((uintptr_t) block);
     if (!block || it == ps.by_base.begin()) return PB200_EINVAL;
     ResultPool * p = (--it)->second;
@@ -150,6 +158,8 @@ extern "C" int pb200_result_give(void * block) {
         if (prev->first + prev->second == at) { at = prev->first; n += prev->second; p->free_.erase(prev); }
     }
     p->free_[at] = n;
-    drop_user(ps, p);
+    p = drop_user(ps, p);
+    g.unlock();
+    unmake(p);
     return 0;
 }
