@@ -293,9 +293,9 @@ typedef struct pb200_batch_entry {
     int32_t n_want;
     const int32_t * want;
 } pb200_batch_entry;
-/* Page-locked host memory for logits_host, out of a pool of fixed size that a layer-list model holds from pb200_model_finalize on: the rows arrive in it without a
- * copy through a staging buffer (as in any page-locked memory of the caller's).  NULL: the pool has no room, use any other memory.  A block stays valid until it is
- * given back, also beyond the model's end.  Both calls may come from any thread. */
+/* Page-locked host memory for logits_host, out of a pool of bounded size that a layer-list model takes from the system as blocks are asked for and holds until its end:
+ * the rows arrive in it without a copy through a staging buffer (as in any page-locked memory of the caller's).  NULL: the pool has no room, or there is no memory that can
+ * be page-locked; use any other memory.  A block stays valid until it is given back, also beyond the model's end.  Both calls may come from any thread. */
 PB200_API void * pb200_result_take(pb200_model * m, size_t bytes);
 PB200_API int    pb200_result_give(void * block);
 PB200_API int pb200_batch_step(pb200_model * m, int n_entries, const pb200_batch_entry * entries, float * logits_host, int32_t * greedy_host);

@@ -1802,7 +1802,7 @@ int ll_finalize(pb200_model * m) {
     ll.seq_prev.assign((size_t) ll.n_seq, -1);
     m->n_seq = ll.n_seq;
     m->weight_bytes = ll.weight_bytes;
-    ll.results = result_pool_create(LayerList::RESULT_BYTES);   // none: every step's logits go through the staging buffer
+    ll.results = result_pool_create(LayerList::RESULT_BYTES);
     m->finalized = true;
     return 0;
 }
@@ -3082,7 +3082,13 @@ int pb200_seq_length(pb200_model * m, int slot) {
     if (!m->ll) return PB200_ENOTSUP;
     return ll_seq_length(m, slot);
 }
-void * pb200_result_take(pb200_model * m, size_t bytes) { return m && m->ll ? result_take(m->ll->results, bytes) : nullptr; }
+void * pb200_result_take(pb200_model * m, size_t bytes) try {
+    if (!m || !m->ll) return nullptr;
+    cudaSetDevice(m->device);
+    return result_take(m->ll->results, bytes);
+} catch (...) {   // no memory for the bookkeeping
+    return nullptr;
+}
 int pb200_batch_step(pb200_model * m, int n_entries, const pb200_batch_entry * entries, float * logits_host, int32_t * greedy_host) {
     if (!m) return PB200_EINVAL;
     if (!m->ll) return PB200_ENOTSUP;

@@ -465,7 +465,7 @@ int launch_conv4(const float * u, int64_t ldu, const BatchView & b, int channels
 
 // page-locked memory for the logits of batch steps (results.cu)
 struct ResultPool;
-ResultPool * result_pool_create(size_t bytes);              // NULL: no memory that can be page-locked
+ResultPool * result_pool_create(size_t bytes);              // of up to so many bytes, none yet
 void result_pool_release(ResultPool * p);                   // the model's share; blocks that are out keep the pool
 void * result_take(ResultPool * p, size_t bytes);
 bool result_direct(const void * p, size_t bytes);           // the device can write [p, p + bytes) itself
