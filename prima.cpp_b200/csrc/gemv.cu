@@ -839,11 +839,12 @@ bool gemv_dist_prologue_ok() {
 }
 // Up to this length every CTA quantizes the activation for itself; above it a kernel in front does.  us per call, two launches / one: Q4_K 1000 x 2048
 // 9.1 / 4.6, 4096 x 4096 12.1 / 6.4, 14336 x 4096 14.8 / 9.3, 4096 x 14336 16.5 / 15.2, 28672 x 14336 47.2 / 44.5, Q6_K 1000 x 14336 12.4 / 11.2; but
-// Q5_K 301 x 28672 12.3 / 15.8: there 14 super-blocks a warp, one after the other, are what the call waits for.
+// Q5_K 301 x 28672 12.3 / 15.8: there 14 super-blocks a warp, one after the other, are what the call waits for.  While a trace is taken the product is a launch of its
+// own, which has the stamps.
 constexpr int GEMV_QUANT_MAX_K = 16384;
 bool gemv_quant_prologue_ok(int type, const void * W, int N, int K, const float * x) {
     GemvPlan pl;
-    return is_kquant(type) && K <= GEMV_QUANT_MAX_K && (((uintptr_t) W | (uintptr_t) x) & 15) == 0 && gemv_plan(&type, &N, 1, K, pl);
+    return !g_trace_buf && is_kquant(type) && K <= GEMV_QUANT_MAX_K && (((uintptr_t) W | (uintptr_t) x) & 15) == 0 && gemv_plan(&type, &N, 1, K, pl);
 }
 int gemv_smem_bytes(int type, int K, int N) {
     GemvPlan pl;
