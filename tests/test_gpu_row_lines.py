@@ -1,0 +1,32 @@
+"""-m gpu: prompts at the lengths from which a CTA routes eight tokens, whole groups of them and rests, against the float64 oracles."""
+import numpy as np
+import pytest
+
+import ref_sapudra as RS
+import test_gpu_sapudra as S
+
+pytestmark = pytest.mark.gpu
+
+
+def lines(lib, rows):
+    """tokens up to which a token has a CTA of its own (a warp a router row, 8 to 32 of them)"""
+    per_sm = 2048 // (256 if rows <= 8 else 1024 if rows >= 32 else 32 * rows)
+    return lib.c.pb200_sm_count() * (per_sm if per_sm > 2 else 2 * per_sm)
+
+
+@pytest.mark.parametrize("moe", [dict(experts=15, top=3, count=5, keep=2), dict(experts=32, top=4, ff=30, count=8, keep=4), dict(experts=24, top=2, ff=36, count=1, keep=1, shared=None)])
+def test_routing(pkg, cuda, lib, moe):
+    cfg = S.config([S.att_layer(heads=2, kv_heads=1, dim=16, vdim=16, window=40, mlp=S.moe_ff(**moe))], width=72, vocab=37, max_positions=1024)
+    bits, W = RS.random_weights(cfg, seed=moe["experts"])
+    m = S.load(pkg, cfg, bits, n_ctx=1024)
+    line = lines(lib, moe["experts"] + (moe.get("shared", 56) is not None))
+    assert line < 1000
+    for n in (line, line + 1, line + 8):
+        t = S.tokens_for(cfg, n, n)
+        want = RS.forward(cfg, W, t)
+        want = want[0] if isinstance(want, tuple) else want
+        s = m.seq_alloc()
+        got = m.batch_step([(s, t, list(range(n)))])[0]
+        m.seq_free(s)
+        assert RS.rel_err(np.asarray(got, dtype=np.float64), want).max() < S.F32_TOL, n
+    m.close()

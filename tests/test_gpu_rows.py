@@ -73,7 +73,7 @@ def test_latents_of_every_size(pkg, cuda, kv_rank, q_rank, dtype, tol):
 @pytest.mark.parametrize("width", [72, 70])   # 70: rows that are gathered and summed an element a thread
 @pytest.mark.parametrize("moe", [dict(), dict(experts=5, top=2, ff=36, count=1, keep=1, shared=None), dict(experts=32, top=4, ff=30, count=8, keep=4)])
 def test_experts_of_a_prompt(pkg, cuda, width, moe):
-    """Prompts around the length from which a CTA routes eight tokens, whole groups of them and rests."""
+    """Prompts of some dozens of tokens: experts with many tokens, few and none."""
     cfg = S.config([S.att_layer(heads=2, kv_heads=1, dim=16, vdim=16, window=300, mlp=S.moe_ff(**moe))], width=width, vocab=37)
     bits, W = RS.random_weights(cfg, seed=width)
     m = S.load(pkg, cfg, bits, n_ctx=256)
