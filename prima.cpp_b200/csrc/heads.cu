@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "launch.h"
 #include "layers.h"
 #include "mixers.cuh"
 #include "rows.cuh"
@@ -220,7 +221,10 @@ int launch_conv4(const float * u, int64_t ldu, const BatchView & b, int channels
     if (channels % 4 != 0 || !rows_ok(u, ldu) || !at16(w) || !rows_ok(conv_state, slot_stride) || !rows_ok(out, ldo)) return (int) cudaErrorNotSupported;
     const unsigned tiles = (unsigned) ((channels / 4 + 127) / 128);
     return ck_launch([&] {
-        if (b.n_tokens >= 128)   // four tokens a thread share the weights and, in L1, the inputs
+        // Four tokens a thread share the weights and, in L1, the inputs, but a quarter of the CTAs keep the SMs busy only from so many on.  us of the convolution and its
+        // state's step, a token a thread / four: 3072 channels 128 tokens 13.1 / 14.9, 256 tokens 15.2 / 15.2, 384 tokens 15.3 / 15.2, 512 tokens 17.2 / 15.7; 2048 channels
+        // 256 tokens 13.4 / 13.9, 512 tokens 15.6 / 15.4, 1024 tokens 19.6 / 17.1
+        if ((int64_t) b.n_tokens * tiles >= 14 * sm_count())
             launch_dep(k_conv4<4>, dim3(tiles, (unsigned) ((b.n_tokens + 3) / 4)), dim3(128), 0, st, u, ldu, b.slot, b.off, b.entry_of, b.n_tokens, channels, w, silu_from, conv_state,
                        slot_stride, out, ldo, advance);
         else

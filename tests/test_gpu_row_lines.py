@@ -1,8 +1,10 @@
-"""-m gpu: prompts at the lengths from which a CTA routes eight tokens, whole groups of them and rests, against the float64 oracles."""
+"""-m gpu: prompts at the lengths from which a CTA routes eight tokens and a thread convolves four, whole groups of them and rests, against the float64 oracles."""
 import numpy as np
 import pytest
 
+import ref_ludusun as RL
 import ref_sapudra as RS
+import test_gpu_ludusun as L
 import test_gpu_sapudra as S
 
 pytestmark = pytest.mark.gpu
@@ -29,4 +31,15 @@ def test_routing(pkg, cuda, lib, moe):
         got = m.batch_step([(s, t, list(range(n)))])[0]
         m.seq_free(s)
         assert RS.rel_err(np.asarray(got, dtype=np.float64), want).max() < S.F32_TOL, n
+    m.close()
+
+
+def test_convolution(pkg, cuda, lib):
+    cfg = L.config([L.par(heads=2, kv_heads=1, dim=16, r_heads=8, r_kv=8, r_dim=128, r_vdim=128, taps=4, ff=0)], width=64, vocab=37)
+    bits, W = RL.random_weights(cfg, seed=5)
+    m = L.load(pkg, cfg, bits, n_ctx=512)
+    line = -(-14 * lib.c.pb200_sm_count() // 6)      # 3072 channels: six tiles of 512
+    for n in (line - 1, line, line + 1, line + 3):
+        t = L.tokens_for(cfg, n, n)
+        L.check(L.run_whole(m, t), RL.forward(cfg, W, t)[0], L.F32_TOL)
     m.close()
