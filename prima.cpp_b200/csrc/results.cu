@@ -25,8 +25,8 @@
 namespace pb {
 
 constexpr size_t RESULT_PAGE = 4096, RESULT_ALIGN = 2u << 20;
-// a slab holds this many blocks of the size that it is made for, as far as the pool's bound allows
-constexpr size_t RESULT_SLAB_BLOCKS = 4;
+// A slab holds this many blocks of the size that it is made for, as far as the pool's bound allows: the first step with results waits for it (blocks of 1 MB: 0.4 ms)
+constexpr size_t RESULT_SLAB_BLOCKS = 2;
 
 namespace {
 struct Slab {
