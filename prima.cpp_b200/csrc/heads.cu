@@ -220,6 +220,7 @@ int launch_conv4(const float * u, int64_t ldu, const BatchView & b, int channels
                  int advance, cudaStream_t st) {
     if (channels % 4 != 0 || !rows_ok(u, ldu) || !at16(w) || !rows_ok(conv_state, slot_stride) || !rows_ok(out, ldo)) return (int) cudaErrorNotSupported;
     const unsigned tiles = (unsigned) ((channels / 4 + 127) / 128);
+    if ((b.n_tokens + 3) / 4 > 65535) return (int) cudaErrorNotSupported;   // a grid's second dimension: more tokens go to the general kernel
     return ck_launch([&] {
         // Four tokens a thread share the weights and, in L1, the inputs, but a quarter of the CTAs keep the SMs busy only from so many on.  us of the convolution and its
         // state's step, a token a thread / four: 3072 channels 128 tokens 13.1 / 14.9, 256 tokens 15.2 / 15.2, 384 tokens 15.3 / 15.2, 512 tokens 17.2 / 15.7; 2048 channels

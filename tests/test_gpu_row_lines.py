@@ -4,8 +4,10 @@ import pytest
 
 import ref_ludusun as RL
 import ref_sapudra as RS
+import ref_zevedra as RZ
 import test_gpu_ludusun as L
 import test_gpu_sapudra as S
+import test_gpu_zevedra as Z
 
 pytestmark = pytest.mark.gpu
 
@@ -42,4 +44,24 @@ def test_convolution(pkg, cuda, lib):
     for n in (line - 1, line, line + 1, line + 3):
         t = L.tokens_for(cfg, n, n)
         L.check(L.run_whole(m, t), RL.forward(cfg, W, t)[0], L.F32_TOL)
+    m.close()
+
+
+def test_more_tokens_than_a_grid_has_rows(pkg, cuda):
+    """Five prompts that have more tokens together than the four-tap convolution's grid takes in groups of four, against each of them alone."""
+    cfg = Z.config([Z.par(heads=1, kv_heads=1, dim=8, vdim=8, rot=4, window=16, conv=4, r_heads=1, r_kv=1, r_dim=8, r_vdim=8, r_conv=4)], width=16, vocab=23)
+    bits, W = RZ.random_weights(cfg, seed=3)
+    m = Z.load(pkg, cfg, bits, n_ctx=53000)
+    ts = [np.random.default_rng(i).integers(0, 23, 53000).astype(np.int32) for i in range(5)]
+
+    def run(ts):
+        slots = [m.seq_alloc() for _ in ts]
+        out = m.batch_step([(s, t, [20, len(t) - 1]) for s, t in zip(slots, ts)])[0].copy()
+        for s in slots:
+            m.seq_free(s)
+        return out
+    together = run(ts)
+    assert np.isfinite(together).all()
+    for i, t in enumerate(ts):
+        assert RS.rel_err(together[2 * i:2 * i + 2].astype(np.float64), run([t]).astype(np.float64)).max() < Z.F32_TOL
     m.close()
