@@ -392,7 +392,8 @@ template <int N>
 int delta_scan_launch(const GatedLinIO & io, const BatchView & b, const GatedLinParams & p, float * state, int64_t slot_stride, float * y, cudaStream_t st) {
     const dim3 grid((unsigned) (p.heads * ((p.vdim + DS_COLS - 1) / DS_COLS)), (unsigned) b.n_entries);
     // Blocks of four where every CTA has an SM of its own: 384 threads and 106 KB a CTA leave room for one or two, and with more CTAs than SMs it is throughput that
-    // counts (eight prompts of 9 to 128 tokens: 26 us token by token, 52 in blocks).  Entries of fewer tokens are not a block.
+    // counts (eight prompts of 9 to 128 tokens: 26 us token by token, 52 in blocks).  Entries of fewer tokens are not a block.  The two forms round differently: a prompt's
+    // last bits depend on how many others share its batch.
     if (b.max_n >= DB_BLOCK && (int64_t) grid.x * grid.y <= sm_count()) {
         const int rc = raise_smem(k_delta_blocks<N>, sizeof(DbSmem<N>));
         if (rc) return rc;

@@ -423,7 +423,7 @@ int launch_moe_route_sigmoid(const void * h, int htype, const float * wr, const 
     const int threads = rows <= 8 ? 256 : rows >= 32 ? 1024 : 32 * rows;
     // Eight tokens a CTA read the router's rows an eighth as often, but their CTAs are few and each takes longer: that pays once the CTAs of one token no longer run
     // in one wave (where an SM holds two of them, in two).  us of the experts of a layer, a token a CTA / eight: 8 rows 456 tokens 70.8 / 75.6, 1200 tokens 99.6 / 97.7;
-    // 17 rows of 2048 64 tokens 95.3 / 99.5, 444 tokens 75.1 / 77.3, 456 tokens 84.2 / 79.0, 1024 tokens 103.5 / 91.5; 25 rows 296 tokens 77.0 / 85.5, 592 tokens
+    // 17 rows of 2048 128 tokens 70.8 / 74.9, 444 tokens 75.1 / 77.3, 456 tokens 84.2 / 79.0, 1024 tokens 103.5 / 91.5; 25 rows 296 tokens 77.0 / 85.5, 592 tokens
     // 91.9 / 91.8, 600 tokens 98.8 / 92.2; 33 rows 592 tokens 105.4 / 107.2, 600 tokens 112.5 / 108.3; 65 rows 256 tokens 124.8 / 147.5, 640 tokens 162.2 / 158.6
     const int per_sm = 2048 / threads, line = sm_count() * (per_sm > 2 ? per_sm : 2 * per_sm);
     const size_t many = ROUTE_TOKENS * ((size_t) width + 2 * (size_t) p.experts + 2 * (size_t) p.groups) * sizeof(float);
