@@ -255,8 +255,8 @@ constexpr int ROWS_MAX_T = 8;
 // Largest batch the weight-streaming kernel takes when the tensor-core kernel could run instead.  PB200_DENSE_ROWS_MAX overrides for A/B runs.  The line was
 // drawn when the tensor-core kernel had 64-token tiles.  With its 16-token tiles and K over a cluster, us on a B200 for 2 / 4 tokens (weights
 // from HBM): 28672 x 4096 51 / 67 here, 39 / 40 there; 4096 x 14336 27 / 36, 22 / 22; 4096 x 4096 11.3 / 14.1, 9.6 / 9.7; 2048 x 2048 5.9 / 7.2,
-// 6.2 / 6.3; 512 x 2048 5.2 / 6.7, 5.2 / 5.2.  One token: 44 here at 28672 x 4096 and 4.9 at 2048 x 2048.  So batches of 2 to 4 would gain by a
-// lower line, which changes the order of their sums.
+// 6.2 / 6.3; 512 x 2048 5.2 / 6.7, 5.2 / 5.2.  One token: 44 here at 28672 x 4096 and 4.9 at 2048 x 2048.  The tensor cores' sums over a long K are
+// less exact than these (1e-5 against 1e-7), so batches of 2 to 4 stay on this side; most of them take dense_stream.cu (41 / 55 at 28672 x 4096).
 int rows_max_t() {
     static const int v = [] {
         const char * e = getenv("PB200_DENSE_ROWS_MAX");
@@ -270,6 +270,12 @@ template <typename WT>
 int dense_typed(const WT * A, int64_t lda, const WT * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
                 const float * resid, int64_t ldr, float alpha, cudaStream_t st, int plane_rows = 0, int64_t a_plane = 0,
                 const DenseAct & act = DenseAct()) {
+    if constexpr (sizeof(WT) == 2) {
+        if (plane_rows == 0) {   // rows one behind the other: streamed through shared memory
+            const int rc = launch_dense_stream(A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st, act);
+            if (rc != (int) cudaErrorNotSupported) return rc;
+        }
+    }
     if (T <= ROWS_MAX_T) {
         const bool glu = act.silu_glu != 0;
         if (glu) N /= 2;   // pairs of rows

@@ -247,6 +247,7 @@ struct LayerList {
     std::vector<int> prof_cat;
     float prof_ms[10] = {0};
     // decode steps replayed as CUDA graphs, one per (entries, wanted rows); the batch's metadata lives at fixed device addresses
+    const float * norm_ahead = nullptr;   // weight of a norm of the stream that the next product makes for itself (stream_product)
     struct StepGraph { cudaGraphExec_t exec = nullptr; int seen = 0; uint64_t launches = 0; };
     std::map<uint64_t, StepGraph> graphs;
     // a dual mixer's recurrent branch runs on a second stream beside the attention branch (fork after the token preparation, join before the
@@ -2050,6 +2051,21 @@ static int tap_prepare(pb200_model * m, int T) {
     return 0;
 }
 
+// C[t] = W h (+ bias), or its activation, h = the sublayer's normed input: ll.act, or still to be made from the stream (norm_ahead)
+static int stream_product(pb200_model * m, int T, const DenseW & w, int N, float * C, const float * bias, const DenseAct * act) {
+    LayerList & ll = *m->ll;
+    const int W = ll.width, ct = ll.ctype;
+    if (ll.norm_ahead) {
+        const float * nw = ll.norm_ahead;
+        ll.norm_ahead = nullptr;
+        const int rc = launch_dense_normed(ct, ll.x, W, nullptr, nw, ll.eps, w.data, W, C, N, T, N, W, bias, m->stream, act ? *act : DenseAct());
+        if (rc != (int) cudaErrorNotSupported) return rc;
+        CK(launch_group_rmsnorm(ll.x, nullptr, nw, 1, ll.eps, ll.act, ct, T, W, m->stream));
+    }
+    if (act) return launch_dense_act(ct, ll.act, W, w.data, W, *act, T, N, W, m->stream);
+    return launch_dense(ct, ll.act, W, w.data, W, C, N, T, N, W, bias, nullptr, 0, 1.f, m->stream);
+}
+
 // ---- mixers: out[t] = (resid ? resid[t] : 0) + mixer(ll.act[t]); ll.act holds the mixer's input in the operand type ----
 static int mix_attention(pb200_model * m, const BatchView & b, bool prefill, const LRun & r, LLayer & L, const float * resid, float * out) {
     LayerList & ll = *m->ll;
@@ -2059,7 +2075,7 @@ static int mix_attention(pb200_model * m, const BatchView & b, bool prefill, con
     const int C = attn_qkvg_cols(a);
     float * sbase = ll.state + r.state_off;       // this layer's rows, or those of the layer it reads
     CAT(CAT_DENSE);
-    CK(launch_dense(ct, ll.act, W, L.qkvg.data, W, ll.big, C, T, C, W, nullptr, nullptr, 0, 1.f, st));
+    CK(stream_product(m, T, L.qkvg, C, ll.big, nullptr, nullptr));
     float * kc = sbase, * vc = sbase + (int64_t) a.cache_rows * a.kv_heads * a.dim;
     CAT(CAT_ATTN);
     if (L.att_prep) {   // norm over the whole projections, rotation, temperatures and the cache store in one launch
@@ -2132,7 +2148,7 @@ static int mix_latent(pb200_model * m, const BatchView & b, bool prefill, const 
     float * q = direct_q ? ll.big : ll.big2;      // [T][heads][dim + rot_dim], rows ldq floats apart
     const int64_t ldq = direct_q ? C : (int64_t) H * DQ;
     CAT(CAT_DENSE);
-    CK(launch_dense(ct, ll.act, W, L.lproj.data, W, ll.big, C, T, C, W, nullptr, nullptr, 0, 1.f, st));
+    CK(stream_product(m, T, L.lproj, C, ll.big, nullptr, nullptr));
     CAT(CAT_LATENT);
     // a layer with a cache of its own: the batch's latents and key parts leave in the same launch that stores them (the query latent takes
     // ll.act2, and the mixer's input in ll.act has been read by then)
@@ -2233,7 +2249,7 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     o = (o + 3) / 4 * 4;
     float * rec_state = ll.state + r.state_off + o;
     CAT(CAT_DENSE);
-    CK(launch_dense(ct, ll.act, W, L.qkvg.data, W, ll.big, C, T, C, W, d.biased ? L.qk_bias.data : nullptr, nullptr, 0, 1.f, st));
+    CK(stream_product(m, T, L.qkvg, C, ll.big, d.biased ? L.qk_bias.data : nullptr, nullptr));
     // where q, k, v of a branch are read from: the projection, or the convolution's output where its columns pass one
     float * lq = ll.big + d.c_q, * lk = ll.big + d.c_k, * lv = a.tied_v ? lk : ll.big + d.c_v, * rq = ll.big + d.c_rq, * rk = ll.big + d.c_rk, * rv = ll.big + d.c_rv;
     int64_t ld = C, ldr = C;
@@ -2408,14 +2424,14 @@ static int ff_xielu(pb200_model * m, int T, LLayer & L, float * x) {
     static const bool unfused = getenv("PB200_FF_UNFUSED") != nullptr;
     CAT(CAT_DENSE);
     if (unfused) {
-        CK(launch_dense(ct, ll.act, W, L.gateup.data, W, ll.big, ff, T, ff, W, nullptr, nullptr, 0, 1.f, st));
+        CK(stream_product(m, T, L.gateup, ff, ll.big, nullptr, nullptr));
         CAT(CAT_ELEM);
         CK(launch_xielu(ll.big, L.ff_act.data, ll.act2, ct, (int64_t) T * ff, st));
         CAT(CAT_DENSE);
     } else {
         DenseAct act;
         act.xielu = L.ff_act.data; act.y = ll.act2; act.ldy = ff;
-        CK(launch_dense_act(ct, ll.act, W, L.gateup.data, W, act, T, ff, W, st));
+        CK(stream_product(m, T, L.gateup, ff, nullptr, nullptr, &act));
     }
     return launch_dense(ct, ll.act2, ff, L.down.data, ff, x, W, T, W, ff, nullptr, x, W, 1.f, st);
 }
@@ -2428,14 +2444,14 @@ static int ff_silu(pb200_model * m, int T, LLayer & L, float * x) {
     static const bool unfused = getenv("PB200_FF_UNFUSED") != nullptr;
     CAT(CAT_DENSE);
     if (unfused) {
-        CK(launch_dense(ct, ll.act, W, L.gateup.data, W, ll.big, 2 * ff, T, 2 * ff, W, nullptr, nullptr, 0, 1.f, st));
+        CK(stream_product(m, T, L.gateup, 2 * ff, ll.big, nullptr, nullptr));
         CAT(CAT_ELEM);
         CK(launch_silu_mul(ll.big, ll.act2, ct, T, ff, nullptr, nullptr, st, 1));
         CAT(CAT_DENSE);
     } else {
         DenseAct act;
         act.silu_glu = 1; act.y = ll.act2; act.ldy = ff;
-        CK(launch_dense_act(ct, ll.act, W, L.gateup.data, W, act, T, 2 * ff, W, st));
+        CK(stream_product(m, T, L.gateup, 2 * ff, nullptr, nullptr, &act));
     }
     return launch_dense(ct, ll.act2, ff, L.down.data, ff, x, W, T, W, ff, nullptr, x, W, 1.f, st);
 }
@@ -2554,6 +2570,8 @@ static int ll_forward_prerms(pb200_model * m, const BatchView & b, bool prefill,
     LayerList & ll = *m->ll;
     cudaStream_t st = m->stream;
     const int T = b.n_tokens, W = ll.width, ct = ll.ctype;
+    const bool ahead = ct == T_BF16 && T <= 4 && !ll.prof_on;   // few tokens: a product norms its input itself
+    ll.norm_ahead = nullptr;
     CAT(CAT_ELEM);
     bool act_ready = false;   // the kernel that closed the previous sublayer has left this one's normed input in ll.act
     if (ll.embed_normed || (ll.bigram.buckets <= 0 && ll.loop_times <= 0)) {
@@ -2570,7 +2588,8 @@ static int ll_forward_prerms(pb200_model * m, const BatchView & b, bool prefill,
             CK(launch_stream_add_rmsnorm(ll.x, r.pass > 0 ? ll.x0 : nullptr, ll.loop_step.data + (int64_t) r.pass * W, L.norm1.data, ll.eps, ll.act, ct, T, W, st));
         } else if (!act_ready && L.kind != MIX_WKV) {   // a WKV mixer norms the stream itself, with the token mix
             CAT(CAT_NORM);
-            CK(launch_group_rmsnorm(ll.x, nullptr, L.norm1.data, 1, ll.eps, ll.act, ct, T, W, st));
+            if (ahead) ll.norm_ahead = L.norm1.data;   // the mixers other than WKV begin with one product of it
+            else CK(launch_group_rmsnorm(ll.x, nullptr, L.norm1.data, 1, ll.eps, ll.act, ct, T, W, st));
         }
         act_ready = false;
         // the norm that follows the mixer: this layer's second one, or the next run's first one unless that run opens a pass
@@ -2587,7 +2606,8 @@ static int ll_forward_prerms(pb200_model * m, const BatchView & b, bool prefill,
         if (L.ff > 0) {
             if (!fused) {
                 CAT(CAT_NORM);
-                CK(launch_group_rmsnorm(ll.x, nullptr, L.norm2.data, 1, ll.eps, ll.act, ct, T, W, st));
+                if (ahead && L.ff_kind != FF_MOE) ll.norm_ahead = L.norm2.data;
+                else CK(launch_group_rmsnorm(ll.x, nullptr, L.norm2.data, 1, ll.eps, ll.act, ct, T, W, st));
             }
             if (L.ff_kind == FF_MOE) CK(ff_moe(m, T, prefill, L, ll.x, true, ll.resid_mult));
             else if (L.ff_kind == FF_XIELU && ll.resid_mult == 1.f) CK(ff_xielu(m, T, L, ll.x));
@@ -2600,9 +2620,14 @@ static int ll_forward_prerms(pb200_model * m, const BatchView & b, bool prefill,
     }
     if (nW > 0) {
         CAT(CAT_HEAD);
-        CK(launch_group_rmsnorm(ll.x, want_dev, ll.final_norm.data, 1, ll.eps, ll.actw, ct, nW, W, st));
         float * lg = ll.logits + (int64_t) lrow0 * ll.vocab;
-        CK(launch_dense(ct, ll.actw, W, (ll.tied_head ? ll.embed : ll.head).data, W, lg, ll.vocab, nW, ll.vocab, W, nullptr, nullptr, 0, ll.logit_scale, st));
+        const void * hw = (ll.tied_head ? ll.embed : ll.head).data;
+        int rc = ahead && ll.logit_scale == 1.f ? launch_dense_normed(ct, ll.x, W, want_dev, ll.final_norm.data, ll.eps, hw, W, lg, ll.vocab, nW, ll.vocab, W, nullptr, st, DenseAct()) : (int) cudaErrorNotSupported;
+        if (rc == (int) cudaErrorNotSupported) {
+            CK(launch_group_rmsnorm(ll.x, want_dev, ll.final_norm.data, 1, ll.eps, ll.actw, ct, nW, W, st));
+            rc = launch_dense(ct, ll.actw, W, hw, W, lg, ll.vocab, nW, ll.vocab, W, nullptr, nullptr, 0, ll.logit_scale, st);
+        }
+        CK(rc);
         CK(launch_softcap(lg, (int64_t) nW * ll.vocab, ll.logit_softcap, st));
     }
     CAT(-1);

@@ -56,6 +56,13 @@ struct DenseAct {
     void * y = nullptr;
     int64_t ldy = 0;
 };
+// bf16, up to four tokens, rows of W one behind the other: weights streamed through shared memory (dense_stream.cu); cudaErrorNotSupported: not taken
+int launch_dense_stream(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
+                        const float * resid, int64_t ldr, float alpha, cudaStream_t stream, const DenseAct & act);
+// launch_dense / launch_dense_act of A[t] = the RMS norm of row t, or rows[t], of x (fp32, ldx apart) with weight norm_w, rounded to the operand type, in one launch:
+// bf16, up to four tokens, K up to 8192; cudaErrorNotSupported otherwise
+int launch_dense_normed(int type, const float * x, int64_t ldx, const int32_t * rows, const float * norm_w, float eps, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K,
+                        const float * bias, cudaStream_t stream, const DenseAct & act);
 int launch_dense_act(int type, const void * A, int64_t lda, const void * W, int64_t ldw, const DenseAct & act, int T, int N, int K, cudaStream_t stream);
 // Several products of one shape over operands of their own, side by side: C[t][p * N + n] = sum_k A[p * a_plane + t * lda + k] * W[p * N + n][k],
 // p < planes (W: one [planes * N][K] matrix).
