@@ -196,6 +196,11 @@ int launch_attn_prefill_io(const AttnIO & io, const BatchView & b, const AttnPar
 int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnParams & a, const float * kcache, const float * vcache, int64_t slot_stride,
                           void * out, int otype, cudaStream_t stream, float * part = nullptr);
 
+// one-token entries with a cluster of CTAs per (entry, kv head) (attn_decode.cu): up to eight query heads to a kv head, heads of up to 128 entries, a multiple of
+// four, at 16 bytes; cudaErrorNotSupported otherwise
+int launch_attn_decode_group(const AttnIO & io, const BatchView & b, const AttnParams & a, const float * kcache, const float * vcache, int64_t slot_stride, void * out,
+                             int otype, cudaStream_t stream);
+
 // prompt attention with every operand as two f16 numbers on the tensor cores (attn_split.cu): head sizes up to 192, value sizes up to 128.  A prompt batch whose
 // longest entry is beyond 16 tokens takes it for all of its entries; shorter ones keep the fp32 FMA kernel
 size_t attn_split_bytes(const AttnParams & a, int n_tokens, int n_entries);   // scratch for a prompt batch (0: the shape is not taken)

@@ -10,6 +10,7 @@
 #include <atomic>
 
 #include "layers.h"
+#include "attn.cuh"
 #include "mixers.cuh"
 #include "rows.cuh"
 
@@ -242,8 +243,7 @@ __global__ void __launch_bounds__(1024) k_argmax_rows(const float * __restrict__
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// attention.  Cache row of position p: p itself below keep_first, else keep_first + (p - keep_first) mod ring.
-__device__ __forceinline__ int cache_row(int p, int keep_first, int ring) { return p < keep_first ? p : keep_first + (p - keep_first) % ring; }
+// attention
 
 // where a prompt kernel finds keys and values of an entry's positions: the entry's rows of the batch, or its slot's cache
 struct AttnKV {
@@ -259,15 +259,6 @@ struct AttnKV {
 __device__ __forceinline__ float attn_key(const AttnKV & kv, const AttnIO & io, int64_t row, int kvh, int d, int DN) {
     return d < DN ? kv.k[row * io.ldk + (int64_t) kvh * DN + d] : kv.ks[row * io.ldks + (d - DN)];
 }
-// score of the sink of head h
-__device__ __forceinline__ float attn_sink(const AttnIO & io, int h) { return io.sink ? io.sink[h] : 0.f; }
-// factor on output element d of head h: sigmoid of a gate logit per head, per element, or none
-__device__ __forceinline__ float attn_gate(const AttnIO & io, int64_t row, int h, int d, int DV) {
-    if (io.gate_mode == 1) return sigmoid_f(io.gate[row * io.ldg + h]);
-    if (io.gate_mode == 2) return sigmoid_f(io.gate[row * io.ldg + (int64_t) h * DV + d]);
-    return 1.f;
-}
-
 __global__ void k_attn_kv_store(const float * qkvg, const int32_t * __restrict__ slot, const int32_t * __restrict__ off,
                                 const int32_t * __restrict__ pos0, const int32_t * __restrict__ entry_of, AttnParams a, float * __restrict__ kcache,
                                 float * __restrict__ vcache, int64_t slot_stride) {
@@ -566,6 +557,7 @@ __global__ void __launch_bounds__(256) k_attn_window_prefill_tiled(const AttnIO 
     }
 }
 
+// What attn_decode.cu does not take (caches below 128 rows, wide or odd heads, many sequences of ungrouped heads):
 // decode: CTA (head, entry, split).  Warp w takes cache rows 4 w .. 4 w + 3 of the split's chunk, then 4 * warps further on, ...: the lanes
 // split the key's dimensions (coalesced row reads, four rows in flight), the score is a warp sum, the running max / sum are uniform over the
 // warp, and every lane accumulates its share of the value dimensions.  The warps' partial softmax states are merged in shared memory.  With
@@ -576,7 +568,6 @@ __global__ void __launch_bounds__(256) k_attn_window_prefill_tiled(const AttnIO 
 // scores are summed.  TIED (a key is its own value, 16-byte rows): the key's registers serve as the value, lane entry 4 c + i of a head being d =
 // 128 c + 4 lane + i.
 constexpr int DEC_WARPS = 16, DEC_ROWS = 4, DEC_SPLIT_WARPS = 8;
-__device__ __forceinline__ int dec_rows_used(const AttnParams & a, int pi) { return min(a.cache_rows, (a.chunk > 0 ? pi % a.chunk : pi) + 1); }   // a chunk's rows start at row 0 of the ring
 template <typename OT, int NV, bool TIED>
 __global__ void __launch_bounds__(DEC_WARPS * 32) k_attn_window_decode(const AttnIO io, const int32_t * __restrict__ slot,
                                                                        const int32_t * __restrict__ off, const int32_t * __restrict__ pos0, AttnParams a,
@@ -1149,6 +1140,10 @@ int launch_attn_decode_io(const AttnIO & io, const BatchView & b, const AttnPara
                           void * out, int otype, cudaStream_t st, float * part) {
     if (b.n_tokens <= 0) return 0;
     if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads != 0 || a.dim <= 0 || a.vdim <= 0) return (int) cudaErrorInvalidValue;
+    if (part && attn_decode_splits(a.cache_rows) > 1) {
+        const int rc = launch_attn_decode_group(io, b, a, kcache, vcache, slot_stride, out, otype, st);
+        if (rc != (int) cudaErrorNotSupported) return rc;
+    }
     const int nv = (a.vdim + 31) / 32;
     if (a.tied_v && kcache == vcache && a.dim <= 128 && a.dim % 4 == 0 && io.k_row % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t) kcache & 15) == 0) {
         if (otype == T_BF16) return attn_decode_typed<__nv_bfloat16, 4, true>(io, b, a, kcache, vcache, slot_stride, (__nv_bfloat16 *) out, part, st);
