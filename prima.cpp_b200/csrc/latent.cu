@@ -10,6 +10,7 @@
 
 #include <algorithm>
 
+#include "latent.cuh"
 #include "layers.h"
 #include "mixers.cuh"
 #include "rows.cuh"
@@ -17,24 +18,7 @@
 namespace pb {
 namespace {
 
-// entries of pair i
-__device__ __forceinline__ void pair_at(const LatentParams & p, int i, int & ia, int & ib) {
-    if (p.rot_layout == ROT_INTERLEAVED) { ia = 2 * i; ib = 2 * i + 1; }
-    else { ia = i; ib = i + p.rot_dims / 2; }
-}
 constexpr int LATENT_ROW_V = 2;   // float4s a thread holds of a latent
-// rotates the pair (u, v) by the angle pos * freq; cos and sin carry the factor mag
-__device__ __forceinline__ void turn(float u, float v, int pos, float f, float mag, float & ou, float & ov) {
-    const float ang = (float) pos * f;
-    const float c = cosf(ang) * mag, s = sinf(ang) * mag;
-    ou = u * c - v * s;
-    ov = v * c + u * s;
-}
-
-// factor on output element (head h, entry dv): sigmoid of the head's gate logit, of the element's, or none
-__device__ __forceinline__ float latent_gate(const LatentParams & p, const float * gate, int64_t at, int h, int dv) {
-    return gate ? sigmoid_f(gate[at + (p.gate_mode == 1 ? h : h * p.vdim + dv)]) : 1.f;
-}
 // turns the rotated part of every query head of one token
 __device__ __forceinline__ void rope_q_row(float * __restrict__ row, int pos, const LatentParams & p, const float * __restrict__ freq) {
     const int half = p.rot_dims / 2, DQ = p.dim + p.rot_dim;

@@ -2182,9 +2182,13 @@ static int mix_latent(pb200_model * m, const BatchView & b, bool prefill, const 
         io.split_ws = ll.split_ws; io.split_bytes = ll.split_bytes;
         CK(launch_attn_prefill_io(io, b, ap, ll.act, ct, st));
     } else if (T == b.n_entries && R <= 512) {   // one token per entry: the key up-projection folded into the query, rows split over CTAs
-        CK(launch_latent_absorb_q(q, ldq, b, wuk, ct, a, L.rot_freq.data, ll.big3, st));
-        CAT(CAT_ATTN);
-        CK(launch_latent_decode(ll.big3, b, a, cache, ll.slot_floats, latent_decode_splits(a.cache_rows), ll.lat_part, wuv, ct, sink, gate, C, ll.act, ct, st));
+        int rc = launch_latent_decode_group(q, ldq, b, wuk, wuv, ct, a, L.rot_freq.data, cache, ll.slot_floats, sink, gate, C, ll.act, st);
+        if (rc == (int) cudaErrorNotSupported) {
+            CK(launch_latent_absorb_q(q, ldq, b, wuk, ct, a, L.rot_freq.data, ll.big3, st));
+            CAT(CAT_ATTN);
+            rc = launch_latent_decode(ll.big3, b, a, cache, ll.slot_floats, latent_decode_splits(a.cache_rows), ll.lat_part, wuv, ct, sink, gate, C, ll.act, ct, st);
+        }
+        CK(rc);
     } else {         // the same through the shared decode kernel: one key / value head, the key is the whole row, the value its latent part
         CK(launch_latent_absorb_q(q, ldq, b, wuk, ct, a, L.rot_freq.data, ll.big3, st));
         CAT(CAT_ATTN);

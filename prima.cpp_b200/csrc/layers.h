@@ -295,6 +295,11 @@ int launch_latent_absorb_q(const float * q, int64_t ldq, const BatchView & b, co
 int launch_latent_up_v(const float * olat, const void * wuv, int wtype, const LatentParams & p, const float * gate, int64_t ldg, void * out, int otype,
                        int n_tokens, cudaStream_t stream);
 
+// both of these and the up-projection in one launch (latent_decode.cu): bf16 weights and output, kv_rank a multiple of 16 up to 512, heads of up to 128 entries;
+// cudaErrorNotSupported otherwise
+int launch_latent_decode_group(const float * q, int64_t ldq, const BatchView & b, const void * wuk, const void * wuv, int wtype, const LatentParams & p, const float * freq,
+                               const float * cache, int64_t slot_stride, const float * sink, const float * gate, int64_t ldg, void * out, cudaStream_t stream);
+
 // decode attention of one-token entries over the slot's rows, split over `splits` CTAs per (entry, 16 heads), then the merge, the
 // value up-projection and the gate (may be null) in a second kernel.  sink (may be null): score per head of one more key in the denominator
 // that has no value.  part: scratch of n_entries * splits * heads * (kv_rank + 2) floats.
