@@ -682,9 +682,13 @@ static int prefill_ubatch(pb200_model * m, const int32_t * tokens_host, const fl
         const bool qkv_fused = pf_tc(L.wq, T) && pf_tc(L.wk, T) && pf_tc(L.wv, T) && is_kquant(L.wq.type) && is_kquant(L.wk.type) && is_kquant(L.wv.type);
         if (qkv_fused) {
             MmqPre pre; pre.kind = 2; pre.aux = L.attn_norm; pre.eps = hp.rms_eps;
-            CK(pf_matmul(m, L.wq, x, T, P.q, L.bq, nullptr, n, nullptr, &pre));
-            CK(pf_matmul(m, L.wk, x, T, P.k, L.bk, nullptr, n, &L.wq));
-            CK(pf_matmul(m, L.wv, x, T, P.v, L.bv, nullptr, n, &L.wk));
+            const MmqDesc d[3] = {{L.wq.type, L.wq.data, L.wq.N, P.q, L.bq}, {L.wk.type, L.wk.data, L.wk.N, P.k, L.bk}, {L.wv.type, L.wv.data, L.wv.N, P.v, L.bv}};
+            const cudaError_t rc = launch_mmq_multi(d, 3, E, x, E, T, P.ws, st, &pre, !no_pdl());
+            if (rc == cudaErrorNotSupported) {
+                CK(pf_matmul(m, L.wq, x, T, P.q, L.bq, nullptr, n, nullptr, &pre));
+                CK(pf_matmul(m, L.wk, x, T, P.k, L.bk, nullptr, n, &L.wq));
+                CK(pf_matmul(m, L.wv, x, T, P.v, L.bv, nullptr, n, &L.wk));
+            } else { CK((int) rc); n += 2; }
         } else {
             CK(launch_rms_norm(x, P.xn, E, T, hp.rms_eps, st, L.attn_norm)); n++;
             CK(pf_matmul(m, L.wq, P.xn, T, P.q, L.bq, nullptr, n));
@@ -703,8 +707,12 @@ static int prefill_ubatch(pb200_model * m, const int32_t * tokens_host, const fl
         // --- FFN block ---
         if (pf_tc(L.gate, T) && pf_tc(L.up, T) && is_kquant(L.gate.type) && is_kquant(L.up.type)) {
             MmqPre pre; pre.kind = 2; pre.aux = L.ffn_norm; pre.eps = hp.rms_eps;
-            CK(pf_matmul(m, L.gate, y, T, P.g, nullptr, nullptr, n, nullptr, &pre));
-            CK(pf_matmul(m, L.up, y, T, P.u, nullptr, nullptr, n, &L.gate));
+            const MmqDesc d[2] = {{L.gate.type, L.gate.data, L.gate.N, P.g, nullptr}, {L.up.type, L.up.data, L.up.N, P.u, nullptr}};
+            const cudaError_t rc = launch_mmq_multi(d, 2, E, y, E, T, P.ws, st, &pre, !no_pdl());
+            if (rc == cudaErrorNotSupported) {
+                CK(pf_matmul(m, L.gate, y, T, P.g, nullptr, nullptr, n, nullptr, &pre));
+                CK(pf_matmul(m, L.up, y, T, P.u, nullptr, nullptr, n, &L.gate));
+            } else { CK((int) rc); n += 2; }
         } else {
             CK(launch_rms_norm(y, P.xn, E, T, hp.rms_eps, st, L.ffn_norm)); n++;
             CK(pf_matmul(m, L.gate, P.xn, T, P.g, nullptr, nullptr, n));

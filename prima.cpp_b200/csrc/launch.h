@@ -141,6 +141,9 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
 // pdl: the kernel in front may be programmatic; the weights, which are then fetched before it ends, must not be its result.
 // resid: [T][N] added in the epilogue (must not alias dst).  reuse_prep: ws already holds this x (same K, T) from the previous launch_mmq
 // on the stream (q|k|v and gate|up share one activation: the q8_K -> fp16 tiling pass runs once)
+// several matrices over one activation in one launch; cudaErrorNotSupported (nothing has been launched): the callers launch them one by one
+struct MmqDesc { int type; const void * W; int64_t N; float * dst; const float * bias; };
+cudaError_t launch_mmq_multi(const MmqDesc * d, int n, int64_t K, const float * x, int64_t ldx, int64_t T, void * ws, cudaStream_t st, const MmqPre * pre, bool pdl);
 int launch_get_rows(const void * table, int type, int K, const int32_t * ids, int n_ids, float * y, cudaStream_t stream, bool pdl);
 
 // element-wise helpers for the plugin

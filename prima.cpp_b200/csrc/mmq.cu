@@ -77,6 +77,19 @@ struct MmqParams {
     uint32_t tmem_cols, idesc;
 };
 
+// Several matrices over one activation in a cut launch: row tiles [rt0, next rt0) belong to a matrix.  `slot` as in MmqParams; `second`: its blocks are of the
+// kernel's second type.
+constexpr int MMQ_MAX_MATS = 3;
+struct MmqMat {
+    const uint8_t * W;
+    float * dst;
+    const float * bias;
+    int64_t row_bytes, total_bytes;
+    int N, rt0, bpb, slot, second;
+};
+template <bool MULTI> struct MmqMats { CUtensorMap map[1]; };
+template <> struct MmqMats<true> { CUtensorMap map[MMQ_MAX_MATS]; MmqMat mat[MMQ_MAX_MATS]; int n; };
+
 struct MmqCtl {
     uint64_t raw_full[3], raw_empty[3];
     uint64_t a_ready[MMQ_A_MAX], b_full[MMQ_B_NST];
@@ -346,8 +359,11 @@ __device__ __forceinline__ void cp_async16(void * smem_dst, const void * gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
 
-template <int TYPE, int CG, bool CUT>
-__global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant__ MmqParams P, const __grid_constant__ CUtensorMap map_w) {
+// TYPE2 > 0 (cut launches): several matrices, whose blocks are of TYPE or TYPE2
+template <int TYPE, int CG, bool CUT, int TYPE2 = 0>
+__global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant__ MmqParams P, const __grid_constant__ MmqMats<(TYPE2 > 0)> mm) {
+    constexpr bool MULTI = TYPE2 > 0, MIXED = MULTI && TYPE2 != TYPE;
+    static_assert(!MULTI || (CUT && CG == 1), "a CTA of a launch of several matrices walks one tile");
     extern __shared__ uint8_t smem_raw[];
     // the swizzle-128B atoms (A and B stages) need 1024-byte alignment in the shared window
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -373,6 +389,15 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         const int units = min(P.chain * P.ngrp, P.total_units - u0), shares = units / P.ngrp + 1;
         w0 = u0 + (int) ((int64_t) units * min(j, shares) / shares);
         w1 = u0 + (int) ((int64_t) units * min(j + 1, shares) / shares);
+    }
+
+    // the matrix: the only one, or that of this CTA's tile
+    MmqMat M{P.W, P.dst, P.bias, P.row_bytes, P.total_bytes, P.N, 0, P.bpb, P.slot, 0};
+    int mi = 0;
+    if constexpr (MULTI) {
+        const int rt = w0 / P.ngrp % P.rtiles;
+        while (mi + 1 < mm.n && rt >= mm.mat[mi + 1].rt0) mi++;
+        M = mm.mat[mi];
     }
 
     if (threadIdx.x == 0) {
@@ -494,8 +519,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
             for (int x = 0; x < nx; x++) {
                 if (x >= P.nraw && !mmq_wait(ctl, &ctl->raw_empty[slot], ph)) break;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&ctl->raw_full[slot], (uint32_t) (MMQ_BM * P.slot));
-                    tma_raw(smem_u32(raw + (size_t) slot * MMQ_BM * P.slot), &map_w, (sb * P.bpb & ~15) >> 1, (rt * CG + (int) rank) * MMQ_BM, smem_u32(&ctl->raw_full[slot]));
+                    mbar_arrive_expect_tx(&ctl->raw_full[slot], (uint32_t) (MMQ_BM * M.slot));
+                    tma_raw(smem_u32(raw + (size_t) slot * MMQ_BM * P.slot), &mm.map[mi], (sb * M.bpb & ~15) >> 1, ((rt - M.rt0) * CG + (int) rank) * MMQ_BM, smem_u32(&ctl->raw_full[slot]));
                 }
                 __syncwarp();
                 if (++slot == P.nraw) { slot = 0; ph ^= 1; }
@@ -508,18 +533,18 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         const int r = dt >> 2, h = (dt >> 1) & 1, hh = dt & 1;
         bool ok = true;
         // this thread fetches its own half of the row's block: 16-byte cp.async pieces of the 16-B aligned window around it
-        const int64_t lim = (P.total_bytes + 15) & ~(int64_t) 15;
-        const int cpr = P.slot >> 4, p_lo = cpr * (dt & 3) / 4, p_hi = cpr * ((dt & 3) + 1) / 4;   // this thread's quarter of the row's window
+        const int64_t lim = (M.total_bytes + 15) & ~(int64_t) 15;
+        const int cpr = M.slot >> 4, p_lo = cpr * (dt & 3) / 4, p_hi = cpr * ((dt & 3) + 1) / 4;   // this thread's quarter of the row's window
         const int nx = w1 - w0;                                 // groups this CTA walks, x = 0 .. nx-1 across its segments
         // fetch cursor: the group nraw-1 ahead of the one being expanded (tile / K group tracked incrementally: no divisions in the loop)
         int f_x = 0, f_sb, f_rt;
         { const int tile = w0 / P.ngrp; f_sb = w0 - tile * P.ngrp; f_rt = tile % P.rtiles; }
         auto fetch_next = [&](int slot) {                       // issues group f_x of this CTA into raw slot `slot`, advances the cursor
-            const int gr = min((f_rt * CG + (int) rank) * MMQ_BM + r, P.N - 1);
-            const int64_t src0 = ((int64_t) gr * P.row_bytes + (int64_t) f_sb * P.bpb) & ~(int64_t) 15;
+            const int gr = min((f_rt * CG + (int) rank) * MMQ_BM + r, M.N - 1);   // never with several matrices: those come by boxes
+            const int64_t src0 = ((int64_t) gr * M.row_bytes + (int64_t) f_sb * M.bpb) & ~(int64_t) 15;
             uint8_t * dst0 = raw + ((size_t) slot * MMQ_BM + r) * P.slot;
             for (int pc = p_lo; pc < p_hi; pc++)
-                if (src0 + pc * 16 + 16 <= lim) cp_async16(dst0 + pc * 16, P.W + src0 + pc * 16);
+                if (src0 + pc * 16 + 16 <= lim) cp_async16(dst0 + pc * 16, M.W + src0 + pc * 16);
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->raw_full[slot])) : "memory");
             f_x++;
             if (++f_sb == P.ngrp) { f_sb = 0; if (++f_rt == P.rtiles) f_rt = 0; }
@@ -533,8 +558,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
         int prs = P.nraw - 1, pph = 1;                          // ... of the group before it (the slot the next fetch goes into)
         for (int w = w0; w < w1 && ok; seg++) {
             const int tile = w / P.ngrp, sbb = w - tile * P.ngrp, sbe = min(P.ngrp, sbb + (w1 - w));
-            const int row0 = ((tile % P.rtiles) * CG + (int) rank) * MMQ_BM;
-            const int gr = min(row0 + r, P.N - 1);
+            const int row0 = ((tile % P.rtiles - M.rt0) * CG + (int) rank) * MMQ_BM;
+            const int gr = min(row0 + r, M.N - 1);
             for (int sb = sbb; sb < sbe && ok; sb++) {
                 // refill the slot the previous group used, once every expansion warp has left it
                 if (!P.tma && f_x < nx) {
@@ -542,22 +567,28 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     fetch_next(prs);
                 }
                 if (!mmq_wait(ctl, &ctl->raw_full[rs], rph)) { ok = false; break; }
-                const int64_t g0 = (int64_t) gr * P.row_bytes + (int64_t) sb * P.bpb;
-                const uint8_t * blk = raw + (size_t) (rs * MMQ_BM + r) * P.slot + (g0 & 15);
+                const int64_t g0 = (int64_t) gr * M.row_bytes + (int64_t) sb * M.bpb;
+                const uint8_t * blk = raw + (size_t) rs * MMQ_BM * P.slot + (size_t) r * M.slot + (g0 & 15);
                 const int nst = min(4, nstep_all - 4 * sb);      // the last group of a K % 256 != 0 row (32-element block types) is short
                 constexpr bool K45 = TYPE == T_Q4_K || TYPE == T_Q5_K;
+                const bool second = MIXED && M.second;           // Q6_K beside Q4_K or Q5_K
                 KGroup<TYPE> kg;
                 if constexpr (K45) {
-                    kg.load(blk, h, hh);
-                    kg.loaded();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
+                    if (!second) {
+                        kg.load(blk, h, hh);
+                        kg.loaded();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     if (c >= nst) break;
                     uint32_t v[8];
-                    if constexpr (K45) kg.expand(c, h, v);
+                    if constexpr (MIXED) {
+                        if (second) expand<TYPE2>(blk, c, h, hh, v);
+                        else kg.expand(c, h, v);
+                    } else if constexpr (K45) kg.expand(c, h, v);
                     else expand<TYPE>(blk, c, h, hh, v);
                     if (g >= P.a_nst) {     // step g - a_nst has consumed this A stage
                         const int f = g - P.a_nst;
@@ -571,7 +602,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     if (lane == 0) mbar_arrive(&ctl->a_ready[g & amask]);
                     g++;
                 }
-                if (!K45) {
+                if (!K45 || second) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&ctl->raw_empty[rs]);
                 }
@@ -587,7 +618,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 const int tt0 = (tile / P.rtiles) * P.nacc, nacc = min(P.nacc, P.ttiles - tt0);
                 const int quad = warp & 3, grp = (warp - MMQ_DQ_WARP0) >> 2, n = row0 + quad * 32 + lane;
                 float * red = reinterpret_cast<float *>(smem) + quad * 32 + lane;
-                const float bias = (P.bias && n < P.N) ? P.bias[n] : 0.f;
+                const float bias = (M.bias && n < M.N) ? M.bias[n] : 0.f;
                 for (int a = 0; a < nacc; a++) {
                     const int t0 = (tt0 + a) * BN, tn = min(BN, P.T - t0);
                     for (int c0 = 16 * grp; c0 < tn && acc_ok; c0 += 64) {
@@ -605,13 +636,13 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                     }
                     __syncwarp();
                     mmq_cluster_sync();
-                    if (n < P.N) {
+                    if (n < M.N) {
                         constexpr int U = 8;                     // tokens of a thread at once, two parts of them on their way: what takes time is the latency
                         const int step = 4 * P.parts;
                         for (int t = part + P.parts * grp; t < tn; t += U * step) {
                             float sum[U], f[2][U];                // bias and residual ride on part 0
 #pragma unroll
-                            for (int i = 0; i < U; i++) sum[i] = P.resid && t + i * step < tn ? P.resid[(size_t) (t0 + t + i * step) * (size_t) P.N + n] : 0.f;
+                            for (int i = 0; i < U; i++) sum[i] = P.resid && t + i * step < tn ? P.resid[(size_t) (t0 + t + i * step) * (size_t) M.N + n] : 0.f;
                             for (int c = 0; c < P.parts; c += 2) {
 #pragma unroll
                                 for (int h = 0; h < 2; h++)
@@ -630,7 +661,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                             }
 #pragma unroll
                             for (int i = 0; i < U; i++)
-                                if (t + i * step < tn) P.dst[(size_t) (t0 + t + i * step) * (size_t) P.N + n] = sum[i];
+                                if (t + i * step < tn) M.dst[(size_t) (t0 + t + i * step) * (size_t) M.N + n] = sum[i];
                         }
                     }
                     __syncwarp();
@@ -650,10 +681,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                 const bool first = sbb == 0, whole = first && sbe == P.ngrp;   // bias / residual ride on the K group 0 segment
                 const int quad = warp & 3;
                 const int n = row0 + quad * 32 + lane;
-                const bool live = acc_ok && n < P.N;
-                const float bias = (P.bias && live && first) ? P.bias[n] : 0.f;
+                const bool live = acc_ok && n < M.N;
+                const float bias = (M.bias && live && first) ? M.bias[n] : 0.f;
                 const float * rp = (P.resid && first && live) ? P.resid + n : nullptr;
-                const size_t ldd = (size_t) P.N;
+                const size_t ldd = (size_t) M.N;
                 for (int ch = (warp - MMQ_DQ_WARP0) >> 2; ch < nch; ch += 4) {
                     const int t0 = tt0 * BN + ch * 16;
                     const int nt = min(16, P.T - t0);            // tokens of the chunk (<= 0: padding only)
@@ -679,7 +710,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) k_mmq_tc(const __grid_constant
                         : "memory");
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (live) {
-                        float * d = P.dst + (size_t) t0 * ldd + n;
+                        float * d = M.dst + (size_t) t0 * ldd + n;
 #pragma unroll
                         for (int i = 0; i < 16; i++) y[i] = __fadd_rn(__fadd_rn(__uint_as_float(v[i]), bias), y[i]);
                         if (whole && nt == 16) {
@@ -853,10 +884,10 @@ bool mmq_supported(int type, int64_t K) {
     return (type == T_Q8_0 || type == T_Q5_1) && K % 64 == 0 && K >= 256;   // 32-element blocks: two per 64-element step
 }
 
-template <int TYPE, int CG, bool CUT>
-static cudaError_t mmq_launch_typed2(const MmqParams & P, const CUtensorMap & map_w, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
+template <int TYPE, int CG, bool CUT, int TYPE2 = 0>
+static cudaError_t mmq_launch_typed2(const MmqParams & P, const MmqMats<(TYPE2 > 0)> & mats, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
     static FuncAttrCache attr_cache;
-    cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT>, smem, false);
+    cudaError_t e = ensure_dyn_smem(attr_cache, (const void *) k_mmq_tc<TYPE, CG, CUT, TYPE2>, smem, false);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -870,10 +901,10 @@ static cudaError_t mmq_launch_typed2(const MmqParams & P, const CUtensorMap & ma
     attr[1].val.clusterDim.x = CUT ? (unsigned) P.parts : CG; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = CG > 1 || CUT ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT>, P, map_w);
+    return cudaLaunchKernelEx(&cfg, k_mmq_tc<TYPE, CG, CUT, TYPE2>, P, mats);
 }
 template <int TYPE>
-static cudaError_t mmq_launch_typed(const MmqParams & P, const CUtensorMap & map_w, int cg, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
+static cudaError_t mmq_launch_typed(const MmqParams & P, const MmqMats<false> & map_w, int cg, dim3 grid, size_t smem, cudaStream_t st, bool pdl) {
     if (P.parts > 1) return mmq_launch_typed2<TYPE, 1, true>(P, map_w, grid, smem, st, pdl);
     return cg == 2 ? mmq_launch_typed2<TYPE, 2, false>(P, map_w, grid, smem, st, pdl) : mmq_launch_typed2<TYPE, 1, false>(P, map_w, grid, smem, st, pdl);
 }
@@ -901,27 +932,78 @@ static int mmq_clusters(int parts, int nsm) {
 // What the order costs: shares for every SM whose sums meet as they arrive took (512 / 64 tokens, then -> now) 20.0 / 11.9 -> 34.1 / 16.6 at
 // 1024 x 4096, 31.4 / 21.0 -> 37.2 / 21.9 at 4096 x 4096, 25.1 / 14.8 -> 32.4 / 18.8 at 3072 x 3072, 74.0 / 54.9 -> 78.3 / 55.1 at 4096 x 14336,
 // 229 / 169 -> 244 / 183 at 8192 x 28672, 175 / 126 -> 183 / 138 at 12800 x 14336; 37.8 / 29.7 -> 28.9 / 19.9 at 2048 x 2048, where tiles stayed whole.
-struct MmqCut { int parts, chain, upc; };
+struct MmqCut { int parts, chain, upc; double us; };
 static int64_t mmq_chain_ctas(int64_t tiles, int m) { return tiles / m * (m + 1) + (tiles % m ? tiles % m + 1 : 0); }
 static MmqCut mmq_pick_cut(int64_t tiles, int ngrp, int nsm, int max_parts, double tokens) {
     const double unit = 3.05, seg = 8.0, tile_us = 128.0 * 512.0 * 4.0 / 6.2e6, clear = 3.0 + (double) tiles * tile_us;
     const int rounds = (int) ((tiles + nsm - 1) / nsm);
-    MmqCut best{1, 0, rounds * ngrp};
+    MmqCut best{1, 0, rounds * ngrp, 0.0};
     double best_us = rounds * (ngrp * unit + seg);
     auto consider = [&](const MmqCut & c, double us) { if (us < best_us) { best_us = us; best = c; } };
     const int upc = std::max((int) ((tiles * ngrp + nsm - 1) / nsm), ngrp - 1);
-    if (upc % ngrp != 0) consider({1, 0, upc}, upc * unit + ((upc + ngrp - 2) / ngrp + 1) * seg + clear);
+    if (upc % ngrp != 0) consider({1, 0, upc, 0.0}, upc * unit + ((upc + ngrp - 2) / ngrp + 1) * seg + clear);
     for (int m = 2; m <= 8; m++)
-        if (mmq_chain_ctas(tiles, m) <= nsm) consider({1, m, 0}, (m * ngrp + m) / (m + 1) * unit + 2 * seg + clear);
+        if (mmq_chain_ctas(tiles, m) <= nsm) consider({1, m, 0, 0.0}, (m * ngrp + m) / (m + 1) * unit + 2 * seg + clear);
     // two halves: by a cluster or a chain of one tile, whichever is the faster one for these tokens; the bits are the same
     const bool pairs = max_parts >= 2 && tiles <= mmq_clusters(2, nsm);
     if (tiles * 2 <= nsm && ngrp >= 2)
-        consider(pairs && 10.0 * tokens <= 3.0 * 512.0 + (double) tiles * tile_us * tokens ? MmqCut{2, 0, 0} : MmqCut{1, 1, 0}, (ngrp + 1) / 2 * unit + seg + std::min(10.0, clear));
+        consider(pairs && 10.0 * tokens <= 3.0 * 512.0 + (double) tiles * tile_us * tokens ? MmqCut{2, 0, 0, 0.0} : MmqCut{1, 1, 0, 0.0}, (ngrp + 1) / 2 * unit + seg + std::min(10.0, clear));
     for (int p = 3; p <= max_parts && p <= ngrp && tiles * p <= nsm; p++) {
         const double us = (ngrp + p - 1) / p * unit + seg + 7.5 + 1.25 * p;
-        if (us < best_us && tiles <= mmq_clusters(p, nsm)) consider({p, 0, 0}, us);
+        if (us < best_us && tiles <= mmq_clusters(p, nsm)) consider({p, 0, 0, 0.0}, us);
     }
+    best.us = best_us;
     return best;
+}
+
+// bytes of one 256-K group of a row, and the 16-byte aligned window reserved for it (Q6_K and Q8_0 rows are not 16-B aligned)
+static int mmq_group_bytes(int type) { return type == T_Q4_K ? BYTES_Q4_K : type == T_Q5_K ? BYTES_Q5_K : type == T_Q6_K ? BYTES_Q6_K : type == T_Q8_0 ? 8 * BYTES_Q8_0 : 8 * BYTES_Q5_1; }
+static int mmq_slot_bytes(int type) { return type == T_Q6_K ? 240 : type == T_Q8_0 ? 288 : mmq_group_bytes(type); }
+// the raw blocks of a matrix by boxes; false: its rows do not lie at multiples of 16 bytes
+static bool mmq_map(CUtensorMap & map, int type, const void * W, int64_t N, int64_t K) {
+    const int64_t row = row_bytes(type, K);
+    const EncodeTiled fn = row % 16 == 0 && ((uintptr_t) W & 15) == 0 ? encode_tiled() : nullptr;
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t) row / 2, (cuuint64_t) N}, strides[1] = {(cuuint64_t) row};   // 16-bit entries: a box is at most 256 of them wide
+    const cuuint32_t box[2] = {(cuuint32_t) mmq_slot_bytes(type) / 2, MMQ_BM}, one[2] = {1, 1};
+    return fn(&map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void *) W, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+static cudaError_t mmq_prepare(int type, const float * x, int64_t ldx, int64_t T, int64_t K, int BN, void * ws, const MmqPre * pre, bool pdl, cudaStream_t st) {
+    const int kind = pre ? pre->kind : 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned) ((T + BN - 1) / BN * BN), kind != 2 && K >= 32 * 256 ? 2 : 1);   // long rows over two CTAs (a norm wants the whole row)
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_mmq_prep, x, ldx, (int) T, (int) K, BN, (uint8_t *) ws, is_kquant(type) ? 0 : 1, kind, pre ? pre->aux : (const float *) nullptr,
+                              pre ? pre->ld_aux : (int64_t) 0, pre ? pre->eps : 0.f);
+}
+// P's tensor memory, instruction and ring depths; returns the shared memory, 0: more than there is.  3 raw super-block slots (HBM latency) if they fit, and as many
+// activation stages (2..4) as the 227 KB budget leaves; 4 expanded-weight stages when a CTA pair halves the activation stages (the handshake "MMA
+// done -> store the next tile -> MMA" then has three MMA steps of slack instead of one), else 2
+static size_t mmq_rings(MmqParams & P, int cg) {
+    uint32_t cols = 32;
+    while ((int) cols < P.BN) cols <<= 1;
+    P.tmem_cols = P.nacc == 2 ? 512 : cols;
+    // kind::f16 instruction descriptor (cute/arch/mma_sm100_desc.hpp InstrDescriptor): D=f32, A=B=f16, both K-major, N>>3, M>>4
+    P.idesc = (1u << 4) | ((uint32_t) (P.BN >> 3) << 17) | ((uint32_t) ((MMQ_BM * cg) >> 4) << 24);
+    auto smem_for = [&](int nraw, int b_nst) {
+        return 1024 + (size_t) P.a_nst * MMQ_A_BYTES + (size_t) b_nst * P.nacc * (P.BN / cg) * 128 + (size_t) nraw * MMQ_BM * P.slot + MMQ_CTL_BYTES;
+    };
+    static const int force_a = getenv("PB200_MMQ_A_NST") ? atoi(getenv("PB200_MMQ_A_NST")) : 0;
+    P.a_nst = force_a == 2 || force_a == 4 ? force_a : (cg == 2 ? 4 : 2);
+    P.nraw = 3;
+    if (smem_for(3, 2) > 232448) P.nraw = 2;
+    if (smem_for(P.nraw, 2) > 232448) P.a_nst = 2;
+    P.b_nst = MMQ_B_NST;
+    while (P.b_nst > 2 && smem_for(P.nraw, P.b_nst) > 232448) P.b_nst--;
+    const size_t smem = smem_for(P.nraw, P.b_nst);
+    return smem > 232448 ? 0 : smem;
 }
 
 cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const float * x, int64_t ldx, int64_t T, float * dst, const float * bias,
@@ -944,9 +1026,8 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     P.K = (int) K;
     P.T = (int) T;
     P.BN = BN;
-    // bytes of one 256-K group of a row, and the 16-byte aligned window reserved for it (Q6_K and Q8_0 rows are not 16-B aligned)
-    P.bpb = type == T_Q4_K ? BYTES_Q4_K : type == T_Q5_K ? BYTES_Q5_K : type == T_Q6_K ? BYTES_Q6_K : type == T_Q8_0 ? 8 * BYTES_Q8_0 : 8 * BYTES_Q5_1;
-    P.slot = type == T_Q6_K ? 240 : (type == T_Q8_0 ? 288 : P.bpb);
+    P.bpb = mmq_group_bytes(type);
+    P.slot = mmq_slot_bytes(type);
     P.ttiles = tpad / BN;
     // CTA pairs (tcgen05 cta_group::2, PB200_MMQ_CG=2): two row tiles form one M = 256 MMA, each CTA stages only half of the activation tile
     // (L2 -> SM traffic halves, room for 4 expanded-weight stages).  Built and measured: parity green, but 5-7 % SLOWER than one CTA per
@@ -968,43 +1049,14 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
     if (total > 0x7fffffff) return cudaErrorInvalidValue;
     P.total_units = (int) total;
     if (!reuse_prep) {
-        const int kind = pre ? pre->kind : 0;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned) tpad, kind != 2 && K >= 32 * 256 ? 2 : 1);   // long rows over two CTAs (a norm wants the whole row)
-        cfg.blockDim = dim3(256);
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e0 = cudaLaunchKernelEx(&cfg, k_mmq_prep, x, ldx, (int) T, (int) K, BN, (uint8_t *) ws, is_kquant(type) ? 0 : 1, kind, pre ? pre->aux : (const float *) nullptr,
-                                                  pre ? pre->ld_aux : (int64_t) 0, pre ? pre->eps : 0.f);
+        const cudaError_t e0 = mmq_prepare(type, x, ldx, T, K, BN, ws, pre, pdl, st);
         if (e0 != cudaSuccess) return e0;
     }
-    uint32_t cols = 32;
-    while ((int) cols < BN) cols <<= 1;
-    P.tmem_cols = P.nacc == 2 ? 512 : cols;
-    // kind::f16 instruction descriptor (cute/arch/mma_sm100_desc.hpp InstrDescriptor): D=f32, A=B=f16, both K-major, N>>3, M>>4
-    P.idesc = (1u << 4) | ((uint32_t) (BN >> 3) << 17) | ((uint32_t) ((MMQ_BM * cg) >> 4) << 24);
-    // ring depths: 3 raw super-block slots (HBM latency) if they fit, and as many activation stages (2..4) as the 227 KB budget leaves
-    auto smem_for = [&](int nraw, int b_nst) {
-        return 1024 + (size_t) P.a_nst * MMQ_A_BYTES + (size_t) b_nst * P.nacc * (BN / cg) * 128 + (size_t) nraw * MMQ_BM * P.slot + MMQ_CTL_BYTES;
-    };
-    // 4 expanded-weight stages when a CTA pair halves the activation stages (the handshake "MMA done -> store the next tile -> MMA" then
-    // has three MMA steps of slack instead of one), else 2; 3 raw slots if they fit; then as many activation stages (2..4) as are left
-    static const int force_a = getenv("PB200_MMQ_A_NST") ? atoi(getenv("PB200_MMQ_A_NST")) : 0;
-    P.a_nst = force_a == 2 || force_a == 4 ? force_a : (cg == 2 ? 4 : 2);
-    P.nraw = 3;
-    if (smem_for(3, 2) > 232448) P.nraw = 2;
-    if (smem_for(P.nraw, 2) > 232448) P.a_nst = 2;
-    P.b_nst = MMQ_B_NST;
-    while (P.b_nst > 2 && smem_for(P.nraw, P.b_nst) > 232448) P.b_nst--;
-    const size_t smem = smem_for(P.nraw, P.b_nst);
-    if (smem > 232448) return cudaErrorInvalidConfiguration;
+    const size_t smem = mmq_rings(P, cg);
+    if (smem == 0) return cudaErrorInvalidConfiguration;
     const int nsm = sm_count() / cg;           // CTAs (pairs) that can be resident: one CTA per SM
     MmqCut cut = mmq_pick_cut(tiles, P.ngrp, nsm, cg == 1 && (size_t) MMQ_BM * BN * 4 <= smem - 1024 - MMQ_CTL_BYTES ? MMQ_MAX_PARTS : 1, (double) std::min<int64_t>(T, 512));
-    if (whole_tiles) cut = {1, 0, P.ngrp};
+    if (whole_tiles) cut = {1, 0, P.ngrp, 0.0};
     P.parts = cut.parts;
     P.chain = cut.chain;
     P.upc = cut.upc;
@@ -1012,20 +1064,73 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
         cudaError_t e0 = cudaMemsetAsync(dst, 0, (size_t) T * (size_t) N * sizeof(float), st);
         if (e0 != cudaSuccess) return e0;
     }
-    CUtensorMap map_w{};
-    if (P.row_bytes % 16 == 0 && ((uintptr_t) W & 15) == 0) {   // 16-bit entries: a box is at most 256 of them wide
-        const EncodeTiled fn = encode_tiled();
-        const cuuint64_t dims[2] = {(cuuint64_t) P.row_bytes / 2, (cuuint64_t) N}, strides[1] = {(cuuint64_t) P.row_bytes};
-        const cuuint32_t box[2] = {(cuuint32_t) P.slot / 2, MMQ_BM}, one[2] = {1, 1};
-        P.tma = fn && fn(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void *) W, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
+    MmqMats<false> map_w{};
+    P.tma = mmq_map(map_w.map[0], type, W, N, K);
     dim3 grid((unsigned) (cut.parts > 1 ? tiles * cut.parts : cg * (cut.chain > 0 ? mmq_chain_ctas(tiles, cut.chain) : (total + cut.upc - 1) / cut.upc)), 1, 1);
     if (type == T_Q4_K) return mmq_launch_typed<T_Q4_K>(P, map_w, cg, grid, smem, st, pdl);
     if (type == T_Q5_K) return mmq_launch_typed<T_Q5_K>(P, map_w, cg, grid, smem, st, pdl);
     if (type == T_Q6_K) return mmq_launch_typed<T_Q6_K>(P, map_w, cg, grid, smem, st, pdl);
     if (type == T_Q8_0) return mmq_launch_typed<T_Q8_0>(P, map_w, cg, grid, smem, st, pdl);
     return mmq_launch_typed<T_Q5_1>(P, map_w, cg, grid, smem, st, pdl);
+}
+
+// d: up to three k-quant matrices with K columns over the activation x, of one type, or of two where one is Q6_K.  One after the other each of them has a
+// few tiles to cut into many parts, whose joins and starts take most of the time, and waits for the one in front; together they take a launch.  Not
+// supported: where the tiles of all are too many for clusters, or the launches one by one are the faster way by mmq_pick_cut's costs.
+// 512 tokens, K 4096, rows 4096 + 1024 + 1024, us: one by one 86, together 42.
+cudaError_t launch_mmq_multi(const MmqDesc * d, int n, int64_t K, const float * x, int64_t ldx, int64_t T, void * ws, cudaStream_t st, const MmqPre * pre, bool pdl) {
+    if (n < 2 || n > MMQ_MAX_MATS || T <= 0 || K % 256 || K < 256) return cudaErrorNotSupported;
+    if (pre && pre->kind != 0 && (!pre->aux || pre->kind < 0 || pre->kind > 2)) return cudaErrorInvalidValue;
+    int type = d[0].type, type2 = 0;
+    for (int i = 0; i < n; i++) {
+        if (!is_kquant(d[i].type) || d[i].N <= 0) return cudaErrorNotSupported;
+        if (d[i].type != T_Q6_K) type = d[i].type;
+    }
+    for (int i = 0; i < n; i++)
+        if (d[i].type != type) {
+            if (d[i].type != T_Q6_K) return cudaErrorNotSupported;
+            type2 = T_Q6_K;
+        }
+    MmqParams P{};
+    MmqMats<true> mats{};
+    mats.n = n;
+    P.abort_flag = abort_flag();
+    P.B = (const uint8_t *) ws;
+    P.K = (int) K;
+    P.T = (int) T;
+    P.BN = mmq_pick_bn((int) T);
+    P.ttiles = (int) ((T + P.BN - 1) / P.BN);
+    P.nacc = P.ttiles >= 2 ? 2 : 1;
+    P.ngrp = (int) (K / 256);
+    P.tma = 1;
+    const int tgroups = (P.ttiles + P.nacc - 1) / P.nacc, nsm = sm_count();
+    const double tokens = (double) std::min<int64_t>(T, 512);
+    double apart = 0.0;
+    for (int i = 0; i < n; i++) {
+        MmqMat & M = mats.mat[i];
+        M = MmqMat{(const uint8_t *) d[i].W, d[i].dst, d[i].bias, row_bytes(d[i].type, K), row_bytes(d[i].type, K) * d[i].N, (int) d[i].N, P.rtiles, mmq_group_bytes(d[i].type),
+                   mmq_slot_bytes(d[i].type), type2 && d[i].type == type2 ? 1 : 0};
+        const int rt = (int) ((d[i].N + MMQ_BM - 1) / MMQ_BM);
+        P.rtiles += rt;
+        P.slot = std::max(P.slot, M.slot);
+        apart += mmq_pick_cut((int64_t) rt * tgroups, P.ngrp, nsm, MMQ_MAX_PARTS, tokens).us;
+        if (!mmq_map(mats.map[i], d[i].type, d[i].W, d[i].N, K)) return cudaErrorNotSupported;
+    }
+    const int64_t tiles = (int64_t) P.rtiles * tgroups;
+    if (tiles * P.ngrp > 0x7fffffff) return cudaErrorNotSupported;
+    P.total_units = (int) (tiles * P.ngrp);
+    const size_t smem = mmq_rings(P, 1);
+    if (smem == 0 || (size_t) MMQ_BM * P.BN * 4 > smem - 1024 - MMQ_CTL_BYTES) return cudaErrorNotSupported;
+    MmqCut cut = mmq_pick_cut(tiles, P.ngrp, nsm, MMQ_MAX_PARTS, tokens);
+    if (cut.parts == 1 && cut.chain == 1 && tiles <= mmq_clusters(2, nsm)) cut.parts = 2;   // halves by a cluster: the same bits
+    if (cut.parts < 2 || cut.us >= apart) return cudaErrorNotSupported;
+    P.parts = cut.parts;
+    const cudaError_t e = mmq_prepare(type, x, ldx, T, K, P.BN, ws, pre, pdl, st);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned) (tiles * cut.parts));
+    if (type == T_Q4_K) return type2 ? mmq_launch_typed2<T_Q4_K, 1, true, T_Q6_K>(P, mats, grid, smem, st, pdl) : mmq_launch_typed2<T_Q4_K, 1, true, T_Q4_K>(P, mats, grid, smem, st, pdl);
+    if (type == T_Q5_K) return type2 ? mmq_launch_typed2<T_Q5_K, 1, true, T_Q6_K>(P, mats, grid, smem, st, pdl) : mmq_launch_typed2<T_Q5_K, 1, true, T_Q5_K>(P, mats, grid, smem, st, pdl);
+    return mmq_launch_typed2<T_Q6_K, 1, true, T_Q6_K>(P, mats, grid, smem, st, pdl);
 }
 
 }  // namespace pb
