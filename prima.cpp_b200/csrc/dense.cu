@@ -22,7 +22,7 @@ int launch_dense_tc(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * 
                     DenseAct act = DenseAct());   // dense_tc.cu
 bool dense_tc_ok(int T, int N, int K, int64_t lda, int64_t ldw, const void * A, const void * W);
 int launch_dense_tc_grouped(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, int64_t w_stride, float * C, int64_t ldc,
-                            const int32_t * start, const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st);
+                            const int32_t * start, const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st, DenseAct act);
 
 namespace {
 
@@ -318,9 +318,9 @@ int dense_grouped_ok(int type, int N, int K, int64_t lda, int64_t ldw, int64_t w
     return type == T_BF16 && w_stride % 8 == 0 && dense_tc_ok(1, N, K, lda, ldw, A, W) ? 1 : 0;
 }
 int launch_dense_grouped(int type, const void * A, int64_t lda, const void * W, int64_t ldw, int64_t w_stride, float * C, int64_t ldc, const int32_t * start,
-                         const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st) {
-    if (!dense_grouped_ok(type, N, K, lda, ldw, w_stride, A, W)) return (int) cudaErrorInvalidValue;
-    return launch_dense_tc_grouped((const __nv_bfloat16 *) A, lda, (const __nv_bfloat16 *) W, ldw, w_stride, C, ldc, start, count, groups, max_rows, N, K, st);
+                         const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st, const DenseAct & act) {
+    if (!dense_grouped_ok(type, N, K, lda, ldw, w_stride, A, W) || act.xielu || act.silu_glu) return (int) cudaErrorInvalidValue;
+    return launch_dense_tc_grouped((const __nv_bfloat16 *) A, lda, (const __nv_bfloat16 *) W, ldw, w_stride, C, ldc, start, count, groups, max_rows, N, K, st, act);
 }
 
 int launch_dense_planes(int type, const void * A, int64_t a_plane, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int planes, int T, int N,
@@ -347,7 +347,8 @@ int launch_dense_planes(int type, const void * A, int64_t a_plane, int64_t lda, 
 
 int launch_dense_act(int type, const void * A, int64_t lda, const void * W, int64_t ldw, const DenseAct & act, int T, int N, int K, cudaStream_t st) {
     if (T <= 0 || N <= 0) return 0;
-    if (K <= 0 || !A || !W || (!act.xielu && !act.silu_glu) || (act.silu_glu && (act.xielu || N % 2)) || !act.y || (type != 0 && type != T_BF16)) return (int) cudaErrorInvalidValue;
+    if (act.relu2 && !(type == T_BF16 && T > rows_max_t() && dense_tc_ok(T, N, K, lda, ldw, A, W))) return (int) cudaErrorInvalidValue;
+    if (K <= 0 || !A || !W || (!act.xielu && !act.silu_glu && !act.relu2) || (act.silu_glu && (act.xielu || N % 2)) || !act.y || (type != 0 && type != T_BF16)) return (int) cudaErrorInvalidValue;
     if (type == 0) return dense_typed<float>((const float *) A, lda, (const float *) W, ldw, nullptr, 0, T, N, K, nullptr, nullptr, 0, 1.f, st, 0, 0, act);
     const __nv_bfloat16 * a = (const __nv_bfloat16 *) A, * w = (const __nv_bfloat16 *) W;
     if (T > rows_max_t() && dense_tc_ok(T, N, K, lda, ldw, A, W)) return launch_dense_tc(a, lda, w, ldw, nullptr, 0, T, N, K, nullptr, nullptr, 0, 1.f, st, 0, 0, act);

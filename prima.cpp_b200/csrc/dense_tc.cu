@@ -60,7 +60,9 @@ struct TcParams {
 // every load behind a store would wait for it.
 struct Finish {
     float bias, xp, xn;
-    __device__ __forceinline__ Finish(const TcParams & P, int n) {
+    int y0;   // grouped: row of act.y of the group's first token
+    __device__ __forceinline__ Finish(const TcParams & P, int n, int first = 0) {
+        y0 = first;
         bias = (P.bias && n < P.N) ? P.bias[n] : 0.f;
         xp = P.act.xielu ? softplus_f(P.act.xielu[0]) : 0.f;
         xn = P.act.xielu ? 0.5f + softplus_f(P.act.xielu[1]) : 0.f;
@@ -82,6 +84,16 @@ struct Finish {
             return;
         }
         if (n >= P.N) return;
+        if (P.act.relu2) {
+            __nv_bfloat16 * y = (__nv_bfloat16 *) P.act.y + (int64_t) (y0 + t) * P.act.ldy + n;
+#pragma unroll
+            for (int i = 0; i < NT; i++, y += P.act.ldy)
+                if (FULL || t + i < Tn) {
+                    const float r = fmaxf(fmaf(P.alpha, v[i], bias), 0.f);
+                    *y = __float2bfloat16_rn(r * r);
+                }
+            return;
+        }
         if (P.act.xielu) {
             __nv_bfloat16 * y = (__nv_bfloat16 *) P.act.y + (int64_t) t * P.act.ldy + n;
 #pragma unroll
@@ -216,7 +228,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     fence_after();
     {
         const int quad = warp & 3, half = warp >> 2, r = quad * 32 + lane, n = n0 + r;
-        const Finish finish(P, n);
+        const Finish finish(P, n, a_row0);
         const uint32_t tq = tmem + ((uint32_t) (quad * 32) << 16);
         constexpr int HC = BN >= 32 ? BN / 2 : BN;   // columns per warp: halves of the tile, or all of a 16-token tile for the first four warps
         const int c_lo = half * HC, c_hi = c_lo + HC;
@@ -490,10 +502,10 @@ int launch_dense_tc(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * 
 }
 
 int launch_dense_tc_grouped(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, int64_t w_stride, float * C, int64_t ldc,
-                            const int32_t * start, const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st) {
+                            const int32_t * start, const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t st, DenseAct act) {
     if (groups <= 0 || max_rows <= 0) return 0;
     // T bounds the grid only (all groups together hold max_rows rows); the kernel reads each group's own count
-    TcParams P{C, ldc, nullptr, nullptr, 0, 1.f, max_rows, N, K, abort_flag(), start, count, groups, 0, 1, 0, 0, DenseAct()};
+    TcParams P{C, ldc, nullptr, nullptr, 0, 1.f, max_rows, N, K, abort_flag(), start, count, groups, 0, 1, 0, 0, act};
     const TcOperands o{A, lda, max_rows, 1, 0, W, ldw, N, groups, w_stride};
     const TcPlan p = plan_tc((max_rows + groups - 1) / groups, groups, N, K, 0);   // the tile follows the expected rows of a group
     P.splits = 1;

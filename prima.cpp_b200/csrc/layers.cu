@@ -2051,6 +2051,17 @@ static int tap_prepare(pb200_model * m, int T) {
     return 0;
 }
 
+// the second stream goes on from where the first one is
+static int fork_side(pb200_model * m) {
+    LayerList & ll = *m->ll;
+    if (!ll.side) {
+        CK(cudaStreamCreateWithFlags(&ll.side, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&ll.ev_fork, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ll.ev_join, cudaEventDisableTiming));
+    }
+    CK(cudaEventRecord(ll.ev_fork, m->stream));
+    return (int) cudaStreamWaitEvent(ll.side, ll.ev_fork, 0);
+}
 // C[t] = W h (+ bias), or its activation, h = the sublayer's normed input: ll.act, or still to be made from the stream (norm_ahead)
 static int stream_product(pb200_model * m, int T, const DenseW & w, int N, float * C, const float * bias, const DenseAct * act) {
     LayerList & ll = *m->ll;
@@ -2296,14 +2307,8 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
     const bool forked = !ll.prof_on && !one_stream;
     cudaStream_t rst = st;
     if (forked) {
-        if (!ll.side) {
-            CK(cudaStreamCreateWithFlags(&ll.side, cudaStreamNonBlocking));
-            CK(cudaEventCreateWithFlags(&ll.ev_fork, cudaEventDisableTiming));
-            CK(cudaEventCreateWithFlags(&ll.ev_join, cudaEventDisableTiming));
-        }
+        CK(fork_side(m));
         rst = ll.side;
-        CK(cudaEventRecord(ll.ev_fork, st));
-        CK(cudaStreamWaitEvent(rst, ll.ev_fork, 0));
     }
     const float * r_gate = d.rec == REC_DELTA ? ll.big + d.c_rg : nullptr;   // gate logits of the recurrence's result
     int64_t ldrg = C;
@@ -2408,14 +2413,19 @@ static int ff_clamped(pb200_model * m, int T, const DenseW & gateup, const Dense
     return launch_dense(ct, ll.act2, ff, down.data, ff, x, W, T, W, ff, nullptr, x, W, 1.f, st);
 }
 // ---- squared-ReLU feed-forward: out[t] = down(max(up(ll.act[t]), 0)^2); ll.act stays as it is ----
-static int ff_relu2(pb200_model * m, int T, const DenseW & up, const DenseW & down, int ff, float * out) {
+static int ff_relu2(pb200_model * m, int T, const DenseW & up, const DenseW & down, int ff, float * out, cudaStream_t st) {
     LayerList & ll = *m->ll;
-    cudaStream_t st = m->stream;
     const int W = ll.width, ct = ll.ctype;
     CAT(CAT_DENSE);
-    CK(launch_dense(ct, ll.act, W, up.data, W, ll.big, ff, T, ff, W, nullptr, nullptr, 0, 1.f, st));
-    CAT(CAT_ELEM);
-    CK(launch_relu2(ll.big, ll.act2, ct, (int64_t) T * ff, st));
+    if (dense_uses_tensor_cores(ct, T, ff, W, W, W)) {   // the activation is the up product's epilogue
+        DenseAct act;
+        act.relu2 = 1; act.y = ll.act2; act.ldy = ff;
+        CK(launch_dense_act(ct, ll.act, W, up.data, W, act, T, ff, W, st));
+    } else {
+        CK(launch_dense(ct, ll.act, W, up.data, W, ll.big, ff, T, ff, W, nullptr, nullptr, 0, 1.f, st));
+        CAT(CAT_ELEM);
+        CK(launch_relu2(ll.big, ll.act2, ct, (int64_t) T * ff, st));
+    }
     CAT(CAT_DENSE);
     return launch_dense(ct, ll.act2, ff, down.data, ff, out, W, T, W, ff, nullptr, nullptr, 0, 1.f, st);
 }
@@ -2471,12 +2481,21 @@ static int ff_moe(pb200_model * m, int T, bool prefill, LLayer & L, float * x, b
     int base = MOE_ADD;
     const float * xscale = nullptr;
     CAT(CAT_MOE);
+    bool forked = false;
     if (L.route == ROUTE_SIGMOID_GROUPS) {
+        if (L.shared_ff > 0 && p.act == 1 && !accumulate && prefill && (int64_t) T * p.top > 64 && !ll.prof_on) {
+            // a prompt's shared expert, on the second stream beside the choice and the sorting, which leave most SMs idle
+            CK(fork_side(m));
+            forked = true;
+            const PdlScope plain(false);   // the first kernel behind an event of another stream has two dependencies
+            CK(ff_relu2(m, T, L.s_gateup, L.s_down, L.shared_ff, x, ll.side));
+            CK(cudaEventRecord(ll.ev_join, ll.side));
+        }
         CK(launch_moe_route_sigmoid(ll.act, ct, L.router.data, L.router_b.data, p, W, L.shared_ff > 0 ? L.shared_gate.data : nullptr, ll.moe_idx, ll.moe_wt, ll.moe_sg, T, st));
         if (accumulate) return PB200_ENOTSUP;
         if (L.shared_ff > 0) {   // the shared expert's result waits in x; the kernel that sums the experts multiplies it by the token's gate
-            if (p.act == 1) CK(ff_relu2(m, T, L.s_gateup, L.s_down, L.shared_ff, x));
-            else return PB200_ENOTSUP;
+            if (p.act != 1) return PB200_ENOTSUP;
+            if (!forked) CK(ff_relu2(m, T, L.s_gateup, L.s_down, L.shared_ff, x, st));
             base = MOE_SCALE;
             xscale = ll.moe_sg;
         } else {
@@ -2509,9 +2528,13 @@ static int ff_moe(pb200_model * m, int T, bool prefill, LLayer & L, float * x, b
     if (dense_grouped_ok(ct, UR, W, W, W, (int64_t) UR * W, ll.moe_hs, L.e_gateup.data) &&
         dense_grouped_ok(ct, W, p.ff, p.ff, p.ff, (int64_t) W * p.ff, ll.moe_y, L.e_down.data)) {
         // all experts in one launch each way; the row counts never leave the device
-        CK(launch_dense_grouped(ct, ll.moe_hs, W, L.e_gateup.data, W, (int64_t) UR * W, ll.moe_gu, UR, ll.moe_start, ll.moe_count, E, P, UR, W, st));
-        CK(activate(P));
+        DenseAct act;
+        if (p.act == 1) { act.relu2 = 1; act.y = ll.moe_y; act.ldy = p.ff; }   // the activation is the product's epilogue
+        CK(launch_dense_grouped(ct, ll.moe_hs, W, L.e_gateup.data, W, (int64_t) UR * W, ll.moe_gu, UR, ll.moe_start, ll.moe_count, E, P, UR, W, st, act));
+        if (p.act != 1) CK(activate(P));
         CK(launch_dense_grouped(ct, ll.moe_y, p.ff, L.e_down.data, p.ff, (int64_t) W * p.ff, ll.moe_ds, W, ll.moe_start, ll.moe_count, E, P, W, p.ff, st));
+        if (forked) CK(cudaStreamWaitEvent(st, ll.ev_join, 0));
+        const PdlScope joined(g_pdl && !forked);
         return launch_moe_combine(ll.moe_ds, ll.moe_perm, ll.moe_row_of, sum_wt, p.top, W, x, T, st, base, xscale, out_scale);
     }
     CK(cudaMemcpyAsync(ll.moe_count_host, ll.moe_count, (size_t) E * 4, cudaMemcpyDeviceToHost, st));
@@ -2527,6 +2550,8 @@ static int ff_moe(pb200_model * m, int T, bool prefill, LLayer & L, float * x, b
         if (cnt[e] > 0)
             CK(launch_dense(ct, (const uint8_t *) ll.moe_y + (size_t) start[e] * p.ff * es, p.ff, (const uint8_t *) L.e_down.data + (size_t) e * W * p.ff * es, p.ff,
                             ll.moe_ds + (int64_t) start[e] * W, W, cnt[e], W, p.ff, nullptr, nullptr, 0, 1.f, st));
+    if (forked) CK(cudaStreamWaitEvent(st, ll.ev_join, 0));
+    const PdlScope joined(g_pdl && !forked);
     return launch_moe_combine(ll.moe_ds, ll.moe_perm, ll.moe_row_of, sum_wt, p.top, W, x, T, st, base, xscale, out_scale);
 }
 
@@ -2548,7 +2573,7 @@ static int ll_forward_postnorm(pb200_model * m, const BatchView & b, bool prefil
         CK(launch_layernorm_affine_residual(ll.msub, L.norm1.data, L.norm1_bias.data, ll.resid_mult, ll.eps, ll.x, (last && L.ff <= 0) ? nullptr : ll.act, ct, T, W, st));
         if (L.ff > 0) {
             if (L.ff_kind == FF_MOE) CK(ff_moe(m, T, prefill, L, ll.msub, false));
-            else if (L.ff_kind == FF_RELU2) CK(ff_relu2(m, T, L.gateup, L.down, L.ff, ll.msub));
+            else if (L.ff_kind == FF_RELU2) CK(ff_relu2(m, T, L.gateup, L.down, L.ff, ll.msub, m->stream));
             else return PB200_ENOTSUP;
             CAT(CAT_NORM);
             CK(launch_layernorm_affine_residual(ll.msub, L.norm2.data, L.norm2_bias.data, ll.resid_mult, ll.eps, ll.x, last ? nullptr : ll.act, ct, T, W, st));

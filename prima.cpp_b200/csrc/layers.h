@@ -49,10 +49,12 @@ int launch_dense(int type, const void * A, int64_t lda, const void * W, int64_t 
 int dense_grouped_ok(int type, int N, int K, int64_t lda, int64_t ldw, int64_t w_stride, const void * A, const void * W);
 // Epilogue of a product that feeds another one, instead of C[t][n], in the operand type:
 //   xielu (the activation's two numbers, device):  y[t * ldy + n] = xielu(C[t][n])
+//   relu2:  y[t * ldy + n] = max(C[t][n], 0)^2      (tensor-core kernels)
 //   silu_glu (rows 2j of W are gates, rows 2j + 1 the values beside them):  y[t * ldy + j] = silu(C[t][2j]) * C[t][2j + 1]
 struct DenseAct {
     const float * xielu = nullptr;
     int silu_glu = 0;
+    int relu2 = 0;
     void * y = nullptr;
     int64_t ldy = 0;
 };
@@ -69,7 +71,7 @@ int launch_dense_act(int type, const void * A, int64_t lda, const void * W, int6
 int launch_dense_planes(int type, const void * A, int64_t a_plane, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int planes, int T, int N,
                         int K, cudaStream_t stream);
 int launch_dense_grouped(int type, const void * A, int64_t lda, const void * W, int64_t ldw, int64_t w_stride, float * C, int64_t ldc, const int32_t * start,
-                         const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t stream);
+                         const int32_t * count, int groups, int max_rows, int N, int K, cudaStream_t stream, const DenseAct & act = DenseAct());
 // 1: the tensor-core kernel takes this shape (bf16, aligned K / strides); informational (bench, tests)
 int dense_uses_tensor_cores(int type, int T, int N, int K, int64_t lda, int64_t ldw);
 
