@@ -388,8 +388,67 @@ __global__ void __launch_bounds__(DS_COLS / 2 * (N / DS_NREG) + DB_PRODUCERS) k_
     }
 }
 
+// ---- one token per entry ----
+// CTA = one head x 32 value columns of one entry, a lane to a column, a warp to N / 8 key entries: the state comes and goes in whole lines, all of a thread's loads at
+// once, and the two sums over the keys meet in shared memory.  Bound: the state's way from memory and back.  16 heads of 128 x 128, us: one entry 4.0 with the scan
+// above, 2.4 here; eight (17 MB) 18.7, 5.2.
+constexpr int DT_WARPS = 8;
+template <int N>
+__global__ void __launch_bounds__(DT_WARPS * 32) k_delta_token(GatedLinIO io, const int32_t * __restrict__ slot, const int32_t * __restrict__ off, GatedLinParams p,
+                                                               float * state, int64_t slot_stride, float * y) {
+    constexpr int ROWS = N / DT_WARPS;
+    __shared__ float ks[N], gs[N], qs[N], part[2][DT_WARPS][32];
+    pdl_enter();
+    const int P = p.vdim, ptiles = (P + 31) / 32, h = blockIdx.x / ptiles, pt = blockIdx.x - h * ptiles, e = blockIdx.y, hk = h / (p.heads / p.qk_heads);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col = pt * 32 + lane;
+    const bool ok = col < P;
+    const int64_t t = off[e];
+    float * S0 = state + (int64_t) slot[e] * slot_stride + ((int64_t) h * N + warp * ROWS) * P + col;
+    float S[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) S[i] = ok ? S0[(int64_t) i * P] : 0.f;
+    for (int i = tid; i < N; i += DT_WARPS * 32) {
+        ks[i] = io.k[t * io.ldk + hk * N + i];
+        gs[i] = io.decay[t * io.ldd + h * N + i];
+        qs[i] = io.q[t * io.ldq + hk * N + i];
+    }
+    const float v = ok ? io.v[t * io.ldv + h * P + col] : 0.f, beta = io.beta[t * io.ldb + h];
+    __syncthreads();
+    float x = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+        S[i] *= gs[warp * ROWS + i];
+        x = fmaf(S[i], ks[warp * ROWS + i], x);
+    }
+    part[0][warp][lane] = x;
+    __syncthreads();
+    x = 0.f;
+#pragma unroll
+    for (int w = 0; w < DT_WARPS; w++) x += part[0][w][lane];
+    const float u = beta * (v - x);
+    float o = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+        S[i] = fmaf(ks[warp * ROWS + i], u, S[i]);
+        o = fmaf(S[i], qs[warp * ROWS + i], o);
+        if (ok) S0[(int64_t) i * P] = S[i];
+    }
+    part[1][warp][lane] = o;
+    __syncthreads();
+    if (warp == 0 && ok) {
+        o = 0.f;
+#pragma unroll
+        for (int w = 0; w < DT_WARPS; w++) o += part[1][w][lane];
+        y[t * ((int64_t) p.heads * P) + h * P + col] = o;
+    }
+}
+
 template <int N>
 int delta_scan_launch(const GatedLinIO & io, const BatchView & b, const GatedLinParams & p, float * state, int64_t slot_stride, float * y, cudaStream_t st) {
+    if (b.max_n == 1)
+        return ck_launch([&] {
+            launch_dep(k_delta_token<N>, dim3((unsigned) (p.heads * ((p.vdim + 31) / 32)), (unsigned) b.n_entries), dim3(DT_WARPS * 32), 0, st, io, b.slot, b.off, p, state, slot_stride, y);
+        });
     const dim3 grid((unsigned) (p.heads * ((p.vdim + DS_COLS - 1) / DS_COLS)), (unsigned) b.n_entries);
     // Blocks of four where every CTA has an SM of its own: 384 threads and 106 KB a CTA leave room for one or two, and with more CTAs than SMs it is throughput that
     // counts (eight prompts of 9 to 128 tokens: 26 us token by token, 52 in blocks).  Entries of fewer tokens are not a block.  The two forms round differently: a prompt's
