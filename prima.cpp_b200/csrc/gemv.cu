@@ -44,6 +44,7 @@ __device__ __forceinline__ void load8(const float * p, float (&v)[8]) {   // .cg
     const float4 a0 = __ldcg(reinterpret_cast<const float4 *>(p)), a1 = __ldcg(reinterpret_cast<const float4 *>(p + 4));
     v[0] = a0.x; v[1] = a0.y; v[2] = a0.z; v[3] = a0.w; v[4] = a1.x; v[5] = a1.y; v[6] = a1.z; v[7] = a1.w;
 }
+constexpr int NORM_B = 2;  // super-blocks of a warp where every CTA norms the vector for itself (K up to 3840)
 constexpr int PRO_B = 4;   // super-blocks in flight per warp while summing squares (8 warps x 4 = K 8192 in one batch)
 
 __device__ __forceinline__ void tile_info(const GemvParams & P, int t, int & m, int & r0, int & nrows) {
@@ -163,6 +164,44 @@ __device__ __forceinline__ void dist_prologue(const GemvParams & P, GemvSmemCtl 
         quantize_warp_q8K(bx, lane, b, P.act);
     }
 }
+// ---- PRO_RMSNORM: every CTA norms and quantizes the whole vector into its shared memory, super-blocks warp, warp + 8, ... by a warp; sums and roundings as above.
+// w: the norm's weight at these super-blocks ----
+__device__ __forceinline__ void norm_prologue(const GemvParams & P, GemvSmemCtl * ctl, const ActQ & sa, int warp, int lane, const float (&w)[NORM_B][8]) {
+    float x[NORM_B][8];
+#pragma unroll
+    for (int j = 0; j < NORM_B; j++) {
+        const int b = warp + j * GEMV_NW;
+        if (b < P.nblk) load8(P.in0 + b * 256 + lane * 8, x[j]);
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < NORM_B; j++)
+        if (warp + j * GEMV_NW < P.nblk) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) sum += (double) __fmul_rn(x[j][i], x[j][i]);
+        }
+    sum = warp_sum_d(sum);
+    if (lane == 0) ctl->red[warp] = sum;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < GEMV_NW; i++) t += ctl->red[i];
+    const float mean = (float) (t / (double) P.K), scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, P.eps)));
+#pragma unroll
+    for (int j = 0; j < NORM_B; j++) {
+        const int b = warp + j * GEMV_NW;
+        if (b >= P.nblk) break;
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[j][i] = __fmul_rn(__fmul_rn(x[j][i], scale), w[j][i]);
+        quantize_warp_q8K(x[j], lane, b, sa);
+        if (b % (int) gridDim.x == (int) blockIdx.x) {   // what a caller finds in P.act
+            __syncwarp();
+            reinterpret_cast<uint2 *>(P.act.qs + (int64_t) b * 256)[lane] = *reinterpret_cast<const uint2 *>(sa.qs + b * ACT_SMEM_QS_STRIDE + lane * 8);
+            if (lane < 16) P.act.bsums[(int64_t) b * 16 + lane] = sa.bsums[b * ACT_SMEM_BS_STRIDE + lane];
+            if (lane == 0) P.act.d[b] = sa.d[b];
+        }
+    }
+}
 // ---- PRO_QUANT: every CTA quantizes the whole activation in0 into its shared memory; super-block b also goes to P.act, from CTA b mod grid (what a
 // caller finds in its workspace is the same as behind a quantizing kernel).  The weights' first tiles travel meanwhile ----
 __device__ __forceinline__ void quant_prologue(const GemvParams & P, GemvSmemCtl * ctl, uint8_t * stages, const ActQ & sa, int warp, int lane, uint64_t pol) {
@@ -259,6 +298,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
             if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
         }
     }
+    float nw[NORM_B][8];   // PRO_RMSNORM: the norm's weight does not depend on it either
+    if (TYPE != T_Q8_0 && TYPE != T_Q5_1 && VAR != GV_QUANT && P.prologue == PRO_RMSNORM) {
+#pragma unroll
+        for (int j = 0; j < NORM_B; j++)
+            if (warp + j * GEMV_NW < P.nblk) load8(P.in1 + (warp + j * GEMV_NW) * 256 + lane * 8, nw[j]);
+    }
     stamp<TRACE>(P, 1);
     pdl_wait();      // the activation is produced by the previous kernel in the stream
     stamp<TRACE>(P, 2);
@@ -316,6 +361,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
         }
     } else if (VAR == GV_QUANT) {
         quant_prologue(P, ctl, stages, sa, warp, lane, pol);
+        __syncthreads();
+        load_act_regs(r, sa, blk, valid);
+        finish_act_regs(r);
+    } else if (P.prologue == PRO_RMSNORM) {
+        norm_prologue(P, ctl, sa, warp, lane, nw);
+        fill_rest(P, ctl, stages, pol);
         __syncthreads();
         load_act_regs(r, sa, blk, valid);
         finish_act_regs(r);
@@ -892,7 +943,9 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     P.prefill = std::min(pl.nstage_init, tune.prefill);
     P.stage_bytes = pl.stage_bytes;
     P.act = act;
-    P.prologue = pro.kind;
+    // A norm of less than 16 super-blocks: every CTA for itself, beyond that distributed.  us a step of four layers of width 1024, 2048, 3072, 4096 and 8192, distributed /
+    // so: 119.0 / 102.5, 136.5 / 125.7, 196.0 / 186.4, 228.6 / 229.4, 522 / 530 (where 296 CTAs read 19 MB).
+    P.prologue = pro.kind == PRO_RMSNORM_DIST && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
     P.in0 = pro.in0;
     P.in1 = pro.in1;
     P.eps = pro.eps;

@@ -58,6 +58,7 @@ struct GemvMat {
 //   PRO_NONE          already quantized in HBM (`act`): one coalesced copy per CTA into shared memory, then registers
 //   PRO_RMSNORM_DIST  act = q8_K( rms_norm(in0) * in1 )     llm_build_norm + quantize_row_q8_K   (in1 = norm weight)
 //   PRO_SILU_DIST     act = q8_K( silu(in0) * in1 )         llm_build_ffn LLM_FFN_SILU / LLM_FFN_PAR -> ffn_down
+//   PRO_RMSNORM       the same as PRO_RMSNORM_DIST by every CTA for itself: no barrier over the grid, for K up to 3840
 //   PRO_QUANT         act = q8_K( in0 ), by every CTA for itself: the stand-alone product is one launch that depends on nothing of its own
 //   Distributed: CTA c quantizes super-block c into `act` (HBM/L2), ONE grid barrier (all CTAs of the persistent grid are
 //   co-resident), then every CTA stages the finished vector like PRO_NONE.  No tiny kernel + launch boundary in front of the GEMV
@@ -74,7 +75,7 @@ struct GemvMat {
 //     launch has just written, so that the next GEMV starts with PRO_NONE instead of the distributed prologue.  Bit-identical, but the
 //     single CTA needs ~9 us for it (its loads of y and of the norm weights queue behind the next launch's ring fill, which has the HBM
 //     queues full at that moment): 110.1 -> 101.8-103.3 tok/s (profiles/r2_ab_sweeps.txt ab24 / ab25, r2_token_trace_v7).
-enum : int { PRO_NONE = 0, PRO_RMSNORM_DIST = 4, PRO_SILU_DIST = 5, PRO_QUANT = GEMV_PRO_QUANT };
+enum : int { PRO_NONE = 0, PRO_RMSNORM_DIST = 4, PRO_SILU_DIST = 5, PRO_QUANT = GEMV_PRO_QUANT, PRO_RMSNORM = 7 };
 
 struct GemvParams {
     GemvMat mat[GEMV_MAX_MAT];

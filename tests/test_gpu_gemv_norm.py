@@ -1,0 +1,36 @@
+"""Quantized product with the norm in front of it in the same launch, on both sides of the line between every CTA norming for itself and the distributed form: results and the
+activation left in the workspace are those of a norm kernel and the product behind it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle_lib as O
+
+pytestmark = pytest.mark.gpu
+
+
+class Mat(C.Structure):
+    _fields_ = [("type", C.c_int32), ("pad", C.c_int32), ("W", C.c_void_p), ("n", C.c_int64), ("y", C.c_void_p), ("add", C.c_void_p)]
+
+
+@pytest.mark.parametrize("K", [256, 512, 2304, 3840, 4096, 8192])
+@pytest.mark.parametrize("types,Ns", [((O.Q4_K,), (1000,)), ((O.Q4_K, O.Q4_K, O.Q6_K), (512, 128, 96)), ((O.Q6_K,), (3,))])
+def test_norm_and_product(cuda, lib, K, types, Ns):
+    import torch
+    ptr = lambda t: None if t is None else C.c_void_p(t.data_ptr())   # noqa: E731
+    Ws = [torch.cat([torch.from_numpy(np.ascontiguousarray(O.synth_blocks(t, n, K, seed=11 + i)).reshape(-1).view(np.uint8)), torch.zeros(64, dtype=torch.uint8)]).cuda()
+          for i, (t, n) in enumerate(zip(types, Ns))]
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = 3.0 * torch.randn(K, generator=g, device="cuda"), torch.rand(K, generator=g, device="cuda") + 0.5
+    x[7] = 0.0
+    got = []
+    for sync in (torch.zeros(16, dtype=torch.uint8, device="cuda"), None):   # one launch; a norm kernel in front
+        ws = torch.zeros(lib.c.pb200_act_workspace_bytes(K) + 64, dtype=torch.uint8, device="cuda")
+        ys = [torch.full((n,), float("nan"), device="cuda") for n in Ns]
+        mats = (Mat * len(types))(*[Mat(t, 0, W.data_ptr(), n, y.data_ptr(), None) for t, W, n, y in zip(types, Ws, Ns, ys)])
+        lib.check(lib.c.pb200_gemv_fused(len(types), mats, C.c_int64(K), ptr(ws), 1, ptr(x), ptr(w), C.c_float(1e-5), ptr(sync), 0, None), "gemv_fused")
+        torch.cuda.synchronize()
+        got.append((ys, ws[:K]))
+    assert torch.equal(got[0][1], got[1][1]) and bool((got[0][1] != 0).any())
+    assert all(torch.equal(a, b) and bool(torch.isfinite(a).all()) for a, b in zip(got[0][0], got[1][0]))
