@@ -10,8 +10,8 @@
 // Only models that compute in bf16 come here (the result is rounded to 2^-9 next); float32 models keep the fp32 FMA kernels of mixers.cu.
 // Against float64 in models where nothing else rounds below fp32, six kinds of attention (windows, chunks, sinks, caps, gates, shared key tails), head
 // sizes 64 and 128, 40 to 300 keys, three seeds: 2.8e-7 .. 5.6e-7 off, 0.96 to 1.02 times the FMA kernel, 0.99 over all.
-// Measured with the split pass: 2048 tokens, 16 heads of 128 over 4, causal 1516 -> 114 us; 512 tokens 176 -> 48; latent heads, prompts of 1111,
-// 300 and 77 tokens 522 -> 102.
+// Measured with the split pass, FMA kernel -> these: 2048 tokens, 16 heads of 128 over 4, causal 1516 -> 94 us; 512 tokens 176 -> 37; latent heads,
+// prompts of 1111, 300 and 77 tokens 522 -> 84.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -33,7 +33,11 @@ constexpr int SP_MAX_ND = 3, SP_MAX_NV = 2;    // head sizes up to 192, value si
 // of a tile: key scales [128], value scales relative to the tile's largest [128], value exponents [128], [4]: some value is no number; exponents
 // are far apart; the largest value scale
 constexpr int SP_SCALES = 1552, SP_SPREAD = 12;
-constexpr int SP_THREADS = 320, SP_SM_THREADS = 256;
+constexpr int SP_SLOT = 16384, SP_MAX_SLOTS = 11;   // the ring's pieces: hi or lo of a unit
+constexpr int SP_THREADS = 384, SP_SM_THREADS = 256;
+// registers: 168 a thread at the launch, 128 x 88 + 256 x 208 of the same 64512 from the roles on
+constexpr int SP_REGS_FEW = 88, SP_REGS_SM = 208;
+static_assert(128 * SP_REGS_FEW + SP_SM_THREADS * SP_REGS_SM <= SP_THREADS * 168);
 
 __host__ __device__ inline int sp_v_unit(int nv) { return 2 * nv * 64 * 128; }   // 64 positions of a tile's values: hi, lo, each nv blocks of 64 rows of 128 bytes
 __host__ __device__ inline int64_t sp_tile_bytes(int nd, int nv) { return (int64_t) nd * SP_K_UNIT + 2 * sp_v_unit(nv) + SP_SCALES; }
@@ -45,7 +49,7 @@ struct SplitParams {
     uint8_t * ws;              // [kv head][tile slot][sp_tile_bytes]; entry e's first slot: off[e] / 128 + e
     int slots, kv_first;       // kv heads go through the scratch in groups: this launch's first one
     void * out;
-    int nd, nv, gqa, tok_per_cta, stages;
+    int nd, nv, gqa, tok_per_cta, slots_ring;
     int * abort_flag;
 };
 
@@ -216,7 +220,7 @@ __global__ void __launch_bounds__(256, 2) k_split_kv(const __grid_constant__ Spl
 }
 
 struct SpCtl {
-    uint64_t full[4], empty[4], sc_full[2], sc_empty[2], s_full[2], p_full[2], o_full[2], o_free[2];
+    uint64_t full[SP_MAX_SLOTS], empty[SP_MAX_SLOTS], sc_full[2], sc_empty[2], s_full[2], p_full[2], o_full[2], o_free[2];
     uint32_t tmem_base;
     int abort;
     float2 row_max[2][2][128];     // [tile parity][half of the keys][row]: largest score, largest exponent of weight x value scale
@@ -250,6 +254,8 @@ __device__ __noinline__ float not_numbers(const SplitParams & P, const uint8_t *
 }
 // 2^d for an integer d <= 0 (0 from 2^-127 on, and for what is no number)
 __device__ __forceinline__ float pow2_down(float d) { return d > -126.5f ? __uint_as_float((uint32_t) (127 + (int) d) << 23) : 0.f; }
+// the n low ones of 64 bits
+__device__ __forceinline__ uint64_t below(int n) { return n >= 64 ? ~0ull : n <= 0 ? 0ull : (1ull << n) - 1; }
 __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int h, int d, int DV) {
     if (io.gate_mode == 1) return sigmoid_f(io.gate[row * io.ldg + h]);
     if (io.gate_mode == 2) return sigmoid_f(io.gate[row * io.ldg + (int64_t) h * DV + d]);
@@ -258,12 +264,16 @@ __device__ __forceinline__ float gate_factor(const AttnIO & io, int64_t row, int
 
 // One CTA: 128 query rows (the heads of a GQA group x 128 / group consecutive tokens) of one entry and kv head.  Tensor memory: S twice (2 x 128
 // columns; the split weights go over the scores they come from), the tile's weighted sum twice (2 x 128).
-//   warp 0       key units (64 head entries of 128 keys, hi and lo: 32 KB), value units (64 positions, hi and lo) by bulk copies of the split images
+//   warp 0       lo and hi pieces of key units (64 head entries of 128 keys, 16 KB each) and value units (64 positions) by bulk copies of the split
+//                images; the first ones arrive while the others split the queries
 //   warp 1       MMA issuer, owner of the tensor memory; S(j + 1) goes before P(j) V(j)
-//   warps 2 - 9  softmax: thread = (row, half of the tile's keys); the weighted sum [row][half of the value columns] in registers
-// Bound: 24 MMAs of 107 clocks for S (operand A from shared memory) and 24 of 74 for P V a 128 x 128 tile of 128-wide heads, 4300 clocks; the
-// softmax warps take about half of that.  Their 64 scores and 64 sums a thread do not fit 168 registers (ten warps to an SM): 170 to 180
-// bytes of them go through local memory once a tile.
+//   warps 4 - 11 softmax: thread = (row, half of the tile's keys); the weighted sum [row][half of the value columns] in registers.  64 scores and
+//                64 sums a thread do not fit the 168 registers of twelve warps (180 bytes went through local memory once a tile): the other warpgroup
+//                gives up 80 of its own
+// Bound: in the steady state S takes 1900 and P V 2500 clocks of the tensor cores (24 MMAs each), the softmax warps 4200 beside them, and a tile
+// 4400 to 4600.  It took 7300 to 8200 while every score was tested against the mask (2500 of them) and a unit's memory came free only behind all
+// of its products (900 of waiting for copies).  A CTA that is the first on its SM loses about 13000 clocks more to code that is not there yet.
+// Measured in one run, start to end: 2048 tokens, 16 heads of 128 over 4, causal 119 -> 91 us; 512 tokens 45 -> 31; the latent prompts above 95 -> 77.
 template <typename OT, bool CAP>
 __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_constant__ SplitParams P) {
     extern __shared__ uint8_t smem_raw[];
@@ -275,10 +285,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
     if (q0 >= n) return;
     const int toks = min(P.tok_per_cta, n - q0), rows = toks * P.gqa;
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int nd = P.nd, nv = P.nv, stages = P.stages, v_unit = sp_v_unit(nv), q_piece = nd * 16384;
+    const int nd = P.nd, nv = P.nv, slots = P.slots_ring, v_unit = sp_v_unit(nv), q_piece = nd * 16384;
     uint8_t * q_s = smem, * ring = smem + 2 * q_piece;                            // queries: hi, lo, each nd blocks of 128 rows of 128 bytes
-    float * scales = reinterpret_cast<float *>(ring + stages * SP_K_UNIT);       // [2][SP_SCALES]
-    SpCtl * ctl = reinterpret_cast<SpCtl *>(ring + stages * SP_K_UNIT + 2 * SP_SCALES);
+    float * scales = reinterpret_cast<float *>(ring + slots * SP_SLOT);       // [2][SP_SCALES]
+    SpCtl * ctl = reinterpret_cast<SpCtl *>(ring + slots * SP_SLOT + 2 * SP_SCALES);
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     volatile int * cta_abort = &ctl->abort;
     // key tiles some row sees: the kept first tokens' ones, then from the window's (chunk's) first position to the last query
@@ -288,7 +298,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
     auto tile_of = [&](int j) { return j < kept ? j : first + j - kept; };
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; i++) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], 1); }
+        for (int i = 0; i < SP_MAX_SLOTS; i++) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], 1); }
         for (int i = 0; i < 2; i++) {
             mbar_init(&ctl->sc_full[i], 1); mbar_init(&ctl->sc_empty[i], 8); mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_full[i], 8);
             mbar_init(&ctl->o_full[i], 1); mbar_init(&ctl->o_free[i], 8);
@@ -302,9 +312,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         pdl_trigger();   // behind the allocation: a later kernel's CTA on this SM must not take the columns first and wait for this one
     }
+    __syncthreads();
     pdl_wait();          // queries and the split images are the kernels' in front
-    if (warp >= 2) {
-        const int w = warp - 2, D = a.dim;
+    if (warp >= 4) {
+        const int w = warp - 4, D = a.dim;
         for (int r0 = w * 16; r0 < w * 16 + 16; r0 += 4) {
             float x[4][SP_MAX_ND][2];
 #pragma unroll
@@ -344,112 +355,158 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    fence_before();
-    __syncthreads();
-    fence_after();
+    if (warp == 1 || warp >= 4) {      // the first keys are on their way while the queries are split
+        fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"(SP_SM_THREADS + 32) : "memory");
+        fence_after();
+    }
     const uint32_t tmem = *(volatile uint32_t *) &ctl->tmem_base;
     constexpr uint32_t O0 = 256;
 
-    if (warp == 0) {
-        const uint8_t * src0 = P.ws + ((int64_t) blockIdx.x * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
-        int u = 0;
-        auto load = [&](const uint8_t * src, uint32_t bytes) {
-            const int s = u % stages;
-            if (u >= stages) mbar_wait(&ctl->empty[s], (uint32_t) ((u / stages - 1) & 1), cta_abort, P.abort_flag);
-            __syncwarp();
-            if (elect_one()) {
-                mbar_arrive_expect_tx(&ctl->full[s], bytes);
-                bulk_load(smem_u32(ring + s * SP_K_UNIT), src, bytes, smem_u32(&ctl->full[s]));
-            }
-            __syncwarp();
-            u++;
-        };
-        for (int j = 0; j <= nt && !*cta_abort; j++) {   // K(0) K(1) V(0) K(2) V(1) ...
-            if (j < nt) {
-                const uint8_t * src = src0 + (int64_t) tile_of(j) * sp_tile_bytes(nd, nv);
-                if (j >= 2) mbar_wait(&ctl->sc_empty[j & 1], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SP_REGS_FEW));
+        if (warp == 0) {
+            const uint8_t * src0 = P.ws + ((int64_t) blockIdx.x * P.slots + t_begin / SP_KEYS + e) * sp_tile_bytes(nd, nv);
+            int slot = 0;
+            uint32_t turn = 0u;                             // parity of the round in which the ring is filled
+            bool wrapped = false;
+            auto load = [&](const uint8_t * src, uint32_t bytes) {
+                if (wrapped) mbar_wait(&ctl->empty[slot], turn ^ 1u, cta_abort, P.abort_flag);
                 __syncwarp();
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&ctl->sc_full[j & 1], SP_SCALES);
-                    bulk_load(smem_u32(scales) + (j & 1) * SP_SCALES, src + nd * SP_K_UNIT + 2 * v_unit, SP_SCALES, smem_u32(&ctl->sc_full[j & 1]));
+                    mbar_arrive_expect_tx(&ctl->full[slot], bytes);
+                    bulk_load(smem_u32(ring + slot * SP_SLOT), src, bytes, smem_u32(&ctl->full[slot]));
                 }
                 __syncwarp();
-                for (int c = 0; c < nd; c++) load(src + c * SP_K_UNIT, SP_K_UNIT);
-            }
-            if (j > 0) {
-                const uint8_t * src = src0 + (int64_t) tile_of(j - 1) * sp_tile_bytes(nd, nv) + nd * SP_K_UNIT;
-                for (int c = 0; c < 2; c++) load(src + c * v_unit, (uint32_t) v_unit);
-            }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        constexpr uint32_t idesc = (1u << 4) | ((uint32_t) (SP_KEYS >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
-        const uint32_t idesc_v = (1u << 4) | (1u << 16) | ((uint32_t) (nv * 64 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
-        const uint64_t dq = desc_sw128(smem_u32(q_s));
-        const uint32_t q_lo = (uint32_t) (q_piece >> 4);
-        int u = 0;
-        // the small products of all units go first: what the tensor cores cut off at each step is a share of the sum so far
-        auto scores = [&](int j) {
-            const uint32_t d = tmem + (uint32_t) ((j & 1) * 128);
-            for (int c = 0; c < nd; c++) mbar_wait(&ctl->full[(u + c) % stages], (uint32_t) (((u + c) / stages) & 1), cta_abort, P.abort_flag);
-            __syncwarp();
-            fence_after();
-            if (elect_one()) {
-                for (int c = 0; c < nd; c++) {
-                    const uint64_t hk = desc_sw128(smem_u32(ring + (u + c) % stages * SP_K_UNIT)), lk = hk + (SP_K_UNIT / 2 >> 4), hq = dq + c * (16384 >> 4), lq = hq + q_lo;
-#pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16<1>(d, lq + 2 * k, hk + 2 * k, idesc, (uint32_t) ((c | k) != 0));
-#pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, lk + 2 * k, idesc, 1u);
+                if (++slot == slots) { slot = 0; turn ^= 1u; wrapped = true; }
+            };
+            for (int j = 0; j <= nt && !*cta_abort; j++) {   // K(0) K(1) V(0) K(2) V(1) ...
+                if (j < nt) {
+                    const uint8_t * src = src0 + (int64_t) tile_of(j) * sp_tile_bytes(nd, nv);
+                    if (j >= 2) mbar_wait(&ctl->sc_empty[j & 1], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+                    __syncwarp();
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&ctl->sc_full[j & 1], SP_SCALES);
+                        bulk_load(smem_u32(scales) + (j & 1) * SP_SCALES, src + nd * SP_K_UNIT + 2 * v_unit, SP_SCALES, smem_u32(&ctl->sc_full[j & 1]));
+                    }
+                    __syncwarp();
+                    for (int p = 1; p >= 0; p--)            // lo of all units, then hi
+                        for (int c = 0; c < nd; c++) load(src + c * SP_K_UNIT + p * (SP_K_UNIT / 2), SP_K_UNIT / 2);
                 }
-                for (int c = 0; c < nd; c++) {
-                    const uint64_t hk = desc_sw128(smem_u32(ring + (u + c) % stages * SP_K_UNIT)), hq = dq + c * (16384 >> 4);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, hk + 2 * k, idesc, 1u);
-                    mma_commit(&ctl->empty[(u + c) % stages]);
+                if (j > 0) {
+                    const uint8_t * src = src0 + (int64_t) tile_of(j - 1) * sp_tile_bytes(nd, nv) + nd * SP_K_UNIT;
+                    for (int p = 1; p >= 0; p--)
+                        for (int c = 0; c < 2; c++) load(src + c * v_unit + p * (v_unit / 2), (uint32_t) v_unit / 2);
                 }
-                mma_commit(&ctl->s_full[j & 1]);
             }
             __syncwarp();
-            u += nd;
-        };
-        scores(0);
-        for (int j = 0; j < nt && !*cta_abort; j++) {
-            if (j + 1 < nt) scores(j + 1);       // its columns held P(j - 1), whose products precede it in the pipe
-            const int buf = j & 1;
-            mbar_wait(&ctl->p_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
-            if (j >= 2) mbar_wait(&ctl->o_free[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
-            __syncwarp();
-            const uint32_t d = tmem + O0 + (uint32_t) (buf * 128);
-            for (int h = 0; h < 2; h++) mbar_wait(&ctl->full[(u + h) % stages], (uint32_t) (((u + h) / stages) & 1), cta_abort, P.abort_flag);
-            __syncwarp();
-            fence_after();
-            if (elect_one()) {
+        } else if (warp == 1) {
+            constexpr uint32_t idesc = (1u << 4) | ((uint32_t) (SP_KEYS >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+            const uint32_t idesc_v = (1u << 4) | (1u << 16) | ((uint32_t) (nv * 64 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+            const uint64_t dq = desc_sw128(smem_u32(q_s));
+            const uint32_t q_lo = (uint32_t) (q_piece >> 4);
+            const bool leader = elect_one();
+            int slot = 0;
+            uint32_t turn = 0u;
+            // the next piece of the ring, arrived
+            auto next = [&]() {
+                const int at = slot;
+                mbar_wait(&ctl->full[at], turn, cta_abort, P.abort_flag);
+                __syncwarp();
+                if (++slot == slots) { slot = 0; turn ^= 1u; }
+                return at;
+            };
+            // the small products of all units go first: what the tensor cores cut off at each step is a share of the sum so far; lo pieces before hi, so
+            // that their memory takes the next piece two thirds of the products earlier
+            auto scores = [&](int j) {
+                const uint32_t d = tmem + (uint32_t) ((j & 1) * 128);
+                int at[SP_MAX_ND];
+                for (int c = 0; c < nd; c++) {
+                    const int s = next();
+                    const uint64_t lk = desc_sw128(smem_u32(ring + s * SP_SLOT)), hq = dq + c * (16384 >> 4);
+                    if (c == 0) fence_after();
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, lk + 2 * k, idesc, (uint32_t) ((c | k) != 0));
+                        mma_commit(&ctl->empty[s]);
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int c = 0; c < SP_MAX_ND; c++) {
+                    if (c >= nd) break;
+                    at[c] = next();
+                    const uint64_t hk = desc_sw128(smem_u32(ring + at[c] * SP_SLOT)), lq = dq + c * (16384 >> 4) + q_lo;
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) mma_f16<1>(d, lq + 2 * k, hk + 2 * k, idesc, 1u);
+                    }
+                    __syncwarp();
+                }
+                if (leader) {
+#pragma unroll
+                    for (int c = 0; c < SP_MAX_ND; c++) {
+                        if (c >= nd) break;
+                        const uint64_t hk = desc_sw128(smem_u32(ring + at[c] * SP_SLOT)), hq = dq + c * (16384 >> 4);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) mma_f16<1>(d, hq + 2 * k, hk + 2 * k, idesc, 1u);
+                        mma_commit(&ctl->empty[at[c]]);
+                    }
+                    mma_commit(&ctl->s_full[j & 1]);
+                }
+                __syncwarp();
+            };
+            scores(0);
+            for (int j = 0; j < nt && !*cta_abort; j++) {
+                if (j + 1 < nt) scores(j + 1);       // its columns held P(j - 1), whose products precede it in the pipe
+                const int buf = j & 1;
+                mbar_wait(&ctl->p_full[buf], (uint32_t) ((j / 2) & 1), cta_abort, P.abort_flag);
+                if (j >= 2) mbar_wait(&ctl->o_free[buf], (uint32_t) ((j / 2 - 1) & 1), cta_abort, P.abort_flag);
+                __syncwarp();
+                fence_after();
+                const uint32_t d = tmem + O0 + (uint32_t) (buf * 128), p0 = tmem + (uint32_t) (buf * 128);      // 16 columns hi, 16 columns lo of 32 keys, then the next 32
+                int at[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const uint64_t hv = desc_sw128_mn(smem_u32(ring + (u + h) % stages * SP_K_UNIT), 8192), lv = hv + (v_unit / 2 >> 4);
-                    const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);      // 16 columns hi, 16 columns lo of 32 keys, then the next 32
+                    const int s = next();
+                    const uint64_t lv = desc_sw128_mn(smem_u32(ring + s * SP_SLOT), 8192);
+                    const uint32_t p = p0 + (uint32_t) (h * 64);
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + 16 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, (uint32_t) ((h | k) != 0));
-#pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, lv + k * (2048 >> 4), idesc_v, 1u);
+                        for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, lv + k * (2048 >> 4), idesc_v, (uint32_t) ((h | k) != 0));
+                        mma_commit(&ctl->empty[s]);
+                    }
+                    __syncwarp();
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const uint64_t hv = desc_sw128_mn(smem_u32(ring + (u + h) % stages * SP_K_UNIT), 8192);
-                    const uint32_t p = tmem + (uint32_t) (buf * 128 + h * 64);
+                    at[h] = next();
+                    const uint64_t hv = desc_sw128_mn(smem_u32(ring + at[h] * SP_SLOT), 8192);
+                    const uint32_t p = p0 + (uint32_t) (h * 64);
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, 1u);
-                    mma_commit(&ctl->empty[(u + h) % stages]);
+                        for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + 16 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, 1u);
+                    }
+                    __syncwarp();
                 }
-                mma_commit(&ctl->o_full[buf]);
+                if (leader) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint64_t hv = desc_sw128_mn(smem_u32(ring + at[h] * SP_SLOT), 8192);
+                        const uint32_t p = p0 + (uint32_t) (h * 64);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) mma_f16_ts(d, p + (k >> 1) * 32 + (k & 1) * 8, hv + k * (2048 >> 4), idesc_v, 1u);
+                        mma_commit(&ctl->empty[at[h]]);
+                    }
+                    mma_commit(&ctl->o_full[buf]);
+                }
+                __syncwarp();
             }
             __syncwarp();
-            u += 2;
         }
-        __syncwarp();
     } else {
-        const int quad = warp & 3, part = (warp - 2) >> 2, row = quad * 32 + lane;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SP_REGS_SM));
+        const int quad = warp & 3, part = (warp - 4) >> 2, row = quad * 32 + lane;
         const int qi = row < rows ? q0 + row / P.gqa : -1;                       // the row's position; -1: sees nothing
         const int lo_q = qi >= 0 ? attn_first_visible(a, qi) : 0;
         const int h = kvh * P.gqa + (row < rows ? row % P.gqa : 0);
@@ -499,21 +556,28 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
             const int tile0 = tile_of(j) * SP_KEYS;
             const bool whole = tile0 >= all_from && tile0 + SP_KEYS - 1 <= all_to, plain = whole && tail[1] == 0.f;
             float tm = -INFINITY, tw = -INFINITY;
+            // two copies: with the test beside it every score of every tile paid for it (3600 instead of 1100 clocks a tile)
+            auto take = [&](auto sees) {
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
-                const float4 s4 = *reinterpret_cast<const float4 *>(sc + i);
-                const float f[4] = {s4.x, s4.y, s4.z, s4.w};
+                for (int i = 0; i < 64; i += 4) {
+                    const float4 s4 = *reinterpret_cast<const float4 *>(sc + i);
+                    const float f[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float x = t[i + q] * f[q] * qs;
-                    if constexpr (CAP) x = cap * tanhf(x);
-                    if (!whole) {
-                        const int kj = k0 + i + q;
-                        if (!(kj <= qi && (kj >= lo_q || kj < a.keep_first))) x = -INFINITY;
+                    for (int q = 0; q < 4; q++) {
+                        float x = t[i + q] * f[q] * qs;
+                        if constexpr (CAP) x = cap * tanhf(x);
+                        if (!sees(i + q)) x = -INFINITY;
+                        t[i + q] = x;
+                        tm = fmaxf(tm, x);
                     }
-                    t[i + q] = x;
-                    tm = fmaxf(tm, x);
                 }
+            };
+            if (whole) {
+                take([](int) { return true; });
+            } else {
+                const uint64_t seen = below(qi + 1 - k0) & (~below(lo_q - k0) | below(a.keep_first - k0));
+                const uint32_t seen2[2] = {(uint32_t) seen, (uint32_t) (seen >> 32)};
+                take([&](int i) { return (seen2[i >> 5] >> (i & 31) & 1u) != 0u; });
             }
             if (!plain) {
 #pragma unroll
@@ -595,7 +659,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
                 *reinterpret_cast<float4 *>(os + row * 128 + ((part * 16 + i + row) & 31) * 4) = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
         }
         asm volatile("bar.sync 1, %0;" ::"n"(SP_SM_THREADS) : "memory");
-        const int DV = a.vdim, w = warp - 2;
+        const int DV = a.vdim, w = warp - 4;
         for (int r = w * 16; r < w * 16 + 16 && r < rows; r++) {
             const int64_t tok = t_begin + q0 + r / P.gqa;
             const int hh = kvh * P.gqa + r % P.gqa;
@@ -665,10 +729,10 @@ int launch_attn_split(const AttnIO & io, const BatchView & b, const AttnParams &
     P.nd = (a.dim + 63) / 64; P.nv = (a.vdim + 63) / 64;
     P.gqa = a.heads / a.kv_heads;
     P.tok_per_cta = 128 / P.gqa;
-    P.stages = P.nd == 3 ? 3 : 4;
+    P.slots_ring = 13 - 2 * P.nd;   // with the queries' 2 nd pieces what an SM's shared memory holds
     P.abort_flag = abort_flag();
     const int group = (int) (attn_split_bytes(a, b.n_tokens, b.n_entries) / split_head_bytes(a, b.n_tokens, b.n_entries));
-    const size_t smem = 1024 + (size_t) P.nd * 32768 + (size_t) P.stages * SP_K_UNIT + 2 * SP_SCALES + sizeof(SpCtl);
+    const size_t smem = 1024 + (size_t) P.nd * 32768 + (size_t) P.slots_ring * SP_SLOT + 2 * SP_SCALES + sizeof(SpCtl);
     for (P.kv_first = 0; P.kv_first < a.kv_heads; P.kv_first += group) {
         const unsigned heads = (unsigned) std::min(group, a.kv_heads - P.kv_first);
         g_launches += 2;
