@@ -181,7 +181,8 @@ int launch_attn_qknorm_kv_store(float * qkvg, const BatchView & b, const AttnPar
 int launch_attn_window_prefill(const float * qkvg, const BatchView & b, const AttnParams & a, void * out, int otype, cudaStream_t stream);
 // one-token entries: keys and values come from the cache (the token's own row already stored).  part (may be null): scratch of
 // attn_decode_part_floats floats; with it and a cache of 128 rows or more the rows are split over several CTAs per (head, entry) in chunks
-// of attn_decode_chunk rows, and a second kernel merges the partial softmax states.  The split depends on the cache's row count alone.
+// of attn_decode_chunk rows, and a second kernel merges the partial softmax states.  The split depends on the cache's row count alone.  Where
+// attn_decode.cu takes the call, a cluster per (entry, kv head) does both in one launch.
 inline int attn_decode_chunk(int cache_rows) {
     const int c = (cache_rows + 63) / 64;                 // at most 64 splits ...
     return c < 64 ? 64 : (c + 31) / 32 * 32;              // ... of at least 64 rows
