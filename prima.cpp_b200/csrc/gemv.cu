@@ -22,8 +22,9 @@ static_assert(sizeof(GemvSmemCtl) <= GEMV_CTL_BYTES, "ctl block");
 
 __device__ __forceinline__ float silu_f(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }   // ggml.c:2560
 
-// instantiations of the kernel: plain; with time stamps; quantizing its own activation (PRO_QUANT, gemv.cuh)
-enum : int { GV_PLAIN = 0, GV_TRACE = 1, GV_QUANT = 2 };
+// instantiations of the kernel: plain; with time stamps; quantizing its own activation (PRO_QUANT, gemv.cuh); norming it first (PRO_RMSNORM: as a branch of the
+// plain one its code cost the longer vectors' steps 0.6 %)
+enum : int { GV_PLAIN = 0, GV_TRACE = 1, GV_QUANT = 2, GV_NORM = 3 };
 
 // TRACE instantiation only: slot k (0..5) of this CTA's 8-entry row = %globaltimer (ns) at stamp k; slots 6 / 7 = clock64 at
 // the first / last stamp (the SM clock during the launch follows from the two)
@@ -298,8 +299,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
             if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
         }
     }
-    float nw[NORM_B][8];   // PRO_RMSNORM: the norm's weight does not depend on it either
-    if (TYPE != T_Q8_0 && TYPE != T_Q5_1 && VAR != GV_QUANT && P.prologue == PRO_RMSNORM) {
+    float nw[NORM_B][8];   // the norm's weight does not depend on it either
+    if (VAR == GV_NORM) {
 #pragma unroll
         for (int j = 0; j < NORM_B; j++)
             if (warp + j * GEMV_NW < P.nblk) load8(P.in1 + (warp + j * GEMV_NW) * 256 + lane * 8, nw[j]);
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
         __syncthreads();
         load_act_regs(r, sa, blk, valid);
         finish_act_regs(r);
-    } else if (P.prologue == PRO_RMSNORM) {
+    } else if (VAR == GV_NORM) {
         norm_prologue(P, ctl, sa, warp, lane, nw);
         fill_rest(P, ctl, stages, pol);
         __syncthreads();
@@ -945,7 +946,8 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     P.act = act;
     // A norm of less than 16 super-blocks: every CTA for itself, beyond that distributed.  us a step of four layers of width 1024, 2048, 3072, 4096 and 8192, distributed /
     // so: 119.0 / 102.5, 136.5 / 125.7, 196.0 / 186.4, 228.6 / 229.4, 522 / 530 (where 296 CTAs read 19 MB).
-    P.prologue = pro.kind == PRO_RMSNORM_DIST && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
+    // While a trace is taken the distributed one has the stamps.
+    P.prologue = pro.kind == PRO_RMSNORM_DIST && !g_trace_buf && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
     P.in0 = pro.in0;
     P.in1 = pro.in1;
     P.eps = pro.eps;
@@ -973,22 +975,22 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     int ty = types[0];
     for (int i = 1; i < nmat; i++) if (types[i] != ty) ty = 0;
     const int ti = ty == T_Q4_K ? 1 : ty == T_Q5_K ? 2 : ty == T_Q6_K ? 3 : ty == T_Q8_0 ? 4 : ty == T_Q5_1 ? 5 : 0;
-    const int var = pro.kind == PRO_QUANT ? GV_QUANT : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
+    const int var = pro.kind == PRO_QUANT ? GV_QUANT : P.prologue == PRO_RMSNORM ? GV_NORM : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
     typedef void (*kern_t)(const GemvParams);
-    static const kern_t table[6][2][3] = {
-        {{k_gemv_kquant<0, false, GV_PLAIN>, k_gemv_kquant<0, false, GV_TRACE>, nullptr},
+    static const kern_t table[6][2][4] = {   // rows of a norm by every CTA are never split
+        {{k_gemv_kquant<0, false, GV_PLAIN>, k_gemv_kquant<0, false, GV_TRACE>, nullptr, k_gemv_kquant<0, false, GV_NORM>},
          {k_gemv_kquant<0, true, GV_PLAIN>, k_gemv_kquant<0, true, GV_TRACE>, nullptr}},
-        {{k_gemv_kquant<T_Q4_K, false, GV_PLAIN>, k_gemv_kquant<T_Q4_K, false, GV_TRACE>, k_gemv_kquant<T_Q4_K, false, GV_QUANT>},
+        {{k_gemv_kquant<T_Q4_K, false, GV_PLAIN>, k_gemv_kquant<T_Q4_K, false, GV_TRACE>, k_gemv_kquant<T_Q4_K, false, GV_QUANT>, k_gemv_kquant<T_Q4_K, false, GV_NORM>},
          {k_gemv_kquant<T_Q4_K, true, GV_PLAIN>, k_gemv_kquant<T_Q4_K, true, GV_TRACE>, k_gemv_kquant<T_Q4_K, true, GV_QUANT>}},
-        {{k_gemv_kquant<T_Q5_K, false, GV_PLAIN>, k_gemv_kquant<T_Q5_K, false, GV_TRACE>, k_gemv_kquant<T_Q5_K, false, GV_QUANT>},
+        {{k_gemv_kquant<T_Q5_K, false, GV_PLAIN>, k_gemv_kquant<T_Q5_K, false, GV_TRACE>, k_gemv_kquant<T_Q5_K, false, GV_QUANT>, k_gemv_kquant<T_Q5_K, false, GV_NORM>},
          {k_gemv_kquant<T_Q5_K, true, GV_PLAIN>, k_gemv_kquant<T_Q5_K, true, GV_TRACE>, k_gemv_kquant<T_Q5_K, true, GV_QUANT>}},
-        {{k_gemv_kquant<T_Q6_K, false, GV_PLAIN>, k_gemv_kquant<T_Q6_K, false, GV_TRACE>, k_gemv_kquant<T_Q6_K, false, GV_QUANT>},
+        {{k_gemv_kquant<T_Q6_K, false, GV_PLAIN>, k_gemv_kquant<T_Q6_K, false, GV_TRACE>, k_gemv_kquant<T_Q6_K, false, GV_QUANT>, k_gemv_kquant<T_Q6_K, false, GV_NORM>},
          {k_gemv_kquant<T_Q6_K, true, GV_PLAIN>, k_gemv_kquant<T_Q6_K, true, GV_TRACE>, k_gemv_kquant<T_Q6_K, true, GV_QUANT>}},
         {{k_gemv_kquant<T_Q8_0, false, GV_PLAIN>, k_gemv_kquant<T_Q8_0, false, GV_TRACE>, nullptr},
          {k_gemv_kquant<T_Q8_0, true, GV_PLAIN>, k_gemv_kquant<T_Q8_0, true, GV_TRACE>, nullptr}},
         {{k_gemv_kquant<T_Q5_1, false, GV_PLAIN>, k_gemv_kquant<T_Q5_1, false, GV_TRACE>, nullptr},
          {k_gemv_kquant<T_Q5_1, true, GV_PLAIN>, k_gemv_kquant<T_Q5_1, true, GV_TRACE>, nullptr}}};
-    static FuncAttrCache attr_cache[6][2][3];
+    static FuncAttrCache attr_cache[6][2][4];
     const int si = pl.wpr > 1 ? 1 : 0;
     if (pro.kind == PRO_QUANT && ti == 0) return (int) cudaErrorInvalidValue;
     const kern_t fn = table[ti][si][var];
