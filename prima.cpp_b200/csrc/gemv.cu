@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
         }
     }
     float nw[NORM_B][8];   // the norm's weight does not depend on it either
-    if (VAR == GV_NORM) {
+    if (VAR == GV_NORM && P.prologue == PRO_RMSNORM) {
 #pragma unroll
         for (int j = 0; j < NORM_B; j++)
             if (warp + j * GEMV_NW < P.nblk) load8(P.in1 + (warp + j * GEMV_NW) * 256 + lane * 8, nw[j]);
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
         __syncthreads();
         load_act_regs(r, sa, blk, valid);
         finish_act_regs(r);
-    } else if (VAR == GV_NORM) {
+    } else if (VAR == GV_NORM && P.prologue == PRO_RMSNORM) {
         norm_prologue(P, ctl, sa, warp, lane, nw);
         fill_rest(P, ctl, stages, pol);
         __syncthreads();
@@ -975,7 +975,10 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     int ty = types[0];
     for (int i = 1; i < nmat; i++) if (types[i] != ty) ty = 0;
     const int ti = ty == T_Q4_K ? 1 : ty == T_Q5_K ? 2 : ty == T_Q6_K ? 3 : ty == T_Q8_0 ? 4 : ty == T_Q5_1 ? 5 : 0;
-    const int var = pro.kind == PRO_QUANT ? GV_QUANT : P.prologue == PRO_RMSNORM ? GV_NORM : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
+    // Short products share the instantiation with the norm, whether they have one or not: a step that changed code at every launch lost half of the gain
+    // (widths 1024, 2048 and 3072 against the distributed norm: 119.6 -> 110.0 and 102.7 so, 138.7 -> 137.2 and 127.1, 197.4 -> 189.0 and 185.4 us).
+    const bool norms = P.prologue == PRO_RMSNORM || (is_kquant(types[0]) && !g_trace_buf && pl.wpr == 1 && std::min(K, d[0].N) < GEMV_NW * NORM_B * 256);
+    const int var = pro.kind == PRO_QUANT ? GV_QUANT : norms ? GV_NORM : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
     typedef void (*kern_t)(const GemvParams);
     static const kern_t table[6][2][4] = {   // rows of a norm by every CTA are never split
         {{k_gemv_kquant<0, false, GV_PLAIN>, k_gemv_kquant<0, false, GV_TRACE>, nullptr, k_gemv_kquant<0, false, GV_NORM>},
