@@ -696,6 +696,14 @@ int launch_typed(const SplitParams & P, const dim3 & grid, size_t smem, cudaStre
     static FuncAttrCache cache;
     const cudaError_t e = ensure_dyn_smem(cache, (const void *) k_attn_split<OT, CAP>, smem, true);
     if (e != cudaSuccess) return (int) e;
+    static std::atomic<bool> fits{false};   // the roles' registers are within the launch's: beyond them the softmax warps would wait without end
+    if (!fits.load(std::memory_order_relaxed)) {
+        cudaFuncAttributes f;
+        const cudaError_t ea = cudaFuncGetAttributes(&f, k_attn_split<OT, CAP>);
+        if (ea != cudaSuccess) return (int) ea;
+        if (f.numRegs * SP_THREADS < 128 * SP_REGS_FEW + SP_SM_THREADS * SP_REGS_SM) return (int) cudaErrorLaunchOutOfResources;
+        fits.store(true, std::memory_order_relaxed);
+    }
     return launch_dep(k_attn_split<OT, CAP>, grid, dim3(SP_THREADS), smem, st, P);
 }
 int split_slots(int n_tokens, int n_entries) { return n_tokens / SP_KEYS + n_entries; }   // floor(off / 128) + e are distinct runs of slots
