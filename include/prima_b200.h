@@ -138,8 +138,8 @@ typedef struct pb200_gemv_mat {
  *   0  act_ws already holds the q8_K activation (pb200_quantize_act, or pb200_attn_ggml with act_ws_out)
  *   1  act = q8_K( rms_norm(in0, eps) * in1 )     ggml RMS_NORM + MUL by the norm weight   (llm_build_norm, src/llama.cpp:9772-9802)
  *   2  act = q8_K( silu(in0) * in1 )              ggml UNARY(SILU) + MUL                    (llm_build_ffn, src/llama.cpp:9858-9907)
- * computed once, distributed over the launch's CTAs (one in-kernel grid barrier); norms of up to 3840 entries by every CTA for itself.  Left in
- * act_ws either way.  sync_ws: 16 bytes of zero-initialised
+ * computed once, distributed over the launch's CTAs (one in-kernel grid barrier); norms of up to 3840 entries by every CTA for itself, unless
+ * a y lies over in0 or in1 (which it may).  Left in act_ws either way.  sync_ws: 16 bytes of zero-initialised
  * device memory owned by the caller (barrier state, self-resetting; one per stream).  pdl != 0: the launch may start while the
  * previous kernel of the stream drains (programmatic dependent launch); its inputs are read only after that kernel has completed.
  * Returns PB200_ENOTSUP for types / shapes outside the fast kernel (callers fall back to the single ops). */

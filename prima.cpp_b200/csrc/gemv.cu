@@ -946,8 +946,8 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     P.act = act;
     // A norm of less than 16 super-blocks: every CTA for itself, beyond that distributed.  us a step of four layers of width 1024, 2048, 3072, 4096 and 8192, distributed /
     // so: 119.0 / 102.5, 136.5 / 125.7, 196.0 / 186.4, 228.6 / 229.4, 522 / 530 (where 296 CTAs read 19 MB).
-    // While a trace is taken the distributed one has the stamps.
-    P.prologue = pro.kind == PRO_RMSNORM_DIST && !g_trace_buf && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
+    // While a trace is taken the distributed one has the stamps.  A result over in0 or in1 takes the distributed one, too: its barrier ends all reads of them.
+    P.prologue = pro.kind == PRO_RMSNORM_DIST && !pro.in_place && !g_trace_buf && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
     P.in0 = pro.in0;
     P.in1 = pro.in1;
     P.eps = pro.eps;

@@ -24,6 +24,7 @@ struct GemvFused {       // fused activation prologue of the k-quant GEMV (PRO_*
     const float * in1 = nullptr;
     float eps = 0.f;
     unsigned int * gbar = nullptr;   // kinds 4, 5: two zero-initialised words of device memory owned by the caller (grid barrier state)
+    bool in_place = false;           // kind 4: a result lies over in0 or in1, whose reads then have to end in all CTAs before one stores
 };
 
 // ---- per-device host state (gemv.cu): cudaFuncSetAttribute / SM count are per device, one process may drive several ----

@@ -34,3 +34,26 @@ def test_norm_and_product(cuda, lib, K, types, Ns):
         got.append((ys, ws[:K]))
     assert torch.equal(got[0][1], got[1][1]) and bool((got[0][1] != 0).any())
     assert all(torch.equal(a, b) and bool(torch.isfinite(a).all()) for a, b in zip(got[0][0], got[1][0]))
+
+
+# y over the vector or over the norm's weight: in place, over its end, over its start, two matrices of which the second one lies there
+@pytest.mark.parametrize("K", [2048, 3840, 4096])
+@pytest.mark.parametrize("over", [0, 1])
+@pytest.mark.parametrize("N,at", [(4096, 0), (300, 0), (4096, 2044), (5000, -600)])
+def test_result_over_an_operand(cuda, lib, K, over, N, at):
+    import torch
+    ptr = lambda t: C.c_void_p(t.data_ptr())   # noqa: E731
+    Ws = [torch.from_numpy(np.ascontiguousarray(O.synth_blocks(O.Q4_K, n, K, seed=n)).reshape(-1).view(np.uint8)).cuda() for n in (64, N)]
+    buf = torch.zeros(5 * 4096, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    ops = [3.0 * torch.randn(K, generator=g, device="cuda"), torch.rand(K, generator=g, device="cuda") + 0.5]
+    buf[8192:8192 + K] = ops[over]
+    ops[over] = buf[8192:8192 + K]
+    ws, sync = torch.zeros(lib.c.pb200_act_workspace_bytes(K) + 64, dtype=torch.uint8, device="cuda"), torch.zeros(16, dtype=torch.uint8, device="cuda")
+    got = []
+    for ys in ((torch.empty(64, device="cuda"), torch.empty(N, device="cuda")), (torch.empty(64, device="cuda"), buf[8192 + at:8192 + at + N])):
+        mats = (Mat * 2)(*[Mat(O.Q4_K, 0, W.data_ptr(), y.numel(), y.data_ptr(), None) for W, y in zip(Ws, ys)])
+        lib.check(lib.c.pb200_gemv_fused(2, mats, C.c_int64(K), ptr(ws), 1, ptr(ops[0]), ptr(ops[1]), C.c_float(1e-5), ptr(sync), 0, None), "gemv_fused")
+        torch.cuda.synchronize()
+        got.append(ys)
+    assert all(torch.equal(a, b) for a, b in zip(*got))
