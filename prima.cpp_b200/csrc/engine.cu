@@ -353,7 +353,7 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
                              {L.wv.data, m->v, L.bv, nullptr, L.wv.type, EK}};
             GemvFused pro;
             if (dist) {   // rms_norm * attn_norm -> q8_K inside the GEMV: CTA c produces super-block c, one grid barrier (short norms: each CTA all of it)
-                pro.kind = 4; pro.in0 = x; pro.in1 = L.attn_norm; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
+                pro.kind = 4; pro.in0 = x; pro.in1 = L.attn_norm; pro.in1_weight = true; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
             } else {      // ... or once by a single-CTA kernel in front of it
                 CK(launch_rmsnorm_quant(x, L.attn_norm, E, hp.rms_eps, ACT_Q8_K, m->actE.q, nullptr, st, dep())); n++;
             }
@@ -396,7 +396,7 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
             GemvDesc d[2] = {{L.gate.data, m->g, nullptr, nullptr, L.gate.type, F}, {L.up.data, m->u, nullptr, nullptr, L.up.type, F}};
             GemvFused pro;
             if (dist) {
-                pro.kind = 4; pro.in0 = x1; pro.in1 = L.ffn_norm; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
+                pro.kind = 4; pro.in0 = x1; pro.in1 = L.ffn_norm; pro.in1_weight = true; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
             } else {
                 CK(launch_rmsnorm_quant(x1, L.ffn_norm, E, hp.rms_eps, ACT_Q8_K, m->actE.q, nullptr, st, pdl)); n++;
             }
@@ -437,7 +437,7 @@ static int enqueue_step(pb200_model * m, int seq, uint64_t * nlaunch) {
         CK(prof_begin(m, tbytes(m->output)));
         const bool head_pdl = pdl && m->l1 > m->l0;   // a stage without layers starts with a copy node: no programmatic edge
         if (is_kquant(m->output.type) && gemv_fused_prologue_ok(E) && dist) {
-            GemvFused pro; pro.kind = 4; pro.in0 = m->x_out; pro.in1 = m->output_norm; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
+            GemvFused pro; pro.kind = 4; pro.in0 = m->x_out; pro.in1 = m->output_norm; pro.in1_weight = true; pro.eps = hp.rms_eps; pro.gbar = m->gbar;
             CK(launch_gemv_kquant_fused(&d1, 1, E, m->actE.q, pro, st, head_pdl)); n++;
         } else {
             CK(launch_rmsnorm_quant(m->x_out, m->output_norm, E, hp.rms_eps, act_mode_for(m->output.type), m->actE.q, nullptr, st, head_pdl)); n++;

@@ -299,14 +299,18 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
             if (t < P.ntiles) issue_tile(P, ctl, stages, it, t, pol);
         }
     }
-    float nw[NORM_B][8];   // the norm's weight does not depend on it either
-    if (VAR == GV_NORM && P.prologue == PRO_RMSNORM) {
+    // the norm's weight does not depend on it either where the caller says so; a factor that may be the previous kernel's result is read behind the wait
+    float nw[NORM_B][8];
+    const bool norms = VAR == GV_NORM && P.prologue == PRO_RMSNORM;
+    auto load_weight = [&]() {
 #pragma unroll
         for (int j = 0; j < NORM_B; j++)
             if (warp + j * GEMV_NW < P.nblk) load8(P.in1 + (warp + j * GEMV_NW) * 256 + lane * 8, nw[j]);
-    }
+    };
+    if (norms && P.in1_weight) load_weight();
     stamp<TRACE>(P, 1);
     pdl_wait();      // the activation is produced by the previous kernel in the stream
+    if (norms && !P.in1_weight) load_weight();
     stamp<TRACE>(P, 2);
 
     const int wpr = SPLIT ? P.wpr : 1;
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
         __syncthreads();
         load_act_regs(r, sa, blk, valid);
         finish_act_regs(r);
-    } else if (VAR == GV_NORM && P.prologue == PRO_RMSNORM) {
+    } else if (norms) {
         norm_prologue(P, ctl, sa, warp, lane, nw);
         fill_rest(P, ctl, stages, pol);
         __syncthreads();
@@ -950,6 +954,7 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     P.prologue = pro.kind == PRO_RMSNORM_DIST && !pro.in_place && !g_trace_buf && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
     P.in0 = pro.in0;
     P.in1 = pro.in1;
+    P.in1_weight = pro.in1_weight;
     P.eps = pro.eps;
     P.abort_flag = abort_flag();
     P.trace = g_trace_buf ? g_trace_buf + (size_t) (g_trace_idx++ % (uint64_t) g_trace_slots) * GEMV_TRACE_ROW : nullptr;

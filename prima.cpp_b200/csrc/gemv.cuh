@@ -96,6 +96,7 @@ struct GemvParams {
     const float * in0;
     const float * in1;
     float eps;
+    int in1_weight;                // PRO_RMSNORM: in1 depends on no kernel in front
     unsigned int * gbar;           // distributed prologues: {arrivals, departures} of the grid barrier (self-resetting)
     int * abort_flag;              // host-mapped: set by the wait watchdog (never on a healthy run)
     unsigned long long * trace;    // per-CTA %globaltimer stamps (TRACE instantiation only)

@@ -57,3 +57,36 @@ def test_result_over_an_operand(cuda, lib, K, over, N, at):
         torch.cuda.synchronize()
         got.append(ys)
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+# a programmatic launch reads neither operand before the kernel in front, a product that wrote it just now, has ended
+@pytest.mark.parametrize("K", [2048, 3840, 4096])
+@pytest.mark.parametrize("made", [0, 1])
+def test_operand_from_the_kernel_in_front(cuda, lib, K, made):
+    import torch
+    ptr = lambda t: C.c_void_p(t.data_ptr())   # noqa: E731
+    blocks = lambda n, k, seed: torch.from_numpy(np.ascontiguousarray(O.synth_blocks(O.Q4_K, n, k, seed=seed)).reshape(-1).view(np.uint8)).cuda()   # noqa: E731
+    Kin = 8192                                       # the kernel in front takes a while
+    W0, W1 = blocks(K, Kin, 3), blocks(500, K, 4)
+    space = lambda k: torch.zeros(lib.c.pb200_act_workspace_bytes(k) + 64, dtype=torch.uint8, device="cuda")   # noqa: E731
+    ws0, ws1, sync = space(Kin), space(K), torch.zeros(16, dtype=torch.uint8, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(K)
+    xs = [torch.randn(Kin, generator=g, device="cuda") for _ in range(12)]
+    other, mid = torch.rand(K, generator=g, device="cuda") + 0.5, torch.empty(K, device="cuda")
+
+    def step(x, y, together):
+        lib.check(lib.c.pb200_quantize_act(O.Q4_K, ptr(x), C.c_int64(Kin), ptr(ws0), None), "quantize_act")
+        m0 = (Mat * 1)(Mat(O.Q4_K, 0, W0.data_ptr(), K, mid.data_ptr(), None))
+        lib.check(lib.c.pb200_gemv_fused(1, m0, C.c_int64(Kin), ptr(ws0), 0, None, None, C.c_float(0.0), None, 1, None), "gemv_fused")
+        if not together:
+            torch.cuda.synchronize()
+        m1 = (Mat * 1)(Mat(O.Q4_K, 0, W1.data_ptr(), 500, y.data_ptr(), None))
+        in0, in1 = (mid, other) if made == 0 else (other, mid)
+        lib.check(lib.c.pb200_gemv_fused(1, m1, C.c_int64(K), ptr(ws1), 1, ptr(in0), ptr(in1), C.c_float(1e-5), ptr(sync), 1 if together else 0, None), "gemv_fused")
+
+    got, want = torch.empty(len(xs), 500, device="cuda"), torch.empty(len(xs), 500, device="cuda")
+    for out, together in ((want, False), (got, True)):
+        for x, y in zip(xs, out):
+            step(x, y, together)
+        torch.cuda.synchronize()
+    assert bool(torch.isfinite(want).all()) and torch.equal(got, want)
