@@ -192,6 +192,13 @@ __device__ __forceinline__ void bulk_g2s(void * smem_dst, const void * gsrc, uin
         : "memory");
 }
 
+// What has been loaded from shared memory is in registers: an instruction takes w, made of a word of every load.  A barrier's arrival, or the copy that is issued next, does not wait
+// for loads of shared memory that nothing has used yet, and warps that load at once keep some of them queued for longer than a copy from L2 takes.  So this stands in front of
+// handing back memory that an asynchronous copy fills again.
+__device__ __forceinline__ void loads_done(uint32_t w) {
+    asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %0, 0x9e3779b9;\n@p nanosleep.u32 20;\n}" ::"r"(w) : "memory");
+}
+
 // fire-and-forget prefetch of a 16-B-granular global range into L2 (no destination, no barrier)
 __device__ __forceinline__ void bulk_prefetch_l2(const void * gsrc, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");

@@ -4,7 +4,7 @@
 // Bound: the weights' way from HBM, and for a few MB the start and end of a kernel.  One CTA per SM takes an equal share of the rows, which lie one
 // behind the other in memory.  Each of its 16 warps brings pieces of 4 KB by bulk copies into a ring of its own, two pieces deep, so that 128 KB
 // are on their way whatever the registers hold; the ring fills before the kernel in front has ended (weights depend on nothing).  A CTA asks for more than
-// half of an SM's shared memory: two of one launch on one SM would finish last.  A piece is read and its successor asked for before it is multiplied.
+// half of an SM's shared memory: two of one launch on one SM would finish last.  A piece is in registers, and its successor asked for, before it is multiplied.
 // The pieces' sums of a row meet in their order at the end.
 // A token of a six-layer model of width 2048 (generate, one request): 435 us with a warp to a row and norms of their own, 397 with this.
 #include <cuda_bf16.h>
@@ -178,6 +178,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_dense_stream(const __grid_con
             for (int c = 0; c < NC; c++)
 #pragma unroll
                 for (int i = 0; i < RB; i++) w[i][c] = c * 256 < left ? *reinterpret_cast<const uint4 *>(w8 + i * (2 * SEG) + c * 512) : make_uint4(0u, 0u, 0u, 0u);
+            uint32_t some = 0u;
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+#pragma unroll
+                for (int i = 0; i < RB; i++) some ^= w[i][c].x;
+            loads_done(some);
             __syncwarp();
             if (in.r < nrows) {
                 if (lane == 0) fetch();

@@ -319,13 +319,12 @@ struct KGroup {
         s[1] = ((hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u)) >> (8 * h);
         m[1] = (((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u)) >> (8 * h);
     }
-    // What has been loaded is in registers: an instruction takes a word of every load.  A barrier's arrival alone does not wait for loads of shared memory that nothing has
-    // used yet, and 16 warps that load at once keep some of them queued for longer than a copy from L2 into the slot takes: blocks came out as a mixture of this group
-    // and the one that follows in the slot, where the activations were late and all warps went on together.
+    // What has been loaded is in registers (common.cuh): without this, blocks came out as a mixture of this group and the one that follows in the slot, where the activations
+    // were late and all 16 warps went on together.
     __device__ __forceinline__ void loaded() const {
         uint32_t w = q[0].x ^ q[1].x ^ q[2].x ^ q[3].x ^ s[0];
         if (TYPE == T_Q5_K) w ^= hb[0];
-        asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %0, 0x9e3779b9;\n@p nanosleep.u32 20;\n}" ::"r"(w) : "memory");
+        loads_done(w);
     }
     static __device__ __forceinline__ float byte_f(uint32_t w, int c) {   // exact: 2^23 + byte less 2^23
         return __fadd_rn(__uint_as_float(and_or((c & 1) ? w >> 16 : w, 0xffu, 0x4b000000u)), -8388608.f);

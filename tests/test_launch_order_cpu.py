@@ -49,3 +49,15 @@ def test_results_of_earlier_kernels_are_no_constants(kernel):
     taken = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", kernel[2]))
     assert taken <= CONSTANT, taken - CONSTANT
     assert "__ldg(" not in kernel[3] and "ld.global.nc" not in kernel[3]
+
+
+# where a role hands memory back that an asynchronous copy fills again, behind loads into registers whose values come into use later: kernel, the end of the loads, the handing back
+HANDED_BACK = [("k_mmq_tc", "kg.load(", "mbar_arrive(&ctl->raw_empty"), ("k_dense_stream", "uint4 w[RB][NC];", "fetch();")]
+
+
+@pytest.mark.parametrize("name,loads,back", HANDED_BACK, ids=lambda v: v if v.startswith("k_") else "")
+def test_memory_is_handed_back_behind_its_loads(name, loads, back):
+    """Neither a barrier's arrival nor the next copy waits for loads of shared memory that nothing has used yet."""
+    (body,) = [k[3] for k in KERNELS if k[1] == name]
+    start = body.index(loads)
+    assert re.search(r"\bloads_done\(|\bkg\.loaded\(", body[start:body.index(back, start)])
