@@ -25,7 +25,6 @@ struct GemvFused {       // fused activation prologue of the k-quant GEMV (PRO_*
     float eps = 0.f;
     unsigned int * gbar = nullptr;   // kinds 4, 5: two zero-initialised words of device memory owned by the caller (grid barrier state)
     bool in1_weight = false;         // kind 4: in1 is a weight of the model, which no kernel in front writes: it may be read ahead of the wait for that kernel
-    bool in1_weight = false;         // kind 4: in1 is a weight of the model, which no kernel in front writes: it may be read ahead of the wait for that kernel
     bool in_place = false;           // kind 4: a result lies over in0 or in1, whose reads then have to end in all CTAs before one stores
 };
 
