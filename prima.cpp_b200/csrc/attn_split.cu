@@ -634,10 +634,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_attn_split(const __grid_const
             }
             if (plain) sum = (e4[0] + e4[1]) + (e4[2] + e4[3]);
             tmem_wait_st();
-            const float odd = tail[0], largest = tail[2];
-            const float f = (plain ? largest : __uint_as_float((uint32_t) (top + 100) << 23)) * part_f;   // of the sums: 2^(top - 14 - 13)
-            bad = bad || odd != 0.f;
-            loads_done(__float_as_uint(odd) ^ __float_as_uint(largest));   // first used in the next round, when the scales may be another tile's
+            const float f = (plain ? tail[2] : __uint_as_float((uint32_t) (top + 100) << 23)) * part_f;   // of the sums: 2^(top - 14 - 13)
+            bad = bad || tail[0] != 0.f;
+            loads_done(__float_as_uint(f) + (bad ? 1u : 0u));   // both are first used in the next round, when the scales may be another tile's
             fence_before();
             __syncwarp();
             if (lane == 0) { mbar_arrive(&ctl->p_full[buf]); mbar_arrive(&ctl->sc_empty[buf]); }

@@ -53,7 +53,7 @@ def test_results_of_earlier_kernels_are_no_constants(kernel):
 
 # where a role hands memory back that an asynchronous copy fills again, behind loads into registers whose values come into use later: kernel, the end of the loads, the handing back
 HANDED_BACK = [("k_mmq_tc", "kg.load(", "mbar_arrive(&ctl->raw_empty"), ("k_dense_stream", "uint4 w[RB][NC];", "fetch();"),
-               ("k_attn_split", "= tail[0]", "mbar_arrive(&ctl->sc_empty")]
+               ("k_attn_split", "tail[2] :", "mbar_arrive(&ctl->sc_empty")]
 
 
 @pytest.mark.parametrize("name,loads,back", HANDED_BACK, ids=lambda v: v if v.startswith("k_") else "")
