@@ -943,7 +943,7 @@ int pb200_set_hidden(pb200_model * m, const float * hidden_host) {
     CK(cudaStreamSynchronize(m->stream));
     return (int) cudaMemcpy(m->x_in, hidden_host, (size_t) m->hp.n_embd * 4, cudaMemcpyHostToDevice);
 }
-// debugging / white-box tests: copy a named internal activation buffer of the LAST step to the host
+// debugging / white-box tests: copy a named internal activation buffer of the LAST step (prompt_*: of the last prompt's last layer, token by token) to the host
 int pb200_debug_read(pb200_model * m, const char * name, float * host, int64_t n) {
     if (m && m->ll && m->finalized && name && host) return ll_debug_read(m, name, host, n);
     if (!m || !m->finalized || !name || !host) return PB200_EINVAL;
@@ -951,7 +951,8 @@ int pb200_debug_read(pb200_model * m, const char * name, float * host, int64_t n
     CK(cudaStreamSynchronize(m->stream));
     const std::string s(name);
     const float * p = s == "q" ? m->q : s == "k" ? m->k : s == "v" ? m->v : s == "att" ? m->att : s == "g" ? m->g : s == "u" ? m->u :
-                      s == "x_a" ? m->x_a : s == "x_b" ? m->x_b : s == "x_out" ? m->x_out : s == "xn" ? m->xn : s == "x_in" ? m->x_in : s == "logits" ? m->logits : nullptr;
+                      s == "x_a" ? m->x_a : s == "x_b" ? m->x_b : s == "x_out" ? m->x_out : s == "xn" ? m->xn : s == "x_in" ? m->x_in : s == "logits" ? m->logits :
+                      s == "prompt_q" ? m->pf.q : s == "prompt_k" ? m->pf.k : s == "prompt_v" ? m->pf.v : s == "prompt_g" ? m->pf.g : s == "prompt_u" ? m->pf.u : nullptr;
     if (!p) return PB200_EINVAL;
     return (int) cudaMemcpy(host, p, (size_t) n * 4, cudaMemcpyDeviceToHost);
 }
