@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_dense_stream(const __grid_con
         next(in);
     }
     const int apad = P.segs * SEG, keep = ST_PARTS / (TB * P.segs * RB) * RB & ~1;   // rows whose sums fit
-    // one token: what a result meets arrives beside the weights
-    const bool early = TB == 1 && R == 1 && nrows <= min(keep, ST_THREADS);
+    // one token: what a result meets arrives beside the weights (a product that makes its norm meets nothing)
+    const bool early = !NORM && TB == 1 && R == 1 && nrows <= min(keep, ST_THREADS);
     float meet = 0.f;
     if constexpr (NORM) {
         float4 wn[ST_NORM_V];
@@ -113,7 +113,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_dense_stream(const __grid_con
                 const int k = 4 * (tid + i * ST_THREADS);
                 v[i] = k < P.K ? *reinterpret_cast<const float4 *>(xr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            if (t == 0 && early && tid < nrows && P.resid) meet = P.resid[u_lo + tid];
 #pragma unroll
             for (int i = 0; i < ST_NORM_V; i++) s += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
             const float inv = 1.f / sqrtf(block_sum(s, ctl.red) / (float) P.K + P.eps);
@@ -160,8 +159,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_dense_stream(const __grid_con
                 }
                 float v = sum(u);
                 if (P.bias) v += P.bias[n];
-                if (early) v += meet;
-                else if (P.resid) v += P.resid[(int64_t) t * P.ldr + n];
+                if constexpr (!NORM) {
+                    if (early) v += meet;
+                    else if (P.resid) v += P.resid[(int64_t) t * P.ldr + n];
+                }
                 if (P.act.xielu) put((__nv_bfloat16 *) P.act.y, (int64_t) t * P.act.ldy + n, xielu_f(v, softplus_f(P.act.xielu[0]), 0.5f + softplus_f(P.act.xielu[1])));
                 else P.C[(int64_t) t * P.ldc + n] = v;
             }

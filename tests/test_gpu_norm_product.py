@@ -1,0 +1,72 @@
+"""-m gpu: products of one to four bf16 tokens that make the RMS norm in front of them themselves: through models whose width does not fill a piece of a row, with biases, gated
+and xIELU epilogues and gathered rows, against the float64 oracle and against the same requests in a batch of five, whose norms are kernels of their own."""
+import numpy as np
+import pytest
+
+import ref_ludusun as RL
+import ref_ruvuvik as RR
+import test_gpu_ludusun as L
+import test_gpu_ruvuvik as U
+
+pytestmark = pytest.mark.gpu
+
+
+def models(width):
+    yield L, RL, L.config([L.att(heads=4, kv_heads=2, dim=64, vdim=64, rot=32, ff=300), L.lat(heads=3, dim=24, vdim=96, kv_rank=64, q_rank=32, ff=264), L.par(heads=4, r_vdim=64, ff=520)], width=width)
+    yield U, RR, U.config([U.att(heads=4, kv_heads=4, dim=64, vdim=64, chunk=0, ff=264), U.lat(vdim=96, ff=296)], width=width)
+
+
+@pytest.mark.parametrize("width", [256, 264, 520, 2056])
+@pytest.mark.parametrize("which", [0, 1])
+def test_batches_of_one_to_five(pkg, cuda, which, width):
+    M, R, cfg = list(models(width))[which]
+    bits, W = R.random_weights(cfg, seed=width)
+    m = M.load(pkg, cfg, bits, "bfloat16", n_ctx=64)
+    reqs = [M.tokens_for(cfg, 14, 30 + i) for i in range(5)]
+    want = [R.forward(cfg, W, t)[0] for t in reqs]
+
+    def steps(n):
+        """prompts of one to four tokens, each alone, with wanted rows out of their middle, then steps of n requests beside each other"""
+        slots, rows = [m.seq_alloc() for _ in range(n)], [[] for _ in range(n)]
+        for i, s in enumerate(slots):
+            k = 1 + i % 4
+            rows[i] = list(m.batch_step([(s, reqs[i][:k], [k - 1] if k < 3 else [1, k - 1])])[0])
+        for t in range(8):
+            before = m.lib.c.pb200_kernel_launches()
+            out = m.batch_step([(s, [reqs[i][1 + i % 4 + t]], [0]) for i, s in enumerate(slots)])[0]
+            count = m.lib.c.pb200_kernel_launches() - before
+            for i in range(n):
+                rows[i].append(out[i])
+        for s in slots:
+            m.seq_free(s)
+        return [np.stack(r) for r in rows], count
+
+    apart, most = steps(5)
+    for n in range(1, 6):
+        rows, count = steps(n)
+        assert count < most if n < 5 else count == most          # norms without launches of their own
+        for i, got in enumerate(rows):
+            k = 1 + i % 4
+            at = ([k - 1] if k < 3 else [1, k - 1]) + list(range(k, k + 8))
+            M.check(got, want[i][at], M.BF16_TOL)
+            # fp32 numbers summed in another order; of the operands rounded to bf16 behind them, a dozen in a row, some fall the other way, by 2 ** -8 of an entry each
+            assert np.linalg.norm(got - apart[i]) <= 2.0 ** -7 * np.linalg.norm(apart[i])
+    m.close()
+
+
+def test_steps_repeat(pkg, cuda):
+    """The same bits however the kernels overlap: steps of one, two and four requests in turns, at a width whose pieces come from L2."""
+    cfg = L.config([L.att(heads=16, kv_heads=4, dim=128, vdim=128, rot=64, ff=8192), L.lat(heads=16, dim=64, vdim=128, kv_rank=512, q_rank=256, ff=8192)], width=2048, vocab=2000)
+    m = pkg.Model.from_config(cfg, dtype="bfloat16", n_ctx=64, n_seq=4)
+    m.synth(0, 7)
+    m.finalize()
+    first = {}
+    for _ in range(24):
+        for n in (1, 2, 4):
+            slots = [m.seq_alloc() for _ in range(n)]
+            out = [m.batch_step([(s, [(31 * i + 7 * t) % 2000], [0]) for i, s in enumerate(slots)])[0].copy() for t in range(4)]
+            for s in slots:
+                m.seq_free(s)
+            out = np.stack(out)
+            assert np.isfinite(out).all() and np.array_equal(first.setdefault(n, out), out)
+    m.close()
