@@ -1,7 +1,13 @@
 """Attention of single tokens with a cluster per (entry, kv head): contexts on both sides of a cluster's and of a stage's rows, wrapped windows with kept first tokens, group sizes,
-heads narrower than a warp's lanes, sinks and gates, against the prompt path of the same model, which reads no cache."""
+heads narrower than a warp's lanes, against the prompt path of the same model, which reads no cache; sinks, chunks that are crossed, keys that are their own values over more rows than
+the stages of a cluster hold, and bf16, against the float64 oracles."""
 import numpy as np
 import pytest
+
+import ref_ludusun as RL
+import ref_ruvuvik as RR
+import test_gpu_ludusun as L
+import test_gpu_ruvuvik as U
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +50,30 @@ def test_steps_give_what_the_prompt_gives(cuda, heads, kv, dim, vdim, mask, soft
             have = np.stack([g[k] for g in got])
             # fp32 throughout, sums of up to 560 terms in another order: 560 / 2 ** 24 = 3e-5 a side in the mixer, and as much again in the products behind it
             assert np.linalg.norm(have - want) <= 1e-4 * np.linalg.norm(want)
+
+
+# a cluster holds 1024 rows of keys that are their own values, 512 of keys and values: starts on both sides; chunks of 130 and 200 whose ends are crossed
+CASES = {"tied": (L, RL, lambda: L.config([L.par(heads=4, kv_heads=2, dim=64, every=300, ff=0)]), (1021, 1085, 127)),
+         "tied_one_head": (L, RL, lambda: L.config([L.par(heads=3, kv_heads=3, dim=128, every=0, ff=0)]), (1024, 1281)),
+         "sinks": (L, RL, lambda: L.config([L.att(heads=8, kv_heads=1, dim=96, vdim=64, ff=0)]), (508, 545, 31)),
+         "sinks_read_by_another_layer": (L, RL, lambda: L.config([L.att(heads=4, kv_heads=2, dim=32, vdim=128, ff=0), L.att(heads=8, kv_heads=2, dim=32, vdim=128, of=0, scale=0.7, ff=24)]), (255, 513)),
+         "chunks": (U, RR, lambda: U.config([U.att(heads=4, kv_heads=2, dim=64, vdim=64, chunk=130, rot=0, ff=0)]), (127, 257, 387)),
+         "chunks_of_200": (U, RR, lambda: U.config([U.att(heads=6, kv_heads=6, dim=32, vdim=40, chunk=200, ff=0)]), (196, 200, 397))}
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_steps_give_what_the_oracle_gives(pkg, cuda, name, dtype):
+    M, R, cfg, starts = CASES[name]
+    cfg = cfg()
+    bits, W = R.random_weights(cfg, seed=17)
+    m = M.load(pkg, cfg, bits, dtype, n_ctx=1300)
+    toks = M.tokens_for(cfg, max(starts) + 6, 3)
+    want = R.forward(cfg, W, toks)[0]
+    slots = [m.seq_alloc() for _ in starts]
+    for s, n in zip(slots, starts):
+        m.batch_step([(s, toks[:n], [n - 1])])
+    for i in range(6):
+        got = m.batch_step([(s, [toks[n + i]], [0]) for s, n in zip(slots, starts)])[0]
+        M.check(got, want[[n + i for n in starts]], M.F32_TOL if dtype == "float32" else M.BF16_TOL)
+    m.close()
