@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, GEMV_CTAS_PER_SM) k_gemv_kquant(
     }
     // the norm's weight does not depend on it either where the caller says so; a factor that may be the previous kernel's result is read behind the wait
     float nw[NORM_B][8];
-    const bool norms = VAR == GV_NORM && P.prologue == PRO_RMSNORM;
+    const bool norms = (VAR == GV_NORM || TRACE) && P.prologue == PRO_RMSNORM;
     auto load_weight = [&]() {
 #pragma unroll
         for (int j = 0; j < NORM_B; j++)
@@ -950,8 +950,8 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     P.act = act;
     // A norm of less than 16 super-blocks: every CTA for itself, beyond that distributed.  us a step of four layers of width 1024, 2048, 3072, 4096 and 8192, distributed /
     // so: 119.0 / 102.5, 136.5 / 125.7, 196.0 / 186.4, 228.6 / 229.4, 522 / 530 (where 296 CTAs read 19 MB).
-    // While a trace is taken the distributed one has the stamps.  A result over in0 or in1 takes the distributed one, too: its barrier ends all reads of them.
-    P.prologue = pro.kind == PRO_RMSNORM_DIST && !pro.in_place && !g_trace_buf && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
+    // A result over in0 or in1 takes the distributed one: its barrier ends all reads of them.
+    P.prologue = pro.kind == PRO_RMSNORM_DIST && !pro.in_place && P.nblk < GEMV_NW * NORM_B && (((uintptr_t) pro.in0 | (uintptr_t) pro.in1) & 15) == 0 ? PRO_RMSNORM : pro.kind;
     P.in0 = pro.in0;
     P.in1 = pro.in1;
     P.in1_weight = pro.in1_weight;
@@ -982,8 +982,8 @@ int launch_gemv_kquant_fused(const GemvDesc * d, int nmat, int K, const ActQ & a
     const int ti = ty == T_Q4_K ? 1 : ty == T_Q5_K ? 2 : ty == T_Q6_K ? 3 : ty == T_Q8_0 ? 4 : ty == T_Q5_1 ? 5 : 0;
     // Short products share the instantiation with the norm, whether they have one or not: a step that changed code at every launch lost half of the gain
     // (widths 1024, 2048 and 3072 against the distributed norm: 119.6 -> 110.0 and 102.7 so, 138.7 -> 137.2 and 127.1, 197.4 -> 189.0 and 185.4 us).
-    const bool norms = P.prologue == PRO_RMSNORM || (is_kquant(types[0]) && !g_trace_buf && pl.wpr == 1 && std::min(K, d[0].N) < GEMV_NW * NORM_B * 256);
-    const int var = pro.kind == PRO_QUANT ? GV_QUANT : norms ? GV_NORM : g_trace_buf != nullptr ? GV_TRACE : GV_PLAIN;
+    const bool norms = P.prologue == PRO_RMSNORM || (is_kquant(types[0]) && pl.wpr == 1 && std::min(K, d[0].N) < GEMV_NW * NORM_B * 256);
+    const int var = pro.kind == PRO_QUANT ? GV_QUANT : g_trace_buf != nullptr ? GV_TRACE : norms ? GV_NORM : GV_PLAIN;
     typedef void (*kern_t)(const GemvParams);
     static const kern_t table[6][2][4] = {   // rows of a norm by every CTA are never split
         {{k_gemv_kquant<0, false, GV_PLAIN>, k_gemv_kquant<0, false, GV_TRACE>, nullptr, k_gemv_kquant<0, false, GV_NORM>},
