@@ -2071,7 +2071,9 @@ static int stream_product(pb200_model * m, int T, const DenseW & w, int N, float
         ll.norm_ahead = nullptr;
         const int rc = launch_dense_normed(ct, ll.x, W, nullptr, nw, ll.eps, w.data, W, C, N, T, N, W, bias, m->stream, act ? *act : DenseAct());
         if (rc != (int) cudaErrorNotSupported) return rc;
+        CAT(CAT_NORM);
         CK(launch_group_rmsnorm(ll.x, nullptr, nw, 1, ll.eps, ll.act, ct, T, W, m->stream));
+        CAT(CAT_DENSE);
     }
     if (act) return launch_dense_act(ct, ll.act, W, w.data, W, *act, T, N, W, m->stream);
     return launch_dense(ct, ll.act, W, w.data, W, C, N, T, N, W, bias, nullptr, 0, 1.f, m->stream);
@@ -2599,7 +2601,7 @@ static int ll_forward_prerms(pb200_model * m, const BatchView & b, bool prefill,
     LayerList & ll = *m->ll;
     cudaStream_t st = m->stream;
     const int T = b.n_tokens, W = ll.width, ct = ll.ctype;
-    const bool ahead = ct == T_BF16 && T <= 4 && !ll.prof_on;   // few tokens: a product norms its input itself
+    const bool ahead = ct == T_BF16 && T <= 4;   // few tokens: a product norms its input itself
     ll.norm_ahead = nullptr;
     CAT(CAT_ELEM);
     bool act_ready = false;   // the kernel that closed the previous sublayer has left this one's normed input in ll.act

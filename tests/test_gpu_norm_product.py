@@ -54,6 +54,28 @@ def test_batches_of_one_to_five(pkg, cuda, which, width):
     m.close()
 
 
+@pytest.mark.parametrize("n", [1, 3])
+def test_a_profile_shows_the_kernels_that_run(pkg, cuda, n):
+    cfg = list(models(520))[0][2]
+    cfg["layers"] = cfg["layers"][:2]           # branches beside each other are taken one after the other while every launch is timed
+    m = pkg.Model.from_config(cfg, dtype="bfloat16", n_ctx=64, n_seq=4)
+    m.synth(0, 5)
+    m.finalize()
+    counts, rows = [], []
+    for on in (False, True):
+        slots = [m.seq_alloc() for _ in range(n)]
+        m.batch_step([(s, [7, 9], [0]) for s in slots])
+        m.profile(on)
+        before = m.lib.c.pb200_kernel_launches()
+        rows.append(m.batch_step([(s, [11], [0]) for s in slots])[0].copy())
+        counts.append(m.lib.c.pb200_kernel_launches() - before)
+        m.profile(False)
+        for s in slots:
+            m.seq_free(s)
+    m.close()
+    assert counts[0] == counts[1] and np.array_equal(rows[0], rows[1])
+
+
 def test_steps_repeat(pkg, cuda):
     """The same bits however the kernels overlap: steps of one, two and four requests in turns, at a width whose pieces come from L2."""
     cfg = L.config([L.att(heads=16, kv_heads=4, dim=128, vdim=128, rot=64, ff=8192), L.lat(heads=16, dim=64, vdim=128, kv_rank=512, q_rank=256, ff=8192)], width=2048, vocab=2000)
