@@ -2051,6 +2051,11 @@ static int tap_prepare(pb200_model * m, int T) {
     return 0;
 }
 
+// branches run beside each other, unless every launch is being timed or one stream is asked for (A/B)
+static bool two_streams(const LayerList & ll) {
+    static const bool one = getenv("PB200_ONE_STREAM") != nullptr;
+    return !ll.prof_on && !one;
+}
 // the second stream goes on from where the first one is
 static int fork_side(pb200_model * m) {
     LayerList & ll = *m->ll;
@@ -2304,9 +2309,8 @@ static int mix_dual(pb200_model * m, const BatchView & b, bool prefill, const LR
         CK(launch_dual_prep_store(1, rq, ldr, rk, ldr, nullptr, 0, nullptr, 0, L.f_bias.data, L.f_lower.data, rp.qk_heads, rp.heads, rp.dim, lq, ld, lk, ld, lv, ld, b, a,
                                   pr, kc, vc, ll.slot_floats, st));
     const bool sum = d.join == JOIN_SCALED_SUM;
-    // ---- recurrent branch: on the second stream beside the attention branch, unless every launch is being timed ----
-    static const bool one_stream = getenv("PB200_ONE_STREAM") != nullptr;   // A/B: both branches in a row on one stream
-    const bool forked = !ll.prof_on && !one_stream;
+    // ---- recurrent branch: on the second stream beside the attention branch ----
+    const bool forked = two_streams(ll);
     cudaStream_t rst = st;
     if (forked) {
         CK(fork_side(m));
@@ -2485,7 +2489,7 @@ static int ff_moe(pb200_model * m, int T, bool prefill, LLayer & L, float * x, b
     CAT(CAT_MOE);
     bool forked = false;
     if (L.route == ROUTE_SIGMOID_GROUPS) {
-        if (L.shared_ff > 0 && p.act == 1 && !accumulate && prefill && (int64_t) T * p.top > 64 && !ll.prof_on) {
+        if (L.shared_ff > 0 && p.act == 1 && !accumulate && prefill && (int64_t) T * p.top > 64 && two_streams(ll)) {
             // a prompt's shared expert, on the second stream beside the choice and the sorting, which leave most SMs idle
             CK(fork_side(m));
             forked = true;

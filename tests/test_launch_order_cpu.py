@@ -62,3 +62,8 @@ def test_memory_is_handed_back_behind_its_loads(name, loads, back):
     (body,) = [k[3] for k in KERNELS if k[1] == name]
     start = body.index(loads)
     assert re.search(r"\bloads_done\(|\bkg\.loaded\(", body[start:body.index(back, start)])
+
+
+def test_every_fork_heeds_the_switch_for_one_stream():
+    s = (CSRC / "layers.cu").read_text()
+    assert s.count("CK(fork_side(m))") == s.count("two_streams(ll)") == 2 and s.count('getenv("PB200_ONE_STREAM")') == 1
