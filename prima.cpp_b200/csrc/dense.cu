@@ -269,10 +269,10 @@ int rows_max_t() {
 template <typename WT>
 int dense_typed(const WT * A, int64_t lda, const WT * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
                 const float * resid, int64_t ldr, float alpha, cudaStream_t st, int plane_rows = 0, int64_t a_plane = 0,
-                const DenseAct & act = DenseAct()) {
+                const DenseAct & act = DenseAct(), bool alone = false) {
     if constexpr (sizeof(WT) == 2) {
         if (plane_rows == 0) {   // rows one behind the other: streamed through shared memory
-            const int rc = launch_dense_stream(A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st, act);
+            const int rc = launch_dense_stream(A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st, act, alone);
             if (rc != (int) cudaErrorNotSupported) return rc;
         }
     }
@@ -356,14 +356,14 @@ int launch_dense_act(int type, const void * A, int64_t lda, const void * W, int6
 }
 
 int launch_dense(int type, const void * A, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
-                 const float * resid, int64_t ldr, float alpha, cudaStream_t st) {
+                 const float * resid, int64_t ldr, float alpha, cudaStream_t st, bool alone) {
     if (T <= 0 || N <= 0) return 0;
     if (K <= 0 || !A || !W || !C) return (int) cudaErrorInvalidValue;
     if (type == 0 /* T_F32 */) return dense_typed<float>((const float *) A, lda, (const float *) W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st);
     if (type != T_BF16) return (int) cudaErrorInvalidValue;
     if (T > rows_max_t() && dense_tc_ok(T, N, K, lda, ldw, A, W))
         return launch_dense_tc((const __nv_bfloat16 *) A, lda, (const __nv_bfloat16 *) W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st);
-    return dense_typed<__nv_bfloat16>((const __nv_bfloat16 *) A, lda, (const __nv_bfloat16 *) W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st);
+    return dense_typed<__nv_bfloat16>((const __nv_bfloat16 *) A, lda, (const __nv_bfloat16 *) W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, st, 0, 0, DenseAct(), alone);
 }
 
 }  // namespace pb

@@ -251,11 +251,20 @@ bool stream_ok(const __nv_bfloat16 * W, int64_t ldw, int T, int K) {
     return T >= 1 && T <= 4 && K >= 256 && K <= (T <= 2 ? 16384 : 6144) && K % 8 == 0 && ldw == K && ((uintptr_t) W & 15) == 0;
 }
 
+// A product by itself has no kernel in front beside whose end its rings could fill, which is what it gains in a pass (generate with ff 4096 to 8192, widths 1024 to 2048, one to four requests:
+// 0 to 9 % of a call).  What is left are few rounds of pieces, where a launch counts, and many bytes.  The same times as above, 1 / 2 / 4 tokens, rows over this: 300 x 3072 1.46 / 1.34 / 1.59;
+// 1000 x 3072 1.32 / 1.12 / 1.28; 2048 x 2048 0.99 / 1.09 / 1.04; 4096 x 2048 0.99 / 0.91 / 0.94; 2048 x 5504 0.90 / 0.84 / 0.88; 1000 x 11008 0.83 / 0.84; 8192 x 1024 (half of a piece) 0.83 / 0.80 / 0.99;
+// 4096 x 4096 0.92 / 1.00 / 1.11; 8192 x 4096 1.02 / 1.04 / 1.21; 16384 x 4096 1.00 / 1.24 / 1.44.
+bool alone_ok(int T, int N, int K) {
+    const int seg = T <= 2 ? ST_PIECE / 2 : ST_PIECE / 4;
+    return (int64_t) N * ((K + seg - 1) / seg * seg) <= (T <= 2 ? 5 << 20 : 6 << 20) || (K >= 2048 && (int64_t) N * K >= (T == 4 ? 16 << 20 : 32 << 20));
+}
+
 }  // namespace
 
 int launch_dense_stream(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
-                        const float * resid, int64_t ldr, float alpha, cudaStream_t st, const DenseAct & act) {
-    if (!stream_ok(W, ldw, T, K) || lda % 8 || ((uintptr_t) A & 15)) return (int) cudaErrorNotSupported;
+                        const float * resid, int64_t ldr, float alpha, cudaStream_t st, const DenseAct & act, bool alone) {
+    if (!stream_ok(W, ldw, T, K) || (alone && !alone_ok(T, N, K)) || lda % 8 || ((uintptr_t) A & 15)) return (int) cudaErrorNotSupported;
     return launch_tokens<false>(StreamParams{A, lda, nullptr, nullptr, nullptr, 0.f, W, C, ldc, bias, resid, ldr, alpha, T, act.silu_glu ? N / 2 : N, K, 1, abort_flag(), act}, st);
 }
 

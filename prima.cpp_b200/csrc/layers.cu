@@ -3160,7 +3160,7 @@ int pb200_dense(int type, const void * A, int64_t lda, const void * W, int64_t l
                 const float * resid, int64_t ldr, float alpha, void * stream) {
     if (type != T_F32 && type != T_BF16) return PB200_ENOTSUP;
     if (!A || !W || !C || T < 0 || N < 0 || K <= 0 || lda < K || ldw < K || ldc < N || (resid && ldr < N)) return PB200_EINVAL;
-    return launch_dense(type, A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, (cudaStream_t) stream);
+    return launch_dense(type, A, lda, W, ldw, C, ldc, T, N, K, bias, resid, ldr, alpha, (cudaStream_t) stream, true);
 }
 int pb200_debug_profile(pb200_model * m, int on) {
     if (!m || !m->ll) return PB200_EINVAL;

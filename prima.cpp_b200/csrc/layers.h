@@ -42,7 +42,7 @@ struct BatchView {
 // The result of a row does not depend on what the other rows of the call hold.  Their number chooses the kernel, and in the tensor-core kernel how K is cut
 // (plan_tc in dense_tc.cu): the order of the fp32 sum may change with it, its error bound does not.
 int launch_dense(int type, const void * A, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K,
-                 const float * bias, const float * resid, int64_t ldr, float alpha, cudaStream_t stream);
+                 const float * bias, const float * resid, int64_t ldr, float alpha, cudaStream_t stream, bool alone = false);   // alone: no part of a pass
 // Grouped product in one launch: rows [start[g], start[g] + count[g]) of A times the g-th matrix of W (w_stride elements apart, [N][K]
 // each) into the same rows of C, g < groups; start / count are device arrays and no group has more than max_rows rows.  Tensor-core
 // kernel only (bf16, aligned shapes): dense_grouped_ok says whether it applies; otherwise the caller multiplies group by group.
@@ -60,7 +60,7 @@ struct DenseAct {
 };
 // bf16, up to four tokens, rows of W one behind the other: weights streamed through shared memory (dense_stream.cu); cudaErrorNotSupported: not taken
 int launch_dense_stream(const __nv_bfloat16 * A, int64_t lda, const __nv_bfloat16 * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K, const float * bias,
-                        const float * resid, int64_t ldr, float alpha, cudaStream_t stream, const DenseAct & act);
+                        const float * resid, int64_t ldr, float alpha, cudaStream_t stream, const DenseAct & act, bool alone);
 // launch_dense / launch_dense_act of A[t] = the RMS norm of row t, or rows[t], of x (fp32, ldx apart) with weight norm_w, rounded to the operand type, in one launch:
 // bf16, up to four tokens, K up to 8192; cudaErrorNotSupported otherwise
 int launch_dense_normed(int type, const float * x, int64_t ldx, const int32_t * rows, const float * norm_w, float eps, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K,

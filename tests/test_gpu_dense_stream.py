@@ -1,5 +1,5 @@
 """The product that streams weights through shared memory (one to four tokens of bf16): pieces of a row that end inside one, CTAs without rows, odd rows of a piece
-of two, more rows than a CTA keeps sums for, rows one behind the other and apart."""
+of two, more rows than a CTA keeps sums for, rows one behind the other and apart; products by themselves on both sides of the lines between it and a warp to a row."""
 import ctypes as C
 
 import pytest
@@ -57,3 +57,19 @@ def test_what_the_rows_behind_hold_stays_there(lib, cuda, T):
     torch.cuda.synchronize()
     keep = torch.arange(599, device="cuda") != 100
     assert torch.equal(out[:, keep], clean[:, keep]) and not bool(torch.isfinite(out[:, 100]).any())
+
+
+@pytest.mark.parametrize("N,K", [(2560, 2048), (2561, 2048), (3072, 2048), (3073, 2048), (4096, 1024), (1000, 11008), (4095, 4096), (4096, 4096), (16383, 2048), (16384, 2048), (20000, 2040)])
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+def test_both_sides_of_the_lines(lib, cuda, T, N, K):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(T * 7 + N * 3 + K)
+    A, W = torch.randn(T, K, generator=g, device="cuda").bfloat16(), torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    resid = torch.randn(T, N, generator=g, device="cuda")
+    out = torch.full((T, N + 3), 7.0, device="cuda")
+    lib.check(lib.c.pb200_dense(30, ptr(A), K, ptr(W), K, ptr(out), N + 3, T, N, K, None, ptr(resid), N, 1.0, None), "dense")
+    torch.cuda.synchronize()
+    want = A.double() @ W.double().T + resid.double()
+    # exact products, fp32 sums: a lane's chain of a row alone in its warp, five halvings of a warp, the warps or pieces of a row, the residual
+    bound = (K // 32 + 5 + 8 + 1) * 2.0 ** -24 * (A.double().abs() @ W.double().abs().T + resid.double().abs())
+    assert bool(((out[:, :N].double() - want).abs() <= bound).all()) and bool((out[:, N:] == 7.0).all())

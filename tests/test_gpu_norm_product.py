@@ -54,6 +54,29 @@ def test_batches_of_one_to_five(pkg, cuda, which, width):
     m.close()
 
 
+def test_more_rows_than_a_cta_keeps_sums_for(pkg, cuda):
+    """A head of 152 000 rows of 256 entries: 1024 rows of two tokens' sums and 512 of four tokens' fit a CTA, which has 1028 rows."""
+    cfg = L.config([L.att(heads=2, kv_heads=1, dim=32, vdim=32, ff=0)], width=256, vocab=152000)
+    bits, W = RL.random_weights(cfg, seed=8)
+    m = L.load(pkg, cfg, bits, "bfloat16", n_ctx=32)
+    reqs = [L.tokens_for(cfg, 3, 40 + i) for i in range(5)]
+    want = np.stack([RL.forward(cfg, W, t)[0][2] for t in reqs])
+
+    def last(n):
+        slots = [m.seq_alloc() for _ in range(n)]
+        m.batch_step([(s, r[:2], []) for s, r in zip(slots, reqs)])
+        out = m.batch_step([(s, r[2:], [0]) for s, r in zip(slots, reqs)])[0].copy()
+        for s in slots:
+            m.seq_free(s)
+        return out
+    apart = last(5)
+    for n in range(1, 5):
+        got = last(n)
+        L.check(got, want[:n], L.BF16_TOL)
+        assert np.linalg.norm(got - apart[:n]) <= 2.0 ** -7 * np.linalg.norm(apart[:n])      # as above
+    m.close()
+
+
 @pytest.mark.parametrize("n", [1, 3])
 def test_a_profile_shows_the_kernels_that_run(pkg, cuda, n):
     cfg = list(models(520))[0][2]
