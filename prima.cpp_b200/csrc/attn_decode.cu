@@ -4,7 +4,7 @@
 // kv head, so that a row is read once; it asks for the rows of earlier tokens before the kernel in front has ended (only the token's own row is
 // written in this pass, by a kernel in front).  A stage of 32 rows: scores with a warp to a row, softmax with a warp to a head, weighted values with a warp
 // to a head and a share of the rows.  The CTAs send their sums to the CTA that finishes an output entry: one cluster barrier and no second kernel.
-// The cut of the rows follows the sequence's own length, so that its result does not depend on the batch around it.
+// The cut of the rows follows the sequence's own length.  Which kernel takes a call follows the sequences beside it (launch_attn_decode_group below), and with it the order of the fp32 sums.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>

@@ -243,9 +243,9 @@ int launch_tokens(const StreamParams & P, cudaStream_t st) {
     return launch_stream<4, 2, NORM>(P, st);
 }
 
-// Calls one by one from HBM, us, a warp to a row with its loads in registers (dense.cu) / this, for 1, 2 and 4 tokens: 2048 x 2048 6.9, 8.2, 8.6 / 6.2, 7.9,
-// 8.3; 16384 x 2048 16.5, 18.7, 24.9 / 14.6, 16.7, 21.4; 2048 x 8192 10.3, 12.4, 14.8 / 10.4, 12.3, 16.4; 4096 x 14336 24.7, 28.8, - / 23.6, 25.3, -;
-// 28672 x 4096 45.6, 53.1, 69.1 / 40.8, 41.1, 55.3; 1000 x 5504 8.2, 8.4, 12.2 / 8.2, 8.6, 10.3; 388 x 2048 6.2 / 5.0.  So three and four tokens of rows
+// Calls one by one from HBM, us, a warp to a row with its loads in registers (dense.cu) / this, for 1, 2 and 4 tokens: 2048 x 2048 6.3, 8.3, 8.7 / 6.3, 7.6,
+// 8.3; 16384 x 2048 17.4, 21.1, 27.7 / 17.0, 19.0, 23.1; 2048 x 8192 10.9, 12.8, 14.8 / 11.6, 12.8, 16.4; 4096 x 14336 26.3, 31.8, - / 26.3, 28.3, -;
+// 28672 x 4096 49.7, 53.1, 69.1 / 45.6, 41.1, 55.3; 1000 x 5504 8.3, 8.6, 12.4 / 8.3, 9.1, 10.4; 388 x 2048 6.2 / 5.1.  So three and four tokens of rows
 // beyond 6144 entries, whose operands every CTA would stage for a few rows, stay there.
 bool stream_ok(const __nv_bfloat16 * W, int64_t ldw, int T, int K) {
     return T >= 1 && T <= 4 && K >= 256 && K <= (T <= 2 ? 16384 : 6144) && K % 8 == 0 && ldw == K && ((uintptr_t) W & 15) == 0;

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) k_latent_up_v(const float * olat, const W
 // the key), the 16 lanes of a head keep its running max / sum, and every thread accumulates two latent columns of all 16 heads (the
 // value is the row's latent part) -- a row is read once for all heads of the group.  Partial (sum, max, normaliser) per split go to
 // `part` [entry][split][head][kv_rank + 2]; k_latent_merge_up_v combines them.  The share of a split depends on the sequence's own
-// length only, so a token's result does not depend on the batch around it.
+// length only; whether these kernels or the one of latent_decode.cu, which sums in another order, serve a batch depends on how many sequences it has.
 // VEC: rows whose size is a multiple of 4 travel and are scored in 16-byte pieces (the padded row stride is an odd number of pieces: no bank
 // conflicts between the 16 rows a warp scores).
 constexpr int LT_ROWS = 16, LT_HEADS = 16;

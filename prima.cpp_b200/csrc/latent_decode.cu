@@ -4,7 +4,8 @@
 // W_uk and a quarter of the rows of W_uv each, in registers and on their way before the kernel in front has ended, as are the cache rows of earlier
 // tokens (only the token's own row is written in this pass, by a kernel in front).  The folded queries go to all CTAs of the cluster, each of
 // which walks an eighth of the rows in stages of 16: scores with a warp to two rows, weighted sums with a thread to four entries of a head.  The sums go to the
-// four CTAs of their head, which join them and apply W_uv.  The cut of the rows follows the sequence's own length.
+// four CTAs of their head, which join them and apply W_uv.  The cut of the rows follows the sequence's own length, the choice
+// between this kernel and those three the number of sequences: the order of the fp32 sums may change with it.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>

@@ -39,8 +39,9 @@ struct BatchView {
 // ---- dense products ----
 // C[t][n] = alpha * sum_k A[t][k] * W[n][k] (+ bias[n]) (+ resid[t][n]);  A and W share `type` (T_F32: true fp32 multiply-add;
 // T_BF16: bf16 operands, fp32 accumulation), C / bias / resid are f32.  resid may alias C.  lda / ldw / ldc / ldr in elements.
-// The result of a row does not depend on what the other rows of the call hold.  Their number chooses the kernel, and in the tensor-core kernel how K is cut
-// (plan_tc in dense_tc.cu): the order of the fp32 sum may change with it, its error bound does not.
+// The result of a row does not depend on what the other rows of the call hold.  Their number chooses the kernel, in the tensor-core kernel how K is cut (plan_tc in
+// dense_tc.cu) and in the streamed one the pieces of a row (2048 entries for one and two rows, 1024 for three and four): the order of the fp32 sum may change with it, its error
+// bound does not.  A product by itself (`alone`) may take another kernel than the same one in a pass (dense_stream.cu).
 int launch_dense(int type, const void * A, int64_t lda, const void * W, int64_t ldw, float * C, int64_t ldc, int T, int N, int K,
                  const float * bias, const float * resid, int64_t ldr, float alpha, cudaStream_t stream, bool alone = false);   // alone: no part of a pass
 // Grouped product in one launch: rows [start[g], start[g] + count[g]) of A times the g-th matrix of W (w_stride elements apart, [N][K]
@@ -182,7 +183,7 @@ int launch_attn_window_prefill(const float * qkvg, const BatchView & b, const At
 // one-token entries: keys and values come from the cache (the token's own row already stored).  part (may be null): scratch of
 // attn_decode_part_floats floats; with it and a cache of 128 rows or more the rows are split over several CTAs per (head, entry) in chunks
 // of attn_decode_chunk rows, and a second kernel merges the partial softmax states.  The split depends on the cache's row count alone.  Where
-// attn_decode.cu takes the call, a cluster per (entry, kv head) does both in one launch.
+// attn_decode.cu takes the call (for ungrouped heads: up to 256 clusters), a cluster per (entry, kv head) does both in one launch.
 inline int attn_decode_chunk(int cache_rows) {
     const int c = (cache_rows + 63) / 64;                 // at most 64 splits ...
     return c < 64 ? 64 : (c + 31) / 32 * 32;              // ... of at least 64 rows

@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(256) k_attn_window_prefill_tiled(const AttnIO 
 // warp, and every lane accumulates its share of the value dimensions.  The warps' partial softmax states are merged in shared memory.  With
 // one split (16 warps over all rows) the CTA writes the output; with several (8 warps over `chunk` rows each) it writes its partial state
 // [max, sum, weighted values] and k_attn_decode_merge finishes.  The number of splits comes from the cache's row count alone (the layer's
-// window and the context size), so a sequence's result does not depend on the batch around it.
+// window and the context size); ungrouped heads change between this kernel and the clusters, whose sums have another order, with the sequences beside each other.
 // A split without rows writes nothing, and the merge does not read it.  NV <= 4: the value entries of a step's rows are on their way before the
 // scores are summed.  TIED (a key is its own value, 16-byte rows): the key's registers serve as the value, lane entry 4 c + i of a head being d =
 // 128 c + 4 lane + i.

@@ -1075,7 +1075,10 @@ cudaError_t launch_mmq(int type, const void * W, int64_t N, int64_t K, const flo
 
 // d: up to three k-quant matrices with K columns over the activation x, of one type, or of two where one is Q6_K.  One after the other each of them has a
 // few tiles to cut into many parts, whose joins and starts take most of the time, and waits for the one in front; together they take a launch.  Not
-// supported: where the tiles of all are too many for clusters, or the launches one by one are the faster way by mmq_pick_cut's costs.
+// supported: where the tiles of all are too many for clusters (74 in halves: K 8192 with 64 + 16 tiles is not), the launches one by one are the faster way by mmq_pick_cut's
+// costs, a Q6_K matrix has rows that do not lie at multiples of 16 bytes (K no multiple of 2048), or Q4_K stands beside Q5_K.
+// Prompts of models of four layers, one by one / together, widths 2048, 4096 and 5120 with grouped heads: 9 tokens 489 / 404, 749 / 716, 923 / 892; 512 tokens 985 / 802, 1464 / 1280,
+// 1788 / 1670.  With as many kv heads as heads at 4096 and 5120, and at 8192, the costs say one by one, and it stays what it was.
 // 512 tokens, K 4096, rows 4096 + 1024 + 1024, us: one by one 86, together 42.
 cudaError_t launch_mmq_multi(const MmqDesc * d, int n, int64_t K, const float * x, int64_t ldx, int64_t T, void * ws, cudaStream_t st, const MmqPre * pre, bool pdl) {
     if (n < 2 || n > MMQ_MAX_MATS || T <= 0 || K % 256 || K < 256) return cudaErrorNotSupported;
