@@ -32,10 +32,6 @@ struct DecodeParams {
     void * out;
 };
 
-__device__ __forceinline__ void send(float v, const float * at, int cta) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(smem_u32(at), (uint32_t) cta)), "f"(v) : "memory");
-}
-
 // GM: query heads of a kv head (at most); TIED: a key is its own value
 template <typename OT, int GM, bool TIED>
 __global__ void __launch_bounds__(AD_WARPS * 32) __cluster_dims__(AD_CTAS, 1, 1) k_attn_decode_group(const __grid_constant__ DecodeParams P) {

@@ -36,9 +36,6 @@ struct LatentDecode {
     void * out;
 };
 
-__device__ __forceinline__ void send(float v, const float * at, int cta) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(smem_u32(at), (uint32_t) cta)), "f"(v) : "memory");
-}
 __device__ __forceinline__ void send4(float4 v, const float * at, int cta) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr(smem_u32(at), (uint32_t) cta)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
